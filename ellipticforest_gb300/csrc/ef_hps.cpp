@@ -7,6 +7,7 @@
 #include "ef_hps.hpp"
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -208,6 +209,45 @@ void Hps::plan() {
         if (mn.leaf()) continue;
         groups_[gidx[{-mn.level, nodes_[id].s}]].nodes.push_back(id);
     }
+
+    // Nodes with the same operators.  A merge reads nothing but its children's (coarsened) T, and a
+    // leaf's T depends on its type alone, so two nodes whose subtrees have the same shape and the same
+    // leaf types at the same places have bitwise equal T, S, X^{-1} and H: on a uniform tree with
+    // constant coefficients every level has one distinct merge (where midpoint halving gives all its
+    // leaves the same spacing), on an adaptive one a few tens.  Leaves with coefficients of their own
+    // have types of their own, so nothing is shared there.
+    std::vector<int> cls(N, -1);
+    std::map<std::array<int, 9>, int> key2cls;
+    int ncls = int(types_.size());
+    for (int id = N - 1; id >= 0; --id) {
+        const MeshNode& mn = mesh_.nodes[id];
+        if (mn.leaf()) { cls[id] = nodes_[id].leaf_type; continue; }
+        std::array<int, 9> key;
+        key[8] = nodes_[id].s;
+        for (int c = 0; c < 4; ++c) {
+            key[2 * c] = cls[mn.child[c]];
+            key[2 * c + 1] = nodes_[mn.child[c]].ncoarsen;
+        }
+        const auto it = key2cls.emplace(key, ncls).first;
+        if (it->second == ncls) ++ncls;
+        cls[id] = it->second;
+    }
+    for (auto& g : groups_) {
+        std::map<int, int> first;  // class -> position among the distinct nodes
+        std::vector<int> own, rest;
+        for (int id : g.nodes) {
+            const auto it = first.emplace(cls[id], int(own.size()));
+            if (it.second) {
+                own.push_back(id);
+            } else {
+                rest.push_back(id);
+                g.same.push_back(it.first->second);
+            }
+        }
+        g.distinct = int(own.size());
+        own.insert(own.end(), rest.begin(), rest.end());
+        g.nodes = own;
+    }
 }
 
 void Hps::allocate() {
@@ -301,6 +341,10 @@ void Hps::allocate() {
             g.d_gB = cv.get<const double*>(8 * cnt);
             g.d_gB2 = cv.get<const double*>(8 * cnt);
             g.d_gC = cv.get<double*>(8 * cnt);
+            g.ncopy = 3 * (cnt - g.distinct);
+            g.d_csrc = cv.get<const double*>(g.ncopy);
+            g.d_cdst = cv.get<double*>(g.ncopy);
+            g.d_clen = cv.get<long long>(g.ncopy);
         }
         tsteps_.clear(); hsteps_.clear(); gsteps_.clear();
         for (auto& kv : tmap) {
@@ -446,6 +490,19 @@ void Hps::upload_tables() {
             check(upload_sync(st_, g.d_gB2, gB2.data(), gB2.size() * sizeof(void*)), "gB2");
             check(upload_sync(st_, g.d_gC, gC.data(), gC.size() * sizeof(void*)), "gC");
         }
+        std::vector<const double*> csrc;
+        std::vector<double*> cdst;
+        std::vector<long long> clen;
+        const long long s2 = (long long)g.s * g.s;
+        for (size_t k = 0; k < g.same.size(); ++k) {
+            const NodeDev &a = nodes_[g.nodes[g.same[k]]], &b = nodes_[g.nodes[g.distinct + k]];
+            csrc.push_back(a.T); cdst.push_back(b.T); clen.push_back(64 * s2);
+            csrc.push_back(a.RHS); cdst.push_back(b.RHS); clen.push_back(48 * s2);
+            csrc.push_back(a.H); cdst.push_back(b.H); clen.push_back(16 * s2);
+        }
+        check(upload_sync(st_, g.d_csrc, csrc.data(), csrc.size() * sizeof(void*)), "copy src");
+        check(upload_sync(st_, g.d_cdst, cdst.data(), cdst.size() * sizeof(void*)), "copy dst");
+        check(upload_sync(st_, g.d_clen, clen.data(), clen.size() * sizeof(long long)), "copy len");
     }
     for (size_t k = 0; k < tsteps_.size(); ++k) {
         const int t = step_index_t_[k];
@@ -538,11 +595,11 @@ void Hps::build() {
     // the merges of every level (a fixed launch sequence for this tree) replay as a CUDA graph from
     // the third build on (first eager, second captured); the leaf DtN maps above stay eager
     const long long l0 = g_kernel_launches.load();
-    graph_build_.run(st_, 1, graphs_ && !prof_, [&] { merge_levels(mesh_.max_level - 1); });
+    graph_build_.run(st_, 1, graphs_ && !prof_, [&] { merge_levels(mesh_.max_level - 1, true); });
     build_launches_ = g_kernel_launches.load() - l0;
     check(cudaGetLastError(), "build launch");
     check(cudaStreamSynchronize(st_), "build sync");
-    singular_ = count_singular(mesh_.max_level) + leaf_singular_;
+    singular_ = count_singular(mesh_.max_level, true) + leaf_singular_;
     if (solver_type_ == SOLVER_FIVE_POINT) {
         std::vector<int> info(num_leaves());
         check(cudaMemcpy(info.data(), d_fpinfo_, info.size() * sizeof(int), cudaMemcpyDeviceToHost), "fp info");
@@ -557,7 +614,7 @@ void Hps::build() {
 
 // every merge of the tree levels top .. 0, deepest first (HPSAlgorithm.hpp:497-518 per node): the
 // children's T of level top + 1 must be in place
-void Hps::merge_levels(int top) {
+void Hps::merge_levels(int top, bool distinct) {
     for (int lvl = top; lvl >= 0; --lvl) {
         for (size_t k = 0; k < tsteps_.size(); ++k)
             if (tsteps_[k].level == lvl + 1) {
@@ -568,12 +625,12 @@ void Hps::merge_levels(int top) {
             }
         for (auto& g : groups_) {
             if (g.level != lvl) continue;
-            const int cnt = int(g.nodes.size()), s = g.s, m = 4 * s;
+            const int all = int(g.nodes.size()), cnt = distinct ? g.distinct : all, s = g.s, m = 4 * s;
             const double c = cnt, dm = m;
             pb("gather_xht");
             merge_gather_xht(st_, g.d_items, cnt, s);
             pe(c * 8 * (dm * dm + 2 * dm * dm + 4 * dm * dm) * 1.5, 0);
-            check(cudaMemsetAsync(g.d_info, 0, cnt * sizeof(int), st_), "memset info");
+            check(cudaMemsetAsync(g.d_info, 0, all * sizeof(int), st_), "memset info");
             pb("getrf");
             dgetrf_batched(st_, m, g.d_X, m, g.d_piv, g.d_info, cnt);
             piv_to_perm(st_, m, g.d_piv, g.d_perm, cnt);
@@ -590,17 +647,24 @@ void Hps::merge_levels(int top) {
             GemmArgs ga{g.d_gA, 0, 2 * s, g.d_gB, 0, 3 * m, g.d_gC, 0, 2 * m, g.d_gB2, 0, s};
             dgemm_batched(st_, s, 2 * m, 2 * s, 1.0, ga, 1.0, 8 * cnt);
             pe(c * 8 * (dm * dm / 2 + dm * 2 * dm + 2 * 4 * dm * dm), c * 2.0 * (2 * dm) * (2 * dm) * (dm / 2));
+            if (distinct && g.ncopy > 0) {
+                pb("copy_equal");
+                copy_batched(st_, g.d_csrc, g.d_cdst, g.d_clen, g.ncopy, 128LL * s * s * (all - cnt));
+                pe(double(all - cnt) * 2 * 8 * 128 * s * s, 0);
+            }
         }
     }
 }
 
 // interface LUs with a zero pivot among the merges of the levels below `below` (synchronous)
-int Hps::count_singular(int below) {
+int Hps::count_singular(int below, bool distinct) {
     int bad = 0;
     for (auto& g : groups_) {
         if (g.level >= below) continue;
         std::vector<int> info(g.nodes.size());
         check(cudaMemcpy(info.data(), g.d_info, info.size() * sizeof(int), cudaMemcpyDeviceToHost), "info");
+        if (distinct)
+            for (size_t k = 0; k < g.same.size(); ++k) info[g.distinct + k] = info[g.same[k]];
         for (int v : info) bad += (v != 0);
     }
     return bad;

@@ -51,6 +51,14 @@ struct NodeDev {
 struct Group {
     int level = 0, s = 0;
     std::vector<int> nodes;
+    // nodes[0 .. distinct) have pairwise different operators, nodes[distinct + k] the same as
+    // nodes[same[k]]: build() merges the former and copies T, RHS and H to the latter
+    int distinct = 0;
+    std::vector<int> same;
+    int ncopy = 0;
+    const double** d_csrc = nullptr;
+    double** d_cdst = nullptr;
+    long long* d_clen = nullptr;
     MergeItem* d_items = nullptr;
     double** d_X = nullptr;
     double** d_RHS = nullptr;
@@ -287,10 +295,11 @@ public:
     void profile_reset();
 
 private:
-    void merge_levels(int top);       // merges of levels top .. 0
+    // merges of levels top .. 0; `distinct`: one merge per distinct operator, copied to its equals
+    void merge_levels(int top, bool distinct);
     void upward_levels(int top);      // upward pass of levels top .. 0
     void downward_levels(int bottom, bool uncoarsen_bottom);  // split from the root to level `bottom`
-    int count_singular(int below);    // zero pivots among the merges of levels < below
+    int count_singular(int below, bool distinct);  // zero pivots among the merges of levels < below
     void plan();
     void allocate();
     void upload_tables();

@@ -6,6 +6,7 @@
 // fresh build() bit for bit.
 #include <cstring>
 #include <map>
+#include <numeric>
 #include <stdexcept>
 #include <string>
 #include <tuple>
@@ -165,7 +166,7 @@ void Hps::build_from(const Hps& old) {
     build_leaf_types();
     // the reused operators first: parents read their children's T when they merge
     copy_batched(st_, reinterpret_cast<const double* const*>(at(c_src)), reinterpret_cast<double* const*>(at(c_dst)),
-                 reinterpret_cast<const long long*>(at(c_len)), int(ncopy));
+                 reinterpret_cast<const long long*>(at(c_len)), int(ncopy), std::accumulate(clen.begin(), clen.end(), 0LL));
     const int maxL = mesh_.max_level;
     for (int lvl = maxL - 1; lvl >= 0; --lvl) {
         for (size_t k = 0; k < tsteps_.size(); ++k)

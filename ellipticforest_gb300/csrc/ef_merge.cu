@@ -395,12 +395,17 @@ __global__ void k_root_same(int m, const double* a, const double* b, const doubl
     if (threadIdx.x == 0) *flag = diff ? 0 : 1;
 }
 
+// Copies of whole operators: src and dst are starts of arena buffers (256-byte aligned), so whole
+// 16-byte pairs move and an odd last element goes by itself.
 __global__ void k_copy_batched(const double* const* src, double* const* dst, const long long* len) {
     const double* a = src[blockIdx.y];
     double* b = dst[blockIdx.y];
-    const long long n = len[blockIdx.y];
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
-        b[e] = a[e];
+    const long long n = len[blockIdx.y], n2 = n >> 1;
+    const double2* a2 = reinterpret_cast<const double2*>(a);
+    double2* b2 = reinterpret_cast<double2*>(b);
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n2; e += (long long)gridDim.x * blockDim.x)
+        b2[e] = a2[e];
+    if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) b[n - 1] = a[n - 1];
 }
 
 __global__ void k_fill_zero(double* p, long long n) {
@@ -542,10 +547,13 @@ void root_same(cudaStream_t st, int m, const double* a, const double* b, const d
     ++g_kernel_launches;
 }
 
-void copy_batched(cudaStream_t st, const double* const* src, double* const* dst, const long long* len, int count) {
+void copy_batched(cudaStream_t st, const double* const* src, double* const* dst, const long long* len, int count,
+                  long long total) {
+    // a block per 4096 elements of the mean buffer (eight pairs per thread), at most 64 per buffer
+    const int per = int(std::max(1LL, std::min(64LL, total / std::max(1, count) / 4096)));
     for (int k0 = 0; k0 < count; k0 += 65535) {
         const int c = count - k0 < 65535 ? count - k0 : 65535;
-        k_copy_batched<<<dim3(64, c), 256, 0, st>>>(src + k0, dst + k0, len + k0);
+        k_copy_batched<<<dim3(per, c), 256, 0, st>>>(src + k0, dst + k0, len + k0);
         ++g_kernel_launches;
     }
 }
