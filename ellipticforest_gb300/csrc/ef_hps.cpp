@@ -5,6 +5,7 @@
 // Dirichlet data, pre-order split1to4, leafSolve).  Each tree level is processed as a whole; the
 // merges of one level are independent, so the result equals the reference's post-order traversal.
 #include "ef_hps.hpp"
+#include "ef_gemm64.hpp"
 
 #include <algorithm>
 #include <array>
@@ -81,6 +82,7 @@ Hps::~Hps() {
     if (arena_) cudaFree(arena_);
     if (arena32_) cudaFree(arena32_);
     if (d_rootA_) cudaFree(d_rootA_);
+    if (d_ws_) cudaFree(d_ws_);
 }
 
 cudaEvent_t Hps::ev_get() {
@@ -595,10 +597,15 @@ void Hps::build() {
     // the merges of every level (a fixed launch sequence for this tree) replay as a CUDA graph from
     // the third build on (first eager, second captured); the leaf DtN maps above stay eager
     const long long l0 = g_kernel_launches.load();
-    graph_build_.run(st_, 1, graphs_ && !prof_, [&] { merge_levels(mesh_.max_level - 1, true); });
+    for (const auto& g : groups_) merge_workspace(g.distinct, g.s);
+    graph_build_.run(st_, 1, graphs_ && !prof_, [&] { merge_levels(mesh_.max_level - 1, true, false); });
     build_launches_ = g_kernel_launches.load() - l0;
     check(cudaGetLastError(), "build launch");
     check(cudaStreamSynchronize(st_), "build sync");
+    if (merges_rejected(mesh_.max_level)) {
+        merge_levels(mesh_.max_level - 1, true, true);
+        check(cudaStreamSynchronize(st_), "build sync");
+    }
     singular_ = count_singular(mesh_.max_level, true) + leaf_singular_;
     if (solver_type_ == SOLVER_FIVE_POINT) {
         std::vector<int> info(num_leaves());
@@ -612,9 +619,96 @@ void Hps::build() {
     built_ = true;
 }
 
+bool Hps::merge_workspace(int cnt, int s) {
+    if (!merge64_supported(s)) return true;
+    const size_t need = merge64_workspace(cnt, s) + 1024;
+    if (need <= ws_bytes_) return true;
+    if (ws_refused_) return false;
+    check(cudaStreamSynchronize(st_), "workspace sync");
+    graph_build_.clear();  // the captured merges point into the old workspace
+    if (d_ws_) cudaFree(d_ws_);
+    d_ws_ = nullptr;
+    ws_bytes_ = 0;
+    if (cudaMalloc(&d_ws_, need) != cudaSuccess) {
+        (void)cudaGetLastError();
+        d_ws_ = nullptr;
+        ws_refused_ = true;
+        return false;
+    }
+    ws_bytes_ = need;
+    d_wserr_ = reinterpret_cast<int*>(d_ws_ + need - 1024);
+    check(cudaMemsetAsync(d_wserr_, 0, sizeof(int), st_), "memset workspace error");
+    return true;
+}
+
+bool Hps::merges_rejected(int below) {
+    if (!d_ws_) return false;
+    int err = 0;
+    check(cudaMemcpy(&err, d_wserr_, sizeof(int), cudaMemcpyDeviceToHost), "merge error");
+    if (err) {
+        check(cudaMemset(d_wserr_, 0, sizeof(int)), "merge error");
+        throw std::runtime_error("CUDA error in build: an operand copy of a merge did not complete");
+    }
+    for (auto& g : groups_) {
+        if (g.level >= below || !merge64_supported(g.s)) continue;
+        std::vector<int> info(g.nodes.size());
+        check(cudaMemcpy(info.data(), g.d_info, info.size() * sizeof(int), cudaMemcpyDeviceToHost), "info");
+        for (int v : info)
+            if (v) return true;
+    }
+    return false;
+}
+
+void Hps::merge_lu(const MergeTables& t, int cnt, int s) {
+    const int m = 4 * s;
+    const double c = cnt, dm = m;
+    pb("getrf");
+    dgetrf_batched(st_, m, t.X, m, t.piv, t.info, cnt);
+    piv_to_perm(st_, m, t.piv, t.perm, cnt);
+    pe(c * 8 * 2 * dm * dm, c * 2.0 / 3.0 * dm * dm * dm);
+    pb("gather_rhs");
+    merge_gather_rhs(st_, t.items, cnt, s);
+    pe(c * 8 * (3 * dm * dm + dm * dm), 0);
+    pb("lu_solve");
+    dlu_solve_permuted(st_, m, 3 * m, (const double* const*)t.X, m, t.RHS, 3 * m, cnt);
+    pe(c * 8 * (dm * dm + 2 * 3 * dm * dm), c * 2.0 * dm * dm * 3 * dm);
+    // T = T_LHS + H S  (HPSAlgorithm.hpp:940-968), S = first 8s columns of RHS; H's zero
+    // blocks are skipped: each s-row block of T takes K = 2s (its child's two interfaces)
+    pb("gemm_T");
+    GemmArgs ga{t.gA, 0, 2 * s, t.gB, 0, 3 * m, t.gC, 0, 2 * m, t.gB2, 0, s};
+    dgemm_batched(st_, s, 2 * m, 2 * s, 1.0, ga, 1.0, 8 * cnt);
+    pe(c * 8 * (dm * dm / 2 + dm * 2 * dm + 2 * 4 * dm * dm), c * 2.0 * (2 * dm) * (2 * dm) * (dm / 2));
+}
+
+void Hps::merge_nodes(const MergeTables& t, int cnt, int s, bool careful) {
+    const double c = cnt, dm = 4.0 * s;
+    pb("gather_xht");
+    merge_gather_xht(st_, t.items, cnt, s);
+    pe(c * 8 * (dm * dm + 2 * dm * dm + 4 * dm * dm) * 1.5, 0);
+    check(cudaMemsetAsync(t.info, 0, cnt * sizeof(int), st_), "memset info");
+    if (!merge64_supported(s) || ws_bytes_ < merge64_workspace(cnt, s) + 1024) {
+        merge_lu(t, cnt, s);
+        return;
+    }
+    pb("merge64");
+    merge64(st_, t.items, cnt, s, t.info, d_ws_, d_wserr_);
+    pe(c * 8 * 12 * dm * dm, c * 8.0 * dm * dm * dm);
+    if (!careful) return;
+    std::vector<int> info(cnt);
+    check(cudaMemcpyAsync(info.data(), t.info, cnt * sizeof(int), cudaMemcpyDeviceToHost, st_), "merge info");
+    check(cudaStreamSynchronize(st_), "merge info");
+    for (int i = 0; i < cnt; ++i) {
+        if (!info[i]) continue;
+        const MergeTables one = t.from(i);
+        merge_gather_xht(st_, one.items, 1, s);
+        check(cudaMemsetAsync(one.info, 0, sizeof(int), st_), "memset info");
+        merge_lu(one, 1, s);
+    }
+}
+
 // every merge of the tree levels top .. 0, deepest first (HPSAlgorithm.hpp:497-518 per node): the
 // children's T of level top + 1 must be in place
-void Hps::merge_levels(int top, bool distinct) {
+void Hps::merge_levels(int top, bool distinct, bool careful) {
     for (int lvl = top; lvl >= 0; --lvl) {
         for (size_t k = 0; k < tsteps_.size(); ++k)
             if (tsteps_[k].level == lvl + 1) {
@@ -625,28 +719,10 @@ void Hps::merge_levels(int top, bool distinct) {
             }
         for (auto& g : groups_) {
             if (g.level != lvl) continue;
-            const int all = int(g.nodes.size()), cnt = distinct ? g.distinct : all, s = g.s, m = 4 * s;
-            const double c = cnt, dm = m;
-            pb("gather_xht");
-            merge_gather_xht(st_, g.d_items, cnt, s);
-            pe(c * 8 * (dm * dm + 2 * dm * dm + 4 * dm * dm) * 1.5, 0);
-            check(cudaMemsetAsync(g.d_info, 0, all * sizeof(int), st_), "memset info");
-            pb("getrf");
-            dgetrf_batched(st_, m, g.d_X, m, g.d_piv, g.d_info, cnt);
-            piv_to_perm(st_, m, g.d_piv, g.d_perm, cnt);
-            pe(c * 8 * 2 * dm * dm, c * 2.0 / 3.0 * dm * dm * dm);
-            pb("gather_rhs");
-            merge_gather_rhs(st_, g.d_items, cnt, s);
-            pe(c * 8 * (3 * dm * dm + dm * dm), 0);
-            pb("lu_solve");
-            dlu_solve_permuted(st_, m, 3 * m, (const double* const*)g.d_X, m, g.d_RHS, 3 * m, cnt);
-            pe(c * 8 * (dm * dm + 2 * 3 * dm * dm), c * 2.0 * dm * dm * 3 * dm);
-            // T = T_LHS + H S  (HPSAlgorithm.hpp:940-968), S = first 8s columns of RHS; H's zero
-            // blocks are skipped: each s-row block of T takes K = 2s (its child's two interfaces)
-            pb("gemm_T");
-            GemmArgs ga{g.d_gA, 0, 2 * s, g.d_gB, 0, 3 * m, g.d_gC, 0, 2 * m, g.d_gB2, 0, s};
-            dgemm_batched(st_, s, 2 * m, 2 * s, 1.0, ga, 1.0, 8 * cnt);
-            pe(c * 8 * (dm * dm / 2 + dm * 2 * dm + 2 * 4 * dm * dm), c * 2.0 * (2 * dm) * (2 * dm) * (dm / 2));
+            const int all = int(g.nodes.size()), cnt = distinct ? g.distinct : all, s = g.s;
+            if (cnt < all) check(cudaMemsetAsync(g.d_info + cnt, 0, (all - cnt) * sizeof(int), st_), "memset info");
+            merge_nodes({g.d_items, g.d_X, g.d_RHS, g.d_piv, g.d_perm, g.d_info, g.d_gA, g.d_gB, g.d_gB2, g.d_gC}, cnt, s,
+                        careful);
             if (distinct && g.ncopy > 0) {
                 pb("copy_equal");
                 copy_batched(st_, g.d_csrc, g.d_cdst, g.d_clen, g.ncopy, 128LL * s * s * (all - cnt));

@@ -75,6 +75,23 @@ struct Group {
     double** d_gC = nullptr;
 };
 
+// device tables of a run of merges (per node, or eight per node for the split product's)
+struct MergeTables {
+    const MergeItem* items;
+    double* const* X;
+    double* const* RHS;
+    int* const* piv;
+    int* const* perm;
+    int* info;
+    const double* const* gA;
+    const double* const* gB;
+    const double* const* gB2;
+    double* const* gC;
+    MergeTables from(int i) const {
+        return {items + i, X + i, RHS + i, piv + i, perm + i, info + i, gA + 8 * i, gB + 8 * i, gB2 + 8 * i, gC + 8 * i};
+    }
+};
+
 struct ResampleStep {  // one batched (un)coarsening step: `count` items of fine size nf
     int level = 0;     // tree level of the nodes
     int nf = 0;
@@ -295,8 +312,13 @@ public:
     void profile_reset();
 
 private:
-    // merges of levels top .. 0; `distinct`: one merge per distinct operator, copied to its equals
-    void merge_levels(int top, bool distinct);
+    // merges of levels top .. 0; `distinct`: one merge per distinct operator, copied to its equals;
+    // `careful`: after every group, the merges that block elimination gave up go through the pivoted LU
+    void merge_levels(int top, bool distinct, bool careful);
+    void merge_nodes(const MergeTables& t, int cnt, int s, bool careful);
+    void merge_lu(const MergeTables& t, int cnt, int s);  // from the gathered X, H and T_LHS on
+    bool merge_workspace(int cnt, int s);  // room for merge64; false: not available, merge by LU
+    bool merges_rejected(int below);       // block elimination set info in some merge of levels < below
     void upward_levels(int top);      // upward pass of levels top .. 0
     void downward_levels(int bottom, bool uncoarsen_bottom);  // split from the root to level `bottom`
     int count_singular(int below, bool distinct);  // zero pivots among the merges of levels < below
@@ -332,6 +354,12 @@ private:
     LeafType* d_types_ = nullptr;
     LeafItem *d_items_dtn_ = nullptr, *d_items_neu_ = nullptr, *d_items_solve_ = nullptr;
     int nitems_dtn_ = 0;
+
+    // digits of the merges' products, grown to what a build needs, and the error word of their waits
+    char* d_ws_ = nullptr;
+    size_t ws_bytes_ = 0;
+    int* d_wserr_ = nullptr;
+    bool ws_refused_ = false;
 
     double *d_f_ = nullptr, *d_u_ = nullptr;
     double *d_bca_ = nullptr, *d_bcb_ = nullptr, *d_bcr_ = nullptr;

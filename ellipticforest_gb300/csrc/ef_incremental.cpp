@@ -168,44 +168,48 @@ void Hps::build_from(const Hps& old) {
     copy_batched(st_, reinterpret_cast<const double* const*>(at(c_src)), reinterpret_cast<double* const*>(at(c_dst)),
                  reinterpret_cast<const long long*>(at(c_len)), int(ncopy), std::accumulate(clen.begin(), clen.end(), 0LL));
     const int maxL = mesh_.max_level;
-    for (int lvl = maxL - 1; lvl >= 0; --lvl) {
-        for (size_t k = 0; k < tsteps_.size(); ++k)
-            if (tsteps_[k].level == lvl + 1) coarsen_T(st_, tsteps_[k].d_in, tsteps_[k].d_out, tsteps_[k].count, tsteps_[k].nf);
-        for (size_t gi = 0; gi < groups_.size(); ++gi) {
-            const Group& g = groups_[gi];
-            if (g.level != lvl) continue;
-            const Sub& sb = sub[gi];
-            if (!sb.cnt) continue;
-            const int cnt = sb.cnt, s = g.s, m = 4 * s;
-            auto* items = reinterpret_cast<const MergeItem*>(at(sb.items));
-            auto* X = reinterpret_cast<double* const*>(at(sb.X));
-            auto* RHS = reinterpret_cast<double* const*>(at(sb.RHS));
-            auto* piv = reinterpret_cast<int* const*>(at(sb.piv));
-            auto* perm = reinterpret_cast<int* const*>(at(sb.perm));
-            int* info = reinterpret_cast<int*>(at(sb.info));
-            merge_gather_xht(st_, items, cnt, s);
-            cki(cudaMemsetAsync(info, 0, cnt * sizeof(int), st_), "memset info");
-            dgetrf_batched(st_, m, X, m, piv, info, cnt);
-            piv_to_perm(st_, m, piv, perm, cnt);
-            merge_gather_rhs(st_, items, cnt, s);
-            dlu_solve_permuted(st_, m, 3 * m, (const double* const*)X, m, RHS, 3 * m, cnt);
-            GemmArgs ga{reinterpret_cast<const double* const*>(at(sb.gA)), 0, 2 * s,
-                        reinterpret_cast<const double* const*>(at(sb.gB)), 0, 3 * m,
-                        reinterpret_cast<double* const*>(at(sb.gC)), 0, 2 * m,
-                        reinterpret_cast<const double* const*>(at(sb.gB2)), 0, s};
-            dgemm_batched(st_, s, 2 * m, 2 * s, 1.0, ga, 1.0, 8 * cnt);
+    for (size_t gi = 0; gi < groups_.size(); ++gi)
+        if (sub[gi].cnt) merge_workspace(sub[gi].cnt, groups_[gi].s);
+    auto merge_dirty = [&](bool careful) {
+        for (int lvl = maxL - 1; lvl >= 0; --lvl) {
+            for (size_t k = 0; k < tsteps_.size(); ++k)
+                if (tsteps_[k].level == lvl + 1) coarsen_T(st_, tsteps_[k].d_in, tsteps_[k].d_out, tsteps_[k].count, tsteps_[k].nf);
+            for (size_t gi = 0; gi < groups_.size(); ++gi) {
+                const Sub& sb = sub[gi];
+                if (groups_[gi].level != lvl || !sb.cnt) continue;
+                const MergeTables t{reinterpret_cast<const MergeItem*>(at(sb.items)), reinterpret_cast<double* const*>(at(sb.X)),
+                                    reinterpret_cast<double* const*>(at(sb.RHS)), reinterpret_cast<int* const*>(at(sb.piv)),
+                                    reinterpret_cast<int* const*>(at(sb.perm)), reinterpret_cast<int*>(at(sb.info)),
+                                    reinterpret_cast<const double* const*>(at(sb.gA)),
+                                    reinterpret_cast<const double* const*>(at(sb.gB)),
+                                    reinterpret_cast<const double* const*>(at(sb.gB2)),
+                                    reinterpret_cast<double* const*>(at(sb.gC))};
+                merge_nodes(t, sb.cnt, groups_[gi].s, careful);
+            }
         }
-    }
+    };
+    merge_dirty(false);
     cki(cudaGetLastError(), "incremental build launch");
     cki(cudaStreamSynchronize(st_), "incremental build sync");
-    singular_ = leaf_singular_;
-    for (size_t gi = 0; gi < groups_.size(); ++gi) {
-        const Sub& sb = sub[gi];
-        if (!sb.cnt) continue;
-        std::vector<int> info(sb.cnt);
-        cki(cudaMemcpy(info.data(), at(sb.info), sb.cnt * sizeof(int), cudaMemcpyDeviceToHost), "info");
-        for (int v : info) singular_ += (v != 0);
+    auto marked = [&] {
+        int n = 0;
+        for (size_t gi = 0; gi < groups_.size(); ++gi) {
+            const Sub& sb = sub[gi];
+            if (!sb.cnt) continue;
+            std::vector<int> info(sb.cnt);
+            cki(cudaMemcpy(info.data(), at(sb.info), sb.cnt * sizeof(int), cudaMemcpyDeviceToHost), "info");
+            for (int v : info) n += (v != 0);
+        }
+        return n;
+    };
+    merges_rejected(0);  // a wait that gave up
+    int bad = marked();
+    if (bad > 0) {
+        merge_dirty(true);
+        cki(cudaStreamSynchronize(st_), "incremental build sync");
+        bad = marked();
     }
+    singular_ = leaf_singular_ + bad;
     cudaFree(dev);
     built_ = true;
 }

@@ -75,9 +75,16 @@ void Hps::build_top(int level, const double* const* T_host) {
         if (!T_host[k]) throw std::invalid_argument("build_top: null T block");
         check(cudaMemcpyAsync(nd.T, T_host[k], m * m * sizeof(double), cudaMemcpyHostToDevice, st_), "copy T block");
     }
-    merge_levels(level - 1, false);  // the T blocks come from outside: no two are known to be equal
+    // the T blocks come from outside: no two are known to be equal
+    for (const auto& g : groups_)
+        if (g.level < level) merge_workspace(int(g.nodes.size()), g.s);
+    merge_levels(level - 1, false, false);
     check(cudaGetLastError(), "top build launch");
     check(cudaStreamSynchronize(st_), "top build sync");
+    if (merges_rejected(level)) {
+        merge_levels(level - 1, false, true);
+        check(cudaStreamSynchronize(st_), "top build sync");
+    }
     singular_ = count_singular(level, false);
     top_level_ = level;
     built_ = true;
