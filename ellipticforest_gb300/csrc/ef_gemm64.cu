@@ -34,11 +34,16 @@ constexpr int kDigits = 8;
 constexpr int kMT = 128, kNT = 32, kKB = 64;             // tile rows, tile columns, k per block
 constexpr int kPlane = kMT * kKB * 2;                    // one digit of an A block: 16 KB
 constexpr int kBBlock = kDigits * kNT * kKB * 2;         // all digits of a B block: 32 KB
-constexpr int kASlots = 9, kBSlots = 2, kSets = 2;       // rings: A digits, B blocks, accumulator sets
+constexpr int kASlots = 6, kBSlots = 2, kSets = 2;       // rings: A digits, B blocks, accumulator sets
 constexpr int kFlush = 2;                                // k blocks per accumulator set (128 values of k)
 constexpr int kNotFinite = 1 << 20;                      // exponent of a row that holds an infinity or NaN
+constexpr int kCollect = 256, kGemmThreads = kCollect + 64;  // collecting threads, then the copy and MMA warps
+constexpr int kHalf = kNT / 2;                           // columns per collecting thread
 constexpr int kMaxOps = 8, kMaxGemms = 4;
-constexpr size_t kSmem = 1024 + size_t(kASlots) * kPlane + size_t(kBSlots) * kBBlock + 512;
+enum Add : int { ADD_NONE = 0, ADD_D = 1, ADD_IDENTITY = 2 };
+constexpr int kSums = kMT * kNT * 16;                    // a tile's integer sums on their way to rows of C
+constexpr size_t kSmem = 1024 + size_t(kASlots) * kPlane + size_t(kBSlots) * kBBlock + kSums + 512;
+static_assert(kSmem <= 227 * 1024, "shared memory of one CTA");
 static_assert(2 * kSmem > 228 * 1024, "one CTA per SM: each takes all of TMEM");
 
 __device__ __forceinline__ double* table_ptr(const PtrTable& t, int b) {
@@ -53,6 +58,8 @@ struct SplitOp {
     long long pstride;
     int* ex;
     int estride, blk0;
+    int* info;  // info[item] = 1 where a row's largest entry is 2^limit or more
+    int limit;
 };
 struct SplitList {
     int n;
@@ -74,69 +81,62 @@ __global__ void __launch_bounds__(256) k_split64(const __grid_constant__ SplitLi
     const long long sr = cols ? 1 : P.v.ld, sk = cols ? P.v.ld : 1;
     __shared__ unsigned s_max[8][32];
     __shared__ uint4 stage[kDigits * 256];
-    auto row_ptr = [&](int r) { return base + r * sr + (r >= P.v.rs ? P.v.dr : 0); };
-    auto high_word = [&](const double* p, int k) {
-        return unsigned(__double2hiint(p[k * sk + (k >= P.v.ks ? P.v.dk : 0)])) & 0x7fffffffu;
+    // rows of this thread: columns of B by lanes (coalesced reads), rows of A by groups of eight threads;
+    // either way eight consecutive k per 64
+    const int rl = cols ? lane : tid >> 3, oct = cols ? warp : tid & 7, r = r0 + rl;
+    const bool in = r < P.rows;
+    const double* p = base + min(r, P.rows - 1) * sr + (r >= P.v.rs ? P.v.dr : 0);
+    auto load = [&](int kb, double (&x)[8]) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int k = kb * kKB + 8 * oct + u;
+            x[u] = in && k < K ? p[k * sk + (k >= P.v.ks ? P.v.dk : 0)] : 0.0;
+        }
     };
-    if (cols) {
-        const int r = r0 + lane;
+    auto largest = [](const double (&x)[8]) {
         unsigned m = 0;
-        if (r < P.rows) {
-            const double* p = row_ptr(r);
-            int k = warp;
-            for (; k + 56 < K; k += 64) {
 #pragma unroll
-                for (int u = 0; u < 8; ++u) m = max(m, high_word(p, k + 8 * u));
-            }
-            for (; k < K; k += 8) m = max(m, high_word(p, k));
-        }
-        s_max[warp][lane] = m;
+        for (int u = 0; u < 8; ++u) m = max(m, unsigned(__double2hiint(x[u])) & 0x7fffffffu);
+        return m;
+    };
+    double x[8], y[8];  // the first two blocks stay in registers
+    load(0, x);
+    load(1, y);
+    unsigned mx = max(largest(x), largest(y));
+    for (int kb = 2; kb < nkb; kb += 2) {
+        double t[8], q[8];
+        load(kb, t);
+        load(kb + 1, q);
+        mx = max(mx, max(largest(t), largest(q)));
+    }
+    if (cols) {
+        s_max[warp][lane] = mx;
         __syncthreads();
-        if (warp == 0) {
 #pragma unroll
-            for (int w = 1; w < 8; ++w) m = max(m, s_max[w][lane]);
-            s_max[0][lane] = m;
-        }
+        for (int w = 0; w < 8; ++w) mx = max(mx, s_max[w][lane]);
     } else {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int r = r0 + 4 * warp + q;
-            unsigned m = 0;
-            if (r < P.rows) {
-                const double* p = row_ptr(r);
-                int k = lane;
-                for (; k + 224 < K; k += 256) {
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) m = max(m, high_word(p, k + 32 * u));
-                }
-                for (; k < K; k += 32) m = max(m, high_word(p, k));
-            }
-            m = __reduce_max_sync(0xffffffffu, m);
-            if (lane == 0) s_max[0][4 * warp + q] = m;
-        }
+        for (int off = 4; off > 0; off >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, off));
     }
-    __syncthreads();
-    // rows of this thread in the second pass: columns of B by lanes (coalesced reads), rows of A by
-    // groups of eight threads that each take eight consecutive k
-    const int rl = cols ? lane : tid >> 3, oct = cols ? warp : tid & 7;
-    const int r = r0 + rl;
-    const unsigned mx = s_max[0][rl];
     const bool finite = mx < 0x7ff00000u;
     const int E = max(int(mx >> 20), 1);  // |x| < 2^(E - 1022)
-    if (tid < 32 && r0 + tid < P.rows) {
-        const unsigned m2 = s_max[0][tid];
-        P.ex[(long long)b * P.estride + r0 + tid] = m2 < 0x7ff00000u ? max(int(m2 >> 20), 1) - 1022 : kNotFinite;
+    if (in && oct == 0) {
+        const int e = finite ? E - 1022 : kNotFinite;
+        P.ex[(long long)b * P.estride + r] = e;
+        if (P.info && e > P.limit) P.info[b] = 1;
     }
-    const bool live = r < P.rows && finite;
-    const double* p = row_ptr(min(r, P.rows - 1));
     unsigned char* out = P.planes + (long long)b * P.pstride;
     for (int kb = 0; kb < nkb; ++kb) {
         const int k0 = kb * kKB + 8 * oct;
-        double x[8];
+        if (kb == 1) {
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int k = k0 + u;
-            x[u] = live && k < K ? p[k * sk + (k >= P.v.ks ? P.v.dk : 0)] : 0.0;
+            for (int u = 0; u < 8; ++u) x[u] = y[u];
+        } else if (kb > 1) {
+            load(kb, x);
+        }
+        if (!finite) {
+#pragma unroll
+            for (int u = 0; u < 8; ++u) x[u] = 0.0;
         }
         unsigned uh[8], ul[8];
 #pragma unroll
@@ -193,14 +193,50 @@ struct GemmOp {
     const int *ea, *eb;
     int eastride, ebstride;
     int M, N, K;
-    MatView c;  // C; rows >= c.rs shifted by c.dr, columns >= c.ks by c.dk
-    int neg, add;  // C = (add ? C : 0) + (neg ? -1 : 1) A B
+    MatView c, d;  // C = (neg ? -1 : 1) A B + D or I or nothing; rows >= rs shifted by dr, columns >= ks by dk
+    int neg, add;
     int mt, nt, tile0;
 };
 struct GemmList {
     int n, tiles;
     GemmOp op[kMaxGemms];
 };
+
+// (h + f 2^-32) 2^k as a double, rounded to nearest even, with integer instructions only (a conversion and
+// two additions per entry would take the FP64 pipe longer than the whole product of a short K) and without a
+// branch, so that several entries overlap.  `odd`: the result is not a normal number (see fixed_to_double_any).
+__device__ __forceinline__ double fixed_to_double(long long h, unsigned f, int k, bool& odd) {
+    const unsigned sign = unsigned(h >> 63);
+    f = (f ^ sign) - sign;
+    h = (h ^ (h >> 63)) + (sign != 0 && f == 0 ? 1 : 0);
+    unsigned a2 = unsigned((unsigned long long)h >> 32), a1 = unsigned(h), a0 = f;
+    int n = 0;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {  // leading zero words
+        const bool z = a2 == 0;
+        n += z ? 32 : 0;
+        a2 = z ? a1 : a2;
+        a1 = z ? a0 : a1;
+        a0 = z ? 0u : a0;
+    }
+    const int l = __clz(int(a2)) & 31;
+    const unsigned b2 = __funnelshift_l(a1, a2, l), b1 = __funnelshift_l(a0, a1, l), b0 = a0 << l;
+    const int e = 1023 + 63 - n - l + k;  // biased exponent of the leading bit
+    unsigned lo = (b2 << 21) | (b1 >> 11);
+    const unsigned up = (b1 & 0x7ffu) + ((b0 | (lo & 1u)) != 0 ? 1u : 0u) > 0x400u ? 1u : 0u;
+    lo += up;
+    const unsigned hi = (unsigned(e - 1) << 20) + (b2 >> 11) + (up != 0 && lo == 0 ? 1u : 0u);
+    odd = b2 != 0 && unsigned(e - 1) > 2044u;
+    return b2 == 0 ? 0.0 : __hiloint2double(int(hi | (sign & 0x80000000u)), int(lo));
+}
+// the same for results beyond the normal range and rows or columns that are not finite
+__device__ __noinline__ double fixed_to_double_any(long long h, unsigned f, int ea, int eb) {
+    if (ea >= kNotFinite || eb >= kNotFinite) return __longlong_as_double(0x7ff8000000000000LL);
+    return scalbn((double)h + (double)f * 0x1p-32, ea + eb - 36);
+}
+__device__ __forceinline__ long long join(const int4& q) {
+    return (long long)(((unsigned long long)unsigned(q.y) << 32) | unsigned(q.x));
+}
 
 struct TileAt {
     int o, b, m, n;
@@ -223,34 +259,35 @@ __device__ __forceinline__ TileAt tile_at(const GemmList& L, int t) {
     return r;
 }
 
-// C tile of 128 x 32 per step, one CTA per SM walking over the tiles.  Warp 4 copies digit blocks (one bulk
-// copy each, the layout is the shared-memory image), warp 5 issues the MMAs, warps 0-3 collect.  For every
+// C tile of 128 x 32 per step, one CTA per SM walking over the tiles.  Warp 8 copies digit blocks (one bulk
+// copy each, the layout is the shared-memory image), warp 9 issues the MMAs, warps 0-7 collect.  For every
 // 16 values of k one MMA per digit i of A multiplies it with digits 0 .. 7 - i of B, which are consecutive
 // rows of one K-major operand, into the consecutive accumulators of weights i .. 7: N = 32 (8 - i), so a
 // digit of A is read from shared memory once.  Two accumulator sets of 256 TMEM columns alternate, so the
 // collecting of 128 values of k (8 sums per entry: convert, multiply-add into 64 bits) hides behind the
 // MMAs of the next.  Bound: the 160 KB of digits per 64 values of k (2304 MMA clocks) from L2.
-__global__ void __launch_bounds__(192, 1) k_gemm64(const __grid_constant__ GemmList L, int* __restrict__ err) {
+__global__ void __launch_bounds__(kGemmThreads, 1) k_gemm64(const __grid_constant__ GemmList L, int* __restrict__ err) {
     extern __shared__ unsigned char g_smem[];
     unsigned char* base = g_smem + ((1024u - (smem_u32(g_smem) & 1023u)) & 1023u);
     unsigned char* bbase = base + size_t(kASlots) * kPlane;
-    unsigned long long* bars = reinterpret_cast<unsigned long long*>(bbase + size_t(kBSlots) * kBBlock);
+    int4* sums = reinterpret_cast<int4*>(bbase + size_t(kBSlots) * kBBlock);
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(sums + kMT * kNT);
     unsigned long long *a_full = bars, *a_empty = a_full + kASlots, *b_full = a_empty + kASlots,
                        *b_empty = b_full + kBSlots, *acc_full = b_empty + kBSlots, *acc_empty = acc_full + kSets,
                        *drain = acc_empty + kSets;
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(drain + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     if (tid == 0) {
         for (int i = 0; i < kASlots; ++i) { mbar_init(a_full + i, 1); mbar_init(a_empty + i, 1); }
         for (int i = 0; i < kBSlots; ++i) { mbar_init(b_full + i, 1); mbar_init(b_empty + i, 1); }
-        for (int i = 0; i < kSets; ++i) { mbar_init(acc_full + i, 1); mbar_init(acc_empty + i, 128); }
+        for (int i = 0; i < kSets; ++i) { mbar_init(acc_full + i, 1); mbar_init(acc_empty + i, kCollect); }
         mbar_init(drain, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     }
-    if (warp == 5) {
+    if (warp == 9) {
         tmem_alloc(tmem_slot, 512u);
         tmem_relinquish();
     }
@@ -259,167 +296,220 @@ __global__ void __launch_bounds__(192, 1) k_gemm64(const __grid_constant__ GemmL
     tc_fence_after();
     const unsigned tmem = *tmem_slot;
 
-    if (warp == 4) {
-        if (lane == 0) {
-            unsigned na = 0, nb = 0;  // copies issued into either ring
-            bool ok = true;
-            for (int t = blockIdx.x; t < L.tiles && ok; t += gridDim.x) {
-                const TileAt at = tile_at(L, t);
-                const GemmOp& g = L.op[at.o];
-                const int nkb = (g.K + kKB - 1) / kKB;
-                const unsigned char* A = g.A + at.b * g.astride + (long long)at.m * nkb * (kDigits * kPlane);
-                const unsigned char* B = g.B + at.b * g.bstride + (long long)at.n * nkb * kBBlock;
-                for (int kb = 0; kb < nkb && ok; ++kb) {
-                    const unsigned sb = nb % kBSlots;
-                    if (nb >= kBSlots) ok = tc_wait(b_empty + sb, (nb / kBSlots - 1) & 1u, abort_flag);
-                    if (!ok) break;
+    // Warps 8 and 9 stay converged and one elected lane issues: a branch on the lane number would have the
+    // compiler move every operand of an instruction into uniform registers through a loop over the active
+    // lanes (109 clocks per MMA measured, against 16 to 128 that the MMA takes).
+    if (warp == 8) {
+        unsigned sa = 0, sb = 0, pa = 0, pb = 0;  // ring positions and the parity of their current round
+        unsigned na = 0, nb = 0;                  // copies issued into either ring
+        bool ok = true;
+        for (int t = blockIdx.x; t < L.tiles && ok; t += gridDim.x) {
+            const TileAt at = tile_at(L, t);
+            const GemmOp& g = L.op[at.o];
+            const int nkb = (g.K + kKB - 1) / kKB;
+            const unsigned char* A = g.A + at.b * g.astride + (long long)at.m * nkb * (kDigits * kPlane);
+            const unsigned char* B = g.B + at.b * g.bstride + (long long)at.n * nkb * kBBlock;
+            for (int kb = 0; kb < nkb && ok; ++kb) {
+                if (nb >= kBSlots) ok = tc_wait(b_empty + sb, pb ^ 1u, abort_flag);
+                if (!(ok = __all_sync(0xffffffffu, ok))) break;
+                if (elect_one()) {
                     mbar_expect_tx(b_full + sb, kBBlock);
-                    bulk_copy(bbase + size_t(sb) * kBBlock, B + (long long)kb * kBBlock, kBBlock, b_full + sb);
-                    ++nb;
-                    for (int i = 0; i < kDigits; ++i) {
-                        const unsigned sa = na % kASlots;
-                        if (na >= kASlots) ok = tc_wait(a_empty + sa, (na / kASlots - 1) & 1u, abort_flag);
-                        if (!ok) break;
+                    bulk_copy(bbase + size_t(sb) * kBBlock, B, kBBlock, b_full + sb);
+                }
+                __syncwarp();
+                B += kBBlock;
+                ++nb;
+                if (++sb == kBSlots) { sb = 0; pb ^= 1u; }
+                for (int i = 0; i < kDigits; ++i) {
+                    if (na >= kASlots) ok = tc_wait(a_empty + sa, pa ^ 1u, abort_flag);
+                    if (!(ok = __all_sync(0xffffffffu, ok))) break;
+                    if (elect_one()) {
                         mbar_expect_tx(a_full + sa, kPlane);
-                        bulk_copy(base + size_t(sa) * kPlane, A + ((long long)kb * kDigits + i) * kPlane, kPlane, a_full + sa);
-                        ++na;
+                        bulk_copy(base + size_t(sa) * kPlane, A, kPlane, a_full + sa);
                     }
+                    __syncwarp();
+                    A += kPlane;
+                    ++na;
+                    if (++sa == kASlots) { sa = 0; pa ^= 1u; }
                 }
-            }
-            if (!ok) {
-                // let the copies still in flight land before the shared memory goes away
-                volatile int never_set = 0;
-                for (unsigned q = na > kASlots ? na - kASlots : 0; q < na; ++q)
-                    (void)tc_wait(a_full + q % kASlots, (q / kASlots) & 1u, &never_set);
-                for (unsigned q = nb > kBSlots ? nb - kBSlots : 0; q < nb; ++q)
-                    (void)tc_wait(b_full + q % kBSlots, (q / kBSlots) & 1u, &never_set);
-                atomicExch(err, 1);
             }
         }
-    } else if (warp == 5) {
-        if (lane == 0) {
-            unsigned na = 0, nb = 0, ns = 0;
-            bool ok = true;
-            const uint32_t a0 = smem_u32(base), b0 = smem_u32(bbase);
-            for (int t = blockIdx.x; t < L.tiles && ok; t += gridDim.x) {
-                const GemmOp& g = L.op[tile_at(L, t).o];
-                const int nkb = (g.K + kKB - 1) / kKB;
-                for (int kb = 0; kb < nkb && ok; ++kb) {
-                    const unsigned set = ns % kSets;
-                    if (kb % kFlush == 0 && ns >= kSets) ok = tc_wait(acc_empty + set, (ns / kSets - 1) & 1u, abort_flag);
-                    const unsigned sb = nb % kBSlots;
-                    if (ok) ok = tc_wait(b_full + sb, (nb / kBSlots) & 1u, abort_flag);
-                    const int steps = min(4, (g.K - kb * kKB + 15) / 16);
-                    for (int i = 0; i < kDigits && ok; ++i) {
-                        const unsigned sa = na % kASlots;
-                        ok = tc_wait(a_full + sa, (na / kASlots) & 1u, abort_flag);
-                        if (!ok) break;
-                        tc_fence_after();
-                        const unsigned d = tmem + set * 256u + unsigned(i * kNT);
-                        const unsigned idesc = tc_idesc(kMT, kNT * (kDigits - i));
-                        for (int kk = 0; kk < steps; ++kk)
-                            tc_mma(d, tc_desc(a0 + sa * kPlane + kk * 32u), tc_desc(b0 + sb * kBBlock + kk * 32u), idesc,
-                                   kb % kFlush == 0 && i == 0 && kk == 0 ? 0u : 1u);
-                        tc_commit(a_empty + sa);
-                        ++na;
-                    }
-                    if (!ok) break;
-                    tc_commit(b_empty + sb);
-                    ++nb;
-                    if (kb % kFlush == kFlush - 1 || kb == nkb - 1) {
-                        tc_commit(acc_full + set);
-                        ++ns;
-                    }
-                }
-            }
-            // every MMA issued has completed before TMEM is freed
-            tc_commit(drain);
+        if (!ok && lane == 0) {
+            // let the copies still in flight land before the shared memory goes away
             volatile int never_set = 0;
-            if (!tc_wait(drain, 0u, &never_set)) ok = false;
-            if (!ok) atomicExch(err, 1);
+            for (unsigned q = na > kASlots ? na - kASlots : 0; q < na; ++q)
+                (void)tc_wait(a_full + q % kASlots, (q / kASlots) & 1u, &never_set);
+            for (unsigned q = nb > kBSlots ? nb - kBSlots : 0; q < nb; ++q)
+                (void)tc_wait(b_full + q % kBSlots, (q / kBSlots) & 1u, &never_set);
+            atomicExch(err, 1);
         }
+    } else if (warp == 9) {
+        unsigned sa = 0, sb = 0, pa = 0, pb = 0, ns = 0;
+        bool ok = true;
+        // operand descriptors differ in their address field only
+        const uint64_t da0 = tc_desc(smem_u32(base)), db0 = tc_desc(smem_u32(bbase));
+        for (int t = blockIdx.x; t < L.tiles && ok; t += gridDim.x) {
+            const int nkb = (L.op[tile_at(L, t).o].K + kKB - 1) / kKB;
+            for (int kb = 0; kb < nkb && ok; ++kb) {
+                const unsigned set = ns % kSets;
+                if (kb % kFlush == 0 && ns >= kSets) ok = tc_wait(acc_empty + set, (ns / kSets - 1) & 1u, abort_flag);
+                if (ok) ok = tc_wait(b_full + sb, pb, abort_flag);
+                const uint64_t db = db0 + uint64_t(sb * (kBBlock >> 4));
+                const unsigned d = tmem + set * 256u;
+#pragma unroll
+                for (int i = 0; i < kDigits; ++i) {
+                    if (ok) ok = tc_wait(a_full + sa, pa, abort_flag);
+                    if (!(ok = __all_sync(0xffffffffu, ok))) break;
+                    tc_fence_after();
+                    const uint64_t da = da0 + uint64_t(sa * (kPlane >> 4));
+                    if (elect_one()) {
+#pragma unroll
+                        for (int kk = 0; kk < kKB / 16; ++kk)
+                            tc_mma(d + unsigned(i * kNT), da + uint64_t(2 * kk), db + uint64_t(2 * kk),
+                                   tc_idesc(kMT, kNT * (kDigits - i)), kb % kFlush == 0 && i == 0 && kk == 0 ? 0u : 1u);
+                        tc_commit(a_empty + sa);
+                        if (i == kDigits - 1) {
+                            tc_commit(b_empty + sb);
+                            if (kb % kFlush == kFlush - 1 || kb == nkb - 1) tc_commit(acc_full + set);
+                        }
+                    }
+                    __syncwarp();
+                    if (++sa == kASlots) { sa = 0; pa ^= 1u; }
+                }
+                if (++sb == kBSlots) { sb = 0; pb ^= 1u; }
+                if (kb % kFlush == kFlush - 1 || kb == nkb - 1) ++ns;
+            }
+        }
+        // every MMA issued has completed before TMEM is freed
+        if (elect_one()) tc_commit(drain);
+        __syncwarp();
+        volatile int never_set = 0;
+        if (!tc_wait(drain, 0u, &never_set)) ok = false;
+        if (!ok && lane == 0) atomicExch(err, 1);
     } else {
-        const unsigned lane_off = unsigned(warp * 32) << 16;
+        // warps w and w + 4 hold the same 32 rows (TMEM lanes 32 (w mod 4) ..), columns 0-15 and 16-31
+        const int wr = warp & 3, c0 = warp < 4 ? 0 : kHalf;
+        const unsigned acc0 = tmem + (unsigned(wr * 32) << 16) + unsigned(c0);
+        int4* own = sums + (warp * 32) * kHalf;
         unsigned ns = 0;
         bool ok = true;
         for (int t = blockIdx.x; t < L.tiles && ok; t += gridDim.x) {
             const TileAt at = tile_at(L, t);
             const GemmOp& g = L.op[at.o];
             const int nkb = (g.K + kKB - 1) / kKB, flushes = (nkb + kFlush - 1) / kFlush;
-            long long hi[kNT], lo[kNT];
+            long long hi[kHalf], lo[kHalf];
 #pragma unroll
-            for (int c = 0; c < kNT; ++c) { hi[c] = 0; lo[c] = 0; }
+            for (int c = 0; c < kHalf; ++c) { hi[c] = 0; lo[c] = 0; }
             for (int f = 0; f < flushes; ++f, ++ns) {
                 const unsigned set = ns % kSets;
                 if (!(ok = tc_wait(acc_full + set, (ns / kSets) & 1u, abort_flag))) break;
                 tc_fence_after();
+                // weights 0-3 into hi, 4-7 into lo; rolled over the weight, since a tile runs through this code
+                // only K / 128 times and fetching straight-line code costs more than running it
 #pragma unroll
-                for (int half = 0; half < 2; ++half)
+                for (int part = 0; part < 2; ++part) {
+                    int scale = 1 << 24;
+#pragma unroll 1
+                    for (int w = 4 * part; w < 4 * part + 4; ++w, scale >>= 8) {
+                        float v[kHalf];
+                        tmem_ld16(acc0 + set * 256u + unsigned(w * kNT), v);
 #pragma unroll
-                    for (int w = 0; w < kDigits; ++w) {
-                        float v[16];
-                        tmem_ld16(tmem + lane_off + set * 256u + unsigned(w * kNT + 16 * half), v);
-#pragma unroll
-                        for (int c = 0; c < 16; ++c) {
-                            const long long q = (long long)__float2int_rn(v[c]) * (1LL << (8 * (3 - (w & 3))));
-                            if (w < 4) hi[16 * half + c] += q;
-                            else lo[16 * half + c] += q;
+                        for (int c = 0; c < kHalf; ++c) {
+                            const long long q = (long long)__float2int_rn(v[c]) * scale;
+                            if (part == 0) hi[c] += q;
+                            else lo[c] += q;
                         }
                     }
+                }
                 tc_fence_before();
                 mbar_arrive(acc_empty + set);
             }
             if (!ok) break;
-            const int row = at.m * kMT + tid, n0 = at.n * kNT;
-            if (row >= g.M) continue;
-            double* C = table_ptr(g.c.base, at.b) + g.c.off + (long long)row * g.c.ld + (row >= g.c.rs ? g.c.dr : 0);
-            const int ea = g.ea[(long long)at.b * g.eastride + row];
-            const int* eb = g.eb + (long long)at.b * g.ebstride + n0;
+            // the sums change hands inside the warp, so that lanes take consecutive columns of two rows: this
+            // thread's row goes to shared memory with its 16-byte entries swizzled by the row
 #pragma unroll
-            for (int c = 0; c < kNT; ++c) {
-                if (n0 + c >= g.N) break;
-                // (hi + lo 2^-32) 2^(ea + eb - 36): the carry of lo first, then both parts as doubles by their
-                // bits (1.5 2^52 + integer, 2^20 + fraction), one rounding in the last addition
-                const long long h = hi[c] + (lo[c] >> 32);
-                const double d1 = __longlong_as_double(0x4338000000000000LL + h);
-                const double d2 = __hiloint2double(0x41300000, int(unsigned(lo[c])));
-                double v = (d1 - (6755399441055744.0 + 1048576.0)) + d2;
-                const int e1 = eb[c], k = ea + e1 - 36;
-                const int hw = __double2hiint(v), e = (hw >> 20) & 0x7ff;
-                if (e != 0) {
-                    if (e + k >= 1 && e + k <= 2046) v = __hiloint2double(hw + (k << 20), __double2loint(v));
-                    else v = scalbn(v, k);
-                }
-                if (ea >= kNotFinite || e1 >= kNotFinite) v = __longlong_as_double(0x7ff8000000000000LL);
-                if (g.neg) v = -v;
-                double* dst = C + n0 + c + (n0 + c >= g.c.ks ? g.c.dk : 0);
-                *dst = g.add ? *dst + v : v;
+            for (int c = 0; c < kHalf; ++c) {
+                const long long h = hi[c] + (lo[c] >> 32);  // the carry of lo first
+                own[lane * kHalf + (c ^ (lane & 15))] = make_int4(int(h), int(h >> 32), int(lo[c]), 0);
             }
+            __syncwarp();
+            const int row0 = at.m * kMT + 32 * wr, n = at.n * kNT + c0 + (lane & 15), odd_row = lane >> 4;
+            const bool col = n < g.N;
+            const int ea = g.ea[(long long)at.b * g.eastride + min(row0 + lane, g.M - 1)];
+            const int eb = g.eb[(long long)at.b * g.ebstride + min(n, g.N - 1)];
+            const int add = g.add, crs = g.c.rs, drs = g.d.rs, rows = min(32, g.M - row0);
+            const long long cld = g.c.ld, cdr = g.c.dr, dld = g.d.ld, ddr = g.d.dr;
+            const unsigned flip = g.neg ? 0x80000000u : 0u;
+            double* C = table_ptr(g.c.base, at.b) + g.c.off + n + (n >= g.c.ks ? g.c.dk : 0);
+            double v[16], old[16];
+            if (add == ADD_D) {
+                const double* D = table_ptr(g.d.base, at.b) + g.d.off + n + (n >= g.d.ks ? g.d.dk : 0);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const int i = 2 * j + odd_row, r = row0 + i;
+                    old[j] = col && i < rows ? D[r * dld + (r >= drs ? ddr : 0)] : 0.0;
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) old[j] = n == row0 + 2 * j + odd_row ? 1.0 : 0.0;
+            }
+            // all sixteen conversions before any branch: a branch per entry would run them one after another
+            unsigned odd = 0;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                const int i = 2 * j + odd_row;
+                const int4 q = own[i * kHalf + ((lane & 15) ^ (i & 15))];
+                const int e1 = __shfl_sync(0xffffffffu, ea, i);
+                bool o;
+                v[j] = fixed_to_double(join(q), unsigned(q.z), e1 + eb - 36, o);  // (h + f 2^-32) 2^(e1 + eb - 36)
+                odd |= o || e1 >= kNotFinite || eb >= kNotFinite ? 1u << j : 0u;
+            }
+            if (__any_sync(0xffffffffu, odd != 0)) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const int i = 2 * j + odd_row;
+                    const int4 q = own[i * kHalf + ((lane & 15) ^ (i & 15))];
+                    const int e1 = __shfl_sync(0xffffffffu, ea, i);
+                    if ((odd >> j) & 1u) v[j] = fixed_to_double_any(join(q), unsigned(q.z), e1, eb);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = __hiloint2double(int(unsigned(__double2hiint(v[j])) ^ flip), __double2loint(v[j]));
+            if (add) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] = old[j] + v[j];
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                const int i = 2 * j + odd_row, r = row0 + i;
+                if (col && i < rows) C[r * cld + (r >= crs ? cdr : 0)] = v[j];
+            }
+            __syncwarp();
         }
         if (!ok) atomicExch(err, 1);
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == 5) tmem_dealloc(tmem, 512u);
+    if (warp == 9) tmem_dealloc(tmem, 512u);
 }
 
-// In-place inverse of one matrix of at most 64 rows per block by Gauss-Jordan steps (row k of the result
-// from the pivot row of step k): 256 threads hold 4 x 4 entries each.  The pivot of column k is the largest
-// entry of the rows not used yet, compared by its leading 26 bits (the row's number in the last six, so one
-// warp reduction finds both); rows are not moved but put in order when they are written.  Bound by the SM's
-// two FP64 multiply-adds per clock (n^3 of them: ~65 us for 64 rows).  A pivot that is zero or not finite
-// sets info.
 struct InvList {
     int nv;
-    MatView v[2];
+    MatView v[2], out[2];
 };
-__global__ void __launch_bounds__(256) k_inv64(const __grid_constant__ InvList L, int n, int* __restrict__ info) {
+
+// Inverse of one matrix of at most 32 rows per block, in place, by Gauss-Jordan steps in FP64 (row k of the
+// result from the pivot row of step k): 64 threads hold 4 x 4 entries each.  The pivot of column k is the
+// largest entry of the rows not used yet, compared by its leading 26 bits (the row's number in the last six,
+// so one warp reduction finds both); rows are not moved but put in order when they are written.  A pivot that
+// is zero or not finite sets info.  Bound by the two block barriers and the division of a step.
+__global__ void __launch_bounds__(64) k_inv_small(const __grid_constant__ InvList L, int n, int* __restrict__ info) {
     const MatView& V = L.v[blockIdx.x];
     double* A = table_ptr(V.base, blockIdx.y) + V.off;
-    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15, lane = tid & 31;
-    __shared__ double s_col[2][64], s_row[2][64];
-    __shared__ int s_p[64], s_k[64];
+    const int tid = threadIdx.x, ty = tid >> 3, tx = tid & 7, lane = tid & 31;
+    __shared__ double s_col[2][32], s_row[2][32];
+    __shared__ int s_p[32], s_k[32];
     double a[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -428,37 +518,35 @@ __global__ void __launch_bounds__(256) k_inv64(const __grid_constant__ InvList L
             const int r = 4 * ty + i, c = 4 * tx + j;
             a[i][j] = r < n && c < n ? A[(long long)r * V.ld + c] : (r == c ? 1.0 : 0.0);
         }
-    unsigned used0 = 0, used1 = 0;
+    unsigned used = 0;
     bool bad = false;
-    for (int k = 0; k < n; ++k) {
-        const int bf = k & 1;
+    // the column inside a thread's four is a constant of the unrolled loop, the pivot row inside its four a chain
+    // of selections: the entries stay in registers
+    for (int k4 = 0; k4 < n; k4 += 4) {
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+        const int k = k4 + kk, bf = kk & 1;
+        if (k >= n) break;
         if (tx == (k >> 2)) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (j == (k & 3)) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) s_col[bf][4 * ty + i] = a[i][j];
-                }
+            for (int i = 0; i < 4; ++i) s_col[bf][4 * ty + i] = a[i][kk];
         }
         __syncthreads();
-        const unsigned h0 = unsigned(__double2hiint(s_col[bf][lane])) & 0x7fffffffu;
-        const unsigned h1 = unsigned(__double2hiint(s_col[bf][lane + 32])) & 0x7fffffffu;
-        const unsigned k0 = (used0 >> lane) & 1u || lane >= n ? 0u : ((h0 << 1) & ~63u) | unsigned(63 - lane);
-        const unsigned k1 = (used1 >> lane) & 1u || lane + 32 >= n ? 0u : ((h1 << 1) & ~63u) | unsigned(31 - lane);
-        const unsigned best = __reduce_max_sync(0xffffffffu, max(k0, k1));
-        const int p = 63 - int(best & 63u);
+        const unsigned h = unsigned(__double2hiint(s_col[bf][lane])) & 0x7fffffffu;
+        const unsigned key = (used >> lane) & 1u || lane >= n ? 0u : ((h << 1) & ~63u) | unsigned(63 - lane);
+        const unsigned best = __reduce_max_sync(0xffffffffu, key);
+        const int p = 63 - int(best & 63u);  // an unused row always has a key above zero
         const double piv = s_col[bf][p];
         if (!(fabs(piv) > 0.0) || best >= 0xffe00000u) bad = true;
-        if (p < 32) used0 |= 1u << p;
-        else used1 |= 1u << (p - 32);
+        used |= 1u << p;
         if (ty == (p >> 2)) {
             const double inv = 1.0 / piv;
+            const int pi = p & 3;
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (i == (p & 3)) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) s_row[bf][4 * tx + j] = 4 * tx + j == k ? inv : a[i][j] * inv;
-                }
+            for (int j = 0; j < 4; ++j) {
+                const double x = pi == 0 ? a[0][j] : pi == 1 ? a[1][j] : pi == 2 ? a[2][j] : a[3][j];
+                s_row[bf][4 * tx + j] = j == kk && tx == (k >> 2) ? inv : x * inv;
+            }
         }
         if (tid == 0) { s_p[k] = p; s_k[p] = k; }
         __syncthreads();
@@ -470,11 +558,9 @@ __global__ void __launch_bounds__(256) k_inv64(const __grid_constant__ InvList L
             const int r = 4 * ty + i;
             const double c = s_col[bf][r];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const bool kc = 4 * tx + j == k;
-                a[i][j] = r == p ? rj[j] : fma(-c, rj[j], kc ? 0.0 : a[i][j]);
-            }
+            for (int j = 0; j < 4; ++j) a[i][j] = r == p ? rj[j] : fma(-c, rj[j], j == kk && tx == (k >> 2) ? 0.0 : a[i][j]);
         }
+    }
     }
     __syncthreads();
 #pragma unroll
@@ -483,6 +569,149 @@ __global__ void __launch_bounds__(256) k_inv64(const __grid_constant__ InvList L
         for (int j = 0; j < 4; ++j) {
             const int r = 4 * ty + i, c = 4 * tx + j;
             if (r < n && c < n) A[(long long)s_k[r] * V.ld + s_p[c]] = a[i][j];
+        }
+    if (tid == 0 && bad) info[blockIdx.y] = 1;
+}
+
+// x 2^k for a finite x, by the exponent bits (zero where the result would be below the smallest normal number)
+__device__ __forceinline__ double shift_exponent(double x, int k) {
+    const int hi = __double2hiint(x), e = (hi >> 20) & 0x7ff;
+    if (e == 0 || e + k < 1) return 0.0;
+    return __hiloint2double(e + k > 2046 ? (hi & int(0x80000000u)) | 0x7fe00000 : hi + (k << 20), __double2loint(x));
+}
+
+// FP32 inverse of one matrix of at most 128 rows per block: the start of the Newton steps of `invert`.  The
+// same Gauss-Jordan steps as k_inv_small on FP32 entries, 8 x 8 per thread; rows are brought to magnitudes
+// below one by powers of two first, so any scaling of the rows is harmless.  The FP64 steps of a 64-row
+// inverse alone take 68 us on one SM (two multiply-adds per clock); these take a 64th of that per entry.
+__global__ void __launch_bounds__(256) k_inv_start(const __grid_constant__ InvList L, int n, int* __restrict__ info) {
+    const MatView &V = L.v[blockIdx.x], &O = L.out[blockIdx.x];
+    const double* A = table_ptr(V.base, blockIdx.y) + V.off;
+    double* out = table_ptr(O.base, blockIdx.y) + O.off;
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15, lane = tid & 31;
+    __shared__ __align__(16) float s_col[2][128];
+    __shared__ __align__(16) float s_row[2][128];
+    __shared__ int s_p[128], s_k[128], s_e[128];
+    // rows and columns of a thread: 4 t .. 4 t + 3 and 64 more, so that 16-byte reads of a row or column by the
+    // 16 threads of a direction touch every bank once
+    auto at8 = [](int t, int i) { return 4 * t + (i & 3) + 16 * (i & 4); };
+    float a[8][8];
+    {
+        double x[8][8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int r = at8(ty, i), c = at8(tx, j);
+                x[i][j] = r < n && c < n ? A[(long long)r * V.ld + c] : (r == c ? 1.0 : 0.0);
+            }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            unsigned m = 0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) m = max(m, unsigned(__double2hiint(x[i][j])) & 0x7fffffffu);
+#pragma unroll
+            for (int off = 8; off > 0; off >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, off));
+            const int e = max(int(m >> 20), 1) - 1022;  // a row that is not finite keeps its infinities and NaNs
+#pragma unroll
+            for (int j = 0; j < 8; ++j) a[i][j] = d2f_rn_bits(m < 0x7ff00000u ? shift_exponent(x[i][j], -e) : x[i][j]);
+            if (tx == 0) s_e[at8(ty, i)] = e;
+        }
+    }
+    // rows 4 lane .. 4 lane + 3: 127 - row, and all ones while a row is unused
+    const unsigned k0 = 127u - 4u * unsigned(lane);
+    unsigned m0 = 4 * lane < n ? ~0u : 0u, m1 = 4 * lane + 1 < n ? ~0u : 0u, m2 = 4 * lane + 2 < n ? ~0u : 0u,
+             m3 = 4 * lane + 3 < n ? ~0u : 0u;
+    bool bad = false;
+    for (int k8 = 0; k8 < 128; k8 += 4) {
+        if (k8 >= n) break;
+        const int tk = (k8 & 63) >> 2;
+        const bool top = k8 >= 64;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+            const int k = k8 + kk, bf = kk & 1;
+            if (k >= n) break;
+            if (tx == tk) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) s_col[bf][at8(ty, i)] = top ? a[i][kk + 4] : a[i][kk];
+            }
+            __syncthreads();
+            const float4 cv = *reinterpret_cast<const float4*>(&s_col[bf][4 * lane]);
+            // leading 25 bits of the magnitude, then 127 - row; nothing for rows that are used (or past the end)
+            const unsigned kx = ((__float_as_uint(cv.x) << 1) & ~127u) | k0, ky = ((__float_as_uint(cv.y) << 1) & ~127u) | (k0 - 1u);
+            const unsigned kz = ((__float_as_uint(cv.z) << 1) & ~127u) | (k0 - 2u), kw = ((__float_as_uint(cv.w) << 1) & ~127u) | (k0 - 3u);
+            const unsigned best = __reduce_max_sync(0xffffffffu, max(max(kx & m0, ky & m1), max(kz & m2, kw & m3)));
+            const int p = 127 - int(best & 127u);
+            const float piv = s_col[bf][p], inv = __fdividef(1.f, piv);
+            if (!(fabsf(piv) > 0.f) || best >= 0xff000000u) bad = true;
+            m0 = p == 4 * lane ? 0u : m0;
+            m1 = p == 4 * lane + 1 ? 0u : m1;
+            m2 = p == 4 * lane + 2 ? 0u : m2;
+            m3 = p == 4 * lane + 3 ? 0u : m3;
+            const int pi = (p & 3) + (p >= 64 ? 4 : 0);
+            const bool mine = ty == ((p & 63) >> 2);
+            if (mine) {
+                // the row inside the thread's eight is the same for the whole block: a jump, not selections
+                auto publish = [&](const float (&row)[8]) {
+                    float x[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) x[j] = row[j] * inv;
+                    if (tx == tk) {
+                        if (top) x[kk + 4] = inv;
+                        else x[kk] = inv;
+                    }
+                    *reinterpret_cast<float4*>(&s_row[bf][4 * tx]) = make_float4(x[0], x[1], x[2], x[3]);
+                    *reinterpret_cast<float4*>(&s_row[bf][64 + 4 * tx]) = make_float4(x[4], x[5], x[6], x[7]);
+                };
+                switch (pi) {
+                    case 0: publish(a[0]); break;
+                    case 1: publish(a[1]); break;
+                    case 2: publish(a[2]); break;
+                    case 3: publish(a[3]); break;
+                    case 4: publish(a[4]); break;
+                    case 5: publish(a[5]); break;
+                    case 6: publish(a[6]); break;
+                    default: publish(a[7]); break;
+                }
+            }
+            if (tid == 0) { s_p[k] = p; s_k[p] = k; }
+            __syncthreads();
+            float rj[8], ci[8];
+#pragma unroll
+            for (int j = 0; j < 8; j += 4) {
+                const float4 t = *reinterpret_cast<const float4*>(&s_row[bf][4 * tx + 16 * j]);
+                rj[j] = t.x; rj[j + 1] = t.y; rj[j + 2] = t.z; rj[j + 3] = t.w;
+                const float4 u = *reinterpret_cast<const float4*>(&s_col[bf][4 * ty + 16 * j]);
+                ci[j] = u.x; ci[j + 1] = u.y; ci[j + 2] = u.z; ci[j + 3] = u.w;
+            }
+            // one update for all: row i loses c_i times the scaled pivot row; the pivot row itself keeps a 1 / piv of
+            // itself with c = piv - 1; the entries of column k count as those of a unit vector
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const bool pr = mine && i == pi;
+                if (pr) ci[i] = piv - 1.f;
+                if (tx == tk) {
+                    const float one = pr ? 1.f : 0.f;
+                    if (top) a[i][kk + 4] = one;
+                    else a[i][kk] = one;
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) a[i][j] = fmaf(-ci[i], rj[j], a[i][j]);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int r = at8(ty, i), c = at8(tx, j);
+            if (r < n && c < n) {
+                const int pc = s_p[c];  // the column of A^-1 takes the scale of that row of A
+                out[(long long)s_k[r] * O.ld + pc] = shift_exponent(f2d_bits(a[i][j]), -s_e[pc]);
+            }
         }
     if (tid == 0 && bad) info[blockIdx.y] = 1;
 }
@@ -573,7 +802,8 @@ public:
         int estride, len, K;
     };
     // role 0: rows of A (len = M); 1: columns of B (len = N)
-    Digits split(const MatView& v, int len, int K, int role, int neg0 = 0, int neg1 = 0) {
+    Digits split(const MatView& v, int len, int K, int role, int neg0 = 0, int neg1 = 0, int* info = nullptr,
+                 int limit = 0) {
         const int nkb = (K + kKB - 1) / kKB;
         Digits d;
         d.pstride = role ? (long long)((len + kNT - 1) / kNT) * nkb * kBBlock
@@ -585,18 +815,21 @@ public:
         d.ex = reinterpret_cast<int*>(take(size_t(len) * 4 * cnt_));
         if (sl_.n == kMaxOps) flush_split();
         SplitOp& op = sl_.op[sl_.n];
-        op = SplitOp{v, len, K, role, neg0, neg1, d.planes, d.pstride, d.ex, d.estride, blocks_};
+        op = SplitOp{v, len, K, role, neg0, neg1, d.planes, d.pstride, d.ex, d.estride, blocks_, info, limit};
         // whole tiles: the rows past the end are written as zeros
         blocks_ += role ? (len + kNT - 1) / kNT : (len + kMT - 1) / kMT * (kMT / 32);
         ++sl_.n;
         return d;
     }
-    void gemm(const Digits& a, const Digits& b, const MatView& c, bool neg, bool add) {
+    // C = (neg ? -1 : 1) A B, plus C or the identity
+    void gemm(const Digits& a, const Digits& b, const MatView& c, bool neg, int add) { gemm(a, b, c, neg, add, c); }
+    // ..., plus D
+    void gemm(const Digits& a, const Digits& b, const MatView& c, bool neg, int add, const MatView& d) {
         if (gl_.n == kMaxGemms) flush();
         GemmOp& g = gl_.op[gl_.n];
         const int mt = (a.len + kMT - 1) / kMT, nt = (b.len + kNT - 1) / kNT;
         g = GemmOp{a.planes, b.planes, a.pstride, b.pstride, a.ex, b.ex, a.estride, b.estride, a.len, b.len, a.K,
-                   c, neg, add, mt, nt, gl_.tiles};
+                   c, d, neg, add, mt, nt, gl_.tiles};
         gl_.tiles += mt * nt * cnt_;
         ++gl_.n;
     }
@@ -612,7 +845,7 @@ public:
         flush_split();
         if (gl_.n && !dry_) {
             cudaFuncSetAttribute(k_gemm64, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmem));
-            k_gemm64<<<unsigned(std::min(gl_.tiles, sm_count())), 192, kSmem, st_>>>(gl_, err_);
+            k_gemm64<<<unsigned(std::min(gl_.tiles, sm_count())), kGemmThreads, kSmem, st_>>>(gl_, err_);
             ++g_kernel_launches;
         }
         gl_.n = 0;
@@ -643,23 +876,68 @@ MatView at(const MatView& v, long long r, long long c) {
     return o;
 }
 
-// Inverses of one or two h x h matrices per item, in place, by 2 x 2 block elimination:
+// Inverses of one or two h x h matrices per item, in place.  tmp: room for 3 h^2 doubles per view.
+//
+// Up to 32 rows: Gauss-Jordan in FP64.  Up to 128: an FP32 inverse Y (error e ~ 1e-7 cond) and two Newton steps
+// Y <- Y + Y (I - A Y), each squaring the error, with accurate products; where the residual before the second
+// is not below 2^-34 per entry (the result would not be accurate to the last bits) info is set.  Beyond, 2 x 2
+// block elimination:
 //   [A B; C D]: G = A^-1 B, F = C A^-1, D <- (D - C G)^-1, B <- -G D, C <- -D F, A <- A^-1 - B F.
-// Every product is an accurate GEMM, so the only FP64 roundings are those of the stored blocks.  tmp: room
-// for G and F of all views and of the blocks below, h^2 doubles per view.
+// Every product is an accurate GEMM, so the only FP64 roundings are those of the stored blocks.
 void invert(Runner& R, const std::vector<MatView>& v, int h, const MatView& tmp, int* info) {
-    if (h <= 64) {
+    const size_t n = v.size(), m0 = R.mark();
+    if (h <= 32) {
         if (!R.dry()) {
             InvList L{};
-            L.nv = int(v.size());
-            for (size_t i = 0; i < v.size(); ++i) L.v[i] = v[i];
-            k_inv64<<<dim3(unsigned(v.size()), unsigned(R.count())), 256, 0, R.stream()>>>(L, h, info);
+            L.nv = int(n);
+            for (size_t i = 0; i < n; ++i) L.v[i] = v[i];
+            k_inv_small<<<dim3(unsigned(n), unsigned(R.count())), 64, 0, R.stream()>>>(L, h, info);
             ++g_kernel_launches;
         }
         return;
     }
+    if (h <= 128) {
+        std::vector<MatView> Y, E;
+        InvList L{};
+        L.nv = int(n);
+        for (size_t i = 0; i < n; ++i) {
+            MatView y = tmp;
+            y.off += 2LL * i * h * h;
+            y.ld = h;
+            MatView e = y;
+            e.off += (long long)h * h;
+            Y.push_back(y);
+            E.push_back(e);
+            L.v[i] = v[i];
+            L.out[i] = y;
+        }
+        if (!R.dry()) {
+            k_inv_start<<<dim3(unsigned(n), unsigned(R.count())), 256, 0, R.stream()>>>(L, h, info);
+            ++g_kernel_launches;
+        }
+        std::vector<Runner::Digits> a, y;
+        for (size_t i = 0; i < n; ++i) {
+            a.push_back(R.split(v[i], h, h, 0));
+            const auto yb = R.split(Y[i], h, h, 1);
+            y.push_back(R.split(Y[i], h, h, 0));
+            R.gemm(a[i], yb, E[i], true, ADD_IDENTITY);
+        }
+        R.flush();
+        for (size_t i = 0; i < n; ++i) R.gemm(y[i], R.split(E[i], h, h, 1), Y[i], false, ADD_D);
+        R.flush();
+        for (size_t i = 0; i < n; ++i) {
+            const auto yb = R.split(Y[i], h, h, 1);
+            y[i] = R.split(Y[i], h, h, 0);
+            R.gemm(a[i], yb, E[i], true, ADD_IDENTITY);
+        }
+        R.flush();
+        for (size_t i = 0; i < n; ++i)
+            R.gemm(y[i], R.split(E[i], h, h, 1, 0, 0, info, -34), v[i], false, ADD_D, Y[i]);
+        R.flush();
+        R.release(m0);
+        return;
+    }
     const int h1 = (h / 2 + 31) / 32 * 32, h2 = h - h1;
-    const size_t n = v.size(), m0 = R.mark();
     std::vector<MatView> A, B, C, D, G, F;
     MatView below = tmp;
     for (const auto& x : v) {
@@ -680,11 +958,11 @@ void invert(Runner& R, const std::vector<MatView>& v, int h, const MatView& tmp,
     for (size_t i = 0; i < n; ++i) {
         const auto aA = R.split(A[i], h1, h1, 0), aB = R.split(A[i], h1, h1, 1), bB = R.split(B[i], h2, h1, 1);
         c0.push_back(R.split(C[i], h2, h1, 0));
-        R.gemm(aA, bB, G[i], false, false);
-        R.gemm(c0[i], aB, F[i], false, false);
+        R.gemm(aA, bB, G[i], false, ADD_NONE);
+        R.gemm(c0[i], aB, F[i], false, ADD_NONE);
     }
     R.flush();
-    for (size_t i = 0; i < n; ++i) R.gemm(c0[i], R.split(G[i], h2, h1, 1), D[i], true, true);
+    for (size_t i = 0; i < n; ++i) R.gemm(c0[i], R.split(G[i], h2, h1, 1), D[i], true, ADD_D);
     R.flush();
     R.release(m0);
     invert(R, D, h2, below, info);
@@ -692,11 +970,11 @@ void invert(Runner& R, const std::vector<MatView>& v, int h, const MatView& tmp,
     for (size_t i = 0; i < n; ++i) {
         const auto dA = R.split(D[i], h2, h2, 0), dB = R.split(D[i], h2, h2, 1), gA = R.split(G[i], h1, h2, 0);
         f0.push_back(R.split(F[i], h1, h2, 1));
-        R.gemm(gA, dB, B[i], true, false);
-        R.gemm(dA, f0[i], C[i], true, false);
+        R.gemm(gA, dB, B[i], true, ADD_NONE);
+        R.gemm(dA, f0[i], C[i], true, ADD_NONE);
     }
     R.flush();
-    for (size_t i = 0; i < n; ++i) R.gemm(R.split(B[i], h1, h2, 0), f0[i], A[i], true, true);
+    for (size_t i = 0; i < n; ++i) R.gemm(R.split(B[i], h1, h2, 0), f0[i], A[i], true, ADD_D);
     R.flush();
     R.release(m0);
 }
@@ -729,14 +1007,14 @@ void merge_steps(Runner& R, const MergeItem* items, int s, int kids, int* info) 
         const auto a0 = R.split(A0, s, s, 0), a0b = R.split(A0, s, s, 1), a1 = R.split(A1, s, s, 0),
                    a1b = R.split(A1, s, s, 1), b0 = R.split(B0, 2 * s, s, 1), b1 = R.split(B1, 2 * s, s, 1),
                    c0 = R.split(C0, 2 * s, s, 0), c1 = R.split(C1, 2 * s, s, 0);
-        R.gemm(a0, b0, G, false, false);
-        R.gemm(a1, b1, at(G, s, 0), false, false);
-        R.gemm(c0, a0b, F, false, false);
-        R.gemm(c1, a1b, at(F, 0, s), false, false);
+        R.gemm(a0, b0, G, false, ADD_NONE);
+        R.gemm(a1, b1, at(G, s, 0), false, ADD_NONE);
+        R.gemm(c0, a0b, F, false, ADD_NONE);
+        R.gemm(c1, a1b, at(F, 0, s), false, ADD_NONE);
         R.flush();
         R.release(0);
         const auto c = R.split(C0, 2 * s, 2 * s, 0), g = R.split(G, 2 * s, 2 * s, 1);
-        R.gemm(c, g, D, true, true);
+        R.gemm(c, g, D, true, ADD_D);
         R.flush();
         R.release(0);
     }
@@ -744,10 +1022,10 @@ void merge_steps(Runner& R, const MergeItem* items, int s, int kids, int* info) 
     {
         const auto dA = R.split(D, 2 * s, 2 * s, 0), dB = R.split(D, 2 * s, 2 * s, 1), g = R.split(G, 2 * s, 2 * s, 0),
                    f = R.split(F, 2 * s, 2 * s, 1);
-        R.gemm(g, dB, B0, true, false);
-        R.gemm(dA, f, C0, true, false);
+        R.gemm(g, dB, B0, true, ADD_NONE);
+        R.gemm(dA, f, C0, true, ADD_NONE);
         R.flush();
-        R.gemm(R.split(B0, 2 * s, 2 * s, 0), f, A0, true, true);
+        R.gemm(R.split(B0, 2 * s, 2 * s, 0), f, A0, true, ADD_D);
         R.flush();
         R.release(0);
     }
@@ -784,7 +1062,7 @@ void merge_steps(Runner& R, const MergeItem* items, int s, int kids, int* info) 
             o.ks = s;
             o.dk = (long long)(q.p1 - q.p0 - 1) * s;
             const auto xa = R.split(x, m, 2 * s, 0), tb = R.split(t, 2 * s, 2 * s, 1, q.nega, q.negb);
-            R.gemm(xa, tb, o, false, false);
+            R.gemm(xa, tb, o, false, ADD_NONE);
         }
         R.flush();
         R.release(0);
@@ -807,7 +1085,7 @@ void merge_steps(Runner& R, const MergeItem* items, int s, int kids, int* info) 
             MatView o = at(T, (long long)q.p0 * s, 0);
             o.rs = s;
             o.dr = (long long)(q.p1 - q.p0 - 1) * s * 2 * m;
-            R.gemm(R.split(h, 2 * s, 2 * s, 0), R.split(b, 2 * m, 2 * s, 1), o, false, true);
+            R.gemm(R.split(h, 2 * s, 2 * s, 0), R.split(b, 2 * m, 2 * s, 1), o, false, ADD_D);
         }
         R.flush();
         R.release(0);
