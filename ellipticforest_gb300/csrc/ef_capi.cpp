@@ -134,9 +134,10 @@ int run_single_patch(int solver_type, int n, double xl, double xu, double yl, do
     int singular = 0;
     if (e == cudaSuccess) {
         if (mode == efgb::LEAF_DTN_COLUMN) {
-            // the DtN map by a pivoted dense LU of the 5-point operator (as in a tree build)
+            // the DtN map as in a tree build
             try {
-                singular = efgb::leaf_dtn_lu(0, n, lambda, {dx}, {dy}, {dout});
+                if (efgb::leaf_dtn_definite(n, lambda, dx, dy)) efgb::leaf_dtn_modes(0, n, lambda, dty, 1, dout);
+                else singular = efgb::leaf_dtn_lu(0, n, lambda, {dx}, {dy}, {dout});
             } catch (...) {
                 cudaFree(buf);
                 throw;

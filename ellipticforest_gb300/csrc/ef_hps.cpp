@@ -575,7 +575,7 @@ void Hps::build_leaf_types() {
         pe(double(types_.size()) * 16 * n * n * 8, double(nitems_dtn_) * (6 * n * n * n + 8 * n * n));
         return;
     }
-    // one DtN per distinct leaf geometry, by a pivoted dense LU of its 5-point operator
+    // one DtN per distinct leaf geometry (the types' T lie one after another)
     std::vector<double> dx, dy;
     std::vector<double*> T;
     for (const auto& ty : types_) {
@@ -584,8 +584,12 @@ void Hps::build_leaf_types() {
         T.push_back(ty.T);
     }
     const double nn = n * n, nt = double(types_.size());
+    bool modes = true;
+    for (size_t t = 0; t < types_.size(); ++t)
+        modes = modes && leaf_dtn_definite(n_, lambda_, dx[t], dy[t]) && T[t] == T[0] + t * 16 * size_t(n_) * n_;
     pb("leaf_dtn");
-    leaf_singular_ = leaf_dtn_lu(st_, n_, lambda_, dx, dy, T);
+    if (modes) leaf_dtn_modes(st_, n_, lambda_, d_types_, int(types_.size()), T[0]);
+    else leaf_singular_ = leaf_dtn_lu(st_, n_, lambda_, dx, dy, T);
     pe(nt * 8 * (2 * nn * nn + 2 * nn * 4 * n + 16 * n * n),
        nt * (2.0 / 3.0 * nn * nn * nn + 2.0 * nn * nn * 4 * n));
 }

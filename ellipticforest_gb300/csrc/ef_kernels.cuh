@@ -108,8 +108,12 @@ void leaf_eigen(cudaStream_t st, int mode, const LeafType* types_dev, const Leaf
 // LeafType table (never the constant-memory 16 x 16 basis): for callers that cannot upload it
 void leaf_eigen_tables(cudaStream_t st, int mode, const LeafType* types_dev, const LeafItem* items_dev,
                        int nitems, int nmax);
-// Leaf DtN maps T[t] (4n x 4n, row-major, WESN) of the constant-coefficient leaf geometries
-// (dx[t], dy[t]) by a pivoted dense LU of their 5-point operators (ef_leaf_dtn.cu); synchronous,
+// Leaf DtN maps (4n x 4n, row-major, WESN, one after another from T) of the constant-coefficient leaf
+// types whose operators are negative definite by a margin (leaf_dtn_definite): sums over sine modes in
+// double-double (ef_leaf_dtn.cu); asynchronous
+bool leaf_dtn_definite(int n, double lambda, double dx, double dy);
+void leaf_dtn_modes(cudaStream_t st, int n, double lambda, const LeafType* types_dev, int nt, double* T);
+// The same of any leaf geometries (dx[t], dy[t]) into T[t] by a pivoted dense LU of their 5-point operators (ef_leaf_dtn.cu); synchronous,
 // returns the number of singular operators (zero pivot)
 int leaf_dtn_lu(cudaStream_t st, int n, double lambda, const std::vector<double>& dx, const std::vector<double>& dy,
                 const std::vector<double*>& T);

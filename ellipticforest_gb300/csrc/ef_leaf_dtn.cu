@@ -1,15 +1,26 @@
-// Leaf Dirichlet-to-Neumann maps of the constant-coefficient (FISHPACK90) leaf types by a pivoted
-// dense LU of the 5-point operator (FiniteVolumeSolver::buildD2N, FiniteVolumeSolver.cpp:355-455).
+// Leaf Dirichlet-to-Neumann maps of the constant-coefficient (FISHPACK90) leaf types
+// (FiniteVolumeSolver::buildD2N, FiniteVolumeSolver.cpp:355-455).
 //
 // Column j of T is mapD2N(e_j, f = 0): the solve of A u = -2 c_side e_j at the edge cell of boundary
-// point j, then h = +-(2/d)(u_edge - g) (cpp:296-353).  The sine eigenbasis solves the same system,
-// but its rounding spreads over every mode, and the DtN applied to smooth data cancels to O(1) from
-// entries of O(1/d): HPS trees built on eigenbasis DtN maps drifted from the LU-based solution by
-// ~N^2 eps at the leaf solutions (1.2e-11 at 1024^2 cells, against 2.6e-13 with an LU).  A tree has
-// one DtN per distinct leaf geometry (n, dx, dy), so the n^2 x n^2 LU costs little: the batched
-// pivoted LU and triangular solves of the merges (ef_linalg.cu) factor every type at once.
+// point j, then h = +-(2/d)(u_edge - g) (cpp:296-353).  Every leaf of a type takes the same T, so its
+// rounding errors add up coherently over the tree, and T applied to smooth data cancels to O(1) from
+// entries of O(1/d): T is wanted as close to the rounded exact map as can be had.
+//
+// Negative definite operators (k_dtn_modes): separation of variables.  With sine modes along the data's
+// side the problem across is one-dimensional with constant coefficients, and each entry of T is a sum over
+// the n modes.  In FP64 that sum spreads its rounding over every mode (trees built on it drifted by ~N^2
+// eps at the leaf solutions, 1.2e-11 at 1024^2 cells); here sines, one-dimensional solutions and sums are
+// double-double (unevaluated sums of two doubles; Dekker, "A floating-point technique for extending the
+// available precision", Numer. Math. 18, 1971), so an entry is the exact one rounded once or twice.
+// For 16 x 16 cells it takes 0.15 ms (the chain of double-double divisions of a mode, then 16 terms per entry)
+// where the pivoted LU of the 256 x 256 operator, a chain of pivots, took 2.9 ms.
+//
+// Others (lambda at or above half the smallest eigenvalue): the pivoted dense LU of the 5-point operator,
+// batched over the types (ef_linalg.cu), which also finds singular operators.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cmath>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -99,11 +110,147 @@ __global__ void k_dtn_extract(int n, const double* __restrict__ dxs, const doubl
     }
 }
 
+// ---- double-double ----
+struct dd {
+    double h, l;
+};
+__host__ __device__ inline dd quick_sum(double a, double b) {  // |a| >= |b|
+    const double s = a + b;
+    return {s, b - (s - a)};
+}
+__host__ __device__ inline dd two_sum(double a, double b) {
+    const double s = a + b, t = s - a;
+    return {s, (a - (s - t)) + (b - t)};
+}
+__host__ __device__ inline dd operator+(dd a, dd b) {
+    const dd s = two_sum(a.h, b.h), t = two_sum(a.l, b.l);
+    const dd u = quick_sum(s.h, s.l + t.h);
+    return quick_sum(u.h, u.l + t.l);
+}
+__host__ __device__ inline dd operator-(dd a) { return {-a.h, -a.l}; }
+__host__ __device__ inline dd operator-(dd a, dd b) { return a + (-b); }
+__host__ __device__ inline dd operator*(dd a, dd b) {
+    const double p = a.h * b.h;
+    return quick_sum(p, fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h));
+}
+__host__ __device__ inline dd operator/(dd a, dd b) {
+    const double q1 = a.h / b.h;
+    dd r = a - b * dd{q1, 0.0};
+    const double q2 = r.h / b.h;
+    r = r - b * dd{q2, 0.0};
+    const dd q = quick_sum(q1, q2);
+    return q + dd{r.h / b.h, 0.0};
+}
+
+constexpr int kMaxSide = 64;
+struct SineTable {
+    dd s[kMaxSide + 1];  // sin(pi k / (2n)), k = 0 .. n
+};
+// Taylor series in double-double; the angle is at most pi / 2, so 30 terms reach 1e-33
+SineTable sine_table(int n) {
+    const dd pi{3.141592653589793116, 1.224646799147353207e-16};
+    SineTable t{};
+    for (int k = 0; k <= n; ++k) {
+        const dd x = pi * dd{double(k), 0.0} / dd{2.0 * n, 0.0}, x2 = x * x;
+        dd term = x, sum = x;
+        for (int j = 1; j < 30; ++j) {
+            term = -(term * x2 / dd{2.0 * j * (2.0 * j + 1.0), 0.0});
+            sum = sum + term;
+        }
+        t.s[k] = sum;
+    }
+    return t;
+}
+
+// One-dimensional problem across the patch for mode l of data on its near side (cell spacing d, along the
+// side e): with kappa = (d/e)^2 4 sin^2(pi (l+1) / 2n) - lambda d^2 the solution m cells from the far side
+// grows like q_0 = 1, q_1 = 3 + kappa, q_{m+1} = (2 + kappa) q_m - q_{m-1} (ghost -q_0 beyond the far side,
+// 2g - u beyond the near one), u_m = 2 q_m / (q_{n-1} + q_n) g.  Carried as the ratios r_m = q_{m-1} / q_m
+// = 1 / (2 + kappa - r_{m-1}), which neither overflow nor cancel.
+// Entry (q, p) of T: the modes' sum of sine at q x sine at p x one-dimensional solution, times 2 / spacing.
+__global__ void __launch_bounds__(256) k_dtn_modes(const __grid_constant__ SineTable S, int n,
+                                                   const LeafType* __restrict__ types, double lambda, double* T) {
+    extern __shared__ dd sm_dd[];
+    dd* V = sm_dd;          // V[l][j] = sin(pi (l+1)(2j+1) / 2n)
+    dd* R = V + n * n;      // [2][l][m]: weight of mode l times u_m; across x (data on W, E), across y
+    dd* D = R + 2 * n * n;  // [2][l]: weight times (u at the near cell - g)
+    const double dx = types[blockIdx.y].dx, dy = types[blockIdx.y].dy;
+    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+        const int l = e / n, j = e - l * n;
+        int k = ((l + 1) * (2 * j + 1)) % (4 * n);
+        const bool neg = k > 2 * n;
+        if (neg) k -= 2 * n;
+        const dd v = S.s[k > n ? 2 * n - k : k];
+        V[e] = neg ? -v : v;
+    }
+    for (int e = threadIdx.x; e < 2 * n; e += blockDim.x) {
+        const int dir = e / n, l = e - dir * n;
+        const double d = dir == 0 ? dx : dy, g = dir == 0 ? dy : dx;
+        const dd d2 = dd{d, 0.0} * dd{d, 0.0}, g2 = dd{g, 0.0} * dd{g, 0.0}, s = S.s[l + 1];
+        const dd kappa = dd{4.0, 0.0} * s * s * (d2 / g2) - d2 * dd{lambda, 0.0};
+        const dd two = dd{2.0, 0.0} + kappa, one{1.0, 0.0};
+        const dd weight = dd{l == n - 1 ? 1.0 : 2.0, 0.0} / dd{double(n), 0.0};
+        dd* r = R + (dir * n + l) * n;
+        dd q = one / (one + two);  // r_1
+        for (int m = 1; m < n; ++m) {
+            r[m - 1] = q;
+            q = one / (two - q);
+        }
+        D[e] = weight * ((q - one) / (q + one));
+        dd u = weight * (dd{2.0, 0.0} * q / (q + one));  // near cell (m = n - 1), then inwards
+        for (int m = n - 1; m > 0; --m) {
+            const dd next = u * r[m - 1];
+            r[m] = u;
+            u = next;
+        }
+        r[0] = u;
+    }
+    __syncthreads();
+    const int m4 = 4 * n;
+    double* out = T + (long long)blockIdx.y * m4 * m4;
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m4 * m4; e += gridDim.x * blockDim.x) {
+        const int q = e / m4, p = e - q * m4, a = q / n, o = q - a * n, b = p / n, c = p - b * n;
+        const int dir = b < 2 ? 0 : 1;           // the data's sides lie across this direction
+        const bool low = (b & 1) == 0;           // W or S
+        const dd* r = R + dir * n * n;
+        dd sum{0.0, 0.0};
+        if (a == b) {
+            for (int l = 0; l < n; ++l) sum = sum + V[l * n + o] * V[l * n + c] * D[dir * n + l];
+        } else if ((a < 2) == (b < 2)) {         // the opposite side: the far cell
+            for (int l = 0; l < n; ++l) sum = sum + V[l * n + o] * V[l * n + c] * r[l * n];
+        } else {                                 // a neighbouring side: its o-th cell, n-1-o or o cells from the far side
+            const int m = low ? n - 1 - o : o, end = (a & 1) ? n - 1 : 0;
+            for (int l = 0; l < n; ++l) sum = sum + V[l * n + end] * V[l * n + c] * r[l * n + m];
+        }
+        const double scale = (a & 1 ? -2.0 : 2.0) / (a < 2 ? dx : dy);
+        const dd t = sum * dd{scale, 0.0};
+        out[e] = t.h + t.l;
+    }
+}
+
 void ck(cudaError_t e, const char* what) {
     if (e != cudaSuccess) throw std::runtime_error(std::string("CUDA error in ") + what + ": " + cudaGetErrorString(e));
 }
 
 }  // namespace
+
+bool leaf_dtn_definite(int n, double lambda, double dx, double dy) {
+    const double q = std::sin(M_PI / (2.0 * n));
+    const double smallest = 4.0 * q * q * (1.0 / (dx * dx) + 1.0 / (dy * dy));  // of the negative Laplacian
+    return n <= kMaxSide && lambda < 0.5 * smallest;
+}
+
+void leaf_dtn_modes(cudaStream_t st, int n, double lambda, const LeafType* types_dev, int nt, double* T) {
+    if (nt <= 0) return;
+    const SineTable S = sine_table(n);
+    const size_t smem = (3 * size_t(n) * n + 2 * n) * sizeof(dd);
+    ck(cudaFuncSetAttribute(k_dtn_modes, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)), "leaf DtN attribute");
+    // a block per 128 entries, every block with its own tables, up to about a block per SM over all types
+    const int slices = std::max(1, std::min(16 * n * n / 128, 152 / nt));
+    k_dtn_modes<<<dim3(slices, nt), 256, smem, st>>>(S, n, types_dev, lambda, T);
+    ++g_kernel_launches;
+    ck(cudaGetLastError(), "leaf DtN launch");
+}
 
 int leaf_dtn_lu(cudaStream_t st, int n, double lambda, const std::vector<double>& dx, const std::vector<double>& dy,
                 const std::vector<double*>& T) {
