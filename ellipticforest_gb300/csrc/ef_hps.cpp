@@ -571,7 +571,11 @@ void Hps::build_leaf_types() {
         fp_factor(st_, d_fp_, num_leaves(), n_);
         pe(L * 8 * (6 * N + N * (2 * n + 1)), L * 2.0 * N * n * n);
         pb("leaf_dtn");
-        leaf_run(LEAF_DTN_COLUMN, d_items_dtn_, nitems_dtn_);
+        const size_t scratch = fp_columns_scratch(num_leaves(), n_);
+        if (scratch && reserve(scratch))
+            fp_columns(st_, d_fp_, d_items_dtn_, num_leaves(), n_, reinterpret_cast<double*>(d_ws_));
+        else
+            leaf_run(LEAF_DTN_COLUMN, d_items_dtn_, nitems_dtn_);
         pe(double(types_.size()) * 16 * n * n * 8, double(nitems_dtn_) * (6 * n * n * n + 8 * n * n));
         return;
     }
@@ -597,11 +601,11 @@ void Hps::build_leaf_types() {
 void Hps::build() {
     root_lu_valid_ = false;
     top_level_ = -1;
+    for (const auto& g : groups_) merge_workspace(g.distinct, g.s);
     build_leaf_types();
     // the merges of every level (a fixed launch sequence for this tree) replay as a CUDA graph from
     // the third build on (first eager, second captured); the leaf DtN maps above stay eager
     const long long l0 = g_kernel_launches.load();
-    for (const auto& g : groups_) merge_workspace(g.distinct, g.s);
     graph_build_.run(st_, 1, graphs_ && !prof_, [&] { merge_levels(mesh_.max_level - 1, true, false); });
     build_launches_ = g_kernel_launches.load() - l0;
     check(cudaGetLastError(), "build launch");
@@ -623,9 +627,8 @@ void Hps::build() {
     built_ = true;
 }
 
-bool Hps::merge_workspace(int cnt, int s) {
-    if (!merge64_supported(s)) return true;
-    const size_t need = merge64_workspace(cnt, s) + 1024;
+bool Hps::reserve(size_t need) {
+    need = (need + 1023) / 1024 * 1024 + 1024;  // and the error word
     if (need <= ws_bytes_) return true;
     if (ws_refused_) return false;
     check(cudaStreamSynchronize(st_), "workspace sync");
@@ -643,6 +646,10 @@ bool Hps::merge_workspace(int cnt, int s) {
     d_wserr_ = reinterpret_cast<int*>(d_ws_ + need - 1024);
     check(cudaMemsetAsync(d_wserr_, 0, sizeof(int), st_), "memset workspace error");
     return true;
+}
+
+bool Hps::merge_workspace(int cnt, int s) {
+    return !merge64_supported(s) || reserve(merge64_workspace(cnt, s));
 }
 
 bool Hps::merges_rejected(int below) {

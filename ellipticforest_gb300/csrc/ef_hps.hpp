@@ -318,6 +318,7 @@ private:
     void merge_nodes(const MergeTables& t, int cnt, int s, bool careful);
     void merge_lu(const MergeTables& t, int cnt, int s);  // from the gathered X, H and T_LHS on
     bool merge_workspace(int cnt, int s);  // room for merge64; false: not available, merge by LU
+    bool reserve(size_t bytes);            // d_ws_ of at least that many bytes
     bool merges_rejected(int below);       // block elimination set info in some merge of levels < below
     void upward_levels(int top);      // upward pass of levels top .. 0
     void downward_levels(int bottom, bool uncoarsen_bottom);  // split from the root to level `bottom`

@@ -134,6 +134,10 @@ struct FpLeaf {
     int* info;             // first zero pivot (1-based) or 0
 };
 void fp_factor(cudaStream_t st, const FpLeaf* leaves, int nleaves, int nmax);
+// DtN maps of leaves of at most 32 x 32 cells: items[4n leaf].out <- T (4n x 4n) from the factors.  scratch:
+// fp_columns_scratch bytes (0: the size is not supported, take fp_solve's LEAF_DTN_COLUMN)
+size_t fp_columns_scratch(int nleaves, int n);
+void fp_columns(cudaStream_t st, const FpLeaf* leaves, const LeafItem* items, int nleaves, int n, double* scratch);
 // items[k].type indexes `leaves`; modes as for leaf_eigen
 void fp_solve(cudaStream_t st, int mode, const FpLeaf* leaves, const LeafItem* items, int nitems,
               int nmax);
