@@ -876,7 +876,10 @@ MatView at(const MatView& v, long long r, long long c) {
     return o;
 }
 
-// Inverses of one or two h x h matrices per item, in place.  tmp: room for 3 h^2 doubles per view.
+// rows of the leading block of the 2 x 2 elimination of h rows
+int first_part(int h) { return (h / 2 + 31) / 32 * 32; }
+
+// Inverses of one or two h x h matrices per item, in place.  tmp: invert64_tmp(h) doubles per view.
 //
 // Up to 32 rows: Gauss-Jordan in FP64.  Up to 128: an FP32 inverse Y (error e ~ 1e-7 cond) and two Newton steps
 // Y <- Y + Y (I - A Y), each squaring the error, with accurate products; where the residual before the second
@@ -937,7 +940,7 @@ void invert(Runner& R, const std::vector<MatView>& v, int h, const MatView& tmp,
         R.release(m0);
         return;
     }
-    const int h1 = (h / 2 + 31) / 32 * 32, h2 = h - h1;
+    const int h1 = first_part(h), h2 = h - h1;
     std::vector<MatView> A, B, C, D, G, F;
     MatView below = tmp;
     for (const auto& x : v) {
@@ -1127,6 +1130,24 @@ void merge64(cudaStream_t st, const MergeItem* items, int cnt, int s, int* info,
         Runner R(st, ws, err, std::min(p.items, cnt - i), false);
         merge_steps(R, items + i, s, p.kids, info + i);
     }
+}
+
+size_t invert64_tmp(int h) {
+    if (h <= 128) return 2 * size_t(h) * h;
+    const size_t h1 = first_part(h), h2 = h - h1;
+    return 2 * h1 * h2 + std::max(invert64_tmp(int(h1)), invert64_tmp(int(h2)));
+}
+
+size_t invert64_workspace(int h) {
+    Runner R(nullptr, nullptr, nullptr, 1, true);
+    const MatView v{PtrTable{nullptr, 0}, 0, h};
+    invert(R, {v}, h, v, nullptr);
+    return R.peak();
+}
+
+void invert64(cudaStream_t st, double* const* A, double* const* tmp, int h, int* info, char* ws, int* err) {
+    Runner R(st, ws, err, 1, false);
+    invert(R, {MatView{PtrTable{A, 0}, 0, h}}, h, MatView{PtrTable{tmp, 0}, 0, h}, info);
 }
 
 }  // namespace efgb

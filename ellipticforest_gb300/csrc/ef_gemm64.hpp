@@ -33,4 +33,10 @@ bool merge64_supported(int s);
 size_t merge64_workspace(int cnt, int s);
 void merge64(cudaStream_t st, const MergeItem* items, int cnt, int s, int* info, char* ws, int* err);
 
+// A <- A^-1 of one h x h row-major matrix in place (A: device address holding its pointer) by the same block
+// elimination; info as above except for the residual, which is the caller's to check.  tmp: invert64_tmp doubles.
+size_t invert64_workspace(int h);
+size_t invert64_tmp(int h);
+void invert64(cudaStream_t st, double* const* A, double* const* tmp, int h, int* info, char* ws, int* err);
+
 }  // namespace efgb

@@ -801,13 +801,14 @@ void Hps::root_from_bc() {
     }
     pb("root_general");
     if (!d_rootA_) {
-        const size_t bytes = align_up(size_t(m) * m * 8) + 3 * align_up(size_t(m) * 8) +
+        const size_t bytes = align_up(size_t(m) * m * 8) + 4 * align_up(size_t(m) * 8) +
                              2 * align_up(size_t(m) * 4) + 2 * align_up(sizeof(int)) + 4 * align_up(sizeof(void*));
         check(cudaMalloc(&d_rootA_, bytes), "cudaMalloc(root)");
         Carver cv;
         cv.base = reinterpret_cast<char*>(d_rootA_);
         cv.get<double>(size_t(m) * m);
         d_rootrhs_ = cv.get<double>(m);
+        d_rootres_ = cv.get<double>(m);
         d_rootpiv_ = cv.get<int>(m);
         d_rootperm_ = cv.get<int>(m);
         d_rootinfo_ = cv.get<int>(1);
@@ -834,19 +835,52 @@ void Hps::root_from_bc() {
         same = root_flag_host_ != 0;
     }
     if (!same) {
+        // A^-1 by the merges' block elimination where its residual is that of a pivoted LU, else the LU: the
+        // factors' 2 x 4M steps of a solve are a chain, a product with A^-1 is not (1280 x 1280: 18 ms for LU and
+        // one solve, 3.8 ms for the inverse, its check and a solve)
         root_assemble(st_, m, d_bca_, d_bcb_, nodes_[0].T, d_rootA_);
         check(cudaMemsetAsync(d_rootinfo_, 0, sizeof(int), st_), "memset root info");
-        dgetrf_batched(st_, m, d_rootA_arr_, m, d_rootpiv_arr_, d_rootinfo_, 1);
-        piv_to_perm(st_, m, d_rootpiv_arr_, d_rootperm_arr_, 1);
+        root_inverse_ = false;
+        const size_t digits = (invert64_workspace(m) + 1023) / 1024 * 1024, tmp = invert64_tmp(m) * sizeof(double);
+        if (m <= 32768 && reserve(digits + tmp)) {
+            double* t = reinterpret_cast<double*>(d_ws_ + digits);
+            check(upload_sync(st_, d_rootrhs_arr_, &t, sizeof(void*)), "root tmp");
+            invert64(st_, d_rootA_arr_, d_rootrhs_arr_, m, d_rootinfo_, d_ws_, d_wserr_);
+            root_check(st_, m, nodes_[0].T, d_bca_, d_bcb_, d_rootA_, d_rootrhs_, nodes_[0].g, d_rootinfo_);
+            int info = 0, err = 0;
+            check(cudaMemcpyAsync(&info, d_rootinfo_, sizeof(int), cudaMemcpyDeviceToHost, st_), "root info");
+            check(cudaMemcpyAsync(&err, d_wserr_, sizeof(int), cudaMemcpyDeviceToHost, st_), "root error");
+            check(upload_sync(st_, d_rootrhs_arr_, &d_rootrhs_, sizeof(void*)), "root arr");
+            if (err) {
+                check(cudaMemsetAsync(d_wserr_, 0, sizeof(int), st_), "root error");
+                throw std::runtime_error("CUDA error in the root solve: an operand copy did not complete");
+            }
+            root_inverse_ = info == 0;
+            if (!root_inverse_) {
+                root_assemble(st_, m, d_bca_, d_bcb_, nodes_[0].T, d_rootA_);
+                check(cudaMemsetAsync(d_rootinfo_, 0, sizeof(int), st_), "memset root info");
+            }
+        }
+        if (!root_inverse_) {
+            dgetrf_batched(st_, m, d_rootA_arr_, m, d_rootpiv_arr_, d_rootinfo_, 1);
+            piv_to_perm(st_, m, d_rootpiv_arr_, d_rootperm_arr_, 1);
+        }
         check(cudaMemcpyAsync(d_roota_, d_bca_, m * sizeof(double), cudaMemcpyDeviceToDevice, st_), "root a");
         check(cudaMemcpyAsync(d_rootb_, d_bcb_, m * sizeof(double), cudaMemcpyDeviceToDevice, st_), "root b");
         root_lu_valid_ = true;
         ++root_factorizations_;
     }
-    root_rhs(st_, m, d_bcb_, d_bcr_, nodes_[0].h, d_rootperm_, d_rootrhs_);
-    dlu_solve_permuted(st_, m, 1, (const double* const*)d_rootA_arr_, m, d_rootrhs_arr_, 1, 1);
-    check(cudaMemcpyAsync(nodes_[0].g, d_rootrhs_, m * sizeof(double), cudaMemcpyDeviceToDevice, st_),
-          "root g");
+    if (root_inverse_) {
+        // g = A^-1 r and one refinement step with the residual from T
+        root_rhs(st_, m, d_bcb_, d_bcr_, nodes_[0].h, nullptr, d_rootrhs_);
+        root_gemv(st_, m, d_rootA_, d_rootrhs_, false, nodes_[0].g);
+        root_residual(st_, m, nodes_[0].T, d_bca_, d_bcb_, d_rootrhs_, nodes_[0].g, d_rootres_);
+        root_gemv(st_, m, d_rootA_, d_rootres_, true, nodes_[0].g);
+    } else {
+        root_rhs(st_, m, d_bcb_, d_bcr_, nodes_[0].h, d_rootperm_, d_rootrhs_);
+        dlu_solve_permuted(st_, m, 1, (const double* const*)d_rootA_arr_, m, d_rootrhs_arr_, 1, 1);
+        check(cudaMemcpyAsync(nodes_[0].g, d_rootrhs_, m * sizeof(double), cudaMemcpyDeviceToDevice, st_), "root g");
+    }
     pe(same ? 8.0 * double(m) * m : 8.0 * 3 * double(m) * m,
        (same ? 0.0 : 2.0 / 3.0 * double(m) * m * m) + 2.0 * double(m) * m);
 }

@@ -365,7 +365,8 @@ private:
     double *d_f_ = nullptr, *d_u_ = nullptr;
     double *d_bca_ = nullptr, *d_bcb_ = nullptr, *d_bcr_ = nullptr;
     // general (b != 0) root solve
-    double *d_rootA_ = nullptr, *d_rootrhs_ = nullptr;
+    double *d_rootA_ = nullptr, *d_rootrhs_ = nullptr, *d_rootres_ = nullptr;
+    bool root_inverse_ = false;  // d_rootA_ holds A^-1, not the LU
     int *d_rootpiv_ = nullptr, *d_rootperm_ = nullptr, *d_rootinfo_ = nullptr, *d_rootflag_ = nullptr;
     double *d_roota_ = nullptr, *d_rootb_ = nullptr;  // (a, b) of the cached root LU
     bool root_lu_valid_ = false;

@@ -391,6 +391,13 @@ void root_assemble(cudaStream_t st, int m, const double* a, const double* b, con
                    double* A);
 void root_rhs(cudaStream_t st, int m, const double* b, const double* r, const double* h,
               const int* perm, double* rhs);
+// out = M x (+ out); out = rhs - (diag(a) + diag(b) T) x
+void root_gemv(cudaStream_t st, int m, const double* M, const double* x, bool add, double* out);
+void root_residual(cudaStream_t st, int m, const double* T, const double* a, const double* b, const double* rhs,
+                   const double* x, double* out);
+// info = 1 where Ainv is not the inverse of diag(a) + diag(b) T to the accuracy of a pivoted LU (v, y: m values)
+void root_check(cudaStream_t st, int m, const double* T, const double* a, const double* b, const double* Ainv, double* v,
+                double* y, int* info);
 // flag = 1 when (a, b) equal (a0, b0) bit for bit, else 0
 void root_same(cudaStream_t st, int m, const double* a, const double* b, const double* a0, const double* b0,
                int* flag);

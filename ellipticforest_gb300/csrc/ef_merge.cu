@@ -375,9 +375,45 @@ __global__ void k_root_assemble(int m, const double* a, const double* b, const d
 __global__ void k_root_rhs(int m, const double* b, const double* r, const double* h, const int* perm,
                            double* rhs) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-        const int k = perm[i];
+        const int k = perm ? perm[i] : i;
         const double bh = (h != nullptr) ? b[k] * h[k] : 0.0;
         rhs[i] = r[k] - bh;
+    }
+}
+
+// out = (add ? out : 0) + M x for a row-major m x m matrix, or out = rhs - (diag(a) + diag(b) T) x when `rhs` is
+// given (then M is T); one warp per row
+__global__ void __launch_bounds__(256) k_root_gemv(int m, const double* __restrict__ M, const double* __restrict__ x,
+                                                   const double* a, const double* b, const double* rhs, int add,
+                                                   double* out) {
+    const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (r >= m) return;  // whole warp
+    double acc = (m & 1) == 0 ? group_dot<true, 32>(M + (long long)r * m, x, x, m, m, lane)
+                              : group_dot<false, 32>(M + (long long)r * m, x, x, m, m, lane);
+    acc = group_sum<32>(acc);
+    if (lane == 0) out[r] = rhs ? rhs[r] - fma(b[r], acc, a[r] * x[r]) : add ? out[r] + acc : acc;
+}
+
+// info = 1 where |v - (diag(a) + diag(b) T) y| > 1e-12 (|v| + |A| |y|) in some row, for v = +-1 and y = A^-1 v
+__device__ __forceinline__ double root_check_entry(int i) { return (unsigned(i) * 2654435761u) >> 31 ? 1.0 : -1.0; }
+__global__ void k_root_check_v(int m, double* v) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) v[i] = root_check_entry(i);
+}
+__global__ void __launch_bounds__(256) k_root_check(int m, const double* __restrict__ T, const double* __restrict__ y,
+                                                    const double* a, const double* b, int* info) {
+    const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (r >= m) return;
+    double acc = 0.0, mag = 0.0;
+    for (int k = lane; k < m; k += 32) {
+        const double p = T[(long long)r * m + k] * y[k];
+        acc += p;
+        mag += fabs(p);
+    }
+    acc = group_sum<32>(acc);
+    mag = group_sum<32>(mag);
+    if (lane == 0) {
+        const double ay = a[r] * y[r], res = root_check_entry(r) - fma(b[r], acc, ay);
+        if (!(fabs(res) <= 1e-12 * (1.0 + fabs(ay) + fabs(b[r]) * mag))) *info = 1;
     }
 }
 
@@ -538,6 +574,26 @@ void root_assemble(cudaStream_t st, int m, const double* a, const double* b, con
 void root_rhs(cudaStream_t st, int m, const double* b, const double* r, const double* h,
               const int* perm, double* rhs) {
     k_root_rhs<<<(m + 255) / 256, 256, 0, st>>>(m, b, r, h, perm, rhs);
+    ++g_kernel_launches;
+}
+
+void root_gemv(cudaStream_t st, int m, const double* M, const double* x, bool add, double* out) {
+    k_root_gemv<<<(m + 7) / 8, 256, 0, st>>>(m, M, x, nullptr, nullptr, nullptr, add, out);
+    ++g_kernel_launches;
+}
+
+void root_residual(cudaStream_t st, int m, const double* T, const double* a, const double* b, const double* rhs,
+                   const double* x, double* out) {
+    k_root_gemv<<<(m + 7) / 8, 256, 0, st>>>(m, T, x, a, b, rhs, 0, out);
+    ++g_kernel_launches;
+}
+
+void root_check(cudaStream_t st, int m, const double* T, const double* a, const double* b, const double* Ainv, double* v,
+                double* y, int* info) {
+    k_root_check_v<<<(m + 255) / 256, 256, 0, st>>>(m, v);
+    ++g_kernel_launches;
+    root_gemv(st, m, Ainv, v, false, y);
+    k_root_check<<<(m + 7) / 8, 256, 0, st>>>(m, T, y, a, b, info);
     ++g_kernel_launches;
 }
 
