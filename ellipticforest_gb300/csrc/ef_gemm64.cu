@@ -580,140 +580,211 @@ __device__ __forceinline__ double shift_exponent(double x, int k) {
     return __hiloint2double(e + k > 2046 ? (hi & int(0x80000000u)) | 0x7fe00000 : hi + (k << 20), __double2loint(x));
 }
 
-// FP32 inverse of one matrix of at most 128 rows per block: the start of the Newton steps of `invert`.  The
-// same Gauss-Jordan steps as k_inv_small on FP32 entries, 8 x 8 per thread; rows are brought to magnitudes
-// below one by powers of two first, so any scaling of the rows is harmless.  The FP64 steps of a 64-row
-// inverse alone take 68 us on one SM (two multiply-adds per clock); these take a 64th of that per entry.
+constexpr int kStartLd = 132;
+constexpr size_t kStartSmem = 192 * kStartLd * sizeof(float);
+
+// two FP32 multiply-adds per instruction: (x, y) += (a, a) * (p, q)
+__device__ __forceinline__ void fma2(float& x, float& y, float a, float p, float q) {
+    asm("{\n .reg .b64 d, m, n;\n mov.b64 d, {%0, %1};\n mov.b64 m, {%2, %2};\n mov.b64 n, {%3, %4};\n"
+        " fma.rn.f32x2 d, m, n, d;\n mov.b64 {%0, %1}, d;\n}\n"
+        : "+f"(x), "+f"(y)
+        : "f"(a), "f"(p), "f"(q));
+}
+
+// FP32 inverse of one matrix of at most 128 rows per block: the start of the iteration of `invert`.  Gauss-Jordan
+// in steps of 32 rows: one warp inverts the diagonal block in registers (a row per lane, pivots inside the
+// block, rows exchanged by shuffles), the block's row panel is multiplied by it, and all 256 threads update
+// their 8 x 8 entries with 32 columns at once.  Rows are brought to magnitudes below one by powers of two
+// first, so any scaling of the rows is harmless.  Column by column over the whole matrix (two block barriers
+// and ~1000 clocks per column) it took 76 us for 128 rows.
 __global__ void __launch_bounds__(256) k_inv_start(const __grid_constant__ InvList L, int n, int* __restrict__ info) {
+    constexpr int PB = 32, LD = kStartLd;  // panel width; row stride (16-byte rows, no bank conflicts)
     const MatView &V = L.v[blockIdx.x], &O = L.out[blockIdx.x];
     const double* A = table_ptr(V.base, blockIdx.y) + V.off;
     double* out = table_ptr(O.base, blockIdx.y) + O.off;
     const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15, lane = tid & 31;
-    __shared__ __align__(16) float s_col[2][128];
-    __shared__ __align__(16) float s_row[2][128];
-    __shared__ int s_p[128], s_k[128], s_e[128];
+    const int warp = tid >> 5;
+    extern __shared__ __align__(16) float is_smem[];
+    float (*s_all)[LD] = reinterpret_cast<float (*)[LD]>(is_smem);             // the matrix on its way in and out
+    float (*s_row)[LD] = reinterpret_cast<float (*)[LD]>(is_smem + 128 * LD);  // row panel, then times the inverse block
+    float (*s_colT)[LD] = reinterpret_cast<float (*)[LD]>(is_smem + 160 * LD); // column panel, transposed
+    __shared__ __align__(16) float s_inv[PB][PB + 4];
+    __shared__ int s_e[128];
     // rows and columns of a thread: 4 t .. 4 t + 3 and 64 more, so that 16-byte reads of a row or column by the
     // 16 threads of a direction touch every bank once
-    auto at8 = [](int t, int i) { return 4 * t + (i & 3) + 16 * (i & 4); };
-    float a[8][8];
-    {
-        double x[8][8];
+    // (the loops over rows and steps stay rolled: the block runs each a few times at most, and fetching
+    // straight-line code would take longer than running it)
+#pragma unroll 4
+    for (int r = warp; r < 128; r += 8) {
+        double x[4];
+        unsigned m = 0;
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int r = at8(ty, i), c = at8(tx, j);
-                x[i][j] = r < n && c < n ? A[(long long)r * V.ld + c] : (r == c ? 1.0 : 0.0);
-            }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            unsigned m = 0;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) m = max(m, unsigned(__double2hiint(x[i][j])) & 0x7fffffffu);
-#pragma unroll
-            for (int off = 8; off > 0; off >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, off));
-            const int e = max(int(m >> 20), 1) - 1022;  // a row that is not finite keeps its infinities and NaNs
-#pragma unroll
-            for (int j = 0; j < 8; ++j) a[i][j] = d2f_rn_bits(m < 0x7ff00000u ? shift_exponent(x[i][j], -e) : x[i][j]);
-            if (tx == 0) s_e[at8(ty, i)] = e;
+        for (int q = 0; q < 4; ++q) {
+            const int c = lane + 32 * q;
+            x[q] = r < n && c < n ? A[(long long)r * V.ld + c] : (r == c ? 1.0 : 0.0);
+            m = max(m, unsigned(__double2hiint(x[q])) & 0x7fffffffu);
         }
+        m = __reduce_max_sync(0xffffffffu, m);
+        const int e = max(int(m >> 20), 1) - 1022;  // a row that is not finite keeps its infinities and NaNs
+#pragma unroll
+        for (int q = 0; q < 4; ++q) s_all[r][lane + 32 * q] = d2f_rn_bits(m < 0x7ff00000u ? shift_exponent(x[q], -e) : x[q]);
+        if (lane == 0) s_e[r] = e;
     }
-    // rows 4 lane .. 4 lane + 3: 127 - row, and all ones while a row is unused
-    const unsigned k0 = 127u - 4u * unsigned(lane);
-    unsigned m0 = 4 * lane < n ? ~0u : 0u, m1 = 4 * lane + 1 < n ? ~0u : 0u, m2 = 4 * lane + 2 < n ? ~0u : 0u,
-             m3 = 4 * lane + 3 < n ? ~0u : 0u;
+    __syncthreads();
+    float a[8][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; j += 4) {
+            const float4 t = *reinterpret_cast<const float4*>(&s_all[4 * ty + (i & 3) + 16 * (i & 4)][4 * tx + 16 * j]);
+            a[i][j] = t.x; a[i][j + 1] = t.y; a[i][j + 2] = t.z; a[i][j + 3] = t.w;
+        }
     bool bad = false;
-    for (int k8 = 0; k8 < 128; k8 += 4) {
-        if (k8 >= n) break;
-        const int tk = (k8 & 63) >> 2;
-        const bool top = k8 >= 64;
+#pragma unroll 1
+    for (int k0 = 0; k0 < n; k0 += PB) {
+        // rows (columns) k0 .. k0 + 31 are entries 4 .. 7 or 0 .. 3 of the threads of eight rows (columns)
+        const int t0 = (k0 & 63) >> 2, hi = k0 >= 64 ? 4 : 0;
+        const bool mine_r = ty >= t0 && ty < t0 + 8, mine_c = tx >= t0 && tx < t0 + 8;
+        if (mine_r) {
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-            const int k = k8 + kk, bf = kk & 1;
-            if (k >= n) break;
-            if (tx == tk) {
+            for (int i = 0; i < 4; ++i) {
+                const int r = 4 * (ty - t0) + i;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) s_col[bf][at8(ty, i)] = top ? a[i][kk + 4] : a[i][kk];
+                for (int j = 0; j < 8; j += 4)
+                    *reinterpret_cast<float4*>(&s_row[r][4 * tx + 16 * j]) =
+                        hi ? make_float4(a[i + 4][j], a[i + 4][j + 1], a[i + 4][j + 2], a[i + 4][j + 3])
+                           : make_float4(a[i][j], a[i][j + 1], a[i][j + 2], a[i][j + 3]);
             }
-            __syncthreads();
-            const float4 cv = *reinterpret_cast<const float4*>(&s_col[bf][4 * lane]);
-            // leading 25 bits of the magnitude, then 127 - row; nothing for rows that are used (or past the end)
-            const unsigned kx = ((__float_as_uint(cv.x) << 1) & ~127u) | k0, ky = ((__float_as_uint(cv.y) << 1) & ~127u) | (k0 - 1u);
-            const unsigned kz = ((__float_as_uint(cv.z) << 1) & ~127u) | (k0 - 2u), kw = ((__float_as_uint(cv.w) << 1) & ~127u) | (k0 - 3u);
-            const unsigned best = __reduce_max_sync(0xffffffffu, max(max(kx & m0, ky & m1), max(kz & m2, kw & m3)));
-            const int p = 127 - int(best & 127u);
-            const float piv = s_col[bf][p], inv = __fdividef(1.f, piv);
-            if (!(fabsf(piv) > 0.f) || best >= 0xff000000u) bad = true;
-            m0 = p == 4 * lane ? 0u : m0;
-            m1 = p == 4 * lane + 1 ? 0u : m1;
-            m2 = p == 4 * lane + 2 ? 0u : m2;
-            m3 = p == 4 * lane + 3 ? 0u : m3;
-            const int pi = (p & 3) + (p >= 64 ? 4 : 0);
-            const bool mine = ty == ((p & 63) >> 2);
-            if (mine) {
-                // the row inside the thread's eight is the same for the whole block: a jump, not selections
-                auto publish = [&](const float (&row)[8]) {
-                    float x[8];
+        }
+        if (mine_c) {
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) x[j] = row[j] * inv;
-                    if (tx == tk) {
-                        if (top) x[kk + 4] = inv;
-                        else x[kk] = inv;
-                    }
-                    *reinterpret_cast<float4*>(&s_row[bf][4 * tx]) = make_float4(x[0], x[1], x[2], x[3]);
-                    *reinterpret_cast<float4*>(&s_row[bf][64 + 4 * tx]) = make_float4(x[4], x[5], x[6], x[7]);
-                };
-                switch (pi) {
-                    case 0: publish(a[0]); break;
-                    case 1: publish(a[1]); break;
-                    case 2: publish(a[2]); break;
-                    case 3: publish(a[3]); break;
-                    case 4: publish(a[4]); break;
-                    case 5: publish(a[5]); break;
-                    case 6: publish(a[6]); break;
-                    default: publish(a[7]); break;
+            for (int j = 0; j < 4; ++j) {
+                const int c = 4 * (tx - t0) + j;
+#pragma unroll
+                for (int i = 0; i < 8; i += 4)
+                    *reinterpret_cast<float4*>(&s_colT[c][4 * ty + 16 * i]) =
+                        hi ? make_float4(a[i][j + 4], a[i + 1][j + 4], a[i + 2][j + 4], a[i + 3][j + 4])
+                           : make_float4(a[i][j], a[i + 1][j], a[i + 2][j], a[i + 3][j]);
+            }
+        }
+        __syncthreads();
+        if (tid < 32) {
+            // inverse of the 32 x 32 diagonal block: lane = row; the pivot of column k is the largest entry of the
+            // rows not used yet (leading 26 bits, then the row), row k of the result comes from that row
+            float d[PB];
+#pragma unroll
+            for (int j = 0; j < PB; ++j) d[j] = s_row[lane][k0 + j];
+            bool used = false;
+            int my_k = 0, my_p = 0;  // the step this row is the pivot of; the pivot row of step `lane`
+#pragma unroll 1
+            for (int k = 0; k < PB; ++k) {
+                // column k is d[0]: every step moves the columns one register down and its own to the end
+                const unsigned h = __float_as_uint(d[0]) & 0x7fffffffu;
+                const unsigned best = __reduce_max_sync(0xffffffffu, used ? 0u : ((h << 1) & ~63u) | unsigned(63 - lane));
+                const int p = 63 - int(best & 63u);
+                const float piv = __shfl_sync(0xffffffffu, d[0], p);
+                if (!(fabsf(piv) > 0.f) || best >= 0xff000000u) bad = true;
+                const float inv = __fdividef(1.f, piv);
+                const bool pr = lane == p;
+                if (pr) { used = true; my_k = k; }
+                if (lane == k) my_p = p;
+                // every row loses c times the scaled pivot row; the pivot row keeps 1 / piv of itself with c = piv - 1;
+                // the entries of column k count as those of a unit vector
+                const float c = (pr ? piv - 1.f : d[0]) * inv;
+#pragma unroll
+                for (int j = 1; j < PB; ++j) d[j - 1] = fmaf(-c, __shfl_sync(0xffffffffu, d[j], p), d[j]);
+                d[PB - 1] = (pr ? 1.f : 0.f) - c;
+            }
+#pragma unroll
+            for (int j = 0; j < PB; ++j) {
+                const int pj = __shfl_sync(0xffffffffu, my_p, j);
+                s_inv[my_k][pj] = d[j];
+            }
+        }
+        __syncthreads();
+        // panel x inverse block (the block itself replaced by the identity): 32 x 128, 4 x 4 entries per thread
+        {
+            const int r0 = 4 * (tid >> 5), c0 = 4 * lane;
+            float s[4][4] = {};
+            const bool inside = c0 >= k0 && c0 < k0 + PB;
+#pragma unroll 8
+            for (int k = 0; k < PB; ++k) {
+                float4 p = *reinterpret_cast<const float4*>(&s_row[k][c0]);
+                if (inside)
+                    p = make_float4(c0 - k0 == k, c0 + 1 - k0 == k, c0 + 2 - k0 == k, c0 + 3 - k0 == k);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float v = s_inv[r0 + i][k];
+                    fma2(s[i][0], s[i][1], v, p.x, p.y);
+                    fma2(s[i][2], s[i][3], v, p.z, p.w);
                 }
             }
-            if (tid == 0) { s_p[k] = p; s_k[p] = k; }
             __syncthreads();
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                *reinterpret_cast<float4*>(&s_row[r0 + i][c0]) = make_float4(s[i][0], s[i][1], s[i][2], s[i][3]);
+        }
+        __syncthreads();
+        // the block's columns start from zero, its rows become the panel: A <- A - C R with C = -I in those rows
+        if (mine_c) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (hi) a[i][j + 4] = 0.f;
+                    else a[i][j] = 0.f;
+                }
+        }
+        if (mine_r) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    if (hi) a[i + 4][j] = 0.f;
+                    else a[i][j] = 0.f;
+                }
+        }
+#pragma unroll 2
+        for (int k = 0; k < PB; ++k) {
             float rj[8], ci[8];
 #pragma unroll
             for (int j = 0; j < 8; j += 4) {
-                const float4 t = *reinterpret_cast<const float4*>(&s_row[bf][4 * tx + 16 * j]);
+                const float4 t = *reinterpret_cast<const float4*>(&s_row[k][4 * tx + 16 * j]);
                 rj[j] = t.x; rj[j + 1] = t.y; rj[j + 2] = t.z; rj[j + 3] = t.w;
-                const float4 u = *reinterpret_cast<const float4*>(&s_col[bf][4 * ty + 16 * j]);
-                ci[j] = u.x; ci[j + 1] = u.y; ci[j + 2] = u.z; ci[j + 3] = u.w;
+                const float4 u = *reinterpret_cast<const float4*>(&s_colT[k][4 * ty + 16 * j]);
+                ci[j] = -u.x; ci[j + 1] = -u.y; ci[j + 2] = -u.z; ci[j + 3] = -u.w;
             }
-            // one update for all: row i loses c_i times the scaled pivot row; the pivot row itself keeps a 1 / piv of
-            // itself with c = piv - 1; the entries of column k count as those of a unit vector
+            if (mine_r) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const bool pr = mine && i == pi;
-                if (pr) ci[i] = piv - 1.f;
-                if (tx == tk) {
-                    const float one = pr ? 1.f : 0.f;
-                    if (top) a[i][kk + 4] = one;
-                    else a[i][kk] = one;
+                for (int i = 0; i < 4; ++i) {
+                    const float one = 4 * (ty - t0) + i == k ? 1.f : 0.f;
+                    if (hi) ci[i + 4] = one;
+                    else ci[i] = one;
                 }
             }
 #pragma unroll
             for (int i = 0; i < 8; ++i)
 #pragma unroll
-                for (int j = 0; j < 8; ++j) a[i][j] = fmaf(-ci[i], rj[j], a[i][j]);
+                for (int j = 0; j < 8; j += 2) fma2(a[i][j], a[i][j + 1], ci[i], rj[j], rj[j + 1]);
         }
+        __syncthreads();
     }
-    __syncthreads();
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int r = at8(ty, i), c = at8(tx, j);
-            if (r < n && c < n) {
-                const int pc = s_p[c];  // the column of A^-1 takes the scale of that row of A
-                out[(long long)s_k[r] * O.ld + pc] = shift_exponent(f2d_bits(a[i][j]), -s_e[pc]);
-            }
+        for (int j = 0; j < 8; j += 4)
+            *reinterpret_cast<float4*>(&s_all[4 * ty + (i & 3) + 16 * (i & 4)][4 * tx + 16 * j]) =
+                make_float4(a[i][j], a[i][j + 1], a[i][j + 2], a[i][j + 3]);
+    __syncthreads();
+#pragma unroll 4
+    for (int r = warp; r < n; r += 8)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int c = lane + 32 * q;
+            // a column of A^-1 takes the scale of that row of A
+            if (c < n) out[(long long)r * O.ld + c] = shift_exponent(f2d_bits(s_all[r][c]), -s_e[c]);
         }
-    if (tid == 0 && bad) info[blockIdx.y] = 1;
+    if (tid < 32 && bad && lane == 0) info[blockIdx.y] = 1;
 }
 
 // X^{-1} from the X buffer to its place behind S in the RHS buffer (columns [8s, 12s))
@@ -881,10 +952,10 @@ int first_part(int h) { return (h / 2 + 31) / 32 * 32; }
 
 // Inverses of one or two h x h matrices per item, in place.  tmp: invert64_tmp(h) doubles per view.
 //
-// Up to 32 rows: Gauss-Jordan in FP64.  Up to 128: an FP32 inverse Y (error e ~ 1e-7 cond) and two Newton steps
-// Y <- Y + Y (I - A Y), each squaring the error, with accurate products; where the residual before the second
-// is not below 2^-34 per entry (the result would not be accurate to the last bits) info is set.  Beyond, 2 x 2
-// block elimination:
+// Up to 32 rows: Gauss-Jordan in FP64.  Up to 128: an FP32 inverse Y with residual E = I - A Y (~1e-7 cond) and
+// Y (I + E)(I + E^2), whose residual is E^4, with accurate products (two Newton steps in three rounds of products
+// instead of four); where E^2 is not below 2^-31 per entry (E^4 below 128 2^-62 = 2^-55) info is set.  Beyond,
+// 2 x 2 block elimination:
 //   [A B; C D]: G = A^-1 B, F = C A^-1, D <- (D - C G)^-1, B <- -G D, C <- -D F, A <- A^-1 - B F.
 // Every product is an accurate GEMM, so the only FP64 roundings are those of the stored blocks.
 void invert(Runner& R, const std::vector<MatView>& v, int h, const MatView& tmp, int* info) {
@@ -915,27 +986,26 @@ void invert(Runner& R, const std::vector<MatView>& v, int h, const MatView& tmp,
             L.out[i] = y;
         }
         if (!R.dry()) {
-            k_inv_start<<<dim3(unsigned(n), unsigned(R.count())), 256, 0, R.stream()>>>(L, h, info);
+            cudaFuncSetAttribute(k_inv_start, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kStartSmem));
+            k_inv_start<<<dim3(unsigned(n), unsigned(R.count())), 256, kStartSmem, R.stream()>>>(L, h, info);
             ++g_kernel_launches;
         }
-        std::vector<Runner::Digits> a, y;
+        // E = I - A Y; Y' = Y + Y E and E^2 together; Y' + Y' E^2
         for (size_t i = 0; i < n; ++i) {
-            a.push_back(R.split(v[i], h, h, 0));
-            const auto yb = R.split(Y[i], h, h, 1);
-            y.push_back(R.split(Y[i], h, h, 0));
-            R.gemm(a[i], yb, E[i], true, ADD_IDENTITY);
+            const auto a = R.split(v[i], h, h, 0), yb = R.split(Y[i], h, h, 1);
+            R.gemm(a, yb, E[i], true, ADD_IDENTITY);
         }
         R.flush();
-        for (size_t i = 0; i < n; ++i) R.gemm(y[i], R.split(E[i], h, h, 1), Y[i], false, ADD_D);
-        R.flush();
         for (size_t i = 0; i < n; ++i) {
-            const auto yb = R.split(Y[i], h, h, 1);
-            y[i] = R.split(Y[i], h, h, 0);
-            R.gemm(a[i], yb, E[i], true, ADD_IDENTITY);
+            const auto eb = R.split(E[i], h, h, 1), ya = R.split(Y[i], h, h, 0), ea = R.split(E[i], h, h, 0);
+            R.gemm(ya, eb, Y[i], false, ADD_D);
+            R.gemm(ea, eb, E[i], false, ADD_NONE);
         }
         R.flush();
-        for (size_t i = 0; i < n; ++i)
-            R.gemm(y[i], R.split(E[i], h, h, 1, 0, 0, info, -34), v[i], false, ADD_D, Y[i]);
+        for (size_t i = 0; i < n; ++i) {
+            const auto eb = R.split(E[i], h, h, 1, 0, 0, info, -31), ya = R.split(Y[i], h, h, 0);
+            R.gemm(ya, eb, v[i], false, ADD_D, Y[i]);
+        }
         R.flush();
         R.release(m0);
         return;
