@@ -536,6 +536,7 @@ private:
     LeafType32* d_types32_ = nullptr;
     MixLeaf* d_leaves_ = nullptr;
     float* q32_ = nullptr;
+    float* fpy_ = nullptr;  // FivePointStencil leaves: values between the sweeps of a leaf solve
     double *u64_ = nullptr, *f_ = nullptr, *a_ = nullptr, *r_ = nullptr, *rmax_ = nullptr;
     int* d_err_ = nullptr;
     float* rleaf_ = nullptr;

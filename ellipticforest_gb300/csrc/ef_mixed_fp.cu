@@ -2,13 +2,15 @@
 //
 // The FP64 band LU of every leaf's 5-point operator (factored once at build time, see ef_leaf_fp.cu)
 // has bandwidth n, so with the cells split into n blocks of n rows the triangular solves are
-//     forward   y_j = L_jj^{-1} (q_j - L_{j,j-1} y_{j-1})
-//     backward  x_j = U_jj^{-1} (y_j - U_{j,j+1} x_{j+1})
-// At set-up the diagonal blocks are inverted in FP64 and the four n x n blocks of every block row
-// are stored in FP32; a block of requests is then solved per leaf by 2n small GEMMs over the
-// requests, with the work vectors in shared memory.  The FP64 stencil coefficients cW, cE, cS, cN,
+//     forward   y_j = L_jj^{-1} q_j - (L_jj^{-1} L_{j,j-1}) y_{j-1}
+//     backward  x_j = U_jj^{-1} y_j - (U_jj^{-1} U_{j,j+1}) x_{j+1}
+// At set-up the four n x n matrices of every block row are formed in FP64 and stored in FP32; a block of
+// requests is then solved per leaf in 2n steps of two products over the requests, only one of which
+// waits for the step before.  The FP64 stencil coefficients cW, cE, cS, cN,
 // cC of FiniteVolumeSolver.cpp:66-100 are tabulated per cell for the residual, which uses the same
 // ghost treatment as the reference's boundary rows (cpp:100-184): a missing neighbour is 2g - u_C.
+#include <algorithm>
+
 #include "ef_kernels.cuh"
 #include "ef_mixed_common.cuh"
 
@@ -34,159 +36,208 @@ __global__ void __launch_bounds__(256) k_mx_fp_convert(const FpLeaf* __restrict_
     }
 }
 
-// Block rows of the band LU (CTA = (block j, leaf), thread = column k of the n x n blocks), in FP64,
-// stored FP32 as blocks[j][4][n][n] = { L_jj^{-1}, L_{j,j-1}, U_jj^{-1}, U_{j,j+1} } (row-major).
-// Band row r holds columns r-n .. r+n at positions 0 .. 2n (L multipliers | U).
+// Block rows of the band LU, CTA = (block j, leaf): each thread takes one column of one of the four matrices
+// { L_jj^{-1}, L_jj^{-1} L_{j,j-1}, U_jj^{-1}, U_jj^{-1} U_{j,j+1} } by substitution in FP64, stored FP32 as
+// blocks[j][4][n][n] with the columns contiguous (entry (a, k) at k n + a).  Band row r holds columns
+// r-n .. r+n at positions 0 .. 2n (L multipliers | U); the block's rows and the columns under way lie in
+// shared memory.
 __global__ void k_mx_fp_blocks(const FpLeaf* __restrict__ src, const MixFp* __restrict__ dst) {
-    const FpLeaf lf = src[blockIdx.y];
-    const int n = lf.n, w = 2 * n + 1, j = blockIdx.x, k = threadIdx.x;
-    if (k >= n) return;
-    const double* band = lf.band + (long long)j * n * w;  // first row of block row j
+    const FpLeaf& lf = src[blockIdx.y];
+    const int n = lf.n, w = 2 * n + 1, j = blockIdx.x, nt = blockDim.x;
+    extern __shared__ double fbk_smem[];
+    double* band = fbk_smem;      // n x w
+    double* X = band + n * w;     // n x nt: a column per thread
+    for (int e = threadIdx.x; e < n * w; e += nt) band[e] = lf.band[(long long)j * n * w + e];
+    __syncthreads();
     float* out = dst[blockIdx.y].blocks + (long long)j * 4 * n * n;
-    float* Linv = out;
-    float* Lsub = out + n * n;
-    float* Uinv = out + 2 * n * n;
-    float* Usup = out + 3 * n * n;
-    // column k of L_jj^{-1} (unit lower): x_a = delta_ak - sum_{b<a} L[a][b] x_b, L[a][b] at n - (a - b)
-    double x[64];
-    for (int a = 0; a < n; ++a) {
-        double v = (a == k) ? 1.0 : 0.0;
-        if (a > k)
-            for (int bb = k; bb < a; ++bb) v = fma(-band[(long long)a * w + n - (a - bb)], x[bb], v);
-        x[a] = a < k ? 0.0 : v;
-        Linv[a * n + k] = float(x[a]);
+    const int kind = threadIdx.x / n, k = threadIdx.x - kind * n;
+    double* x = X + threadIdx.x;
+    if (kind < 2) {
+        // x_a = v_a - sum_{b<a} L[a][b] x_b, L[a][b] at n - (a - b); L_{j,j-1}[a][b] (b >= a) at b - a
+        for (int a = 0; a < n; ++a) {
+            double v = kind == 0 ? (a == k ? 1.0 : 0.0) : (j > 0 && k >= a ? band[a * w + k - a] : 0.0);
+            for (int b = kind == 0 ? k : 0; b < a; ++b) v = fma(-band[a * w + n - (a - b)], x[b * nt], v);
+            x[a * nt] = a < k && kind == 0 ? 0.0 : v;
+        }
+    } else if (kind < 4) {
+        // x_a = (v_a - sum_{b>a} U[a][b] x_b) / U[a][a], U[a][b] at n + (b - a); U_{j,j+1}[a][b] (b <= a) at 2n + b - a
+        for (int a = n - 1; a >= 0; --a) {
+            double v = kind == 2 ? (a == k ? 1.0 : 0.0) : (j < n - 1 && k <= a ? band[a * w + 2 * n + k - a] : 0.0);
+            for (int b = a + 1; b <= (kind == 2 ? k : n - 1); ++b) v = fma(-band[a * w + n + (b - a)], x[b * nt], v);
+            x[a * nt] = a > k && kind == 2 ? 0.0 : v / band[a * w + n];
+        }
     }
-    // column k of U_jj^{-1} (upper): x_a = (delta_ak - sum_{b>a} U[a][b] x_b) / U[a][a], U[a][b] at n + (b - a)
-    for (int a = n - 1; a >= 0; --a) {
-        double v = (a == k) ? 1.0 : 0.0;
-        if (a < k)
-            for (int bb = a + 1; bb <= k; ++bb) v = fma(-band[(long long)a * w + n + (bb - a)], x[bb], v);
-        x[a] = a > k ? 0.0 : v / band[(long long)a * w + n];
-        Uinv[a * n + k] = float(x[a]);
-    }
-    // off-diagonal blocks: L_{j,j-1}[a][b] (b >= a) at position b - a; U_{j,j+1}[a][b] (b <= a) at 2n + b - a
-    for (int a = 0; a < n; ++a) {
-        Lsub[a * n + k] = (j > 0 && k >= a) ? float(band[(long long)a * w + (k - a)]) : 0.0f;
-        Usup[a * n + k] = (j < n - 1 && k <= a) ? float(band[(long long)a * w + 2 * n + k - a]) : 0.0f;
+    __syncthreads();
+    for (int e = threadIdx.x; e < 4 * n * n; e += nt) {
+        const int col = e / n, a = e - col * n;  // column of all four matrices: kind * n + k
+        out[e] = float(X[a * nt + col]);
     }
 }
 
-// Block solve of one leaf for a group of BN requests (blockIdx.y): 2n steps, each two n x n x BN
-// products with the block matrices staged in shared memory.  NEUMANN: g = 0, load q, write
-// h32 = DtN(0, q).  SOLVE: load q + boundary terms of g32, add (or store, accumulate == 0) the
-// solution to u64.
+constexpr int kFpReq = 8;     // requests per warp
+constexpr int kFpWarps = 2;
+constexpr int kFpGroup = kFpReq * kFpWarps;
+constexpr int kFpStages = 3;  // block rows in flight
+
+// Block solve of one leaf for a group of 16 requests (blockIdx.y).  A warp takes eight requests, a lane one
+// row of the block; the two matrices of a step stream through a ring of three stages that both warps
+// read.  Per k a lane reads its two matrix entries and, as broadcasts, the eight right-hand sides and the
+// eight previous values of row k: six shared-memory wavefronts for 512 multiply-adds, which bounds the kernel
+// (the matrices' 512 MB of a 1024-leaf, 32 x 32 tree would take 75 us).  A warp exchanges rows inside itself, so
+// the only block barrier of a step is the ring's.  y goes through `scratch` between the sweeps.
+// NEUMANN: g = 0, load q, write h32 = DtN(0, q).  SOLVE: load q + boundary terms of g32, add (or store,
+// accumulate == 0) the solution to u64.
 template <int MODE>
-__global__ void __launch_bounds__(256) k_mx_fp_leaf32(const MixFp* __restrict__ fps, const MixLeaf* __restrict__ leaves,
-                                                      int L, int B, int n, int BN, const float* __restrict__ q,
-                                                      double* __restrict__ u64, int accumulate) {
+__global__ void __launch_bounds__(32 * kFpWarps) k_mx_fp_leaf32(const MixFp* __restrict__ fps, const MixLeaf* __restrict__ leaves,
+                                                              int L, int B, int n, const float* __restrict__ q,
+                                                              double* __restrict__ u64, float* __restrict__ scratch,
+                                                              int accumulate) {
     extern __shared__ __align__(16) float fsm[];
-    const int N = n * n, ld = BN + 1;
-    float* Y = fsm;                 // N x ld
-    float* M1 = Y + N * ld;         // n x n
-    float* M2 = M1 + n * n;         // n x n
-    float* T = M2 + n * n;          // n x ld
-    const int leaf = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
-    const int b0 = blockIdx.y * BN, nb = min(BN, B - b0);
+    const int N = n * n, n2 = n * n;
+    const int leaf = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int b0 = (blockIdx.y * kFpWarps + warp) * kFpReq, nb = max(0, min(kFpReq, B - b0));
+    const bool row = lane < n;
+    const int a = row ? lane : 0;
+    float* ring = fsm;                                                       // [stage][2][n][n]
+    float* sq = fsm + kFpStages * 2 * n2 + warp * 2 * 32 * kFpReq;           // [32][8] right-hand sides of the block
+    float* sy = sq + 32 * kFpReq;                                            // [32][8] values of the block before
     const MixFp mf = fps[leaf];
     const MixLeaf lf = leaves[leaf];
-    const long long nn = N;
-    // load the group's q: cells along threads (coalesced), transposed into rows x requests
-    for (int e = tid; e < N * nb; e += nt) {
-        const int bb = e / N, r = e - bb * N;
-        Y[r * ld + bb] = q[((long long)(b0 + bb) * L + leaf) * nn + r];
-    }
-    __syncthreads();
-    if (MODE == LEAF_SOLVE) {
-        for (int e = tid; e < 4 * n * nb; e += nt) {
-            const int bb = e % nb, t = e / nb, side = t / n, pos = t - side * n;
-            int r;
-            if (side == 0) r = pos;
-            else if (side == 1) r = (n - 1) * n + pos;
-            else if (side == 2) r = pos * n;
-            else r = pos * n + n - 1;
-            // a corner cell gets two terms from two threads: add them in a fixed order (side 0/1 first)
-            if (side >= 2 && (pos == 0 || pos == n - 1)) continue;
-            float v = -2.0f * mf.bcoef[side * n + pos] * lf.g32[(long long)(side * n + pos) * B + b0 + bb];
-            if (side < 2 && (pos == 0 || pos == n - 1)) {
-                const int s2 = pos == 0 ? 2 : 3, p2 = side == 0 ? 0 : n - 1;
-                v += -2.0f * mf.bcoef[s2 * n + p2] * lf.g32[(long long)(s2 * n + p2) * B + b0 + bb];
+    float* Y = scratch + (((long long)blockIdx.y * L + leaf) * kFpWarps + warp) * N * kFpReq;
+    const float* qb = q + ((long long)b0 * L + leaf) * N;
+    const long long qs = (long long)L * N;
+    auto stage = [&](int j, int half, int slot) {
+        const float* g = mf.blocks + ((long long)j * 4 + 2 * half) * n2;
+        for (int e = 4 * tid; e < 2 * n2; e += 4 * 32 * kFpWarps) cp_async16(ring + slot * 2 * n2 + e, g + e, 16);
+    };
+    // boundary terms of a cell on a W/E face (side 0, 1) and on an S/N face (side 2, 3)
+    auto face = [&](int side, int pos, int r) {
+        return -2.0f * mf.bcoef[side * n + pos] * lf.g32[(long long)(side * n + pos) * B + b0 + r];
+    };
+    auto fetch_q = [&](int j, float (&v)[kFpReq]) {
+#pragma unroll
+        for (int r = 0; r < kFpReq; ++r) v[r] = row && r < nb ? qb[r * qs + j * n + a] : 0.f;
+        if (MODE == LEAF_SOLVE && row) {
+            const bool x = j == 0 || j == n - 1, y = a == 0 || a == n - 1;
+            if (x || y) {
+#pragma unroll
+                for (int r = 0; r < kFpReq; ++r)
+                    if (r < nb) {
+                        float t = x ? face(j == 0 ? 0 : 1, a, r) : 0.f;
+                        if (y) t += face(a == 0 ? 2 : 3, j, r);
+                        v[r] += t;
+                    }
             }
-            Y[r * ld + bb] += v;
-        }
-        __syncthreads();
-    }
-    const float* blocks = mf.blocks;
-    const int outs = n * nb;
-    // one product: dst[a][bb] (= base[a][bb] -) sum_c Mat[a][c] src[c][bb]
-    auto gemm = [&](const float* Mat, const float* src, int src_ld, float* dst, int dst_ld, const float* base,
-                    int base_ld, bool sub) {
-        for (int o = tid; o < outs; o += nt) {
-            const int a = o / nb, bb = o - a * nb;
-            const float* mr = Mat + a * n;
-            float s0 = 0.f, s1 = 0.f;
-            int c = 0;
-            for (; c + 1 < n; c += 2) {
-                s0 = fmaf(mr[c], src[c * src_ld + bb], s0);
-                s1 = fmaf(mr[c + 1], src[(c + 1) * src_ld + bb], s1);
-            }
-            if (c < n) s0 = fmaf(mr[c], src[c * src_ld + bb], s0);
-            const float s = s0 + s1;
-            dst[a * dst_ld + bb] = sub ? base[a * base_ld + bb] - s : s;
         }
     };
-    auto stage = [&](const float* g1, const float* g2) {
-        for (int e = tid; e < n * n; e += nt) {
-            M1[e] = g1[e];
-            M2[e] = g2[e];
+    // one row of both products: acc = M1 rhs - M2 prev
+    auto products = [&](int slot, float (&acc)[kFpReq]) {
+        const float* m1 = ring + slot * 2 * n2 + a;
+        const float* m2 = m1 + n2;
+#pragma unroll
+        for (int r = 0; r < kFpReq; ++r) acc[r] = 0.f;
+#pragma unroll 4
+        for (int k = 0; k < n; ++k) {
+            const float x = m1[k * n], y = -m2[k * n];
+            const float4 p0 = *reinterpret_cast<const float4*>(sq + k * kFpReq), p1 = *reinterpret_cast<const float4*>(sq + k * kFpReq + 4);
+            const float4 t0 = *reinterpret_cast<const float4*>(sy + k * kFpReq), t1 = *reinterpret_cast<const float4*>(sy + k * kFpReq + 4);
+            acc[0] = fmaf(x, p0.x, acc[0]); acc[1] = fmaf(x, p0.y, acc[1]); acc[2] = fmaf(x, p0.z, acc[2]); acc[3] = fmaf(x, p0.w, acc[3]);
+            acc[4] = fmaf(x, p1.x, acc[4]); acc[5] = fmaf(x, p1.y, acc[5]); acc[6] = fmaf(x, p1.z, acc[6]); acc[7] = fmaf(x, p1.w, acc[7]);
+            acc[0] = fmaf(y, t0.x, acc[0]); acc[1] = fmaf(y, t0.y, acc[1]); acc[2] = fmaf(y, t0.z, acc[2]); acc[3] = fmaf(y, t0.w, acc[3]);
+            acc[4] = fmaf(y, t1.x, acc[4]); acc[5] = fmaf(y, t1.y, acc[5]); acc[6] = fmaf(y, t1.z, acc[6]); acc[7] = fmaf(y, t1.w, acc[7]);
         }
     };
+    auto put = [&](float* dst, const float (&v)[kFpReq]) {
+        if (row) {
+            *reinterpret_cast<float4*>(dst + a * kFpReq) = make_float4(v[0], v[1], v[2], v[3]);
+            *reinterpret_cast<float4*>(dst + a * kFpReq + 4) = make_float4(v[4], v[5], v[6], v[7]);
+        }
+    };
+    float v[kFpReq], acc[kFpReq];
+#pragma unroll
+    for (int r = 0; r < kFpReq; ++r) v[r] = 0.f;
+    put(sy, v);
     // forward sweep
+    for (int i = 0; i < kFpStages - 1; ++i) {
+        if (i < n) stage(i, 0, i);
+        cp_async_commit();
+    }
+    fetch_q(0, v);
+    int slot = 0;
     for (int j = 0; j < n; ++j) {
-        const float* bj = blocks + (long long)j * 4 * n * n;
-        stage(bj, bj + n * n);  // L_jj^{-1}, L_{j,j-1}
-        __syncthreads();
-        float* Yj = Y + j * n * ld;
-        if (j > 0) gemm(M2, Yj - n * ld, ld, T, ld, Yj, ld, true);
-        else
-            for (int o = tid; o < outs; o += nt) { const int a = o / nb, bb = o - a * nb; T[a * ld + bb] = Yj[a * ld + bb]; }
-        __syncthreads();
-        gemm(M1, T, ld, Yj, ld, nullptr, 0, false);
-        __syncthreads();
+        cp_async_wait<kFpStages - 2>();
+        __syncthreads();  // the stage has arrived for everyone, and the one before is free
+        if (j + kFpStages - 1 < n) stage(j + kFpStages - 1, 0, slot == 0 ? kFpStages - 1 : slot - 1);
+        cp_async_commit();
+        put(sq, v);
+        __syncwarp();
+        if (j + 1 < n) fetch_q(j + 1, v);
+        products(slot, acc);
+        __syncwarp();
+        put(sy, acc);
+        if (row) {
+            *reinterpret_cast<float4*>(Y + (long long)(j * n + a) * kFpReq) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+            *reinterpret_cast<float4*>(Y + (long long)(j * n + a) * kFpReq + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+        }
+        if (++slot == kFpStages) slot = 0;
     }
+    cp_async_wait<0>();
+    __syncthreads();
     // backward sweep
+    for (int i = 0; i < kFpStages - 1; ++i) {
+        if (n - 1 - i >= 0) stage(n - 1 - i, 1, i);
+        cp_async_commit();
+    }
+    auto fetch_y = [&](int j, float (&t)[kFpReq]) {
+        const float4 t0 = row ? *reinterpret_cast<const float4*>(Y + (long long)(j * n + a) * kFpReq) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 t1 = row ? *reinterpret_cast<const float4*>(Y + (long long)(j * n + a) * kFpReq + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        t[0] = t0.x; t[1] = t0.y; t[2] = t0.z; t[3] = t0.w;
+        t[4] = t1.x; t[5] = t1.y; t[6] = t1.z; t[7] = t1.w;
+    };
+    double* ub = MODE == LEAF_SOLVE ? u64 + ((long long)b0 * L + leaf) * N : nullptr;
+    fetch_y(n - 1, v);
+#pragma unroll
+    for (int r = 0; r < kFpReq; ++r) acc[r] = 0.f;
+    put(sy, acc);
+    slot = 0;
     for (int j = n - 1; j >= 0; --j) {
-        const float* bj = blocks + (long long)j * 4 * n * n;
-        stage(bj + 2 * n * n, bj + 3 * n * n);  // U_jj^{-1}, U_{j,j+1}
+        cp_async_wait<kFpStages - 2>();
         __syncthreads();
-        float* Yj = Y + j * n * ld;
-        if (j < n - 1) gemm(M2, Yj + n * ld, ld, T, ld, Yj, ld, true);
-        else
-            for (int o = tid; o < outs; o += nt) { const int a = o / nb, bb = o - a * nb; T[a * ld + bb] = Yj[a * ld + bb]; }
-        __syncthreads();
-        gemm(M1, T, ld, Yj, ld, nullptr, 0, false);
-        __syncthreads();
-    }
-    if (MODE == LEAF_SOLVE) {
-        for (int e = tid; e < N * nb; e += nt) {
-            const int bb = e / N, r = e - bb * N;
-            double* dst = u64 + ((long long)(b0 + bb) * L + leaf) * nn + r;
-            const double v = f2d_bits(Y[r * ld + bb]);
-            *dst = accumulate ? *dst + v : v;
+        if (j - (kFpStages - 1) >= 0) stage(j - (kFpStages - 1), 1, slot == 0 ? kFpStages - 1 : slot - 1);
+        cp_async_commit();
+        put(sq, v);
+        double old[kFpReq];
+        if (MODE == LEAF_SOLVE) {
+#pragma unroll
+            for (int r = 0; r < kFpReq; ++r) old[r] = accumulate && row && r < nb ? ub[r * qs + j * n + a] : 0.0;
         }
-    } else {
-        // Neumann data of FiniteVolumeSolver.cpp:296-353 with g = 0
-        for (int e = tid; e < 4 * n * nb; e += nt) {
-            const int bb = e % nb, t = e / nb, side = t / n, pos = t - side * n;
-            int cell;
-            if (side == 0) cell = pos;
-            else if (side == 1) cell = (n - 1) * n + pos;
-            else if (side == 2) cell = pos * n;
-            else cell = pos * n + n - 1;
-            const float dtn = float(side < 2 ? mf.dtn_x : mf.dtn_y);
-            const float sg = (side == 0 || side == 2) ? 1.0f : -1.0f;
-            lf.h32[(long long)(side * n + pos) * B + b0 + bb] = sg * dtn * Y[cell * ld + bb];
+        __syncwarp();
+        if (j > 0) fetch_y(j - 1, v);
+        products(slot, acc);
+        __syncwarp();
+        put(sy, acc);
+        if (MODE == LEAF_SOLVE) {
+#pragma unroll
+            for (int r = 0; r < kFpReq; ++r)
+                if (row && r < nb) {
+                    const double t = f2d_bits(acc[r]);
+                    ub[r * qs + j * n + a] = accumulate ? old[r] + t : t;
+                }
+        } else if (row) {
+            // Neumann data of FiniteVolumeSolver.cpp:296-353 with g = 0
+            auto flux = [&](int side, int pos, float scale) {
+#pragma unroll
+                for (int r = 0; r < kFpReq; ++r)
+                    if (r < nb) lf.h32[(long long)(side * n + pos) * B + b0 + r] = scale * acc[r];
+            };
+            if (j == 0) flux(0, a, float(mf.dtn_x));
+            if (j == n - 1) flux(1, a, -float(mf.dtn_x));
+            if (a == 0) flux(2, j, float(mf.dtn_y));
+            if (a == n - 1) flux(3, j, -float(mf.dtn_y));
         }
+        if (++slot == kFpStages) slot = 0;
     }
+    cp_async_wait<0>();
 }
 
 // FP64 residual with the tabulated stencil (see the constant-coefficient kernel in ef_mixed.cu for
@@ -286,8 +337,13 @@ __global__ void __launch_bounds__(256) k_mx_fp_residual(const MixFp* __restrict_
 
 void mx_fp_blocks(cudaStream_t st, const FpLeaf* src, const MixFp* dst, int L, int n) {
     if (L <= 0) return;
-    k_mx_fp_blocks<<<dim3(unsigned(n), unsigned(L)), 32 * ((n + 31) / 32), 0, st>>>(src, dst);
-    ++g_kernel_launches;
+    const int threads = (4 * n + 31) / 32 * 32;
+    const size_t smem = (size_t(n) * (2 * n + 1) + size_t(n) * threads) * sizeof(double);
+    cudaFuncSetAttribute(k_mx_fp_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    for (int k = 0; k < L; k += 65535) {
+        k_mx_fp_blocks<<<dim3(unsigned(n), unsigned(std::min(65535, L - k))), threads, smem, st>>>(src + k, dst + k);
+        ++g_kernel_launches;
+    }
 }
 
 void mx_fp_convert(cudaStream_t st, const FpLeaf* src, const MixFp* dst, int L, int n) {
@@ -297,28 +353,18 @@ void mx_fp_convert(cudaStream_t st, const FpLeaf* src, const MixFp* dst, int L, 
     mx_fp_blocks(st, src, dst, L, n);
 }
 
-int mx_fp_group(int n) { return n <= 16 ? 32 : 16; }
-
-size_t mx_fp_leaf_smem(int n) {
-    const int BN = mx_fp_group(n), ld = BN + 1;
-    return (size_t(n) * n * ld + 2 * size_t(n) * n + size_t(n) * ld) * sizeof(float);
+size_t mx_fp_leaf_scratch(int L, int B, int n) {
+    return size_t(L) * ((B + kFpGroup - 1) / kFpGroup) * kFpGroup * n * n;
 }
 
 void mx_fp_leaf32(cudaStream_t st, int mode, const MixFp* fps, const MixLeaf* leaves, int L, int B, int n,
-                  const float* q, double* u64, int accumulate) {
-    const int BN = mx_fp_group(n);
-    const size_t smem = mx_fp_leaf_smem(n);
-    static size_t configured = 48 * 1024;
-    if (smem > configured) {
-        cudaFuncSetAttribute(k_mx_fp_leaf32<LEAF_NEUMANN>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        cudaFuncSetAttribute(k_mx_fp_leaf32<LEAF_SOLVE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        configured = smem;
-    }
-    dim3 grid(unsigned(L), unsigned((B + BN - 1) / BN));
+                  const float* q, double* u64, float* scratch, int accumulate) {
+    const size_t smem = (size_t(kFpStages) * 2 * n * n + size_t(kFpWarps) * 2 * 32 * kFpReq) * sizeof(float);
+    dim3 grid(unsigned(L), unsigned((B + kFpGroup - 1) / kFpGroup));
     if (mode == LEAF_NEUMANN)
-        k_mx_fp_leaf32<LEAF_NEUMANN><<<grid, 256, smem, st>>>(fps, leaves, L, B, n, BN, q, u64, 0);
+        k_mx_fp_leaf32<LEAF_NEUMANN><<<grid, 32 * kFpWarps, smem, st>>>(fps, leaves, L, B, n, q, u64, scratch, 0);
     else
-        k_mx_fp_leaf32<LEAF_SOLVE><<<grid, 256, smem, st>>>(fps, leaves, L, B, n, BN, q, u64, accumulate);
+        k_mx_fp_leaf32<LEAF_SOLVE><<<grid, 32 * kFpWarps, smem, st>>>(fps, leaves, L, B, n, q, u64, scratch, accumulate);
     ++g_kernel_launches;
 }
 

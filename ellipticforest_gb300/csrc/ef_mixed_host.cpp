@@ -133,6 +133,7 @@ MixedSolver::MixedSolver(Hps& hps, int bmax, const MixedSolver* share)
             m.gf64 = nd.ncoarsen ? m.gs64.back() : m.g64;
         }
         q32_ = cv.get<float>(B * L * nn);
+        if (fp) fpy_ = cv.get<float>(mx_fp_leaf_scratch(L, int(B), n));
         u64_ = cv.get<double>(B * L * nn);
         f_ = cv.get<double>(B * L * nn);
         a_ = cv.get<double>(B * 4 * M);
@@ -709,7 +710,7 @@ void MixedSolver::pass(int B, bool first, bool neumann_done, bool last) {
     const double items = double(L) * B, nn = double(n) * n;
     if (!neumann_done) {
         h.pb("mx_leaf_neumann", st);
-        if (d_fps_) mx_fp_leaf32(st, LEAF_NEUMANN, d_fps_, d_leaves_, L, B, n, q32_, nullptr, 0);
+        if (d_fps_) mx_fp_leaf32(st, LEAF_NEUMANN, d_fps_, d_leaves_, L, B, n, q32_, nullptr, fpy_, 0);
         else mx_leaf32(st, LEAF_NEUMANN, d_types32_, d_leaves_, L, B, n, q32_, nullptr, 0);
         h.pe(items * (nn * 4 + 4 * n * 4), items * 2.0 * (3 * nn * n + 4 * nn), st);
     }
@@ -774,7 +775,7 @@ void MixedSolver::pass(int B, bool first, bool neumann_done, bool last) {
         h.pe(double(nmis_) * B * 20.0, 0, st);
     }
     h.pb("mx_leaf_solve", st);
-    if (d_fps_) mx_fp_leaf32(st, LEAF_SOLVE, d_fps_, d_leaves_, L, B, n, q32_, u64_, first ? 0 : 1);
+    if (d_fps_) mx_fp_leaf32(st, LEAF_SOLVE, d_fps_, d_leaves_, L, B, n, q32_, u64_, fpy_, first ? 0 : 1);
     else mx_leaf32(st, LEAF_SOLVE, d_types32_, d_leaves_, L, B, n, q32_, u64_, first ? 0 : 1);
     // q in, the FP64 state written (and read when accumulating), the Dirichlet rows in
     h.pe(items * (nn * (first ? 12.0 : 20.0) + 4.0 * n * 4), items * 2.0 * 4 * nn * n, st);
