@@ -211,6 +211,7 @@ void Hps::build_mixed(int fp64_levels) {
         ck32(cudaMemcpy(info.data(), g.d_info, info.size() * sizeof(int), cudaMemcpyDeviceToHost), "info");
         for (int v : info) singular_ += (v != 0);
     }
+    equal_operators_ = true;
     built32_ = true;
 }
 

@@ -624,7 +624,16 @@ void Hps::build() {
             indefinite_ += (v < 0);
         }
     }
+    equal_operators_ = true;
     built_ = true;
+}
+
+std::vector<int> Hps::operator_classes(size_t group) const {
+    const Group& g = groups_[group];
+    std::vector<int> cls(g.nodes.size());
+    for (size_t i = 0; i < cls.size(); ++i)
+        cls[i] = equal_operators_ && int(i) >= g.distinct ? g.same[i - g.distinct] : int(i);
+    return cls;
 }
 
 bool Hps::reserve(size_t need) {

@@ -245,6 +245,9 @@ public:
     // the FP32 operator set the mixed block solver reads; the plain FP64 solve needs build().
     void build_mixed(int fp64_levels);
     bool built32() const { return built32_; }
+    // operator class of every node of a group: equal where the operators are known to be equal bit for bit (the
+    // last build merged the tree's leaves itself); else every node has its own
+    std::vector<int> operator_classes(size_t group) const;
     // Local re-factorisation after a mesh change (ef_incremental.cpp): merge nodes whose subtree is the
     // same in `old` copy its operators, the others merge; equal to build() bit for bit.
     void build_from(const Hps& old);
@@ -361,6 +364,7 @@ private:
     size_t ws_bytes_ = 0;
     int* d_wserr_ = nullptr;
     bool ws_refused_ = false;
+    bool equal_operators_ = false;  // nodes of equal subtrees have equal operators
 
     double *d_f_ = nullptr, *d_u_ = nullptr;
     double *d_bca_ = nullptr, *d_bcb_ = nullptr, *d_bcr_ = nullptr;
@@ -458,6 +462,7 @@ public:
     MixedSolver& operator=(const MixedSolver&) = delete;
 
     int bmax() const { return bmax_; }
+    int capacity() const { return cap_; }
     // stream of this solver's launches (default: the tree's stream at construction)
     void set_stream(cudaStream_t st) { st_ = st; }
     cudaStream_t stream() const { return st_; }
@@ -466,7 +471,7 @@ public:
     double* a() const { return a_; }
     double* r() const { return r_; }
     double* u() const { return u64_; }
-    // max |leaf residual| per request before each pass: [passes][bmax]
+    // max |leaf residual| per request before each pass: [passes][capacity]
     double* residual_max() const { return rmax_; }
     size_t device_bytes() const { return bytes_; }
     // 1 + sweeps FP32 passes on B <= bmax requests; asynchronous on the Hps stream.
@@ -502,7 +507,9 @@ private:
         CUtensorMap tmS{}, tmXi{}, tmH{};
         // tensor-core path: three bf16 planes per operator kind, tiled as the kernel's stage images
         bool tc[3] = {false, false, false};  // per kind (W, H, DOWN)
-        void *S3 = nullptr, *Xi3 = nullptr, *H3 = nullptr;
+        TcPlanes pl[3];
+        int* rep[3] = {nullptr, nullptr, nullptr};  // device: source row tile of each stored tile
+        std::vector<int> tile[3], first[3];         // their tables
     };
     struct MStep {
         int level = 0, nf = 0, count = 0;
@@ -519,6 +526,7 @@ private:
     // one node GEMM of a group (kind 0 W, 1 H, 2 DOWN): code > 0 the FP32 CUDA-core kernel with K
     // split `code` (0: its heuristic), code < 0 the tensor-core kernel with K split -code
     void node_gemm(cudaStream_t st, const MGroup& g, int kind, int B, int code);
+    int filled(int B) const;  // requests a block of B is run with
     double gemm_bytes(const MGroup& g, int kind, int B, int code) const;
     // times the K-split candidates of every node GEMM (CUDA events, block of min(bmax, 32)) and keeps
     // the fastest per group and kind in the tree
@@ -526,6 +534,7 @@ private:
 
     Hps& H_;
     int bmax_;
+    int cap_;  // requests the buffers hold
     cudaStream_t st_;
     const MixedSolver* share_;
     char* arena_ = nullptr;

@@ -211,6 +211,7 @@ void Hps::build_from(const Hps& old) {
     }
     singular_ = leaf_singular_ + bad;
     cudaFree(dev);
+    equal_operators_ = false;  // the reused operators come from another tree
     built_ = true;
 }
 

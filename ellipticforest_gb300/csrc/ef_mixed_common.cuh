@@ -108,6 +108,12 @@ __device__ __forceinline__ unsigned long long l2_evict_first() {
     return p;
 }
 
+__device__ __forceinline__ unsigned long long l2_evict_normal() {
+    unsigned long long p;
+    asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;\n" : "=l"(p));
+    return p;
+}
+
 // one TMA tile (32 columns x rows) of A into shared memory, completing on `bar`, with L2 policy `pol`
 __device__ __forceinline__ void tma_load_tile(const CUtensorMap* tm, unsigned long long* bar, float* dst, int x,
                                               int y, unsigned bytes, unsigned long long pol) {

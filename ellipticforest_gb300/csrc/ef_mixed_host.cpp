@@ -68,7 +68,7 @@ CUtensorMap make_map(float* base, long long rows, int cols, int box_rows) {
 }  // namespace
 
 MixedSolver::MixedSolver(Hps& hps, int bmax, const MixedSolver* share)
-    : H_(hps), bmax_(bmax), st_(hps.stream()), share_(share) {
+    : H_(hps), bmax_(bmax), cap_(bmax), st_(hps.stream()), share_(share) {
     if (share && &share->H_ != &hps) throw std::invalid_argument("mixed solver: operators shared across trees");
     if (!hps.built() && !hps.built32()) throw std::invalid_argument("mixed solver: build the tree first");
     const bool fp = hps.solver_type() == SOLVER_FIVE_POINT;
@@ -80,7 +80,10 @@ MixedSolver::MixedSolver(Hps& hps, int bmax, const MixedSolver* share)
         throw std::invalid_argument("mixed solver: FivePointStencil leaves of at most 32 x 32 cells");
     if (n % 4 != 0 || n > 64)
         throw std::invalid_argument("mixed solver: the leaf size must be a multiple of 4 and at most 64");
-    const size_t nn = size_t(n) * n, B = size_t(bmax);
+    // room for the requests that fill a block up to a multiple of four (see filled), where the limits allow it
+    const int up4 = (bmax + 3) / 4 * 4;
+    if (bmax >= 5 && (long long)L * up4 < (1LL << 31) && 12LL * hps.node(0).nx * up4 < (1LL << 31)) cap_ = up4;
+    const size_t nn = size_t(n) * n, B = size_t(cap_);
     const int M = hps.root_M();
     const Mesh& mesh = hps.mesh();
     mn_.assign(N, MNode());
@@ -176,15 +179,23 @@ MixedSolver::MixedSolver(Hps& hps, int bmax, const MixedSolver* share)
             // the last row tile and K chunk, 2 bytes each) (per kind: W, H, DOWN)
             for (int kind = 0; kind < 3; ++kind)
                 groups_[gi].tc[kind] = hps.tensor_cores() != 0 && mx_tc_supported(kind, g.s);
-            if (groups_[gi].tc[2])
-                groups_[gi].S3 = share ? share->groups_[gi].S3
-                                       : (void*)cv.get<uint16_t>(size_t(mx_tc_plane_elems(cnt * 4 * s, int(8 * s))));
-            if (groups_[gi].tc[0])
-                groups_[gi].Xi3 = share ? share->groups_[gi].Xi3
-                                        : (void*)cv.get<uint16_t>(size_t(mx_tc_plane_elems(cnt * 4 * s, int(4 * s))));
-            if (groups_[gi].tc[1])
-                groups_[gi].H3 = share ? share->groups_[gi].H3
-                                       : (void*)cv.get<uint16_t>(size_t(mx_tc_plane_elems(cnt * 8 * s, int(2 * s))));
+            const int Ks[3] = {int(4 * s), int(2 * s), int(8 * s)};
+            for (int kind = 0; kind < 3; ++kind) {
+                MGroup& mg = groups_[gi];
+                if (!mg.tc[kind]) continue;
+                if (share) {
+                    mg.pl[kind] = share->groups_[gi].pl[kind];
+                    continue;
+                }
+                mx_tc_tiles(kind, g.s, hps.operator_classes(gi), mg.tile[kind], mg.first[kind]);
+                const bool fewer = mg.first[kind].size() < mg.tile[kind].size();
+                mg.pl[kind].planes = cv.get<uint16_t>(size_t(mx_tc_plane_elems(int(mg.first[kind].size()), Ks[kind])));
+                mg.pl[kind].count = int(mg.first[kind].size());
+                if (fewer) {
+                    mg.pl[kind].tile = cv.get<int>(mg.tile[kind].size());
+                    mg.rep[kind] = cv.get<int>(mg.first[kind].size());
+                }
+            }
             for (size_t i = 0; i < cnt; ++i) {
                 MNode& m = mn_[g.nodes[i]];
                 m.S = S ? S + i * 32 * s * s : nullptr;
@@ -439,9 +450,17 @@ MixedSolver::MixedSolver(Hps& hps, int bmax, const MixedSolver* share)
         g.tmXi = make_map(g.Xi32, cnt * 4 * s, int(4 * s), mx_tile_rows(0, g.s));
         g.tmH = make_map(g.H32, cnt * 8 * s, int(2 * s), mx_tile_rows(1, g.s));
         // (the arena was zeroed: the planes' padding rows and columns stay zero)
-        if (g.tc[2]) mx_tc_split(st, 2, g.S32, g.S3, cnt * 4 * s, int(8 * s), g.s);
-        if (g.tc[0]) mx_tc_split(st, 0, g.Xi32, g.Xi3, cnt * 4 * s, int(4 * s), g.s);
-        if (g.tc[1]) mx_tc_split(st, 1, g.H32, g.H3, cnt * 8 * s, int(2 * s), g.s);
+        const float* op[3] = {g.Xi32, g.H32, g.S32};
+        const long long rows[3] = {cnt * 4 * s, cnt * 8 * s, cnt * 4 * s};
+        const int Ks[3] = {int(4 * s), int(2 * s), int(8 * s)};
+        for (int kind = 0; kind < 3; ++kind) {
+            if (!g.tc[kind]) continue;
+            if (g.pl[kind].tile) {
+                ck(upload_sync(st, g.pl[kind].tile, g.tile[kind].data(), g.tile[kind].size() * sizeof(int)), "tiles");
+                ck(upload_sync(st, g.rep[kind], g.first[kind].data(), g.first[kind].size() * sizeof(int)), "tiles");
+            }
+            mx_tc_split(st, kind, op[kind], g.pl[kind], g.rep[kind], rows[kind], Ks[kind], g.s);
+        }
     }
     ck(cudaGetLastError(), "mixed convert");
     ck(cudaStreamSynchronize(st), "mixed setup");
@@ -470,7 +489,7 @@ void MixedSolver::tune() {
     // per group and kind, the fastest of the CUDA-core GEMM (K split 1, 2, 4, ...: code > 0) and the
     // tensor-core GEMM (code < 0: split -code), timed with CUDA events on a block of min(bmax, 32)
     Hps& h = H_;
-    const int B = std::min(bmax_, 32);
+    const int B = std::min(filled(bmax_), 32);
     std::vector<std::array<int, 3>> best(groups_.size(), std::array<int, 3>{1, 1, 1});
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     ck(cudaEventCreate(&e0), "tune event");
@@ -534,7 +553,8 @@ void MixedSolver::tune() {
 // the FP64 interface state read and written.
 double MixedSolver::gemm_bytes(const MGroup& g, int kind, int B, int code) const {
     const double c = g.cnt, s = g.s, eb = (g.tc[kind] && code < 0) ? 6.0 : 4.0;
-    const double op = (kind == 2 ? 32.0 : 16.0) * s * s * eb;
+    const double own = g.tc[kind] && code < 0 && !g.tile[kind].empty() ? double(g.first[kind].size()) / g.tile[kind].size() : 1.0;
+    const double op = (kind == 2 ? 32.0 : 16.0) * s * s * eb * own;
     // per request: W 4s in + 4s out (FP32); H 8s + 8s in, 8s out; DOWN 8s + 4s in, 2 x 4s out, 4s
     // FP64 read and written
     const double vec = kind == 0 ? 32.0 * s : kind == 1 ? 96.0 * s : (32.0 + 16.0 + 32.0 + (direct_ ? 0.0 : 64.0)) * s;
@@ -543,8 +563,7 @@ double MixedSolver::gemm_bytes(const MGroup& g, int kind, int B, int code) const
 
 void MixedSolver::node_gemm(cudaStream_t st, const MGroup& g, int kind, int B, int code) {
     if (g.tc[kind] && code < 0) {
-        const void* planes = kind == 0 ? g.Xi3 : (kind == 1 ? g.H3 : g.S3);
-        mx_gemm_tc(st, kind, planes, g.d_items, g.cnt, g.s, B, d_err_, -code);
+        mx_gemm_tc(st, kind, g.pl[kind], g.d_items, g.cnt, g.s, B, d_err_, -code);
     } else {
         const int ksplit = code < 0 ? 0 : code;
         const CUtensorMap& tm = kind == 0 ? g.tmXi : (kind == 1 ? g.tmH : g.tmS);
@@ -584,14 +603,14 @@ void MixedSolver::set_root_operator(const double* a, const double* b) {
     const size_t mm = size_t(m) * m;
     auto up = [](size_t x) { return (x + 255) / 256 * 256; };
     if (!robin_mem_) {
-        const size_t bytes = up(2 * m * 8) + up(m * 4) + up(mm * 4) + 2 * up(size_t(m) * bmax_ * 4) + up(3 * sizeof(void*));
+        const size_t bytes = up(2 * m * 8) + up(m * 4) + up(mm * 4) + 2 * up(size_t(m) * cap_ * 4) + up(3 * sizeof(void*));
         ck(cudaMalloc(&robin_mem_, bytes), "cudaMalloc(mixed Robin root)");
         char* p = robin_mem_;
         ra64_ = reinterpret_cast<double*>(p); rb64_ = ra64_ + m; p += up(2 * m * 8);
         rb32_ = reinterpret_cast<float*>(p); p += up(m * 4);
         Z32_ = reinterpret_cast<float*>(p); p += up(mm * 4);
-        rho32_ = reinterpret_cast<float*>(p); p += up(size_t(m) * bmax_ * 4);
-        rhs32_ = reinterpret_cast<float*>(p); p += up(size_t(m) * bmax_ * 4);
+        rho32_ = reinterpret_cast<float*>(p); p += up(size_t(m) * cap_ * 4);
+        rhs32_ = reinterpret_cast<float*>(p); p += up(size_t(m) * cap_ * 4);
         zA_ = reinterpret_cast<const float**>(p);
         zB_ = reinterpret_cast<const float**>(p + sizeof(void*));
         zC_ = reinterpret_cast<float**>(p + 2 * sizeof(void*));
@@ -781,14 +800,24 @@ void MixedSolver::pass(int B, bool first, bool neumann_done, bool last) {
     h.pe(items * (nn * (first ? 12.0 : 20.0) + 4.0 * n * 4), items * 2.0 * 4 * nn * n, st);
 }
 
-void MixedSolver::solve(int B, int sweeps) {
-    if (B < 1 || B > bmax_) throw std::invalid_argument("mixed solver: batch size out of range");
+int MixedSolver::filled(int B) const {
+    const int up4 = (B + 3) / 4 * 4;
+    return B == bmax_ && B >= 5 && 6 * (up4 - B) <= B && up4 <= cap_ ? up4 : B;
+}
+
+void MixedSolver::solve(int batch, int sweeps) {
+    if (batch < 1 || batch > bmax_) throw std::invalid_argument("mixed solver: batch size out of range");
+    // The interface rows of a block are accessed in 16-byte pieces, and the tensor-core GEMMs' right-hand sides
+    // copied in them, when the request count is a multiple of four: a full block that is nearly one takes the
+    // places behind the caller's along (requests do not mix, and nobody reads those).  Adaptive tree, 23
+    // requests: 3.95 -> 3.34 ms; beyond a sixth more requests the leaf passes would cost more than the rows save.
+    const int B = filled(batch);
     if (sweeps < 0 || sweeps + 1 > kMaxPasses) throw std::invalid_argument("mixed solver: too many sweeps");
     Hps& h = H_;
     graphs_.run(st_, (long long)B * 64 + sweeps, h.graphs() && !h.prof_, [&] {
         cudaStream_t s = st_;
         ck(cudaMemsetAsync(uG_begin_, 0, uG_bytes_, s), "clear interface state");
-        ck(cudaMemsetAsync(rmax_, 0, sizeof(double) * size_t(bmax_) * kMaxPasses, s), "clear residuals");
+        ck(cudaMemsetAsync(rmax_, 0, sizeof(double) * size_t(cap_) * kMaxPasses, s), "clear residuals");
         if (robin_) ck(cudaMemsetAsync(mn_[0].g64, 0, sizeof(double) * 4 * size_t(h.root_M()) * B, s), "root g64");
         else mx_root(s, 4 * h.root_M(), B, a_, r_, mn_[0].g64);
         // 16 x 16 constant-coefficient leaves fuse each residual with the next Neumann step (the
@@ -797,7 +826,7 @@ void MixedSolver::solve(int B, int sweeps) {
         const bool fuse = !d_fps_ && h.leaf_n() == 16 && !g_general_residual.load();
         for (int p = 0; p <= sweeps; ++p) {
             const bool f = fuse && (p == 0 || res_form_ == 0);
-            residual(B, rmax_ + size_t(p) * bmax_, p == 0, f);
+            residual(B, rmax_ + size_t(p) * cap_, p == 0, f);
             pass(B, p == 0, f, p == sweeps);
         }
     });

@@ -40,7 +40,7 @@
 // 32w..32w+31; the operands a row's epilogue reads are prefetched when its tile starts; the
 // exterior rows of DOWN's children are copied by their own launch, k_mx_ext32), warps 4-6
 // stage X (the next chunk's loads in flight while the current one is split and written), warp 7
-// allocates TMEM, its lane 0 issues the bulk copies and its lane 1 the MMAs.  Stages
+// allocates TMEM and issues the bulk copies and the MMAs.  Stages
 // are handed over through mbarriers; the MMA issuer frees a stage with tcgen05.commit.  Every wait
 // gives up after about one second: the kernel then sets the error word, lets its copies and MMAs in
 // flight finish (bounded waits), frees its TMEM and returns.
@@ -49,8 +49,11 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <map>
 #include <stdexcept>
 #include <string>
+#include <utility>
+#include <vector>
 
 #include "ef_kernels.cuh"
 #include "ef_mixed_common.cuh"
@@ -272,7 +275,7 @@ __device__ __forceinline__ void tc_store_row(const MixItem* __restrict__ items, 
 template <int KIND, int NSEG>
 __global__ void __launch_bounds__(kTcThreads, 1)
     k_mx_umma(const __nv_bfloat16* __restrict__ A3, const MixItem* __restrict__ items, int s, int B, int cnt,
-              int ksplit, int ntiles, int* __restrict__ err) {
+              int ksplit, int ntiles, const int* __restrict__ tmap, int nplanes, int* __restrict__ err) {
     const TcShape sh = tc_shape(KIND, s);  // sh.nseg == NSEG (checked by the launcher)
     const int K = sh.K, R = cnt * sh.rows_item;
     const int nsegs_total = KIND == MX_H ? 4 * cnt : cnt;
@@ -293,7 +296,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(drain + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int nkc = (K + kTK - 1) / kTK;
     int first_tile, tile_step, nunits, cpu, cbase;
     if (ksplit > 1) {
@@ -351,82 +354,80 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     bool ep_ok = true;
 
     if (warp == 7) {
-        // ---- lane 0: producer of the three A planes of every stage (bulk copies) ----
-        if (lane == 0) {
-            int st = 0;
-            unsigned ph = 0;
-            int issued = 0;
-            bool ok = true;
-            const long long pstride = (long long)ntiles * nkc * (kTM * kTK);  // elements per plane
-            const unsigned long long pol = l2_evict_first();
-            for (int u = 0; u < nunits && ok; ++u) {
-                const long long blk0 = (long long)tile_of(u) * nkc + cbase;
-                for (int c = 0; c < cpu && ok; ++c) {
-                    if (issued >= NS) ok = tc_wait(&empty[st], ph ^ 1u, abort_flag);
-                    if (!ok) break;
-                    unsigned char* sa = base + size_t(st) * SB;
-                    mbar_expect_tx(&a_full[st], 3u * kPlaneA);
-                    const __nv_bfloat16* src = A3 + (blk0 + c) * (kTM * kTK);
-                    for (int p = 0; p < 3; ++p)
-                        bulk_load(sa + p * kPlaneA, src + p * pstride, kPlaneA, &a_full[st], pol);
-                    ++issued;
-                    if (++st == NS) { st = 0; ph ^= 1u; }
-                }
+        // ---- the warp stays converged and elects a lane for the bulk copies of the A planes and the MMAs: a
+        //      branch on the lane number has the compiler move every operand into uniform registers
+        //      through a loop over the active lanes (~100 clocks per MMA, 12 of them per chunk) ----
+        const long long pstride = (long long)nplanes * nkc * (kTM * kTK);  // elements per plane
+        // planes that several tiles read stay in L2; the others are read once per pass and go first
+        const unsigned long long pol = tmap ? l2_evict_normal() : l2_evict_first();
+        int cur_tile = -1;
+        long long cur_blk = 0;
+        auto copy = [&](int g) {
+            const int u = g / cpu, c = g - u * cpu, tl = tile_of(u), sl = g % NS;
+            if (tl != cur_tile) {
+                cur_tile = tl;
+                cur_blk = (long long)(tmap ? __ldg(tmap + tl) : tl) * nkc + cbase;
             }
-            if (!ok) {
-                // let the loads still in flight land before the shared memory goes away
-                // (only the last NS loads can be pending: a stage is reloaded after its MMAs completed)
-                int s2 = 0;
-                unsigned p2 = 0;
-                volatile int never_set = 0;
-                const int first = issued > NS ? issued - NS : 0;
-                for (int q = 0; q < issued; ++q) {
-                    if (q >= first) (void)tc_wait(&a_full[s2], p2, &never_set);
-                    if (++s2 == NS) { s2 = 0; p2 ^= 1u; }
-                }
-                atomicExch(err, 1);
+            const __nv_bfloat16* src = A3 + (cur_blk + c) * (kTM * kTK);
+            if (elect_one()) {
+                unsigned char* sa = base + size_t(sl) * SB;
+                mbar_expect_tx(&a_full[sl], 3u * kPlaneA);
+                for (int p = 0; p < 3; ++p) bulk_load(sa + p * kPlaneA, src + p * pstride, kPlaneA, &a_full[sl], pol);
             }
-        }
-        // ---- lane 1: MMA issuer (independent thread scheduling lets the two lanes wait apart) ----
-        if (lane == 1) {
-            int st = 0;
-            unsigned ph = 0;
-            bool ok = true;
-            const uint32_t a_base = smem_u32(base);
-            if (g_mx_inject_timeout && nunits > 0) ok = tc_wait(never, 0u, abort_flag, 1000000LL);
-            for (int gch = 0; gch < total && ok; ++gch) {
-                const int c = gch % cpu, bf = gch % NP;
-                // the chunk's accumulator set was drained NP chunks ago
-                if (gch >= NP) ok = tc_wait(&acc_empty[bf], unsigned(gch / NP - 1) & 1u, abort_flag);
-                if (ok) ok = tc_wait(&a_full[st], ph, abort_flag) && tc_wait(&x_full[st], ph, abort_flag);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t sa = a_base + uint32_t(st) * SB;
-                const uint32_t sx = sa + 3u * kPlaneA;
-                const unsigned dhi = tmem + unsigned(bf * 3 * ncol), dlo = dhi + unsigned(ncol);
-                const int kleft = K - (cbase + c) * kTK;
-                const int nk = kleft >= kTK ? kTK / 16 : (kleft + 15) / 16;
-                for (int kk = 0; kk < nk; ++kk) {
-                    const uint32_t ko = uint32_t(kk) * 32u;
-                    const uint64_t a1 = tc_desc(sa + ko), a2 = tc_desc(sa + kPlaneA + ko),
-                                   a3 = tc_desc(sa + 2 * kPlaneA + ko);
-                    // the three X planes are consecutive rows of one K-major operand: [x1 | x2 | x3]
-                    const uint64_t x123 = tc_desc(sx + ko);
-                    const unsigned acc = kk > 0 ? 1u : 0u;  // a fresh accumulator set per chunk
-                    tc_mma(dhi, a1, x123, idesc3, acc);  // D_hi = a1 x1, D_lo_a = a1 x2, D_lo_b = a1 x3
-                    tc_mma(dlo, a2, x123, idesc2, 1u);   // D_lo_a += a2 x1, D_lo_b += a2 x2
-                    tc_mma(dlo, a3, x123, idesc1, 1u);   // D_lo_a += a3 x1
+            __syncwarp();
+        };
+        bool ok = true;
+        int issued = 0;
+        for (; issued < NS && issued < total; ++issued) copy(issued);
+        if (g_mx_inject_timeout && nunits > 0) ok = __all_sync(0xffffffffu, tc_wait(never, 0u, abort_flag, 1000000LL));
+        const uint64_t d0 = tc_desc(smem_u32(base));
+        for (int gch = 0; gch < total && ok; ++gch) {
+            const int c = gch % cpu, bf = gch % NP, st = gch % NS;
+            const unsigned ph = unsigned(gch / NS) & 1u;
+            // the chunk's accumulator set was drained NP chunks ago
+            if (gch >= NP) ok = tc_wait(&acc_empty[bf], unsigned(gch / NP - 1) & 1u, abort_flag);
+            if (ok) ok = tc_wait(&a_full[st], ph, abort_flag) && tc_wait(&x_full[st], ph, abort_flag);
+            if (!(ok = __all_sync(0xffffffffu, ok))) break;
+            tc_fence_after();
+            const uint64_t da = d0 + uint64_t(unsigned(st) * (unsigned(SB) >> 4));
+            const uint64_t dx = da + uint64_t(3 * kPlaneA >> 4);
+            const unsigned dhi = tmem + unsigned(bf * 3 * ncol), dlo = dhi + unsigned(ncol);
+            const int kleft = K - (cbase + c) * kTK;
+            const int nk = kleft >= kTK ? kTK / 16 : (kleft + 15) / 16;
+            if (elect_one()) {
+#pragma unroll
+                for (int kk = 0; kk < kTK / 16; ++kk) {
+                    if (kk < nk) {
+                        const uint64_t ko = uint64_t(2 * kk), x123 = dx + ko;
+                        // the three X planes are consecutive rows of one K-major operand: [x1 | x2 | x3]
+                        tc_mma(dhi, da + ko, x123, idesc3, kk > 0 ? 1u : 0u);  // D_hi = a1 x1, D_lo_a = a1 x2, D_lo_b = a1 x3
+                        tc_mma(dlo, da + uint64_t(kPlaneA >> 4) + ko, x123, idesc2, 1u);      // D_lo_a += a2 x1, D_lo_b += a2 x2
+                        tc_mma(dlo, da + uint64_t(2 * kPlaneA >> 4) + ko, x123, idesc1, 1u);  // D_lo_a += a3 x1
+                    }
                 }
                 tc_commit(&empty[st]);
                 tc_commit(&acc_full[bf]);
-                if (++st == NS) { st = 0; ph ^= 1u; }
             }
-            // every MMA issued has completed before TMEM is freed
-            tc_commit(drain);
-            volatile int never_set = 0;
-            if (!tc_wait(drain, 0u, &never_set)) atomicExch(err, 1);
-            if (!ok) atomicExch(err, 1);
+            __syncwarp();
+            // refill the stage of the chunk before, whose MMAs complete while this chunk's run
+            if (gch > 0 && issued < total) {
+                ok = __all_sync(0xffffffffu, tc_wait(&empty[(gch - 1) % NS], unsigned((gch - 1) / NS) & 1u, abort_flag));
+                if (ok) copy(issued++);
+            }
         }
+        if (!ok) {
+            // let the loads still in flight land before the shared memory goes away
+            // (only the last NS loads can be pending: a stage is reloaded after its MMAs completed)
+            volatile int never_set = 0;
+            for (int q = issued > NS ? issued - NS : 0; q < issued; ++q)
+                (void)tc_wait(&a_full[q % NS], unsigned(q / NS) & 1u, &never_set);
+        }
+        // every MMA issued has completed before TMEM is freed
+        if (elect_one()) tc_commit(drain);
+        __syncwarp();
+        volatile int never_set = 0;
+        if (!tc_wait(drain, 0u, &never_set)) ok = false;
+        if (!ok && lane == 0) atomicExch(err, 1);
     } else if (warp >= 4) {
         // ---- warps 4-6: stage X.  FP32 request rows travel by cp.async into a ring of kXRing
         //      chunks (kXRing - 1 chunks ahead of the one being split, so no global-load latency sits
@@ -614,23 +615,26 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 // one bulk copy of sequential bytes instead of 128 row pieces K columns apart.  Rows past R and
 // columns past K of the last tile and chunk stay as the caller zeroed them.  H rows in the
 // child-major order of tc_h_unpermute.
+// `rep`: the source tile of each stored tile (null: all of them in order).
 __global__ void k_tc_split(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long R, int K,
-                           int s, int permute_h) {
-    const long long tot = R * K;
+                           int s, int permute_h, const int* __restrict__ rep, int ntiles) {
+    const long long tot = (long long)ntiles * kTM * K;
     const int nkc = (K + kTK - 1) / kTK;
-    const long long pstride = (R + kTM - 1) / kTM * nkc * (kTM * kTK);
+    const long long pstride = (long long)ntiles * nkc * (kTM * kTK);
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < tot;
          e += (long long)gridDim.x * blockDim.x) {
-        const long long row = e / K;
-        const int k = int(e - row * K);
+        const long long out_row = e / K;
+        const int k = int(e - out_row * K);
+        const long long tile = out_row / kTM;
+        const int r = int(out_row - tile * kTM), c = k / kTK, kk = k - c * kTK;
+        const long long row = (rep ? rep[tile] : tile) * kTM + r;
+        if (row >= R) continue;
         long long srow = row;
         if (permute_h) {
             const long long node = row / (8 * s);
             const int pr = int(row - node * 8 * s);
             srow = node * 8 * s + tc_h_unpermute(pr, s);
         }
-        const long long tile = row / kTM;
-        const int r = int(row - tile * kTM), c = k / kTK, kk = k - c * kTK;
         const long long off = (tile * nkc + c) * (kTM * kTK) + r * kTK + (((kk >> 3) ^ (r & 7)) << 3) + (kk & 7);
         __nv_bfloat16 p0, p1, p2;
         split3(src[srow * K + k], p0, p1, p2);
@@ -641,7 +645,7 @@ __global__ void k_tc_split(const float* __restrict__ src, __nv_bfloat16* __restr
 }
 
 template <int KIND, int NSEG>
-void launch_umma_n(cudaStream_t st, const void* A3, const MixItem* items, int cnt, int s, int B, int* err,
+void launch_umma_n(cudaStream_t st, const TcPlanes& A, const MixItem* items, int cnt, int s, int B, int* err,
                    int ksplit) {
     const TcShape sh = tc_shape(KIND, s);
     const long long R = (long long)cnt * sh.rows_item;
@@ -667,8 +671,8 @@ void launch_umma_n(cudaStream_t st, const void* A3, const MixItem* items, int cn
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = ksplit > 1 ? 1 : 0;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_mx_umma<KIND, NSEG>, reinterpret_cast<const __nv_bfloat16*>(A3),
-                                             items, s, B, cnt, ksplit, ntiles, err);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_mx_umma<KIND, NSEG>, reinterpret_cast<const __nv_bfloat16*>(A.planes),
+                                             items, s, B, cnt, ksplit, ntiles, A.tile, A.tile ? A.count : ntiles, err);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         throw std::runtime_error(std::string("tensor-core node GEMM launch (K split ") + std::to_string(ksplit) +
@@ -678,11 +682,11 @@ void launch_umma_n(cudaStream_t st, const void* A3, const MixItem* items, int cn
 }
 
 template <int KIND>
-void launch_umma(cudaStream_t st, const void* A3, const MixItem* items, int cnt, int s, int B, int* err,
+void launch_umma(cudaStream_t st, const TcPlanes& A, const MixItem* items, int cnt, int s, int B, int* err,
                  int ksplit) {
     const int nseg = tc_shape(KIND, s).nseg;
-    if (nseg == 1) launch_umma_n<KIND, 1>(st, A3, items, cnt, s, B, err, ksplit);
-    else launch_umma_n<KIND, 2>(st, A3, items, cnt, s, B, err, ksplit);
+    if (nseg == 1) launch_umma_n<KIND, 1>(st, A, items, cnt, s, B, err, ksplit);
+    else launch_umma_n<KIND, 2>(st, A, items, cnt, s, B, err, ksplit);
 }
 
 }  // namespace
@@ -704,14 +708,33 @@ int mx_tc_max_split(int kind, int s) {
     return k;
 }
 
-long long mx_tc_plane_elems(long long R, int K) {
-    return 3 * ((R + kTM - 1) / kTM) * ((K + kTK - 1) / kTK) * (kTM * kTK);
+long long mx_tc_plane_elems(int ntiles, int K) {
+    return 3LL * ntiles * ((K + kTK - 1) / kTK) * (kTM * kTK);
 }
 
-void mx_tc_split(cudaStream_t st, int kind, const float* src, void* dst, long long R, int K, int s) {
-    const long long tot = R * K;
+void mx_tc_tiles(int kind, int s, const std::vector<int>& cls, std::vector<int>& tile, std::vector<int>& rep) {
+    const int rows = tc_shape(kind, s).rows_item, cnt = int(cls.size());
+    const int ntiles = int(((long long)cnt * rows + kTM - 1) / kTM);
+    const int per = rows >= kTM ? 1 : kTM / rows;  // nodes of a tile (rows: a power of two)
+    std::map<std::pair<int, std::vector<int>>, int> first;
+    tile.clear();
+    rep.clear();
+    for (int t = 0; t < ntiles; ++t) {
+        const int node = int((long long)t * kTM / rows), part = rows >= kTM ? t % (rows / kTM) : 0;
+        std::vector<int> key;
+        for (int i = 0; i < per; ++i) key.push_back(node + i < cnt ? cls[node + i] : -1);
+        const auto it = first.emplace(std::make_pair(part, key), int(rep.size()));
+        if (it.second) rep.push_back(t);
+        tile.push_back(it.first->second);
+    }
+}
+
+void mx_tc_split(cudaStream_t st, int kind, const float* src, const TcPlanes& dst, const int* rep, long long R, int K, int s) {
+    const int ntiles = dst.tile ? dst.count : int((R + kTM - 1) / kTM);
+    const long long tot = (long long)ntiles * kTM * K;
     const int grid = int(std::min<long long>((tot + 255) / 256, 8192));
-    k_tc_split<<<grid, 256, 0, st>>>(src, reinterpret_cast<__nv_bfloat16*>(dst), R, K, s, kind == MX_H ? 1 : 0);
+    k_tc_split<<<grid, 256, 0, st>>>(src, reinterpret_cast<__nv_bfloat16*>(dst.planes), R, K, s, kind == MX_H ? 1 : 0,
+                                     dst.tile ? rep : nullptr, ntiles);
     ++g_kernel_launches;
 }
 
@@ -720,7 +743,7 @@ void mx_tc_set_inject_timeout(int on) {
         throw std::runtime_error("tensor-core GEMM: setting the failure-path test switch failed");
 }
 
-void mx_gemm_tc(cudaStream_t st, int kind, const void* planes, const MixItem* items, int nitems, int s, int B,
+void mx_gemm_tc(cudaStream_t st, int kind, const TcPlanes& planes, const MixItem* items, int nitems, int s, int B,
                 int* err, int ksplit) {
     if (!mx_tc_supported(kind, s)) throw std::invalid_argument("tensor-core node GEMM: unsupported interface size");
     if (ksplit < 1) ksplit = 1;

@@ -87,6 +87,7 @@ void Hps::build_top(int level, const double* const* T_host) {
     }
     singular_ = count_singular(level, false);
     top_level_ = level;
+    equal_operators_ = false;  // the T blocks come from outside
     built_ = true;
 }
 
