@@ -831,7 +831,8 @@ int ef_hps_mixed_residuals(ef_hps* h, int passes, double* out) {
     int st = cuda_status(cudaStreamSynchronize(h->hps->stream()), "mixed residuals");
     if (st) return st;
     if (X.take_error()) return fail(EF_ERR_CUDA, "mixed solve: an operator tile copy did not complete");
-    return cuda_status(cudaMemcpy(out, X.residual_max(), size_t(passes) * X.bmax() * 8, cudaMemcpyDeviceToHost),
+    return cuda_status(cudaMemcpy2D(out, size_t(X.bmax()) * 8, X.residual_max(), size_t(X.capacity()) * 8, size_t(X.bmax()) * 8,
+                                    size_t(passes), cudaMemcpyDeviceToHost),
                        "copy residuals");
 }
 
