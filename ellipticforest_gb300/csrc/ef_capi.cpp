@@ -3,6 +3,7 @@
 // Thin layer over efgb::Mesh and efgb::Hps: argument checks, exception-to-status conversion and
 // host<->device copies.  No computation happens on the host here; every numerical step runs in
 // the CUDA kernels of this library.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cstring>
@@ -152,6 +153,36 @@ int run_single_patch(int solver_type, int n, double xl, double xu, double yl, do
     cudaFree(buf);
     if (singular) return fail(EF_ERR_SINGULAR, "the 5-point operator of the patch is singular");
     return cuda_status(e, "single patch");
+}
+
+// [p, p + bytes) is memory of the current device, inside one allocation, and p is aligned to a double
+bool readable_here(const void* p, size_t bytes) {
+    using QueryFn = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const QueryFn query = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult q{};
+        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &fn, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            (void)cudaGetLastError();
+            fn = nullptr;
+        }
+        return reinterpret_cast<QueryFn>(fn);
+    }();
+    int dev = -1;
+    if (!query || (reinterpret_cast<uintptr_t>(p) & 7u) || cudaGetDevice(&dev) != cudaSuccess) return false;
+    // (attributes that do not apply come back as zero)
+    CUmemorytype type = CUmemorytype(0);
+    int ordinal = -1;
+    unsigned managed = 0;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    CUpointer_attribute at[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
+                                 CU_POINTER_ATTRIBUTE_IS_MANAGED, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                 CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* out[5] = {&type, &ordinal, &managed, &start, &size};
+    const CUdeviceptr d = reinterpret_cast<CUdeviceptr>(p);
+    return query(5, at, out, d) == CUDA_SUCCESS && type == CU_MEMORYTYPE_DEVICE && ordinal == dev && !managed &&
+           d >= start && d - start + bytes <= size;
 }
 
 // One-patch run of the variable-coefficient (FivePointStencil) leaf kernels.
@@ -611,12 +642,18 @@ int ef_hps_load_device_async(ef_hps* h, const double* f, const double* a, const 
     cudaStream_t s = H.stream();
     const size_t nf = size_t(H.num_leaves()) * H.leaf_n() * H.leaf_n();
     const size_t m = 4 * size_t(H.root_M());
-    int st = EF_OK;
-    if (f) st = cuda_status(cudaMemcpyAsync(H.leaf_f(), f, nf * 8, cudaMemcpyDeviceToDevice, s), "load f");
-    if (!st && a) st = cuda_status(cudaMemcpyAsync(H.bc_a(), a, m * 8, cudaMemcpyDeviceToDevice, s), "load a");
-    if (!st && b) st = cuda_status(cudaMemcpyAsync(H.bc_b(), b, m * 8, cudaMemcpyDeviceToDevice, s), "load b");
-    if (!st && r) st = cuda_status(cudaMemcpyAsync(H.bc_r(), r, m * 8, cudaMemcpyDeviceToDevice, s), "load r");
-    return st;
+    const double* src[4] = {f, a, b, r};
+    double* const dst[4] = {H.leaf_f(), H.bc_a(), H.bc_b(), H.bc_r()};
+    const long long len[4] = {(long long)nf, (long long)m, (long long)m, (long long)m};
+    // one launch for what a kernel of this device may read; the rest by copies, which check for themselves
+    for (int k = 0; k < 4; ++k) {
+        if (!src[k] || readable_here(src[k], size_t(len[k]) * 8)) continue;
+        const int st = cuda_status(cudaMemcpyAsync(dst[k], src[k], size_t(len[k]) * 8, cudaMemcpyDeviceToDevice, s), "load");
+        if (st) return st;
+        src[k] = nullptr;
+    }
+    efgb::load_inputs(s, src, dst, len);
+    return cuda_status(cudaGetLastError(), "load");
 }
 
 int ef_hps_solve_device_async(ef_hps* h, int b_is_zero) {

@@ -24,6 +24,7 @@
 
 #include "ef_gemm64.hpp"
 #include "ef_kernels.cuh"
+#include "ef_launch.cuh"
 #include "ef_tcgen05.cuh"
 
 namespace efgb {
@@ -70,6 +71,7 @@ struct SplitList {
 // digits of every 64 values of k as the GEMM's shared-memory image (128-byte rows, 16-byte groups swizzled),
 // zeros past the operand's ends.  Memory bound: 8 B in (twice, the second time from L2), 16 B out.
 __global__ void __launch_bounds__(256) k_split64(const __grid_constant__ SplitList L) {
+    pdl_begin();
     int o = 0;
     while (o + 1 < L.n && int(blockIdx.x) >= L.op[o + 1].blk0) ++o;
     const SplitOp& P = L.op[o];
@@ -295,6 +297,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm64(const __grid_constan
     __syncthreads();
     tc_fence_after();
     const unsigned tmem = *tmem_slot;
+    pdl_begin();  // barriers and TMEM are set up while the digits are still being written
 
     // Warps 8 and 9 stay converged and one elected lane issues: a branch on the lane number would have the
     // compiler move every operand of an instruction into uniform registers through a loop over the active
@@ -505,6 +508,7 @@ struct InvList {
 // so one warp reduction finds both); rows are not moved but put in order when they are written.  A pivot that
 // is zero or not finite sets info.  Bound by the two block barriers and the division of a step.
 __global__ void __launch_bounds__(64) k_inv_small(const __grid_constant__ InvList L, int n, int* __restrict__ info) {
+    pdl_begin();
     const MatView& V = L.v[blockIdx.x];
     double* A = table_ptr(V.base, blockIdx.y) + V.off;
     const int tid = threadIdx.x, ty = tid >> 3, tx = tid & 7, lane = tid & 31;
@@ -598,6 +602,7 @@ __device__ __forceinline__ void fma2(float& x, float& y, float a, float p, float
 // first, so any scaling of the rows is harmless.  Column by column over the whole matrix (two block barriers
 // and ~1000 clocks per column) it took 76 us for 128 rows.
 __global__ void __launch_bounds__(256) k_inv_start(const __grid_constant__ InvList L, int n, int* __restrict__ info) {
+    pdl_begin();
     constexpr int PB = 32, LD = kStartLd;  // panel width; row stride (16-byte rows, no bank conflicts)
     const MatView &V = L.v[blockIdx.x], &O = L.out[blockIdx.x];
     const double* A = table_ptr(V.base, blockIdx.y) + V.off;
@@ -789,6 +794,7 @@ __global__ void __launch_bounds__(256) k_inv_start(const __grid_constant__ InvLi
 
 // X^{-1} from the X buffer to its place behind S in the RHS buffer (columns [8s, 12s))
 __global__ void k_place_inverse(const MergeItem* __restrict__ items, int s) {
+    pdl_begin();
     const MergeItem& it = items[blockIdx.y];
     const int m = 4 * s, half = m / 2;
     const long long tot = (long long)m * half;
@@ -802,6 +808,7 @@ __device__ __forceinline__ double check_entry(int i) { return (unsigned(i) * 265
 
 // y = X^{-1} v for a vector v of +-1, into w (free during a build); one warp per row
 __global__ void __launch_bounds__(256) k_check_y(const MergeItem* __restrict__ items, int s) {
+    pdl_begin();
     const MergeItem& it = items[blockIdx.y];
     const int m = 4 * s, r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (r >= m) return;
@@ -815,6 +822,7 @@ __global__ void __launch_bounds__(256) k_check_y(const MergeItem* __restrict__ i
 // block elimination without row exchanges between blocks is accepted only where its residual is that of
 // an elimination with them (~1e-15); info is set otherwise
 __global__ void __launch_bounds__(256) k_check_r(const MergeItem* __restrict__ items, int s, int* __restrict__ info) {
+    pdl_begin();
     const MergeItem& it = items[blockIdx.y];
     const int m = 4 * s, r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (r >= m) return;
@@ -858,11 +866,12 @@ int sm_count() {
 // `dry` nothing runs and only the workspace is added up.
 class Runner {
 public:
-    Runner(cudaStream_t st, char* ws, int* err, int cnt, bool dry) : st_(st), ws_(ws), err_(err), cnt_(cnt), dry_(dry) {}
+    Runner(cudaStream_t st, char* ws, int* err, int cnt, bool dry) : st_(st), ws_(ws), err_(err), cnt_(cnt), dry_(dry), chain_(dry ? Chain::none : merge_chain(st)) {}
     size_t mark() const { return off_; }
     void release(size_t m) { off_ = m; }
     size_t peak() const { return peak_; }
     bool dry() const { return dry_; }
+    Chain chain() const { return chain_; }  // see ef_launch.cuh
     int count() const { return cnt_; }
     cudaStream_t stream() const { return st_; }
 
@@ -906,7 +915,7 @@ public:
     }
     void flush_split() {
         if (sl_.n && !dry_) {
-            k_split64<<<dim3(unsigned(blocks_), unsigned(cnt_)), 256, 0, st_>>>(sl_);
+            launch_chained(chain_, k_split64, dim3(unsigned(blocks_), unsigned(cnt_)), 256, 0, st_, sl_);
             ++g_kernel_launches;
         }
         sl_.n = 0;
@@ -916,7 +925,7 @@ public:
         flush_split();
         if (gl_.n && !dry_) {
             cudaFuncSetAttribute(k_gemm64, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmem));
-            k_gemm64<<<unsigned(std::min(gl_.tiles, sm_count())), kGemmThreads, kSmem, st_>>>(gl_, err_);
+            launch_chained(chain_, k_gemm64, dim3(unsigned(std::min(gl_.tiles, sm_count()))), kGemmThreads, kSmem, st_, gl_, err_);
             ++g_kernel_launches;
         }
         gl_.n = 0;
@@ -935,6 +944,7 @@ private:
     int* err_;
     int cnt_;
     bool dry_;
+    Chain chain_;
     size_t off_ = 0, peak_ = 0;
     int blocks_ = 0;
     SplitList sl_{};
@@ -965,7 +975,7 @@ void invert(Runner& R, const std::vector<MatView>& v, int h, const MatView& tmp,
             InvList L{};
             L.nv = int(n);
             for (size_t i = 0; i < n; ++i) L.v[i] = v[i];
-            k_inv_small<<<dim3(unsigned(n), unsigned(R.count())), 64, 0, R.stream()>>>(L, h, info);
+            launch_chained(R.chain(), k_inv_small, dim3(unsigned(n), unsigned(R.count())), 64, 0, R.stream(), L, h, info);
             ++g_kernel_launches;
         }
         return;
@@ -987,7 +997,7 @@ void invert(Runner& R, const std::vector<MatView>& v, int h, const MatView& tmp,
         }
         if (!R.dry()) {
             cudaFuncSetAttribute(k_inv_start, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kStartSmem));
-            k_inv_start<<<dim3(unsigned(n), unsigned(R.count())), 256, kStartSmem, R.stream()>>>(L, h, info);
+            launch_chained(R.chain(), k_inv_start, dim3(unsigned(n), unsigned(R.count())), 256, kStartSmem, R.stream(), L, h, info);
             ++g_kernel_launches;
         }
         // E = I - A Y; Y' = Y + Y E and E^2 together; Y' + Y' E^2
@@ -1104,8 +1114,8 @@ void merge_steps(Runner& R, const MergeItem* items, int s, int kids, int* info) 
     }
     if (!R.dry()) {
         const dim3 rows(unsigned((m + 7) / 8), unsigned(R.count()));
-        k_check_y<<<rows, 256, 0, R.stream()>>>(items, s);
-        k_check_r<<<rows, 256, 0, R.stream()>>>(items, s, info);
+        launch_chained(R.chain(), k_check_y, rows, 256, 0, R.stream(), items, s);
+        launch_chained(R.chain(), k_check_r, rows, 256, 0, R.stream(), items, s, info);
         g_kernel_launches += 2;
     }
     // ---- S = X^{-1} S_RHS: the columns of child c's exterior sides have entries on c's two interfaces only
@@ -1142,7 +1152,8 @@ void merge_steps(Runner& R, const MergeItem* items, int s, int kids, int* info) 
     }
     if (!R.dry()) {
         const long long tot = 8LL * s * s;
-        k_place_inverse<<<dim3(unsigned(std::min(2048LL, (tot + 255) / 256)), unsigned(R.count())), 256, 0, R.stream()>>>(items, s);
+        launch_chained(R.chain(), k_place_inverse, dim3(unsigned(std::min(2048LL, (tot + 255) / 256)), unsigned(R.count())), 256, 0, R.stream(),
+                       items, s);
         ++g_kernel_launches;
     }
     // ---- T += H S: the exterior rows of child c take the S rows of its two interfaces

@@ -412,6 +412,8 @@ void root_check(cudaStream_t st, int m, const double* T, const double* a, const 
 void root_same(cudaStream_t st, int m, const double* a, const double* b, const double* a0, const double* b0,
                int* flag);
 
+// dst[k] = src[k] (device memory, len[k] values) for the k with a source
+void load_inputs(cudaStream_t st, const double* const src[4], double* const dst[4], const long long len[4]);
 void fill_zero(cudaStream_t st, double* p, long long n);
 // dst[k][0..len[k]) = src[k][0..len[k]) for k < count
 void copy_batched(cudaStream_t st, const double* const* src, double* const* dst, const long long* len, int count,

@@ -14,6 +14,7 @@
 #include <stdexcept>
 
 #include "ef_kernels.cuh"
+#include "ef_launch.cuh"
 
 namespace efgb {
 
@@ -286,6 +287,7 @@ __global__ void __launch_bounds__(256) k_leaf16d(const LeafType* __restrict__ ty
 template <int MODE>
 __global__ void __launch_bounds__(256) k_leaf16d_wide(const LeafType* __restrict__ types,
                                                       const LeafItem* __restrict__ items) {
+    pdl_begin();
     __shared__ double A[16 * 17], C[16 * 17], Vs[8 * 16], Vf[16 * 17];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int t = lane & 15, k = warp + 8 * (lane >> 4);  // row, and output k in [0, 16)
@@ -415,8 +417,8 @@ void leaf_eigen(cudaStream_t st, int mode, const LeafType* types, const LeafItem
     if (nmax == 16 && (mode == LEAF_NEUMANN || mode == LEAF_SOLVE)) {
         // up to about seven leaves per SM a block per leaf is faster (64 leaves 37 -> 9 us, 1024 leaves 40 -> 34 us)
         if (nitems <= 1024) {
-            if (mode == LEAF_NEUMANN) k_leaf16d_wide<LEAF_NEUMANN><<<nitems, 256, 0, st>>>(types, items);
-            else k_leaf16d_wide<LEAF_SOLVE><<<nitems, 256, 0, st>>>(types, items);
+            if (mode == LEAF_NEUMANN) launch_chained(Chain::few, k_leaf16d_wide<LEAF_NEUMANN>, dim3(unsigned(nitems)), 256, 0, st, types, items);
+            else launch_chained(Chain::few, k_leaf16d_wide<LEAF_SOLVE>, dim3(unsigned(nitems)), 256, 0, st, types, items);
             ++g_kernel_launches;
             return;
         }

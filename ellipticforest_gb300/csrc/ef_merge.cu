@@ -8,6 +8,7 @@
 #include <algorithm>
 
 #include "ef_kernels.cuh"
+#include "ef_launch.cuh"
 
 namespace efgb {
 
@@ -45,6 +46,7 @@ __device__ __forceinline__ void child_ifaces(int c, int& Ia, int& Ib) {
 
 template <class Real>
 __global__ void k_gather_xht(const MergeItemT<Real>* __restrict__ items, int s) {
+    pdl_begin();
     const MergeItemT<Real>& it = items[blockIdx.y];
     const long long m2 = 2LL * s, m4 = 4LL * s, m8 = 8LL * s;
     const long long nX = m4 * m4, nH = m8 * m2, nT = m8 * m8;
@@ -128,6 +130,7 @@ __device__ __forceinline__ int l12_col(int j, int nf, int* rows, double* w) {
 
 template <class Real>
 __global__ void k_coarsen_T(const Real* const* Tin, Real* const* Tout, int nf) {
+    pdl_begin();
     const Real* __restrict__ A = Tin[blockIdx.y];
     Real* __restrict__ B = Tout[blockIdx.y];
     const int nc = nf / 2, mf = 4 * nf, mc = 4 * nc;
@@ -159,6 +162,7 @@ __global__ void k_convert_batched(const In* const* in, Out* const* out, long lon
 }
 
 __global__ void k_coarsen_vec(const double* const* vin, double* const* vout, int nf) {
+    pdl_begin();
     const double* __restrict__ a = vin[blockIdx.y];
     double* __restrict__ b = vout[blockIdx.y];
     const int nc = nf / 2;
@@ -169,6 +173,7 @@ __global__ void k_coarsen_vec(const double* const* vin, double* const* vout, int
 }
 
 __global__ void k_uncoarsen_vec(const double* const* vin, double* const* vout, int nf) {
+    pdl_begin();
     const double* __restrict__ a = vin[blockIdx.y];
     double* __restrict__ b = vout[blockIdx.y];
     const int nc = nf / 2;
@@ -261,6 +266,7 @@ __device__ __forceinline__ double group_dot(const double* __restrict__ row, cons
 
 // hDiff = h_upper - h_lower per interface point (HPSAlgorithm.hpp:1061-1081)
 __global__ void k_hdiff(const MergeItem* __restrict__ items, int s) {
+    pdl_begin();
     const long long m4 = 4LL * s;
     const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const int b = blockIdx.y;
@@ -279,6 +285,7 @@ __device__ __forceinline__ long long group_row() {
 // w = X^{-1} hDiff (the X^{-1} block of RHS, columns [8s, 12s))
 template <bool VEC, int LPR>
 __global__ void __launch_bounds__(kGemvThreads) k_gemv_w(const MergeItem* __restrict__ items, int s, long long nrows) {
+    pdl_begin();
     const int sl = threadIdx.x & (LPR - 1);
     const long long g = group_row<LPR>();
     const bool ok = g < nrows;
@@ -294,6 +301,7 @@ __global__ void __launch_bounds__(kGemvThreads) k_gemv_w(const MergeItem* __rest
 // compact H row p is contiguous: its first s entries multiply w on interface Ia, the rest Ib
 template <bool VEC, int LPR>
 __global__ void __launch_bounds__(kGemvThreads) k_gemv_h(const MergeItem* __restrict__ items, int s, long long nrows) {
+    pdl_begin();
     const int sl = threadIdx.x & (LPR - 1);
     const long long g = group_row<LPR>();
     const bool ok = g < nrows;
@@ -313,6 +321,7 @@ __global__ void __launch_bounds__(kGemvThreads) k_gemv_h(const MergeItem* __rest
 template <bool VEC, int LPR>
 __global__ void __launch_bounds__(kGemvThreads) k_gemv_down(const MergeItem* __restrict__ items, int s,
                                                             long long nrows, int nitems, int add_w) {
+    pdl_begin();
     const int m4 = 4 * s, m8 = 8 * s;
     const long long ext = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (ext < (long long)nitems * m8) {
@@ -348,14 +357,15 @@ inline int pick_lpr(int len, bool vec) {
 
 #define EF_LPR_DISPATCH(KERNEL, VEC, LPR, GRID, ...)                                       \
     do {                                                                                    \
-        if (LPR == 32) KERNEL<VEC, 32><<<GRID, kGemvThreads, 0, st>>>(__VA_ARGS__);         \
-        else if (LPR == 16) KERNEL<VEC, 16><<<GRID, kGemvThreads, 0, st>>>(__VA_ARGS__);    \
-        else if (LPR == 8) KERNEL<VEC, 8><<<GRID, kGemvThreads, 0, st>>>(__VA_ARGS__);      \
-        else KERNEL<VEC, 4><<<GRID, kGemvThreads, 0, st>>>(__VA_ARGS__);                    \
+        if (LPR == 32) launch_chained(Chain::few, KERNEL<VEC, 32>, dim3(GRID), kGemvThreads, 0, st, __VA_ARGS__);         \
+        else if (LPR == 16) launch_chained(Chain::few, KERNEL<VEC, 16>, dim3(GRID), kGemvThreads, 0, st, __VA_ARGS__);    \
+        else if (LPR == 8) launch_chained(Chain::few, KERNEL<VEC, 8>, dim3(GRID), kGemvThreads, 0, st, __VA_ARGS__);      \
+        else launch_chained(Chain::few, KERNEL<VEC, 4>, dim3(GRID), kGemvThreads, 0, st, __VA_ARGS__);                    \
     } while (0)
 
 __global__ void k_root_diag(int m, const double* a, const double* b, const double* r,
                             const double* h, double* g) {
+    pdl_begin();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
         const double bh = (h != nullptr) ? b[i] * h[i] : 0.0;
         g[i] = (r[i] - bh) / a[i];
@@ -434,6 +444,7 @@ __global__ void k_root_same(int m, const double* a, const double* b, const doubl
 // Copies of whole operators: src and dst are starts of arena buffers (256-byte aligned), so whole
 // 16-byte pairs move and an odd last element goes by itself.
 __global__ void k_copy_batched(const double* const* src, double* const* dst, const long long* len) {
+    pdl_begin();
     const double* a = src[blockIdx.y];
     double* b = dst[blockIdx.y];
     const long long n = len[blockIdx.y], n2 = n >> 1;
@@ -442,6 +453,33 @@ __global__ void k_copy_batched(const double* const* src, double* const* dst, con
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n2; e += (long long)gridDim.x * blockDim.x)
         b2[e] = a2[e];
     if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) b[n - 1] = a[n - 1];
+}
+
+// The arrays of a request into the resident buffers, all in one launch (a copy each takes longer to start than a
+// small tree's arrays take to move).
+struct LoadList {
+    int n;
+    const double* src[4];
+    double* dst[4];
+    long long len[4];
+    int vec[4];
+};
+__global__ void __launch_bounds__(256) k_load_inputs(const __grid_constant__ LoadList l) {
+    pdl_begin();
+    const int k = blockIdx.y;
+    const double* a = l.src[k];
+    double* b = l.dst[k];
+    const long long n = l.len[k], step = (long long)gridDim.x * blockDim.x;
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (l.vec[k]) {
+        const double2* a2 = reinterpret_cast<const double2*>(a);
+        double2* b2 = reinterpret_cast<double2*>(b);
+#pragma unroll 4
+        for (long long e = t; e < n / 2; e += step) b2[e] = a2[e];
+        if ((n & 1) && t == 0) b[n - 1] = a[n - 1];
+    } else {
+        for (long long e = t; e < n; e += step) b[e] = a[e];
+    }
 }
 
 __global__ void k_fill_zero(double* p, long long n) {
@@ -464,7 +502,7 @@ template <class Real>
 void gather_xht_t(cudaStream_t st, const MergeItemT<Real>* items, int nitems, int s) {
     const long long tot = 16LL * s * s + 32LL * s * s + 64LL * s * s;
     dim3 g(grid_for(tot, nitems), nitems);
-    k_gather_xht<Real><<<g, 256, 0, st>>>(items, s);
+    launch_chained(merge_chain(st), k_gather_xht<Real>, g, 256, 0, st, items, s);
     ++g_kernel_launches;
 }
 
@@ -480,7 +518,7 @@ template <class Real>
 void coarsen_T_t(cudaStream_t st, const Real* const* Tin, Real* const* Tout, int nitems, int nf) {
     const long long tot = 4LL * nf * 4LL * nf / 4;
     dim3 g(grid_for(tot, nitems), nitems);
-    k_coarsen_T<Real><<<g, 256, 0, st>>>(Tin, Tout, nf);
+    launch_chained(merge_chain(st), k_coarsen_T<Real>, g, 256, 0, st, Tin, Tout, nf);
     ++g_kernel_launches;
 }
 
@@ -511,19 +549,19 @@ void narrow_batched(cudaStream_t st, const double* const* in, float* const* out,
 
 void coarsen_vec(cudaStream_t st, const double* const* vin, double* const* vout, int nitems, int nf) {
     dim3 g((2 * nf + 255) / 256, nitems);
-    k_coarsen_vec<<<g, 256, 0, st>>>(vin, vout, nf);
+    launch_chained(Chain::few, k_coarsen_vec, g, 256, 0, st, vin, vout, nf);
     ++g_kernel_launches;
 }
 
 void uncoarsen_vec(cudaStream_t st, const double* const* vin, double* const* vout, int nitems, int nf) {
     dim3 g((4 * nf + 255) / 256, nitems);
-    k_uncoarsen_vec<<<g, 256, 0, st>>>(vin, vout, nf);
+    launch_chained(Chain::few, k_uncoarsen_vec, g, 256, 0, st, vin, vout, nf);
     ++g_kernel_launches;
 }
 
 void upward_hdiff(cudaStream_t st, const MergeItem* items, int nitems, int s) {
     dim3 g((4 * s + 255) / 256, nitems);
-    k_hdiff<<<g, 256, 0, st>>>(items, s);
+    launch_chained(Chain::few, k_hdiff, g, 256, 0, st, items, s);
     ++g_kernel_launches;
 }
 
@@ -562,7 +600,7 @@ void downward(cudaStream_t st, const MergeItem* items, int nitems, int s, int ad
 
 void root_diag(cudaStream_t st, int m, const double* a, const double* b, const double* r,
                const double* h, double* g) {
-    k_root_diag<<<(m + 255) / 256, 256, 0, st>>>(m, a, b, r, h, g);
+    launch_chained(Chain::few, k_root_diag, dim3(unsigned((m + 255) / 256)), 256, 0, st, m, a, b, r, h, g);
     ++g_kernel_launches;
 }
 
@@ -609,9 +647,27 @@ void copy_batched(cudaStream_t st, const double* const* src, double* const* dst,
     const int per = int(std::max(1LL, std::min(64LL, total / std::max(1, count) / 4096)));
     for (int k0 = 0; k0 < count; k0 += 65535) {
         const int c = count - k0 < 65535 ? count - k0 : 65535;
-        k_copy_batched<<<dim3(per, c), 256, 0, st>>>(src + k0, dst + k0, len + k0);
+        launch_chained(merge_chain(st), k_copy_batched, dim3(per, c), 256, 0, st, src + k0, dst + k0, len + k0);
         ++g_kernel_launches;
     }
+}
+
+void load_inputs(cudaStream_t st, const double* const src[4], double* const dst[4], const long long len[4]) {
+    LoadList l{};
+    long long most = 0;
+    for (int k = 0; k < 4; ++k) {
+        if (!src[k]) continue;
+        l.src[l.n] = src[k];
+        l.dst[l.n] = dst[k];
+        l.len[l.n] = len[k];
+        // both ends on 16 bytes: pairs move whole
+        l.vec[l.n] = ((reinterpret_cast<uintptr_t>(src[k]) | reinterpret_cast<uintptr_t>(dst[k])) & 15u) == 0 ? 1 : 0;
+        most = std::max(most, len[k]);
+        ++l.n;
+    }
+    if (l.n == 0) return;
+    launch_chained(Chain::few, k_load_inputs, dim3(unsigned(std::min(1216LL, std::max(1LL, (most + 2047) / 2048))), unsigned(l.n)), 256, 0, st, l);
+    ++g_kernel_launches;
 }
 
 void fill_zero(cudaStream_t st, double* p, long long n) {
