@@ -6,6 +6,7 @@
 // W = [alpha_W; gamma_W], E = [beta_E; omega_E], S = [alpha_S; beta_S], N = [gamma_N; omega_N]
 // (the pi_WESN = {0,4,2,6,1,3,5,7} reorder of HPSAlgorithm.hpp:979-993).
 #include <algorithm>
+#include <type_traits>
 
 #include "ef_kernels.cuh"
 #include "ef_launch.cuh"
@@ -192,76 +193,71 @@ __global__ void k_uncoarsen_vec(const double* const* vin, double* const* vout, i
 // threads per CTA of the interface GEMVs
 constexpr int kGemvThreads = 128;
 
-// Group dot products: LPR consecutive lanes (LPR in {4, 8, 16, 32}) share one matrix row; the
-// row is streamed with evict-first loads, the vector is read through L1.
-template <int LPR>
+// Group dot products.  The sum of a row is defined for LPR lanes (LPR in {2 .. 32}) that take its units (pairs of
+// doubles where VEC) in turns of eight, each lane into four partial sums: unit u of a turn into sum u mod 4.
+// F real lanes share one such lane, 4 / F of its partial sums each, and add in the same order, so a result does not
+// depend on F: long levels take F = 1 (sixteen doubles per lane and turn: the FP64 pipe bounds these kernels, and
+// the additions between lanes are a seventh of its work then, a quarter with half the row per lane), short ones
+// F = 4 or 2 (a shorter chain).  The row is streamed with evict-first loads, the vector is read through L1.  A
+// right-hand side of a 7-level tree of 16 x 16 leaves: 1707 us with half the row per lane and F = 1, 1579 now.
+template <int LPR, int F>
 __device__ __forceinline__ double group_sum(double v) {
+#pragma unroll
+    for (int off = LPR; off < F * LPR; off *= 2) v += __shfl_xor_sync(0xffffffffu, v, off);
 #pragma unroll
     for (int off = LPR / 2; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
     return v;
 }
 
-// This lane's share of row[0:len) . x[0:len) for one group of LPR lanes (sl = lane within the
-// group), where x[i] = xa[i] for i < split and xb[i - split] after (split even when VEC).  Eight
-// independent row loads per lane and step keep enough bytes in flight at the occupancy these
-// kernels run at (a vector load serving four rows, with four times the registers, ran slower).
-// VEC: row, xa and xb 16-byte aligned and len even -> double2 loads.
-template <bool VEC, int LPR>
-__device__ __forceinline__ double group_dot(const double* __restrict__ row, const double* __restrict__ xa,
-                                             const double* __restrict__ xb, int split, int len, int sl) {
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    if (VEC) {
-        const double2* r2 = reinterpret_cast<const double2*>(row);
-        const double2* xa2 = reinterpret_cast<const double2*>(xa);
-        const double2* xb2 = reinterpret_cast<const double2*>(xb) - (split >> 1);
-        const int n2 = len >> 1, s2 = split >> 1;
-        int i = sl;
-        for (; i + 7 * LPR < n2; i += 8 * LPR) {
-            double2 m[8], v[8];
+// One turn of group_dot: eight units from unit `at` on, in U = double2 or double; those from n on count nothing
+// (FULL: there are none).
+template <bool FULL, int LPR, int F, class U>
+__device__ __forceinline__ void group_turn(const U* __restrict__ row, const U* __restrict__ xa, const U* __restrict__ xb,
+                                           int split, int n, int at, int lane, double* a) {
+    constexpr int NA = 4 / F;
+    const int first = at + lane / LPR * NA * LPR, base = first + (lane & (LPR - 1));
+    U m[2 * NA], v[2 * NA];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) m[u] = __ldcs(r2 + i + u * LPR);
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int k = i + u * LPR;
-                v[u] = __ldg((k < s2 ? xa2 : xb2) + k);
-            }
-#pragma unroll
-            for (int u = 0; u < 8; u += 4) {
-                a0 = fma(m[u].x, v[u].x, a0); a0 = fma(m[u].y, v[u].y, a0);
-                a1 = fma(m[u + 1].x, v[u + 1].x, a1); a1 = fma(m[u + 1].y, v[u + 1].y, a1);
-                a2 = fma(m[u + 2].x, v[u + 2].x, a2); a2 = fma(m[u + 2].y, v[u + 2].y, a2);
-                a3 = fma(m[u + 3].x, v[u + 3].x, a3); a3 = fma(m[u + 3].y, v[u + 3].y, a3);
-            }
-        }
-#pragma unroll 7
-        for (; i < n2; i += LPR) {
-            const double2 m0 = __ldcs(r2 + i), v0 = __ldg((i < s2 ? xa2 : xb2) + i);
-            a0 = fma(m0.x, v0.x, a0); a0 = fma(m0.y, v0.y, a0);
-        }
-    } else {
-        const double* xbs = xb - split;
-        int i = sl;
-        for (; i + 7 * LPR < len; i += 8 * LPR) {
-            double m[8], v[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) m[u] = __ldcs(row + i + u * LPR);
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int k = i + u * LPR;
-                v[u] = __ldg((k < split ? xa : xbs) + k);
-            }
-#pragma unroll
-            for (int u = 0; u < 8; u += 4) {
-                a0 = fma(m[u], v[u], a0);
-                a1 = fma(m[u + 1], v[u + 1], a1);
-                a2 = fma(m[u + 2], v[u + 2], a2);
-                a3 = fma(m[u + 3], v[u + 3], a3);
-            }
-        }
-#pragma unroll 7
-        for (; i < len; i += LPR) a0 = fma(__ldcs(row + i), __ldg((i < split ? xa : xbs) + i), a0);
+    for (int u = 0; u < 2 * NA; ++u) {
+        const int i = base + (u % NA + 4 * (u / NA)) * LPR;
+        m[u] = FULL || i < n ? __ldcs(row + i) : U{};
     }
-    return (a0 + a1) + (a2 + a3);
+#pragma unroll
+    for (int u = 0; u < 2 * NA; ++u) {
+        const int i = base + (u % NA + 4 * (u / NA)) * LPR;
+        v[u] = FULL || i < n ? __ldg((i < split ? xa : xb) + i) : U{};
+    }
+#pragma unroll
+    for (int u = 0; u < 2 * NA; ++u) {
+        if (!FULL && first + (u % NA + 4 * (u / NA)) * LPR >= n) continue;
+        if constexpr (sizeof(U) == 16) {
+            a[u % NA] = fma(m[u].x, v[u].x, a[u % NA]);
+            a[u % NA] = fma(m[u].y, v[u].y, a[u % NA]);
+        } else {
+            a[u % NA] = fma(m[u], v[u], a[u % NA]);
+        }
+    }
+}
+
+// This lane's share of row[0:len) . x[0:len) (lane: within the group of F LPR), where x[i] = xa[i] for i < split and
+// xb[i - split] after (split even when VEC).  VEC: row, xa and xb 16-byte aligned and len even.
+template <bool VEC, int LPR, int F>
+__device__ __forceinline__ double group_dot(const double* __restrict__ row, const double* __restrict__ xa,
+                                             const double* __restrict__ xb, int split, int len, int lane) {
+    using U = std::conditional_t<VEC, double2, double>;
+    constexpr int NA = 4 / F, W = sizeof(U) / sizeof(double);
+    const U* r = reinterpret_cast<const U*>(row);
+    const U* ua = reinterpret_cast<const U*>(xa);
+    const U* ub = reinterpret_cast<const U*>(xb) - split / W;
+    const int n = len / W;
+    double a[NA];
+#pragma unroll
+    for (int k = 0; k < NA; ++k) a[k] = 0.0;
+    int at = 0;
+#pragma unroll F
+    for (; at + 8 * LPR <= n; at += 8 * LPR) group_turn<true, LPR, F>(r, ua, ub, split / W, n, at, lane, a);
+    if (at < n) group_turn<false, LPR, F>(r, ua, ub, split / W, n, at, lane, a);
+    return NA == 4 ? (a[0] + a[1]) + (a[NA - 2] + a[NA - 1]) : NA == 2 ? a[0] + a[NA - 1] : a[0];
 }
 
 // hDiff = h_upper - h_lower per interface point (HPSAlgorithm.hpp:1061-1081)
@@ -277,33 +273,33 @@ __global__ void k_hdiff(const MergeItem* __restrict__ items, int s) {
 }
 
 // Row handled by this thread's lane group; groups never leave early (full-warp shuffles).
-template <int LPR>
+template <int G>
 __device__ __forceinline__ long long group_row() {
-    return blockIdx.x * (long long)(kGemvThreads / LPR) + threadIdx.x / LPR;
+    return blockIdx.x * (long long)(kGemvThreads / G) + threadIdx.x / G;
 }
 
 // w = X^{-1} hDiff (the X^{-1} block of RHS, columns [8s, 12s))
-template <bool VEC, int LPR>
+template <bool VEC, int LPR, int F>
 __global__ void __launch_bounds__(kGemvThreads) k_gemv_w(const MergeItem* __restrict__ items, int s, long long nrows) {
     pdl_begin();
-    const int sl = threadIdx.x & (LPR - 1);
-    const long long g = group_row<LPR>();
+    const int sl = threadIdx.x & (F * LPR - 1);
+    const long long g = group_row<F * LPR>();
     const bool ok = g < nrows;
     const int m4 = 4 * s;
     const int item = ok ? int(g / m4) : 0, r = ok ? int(g - (long long)item * m4) : 0;
     const MergeItem& it = items[item];
-    const double part = ok ? group_dot<VEC, LPR>(it.RHS + (long long)r * (12LL * s) + 8 * s, it.hd, it.hd, m4, m4, sl) : 0.0;
-    const double acc = group_sum<LPR>(part);
+    const double part = ok ? group_dot<VEC, LPR, F>(it.RHS + (long long)r * (12LL * s) + 8 * s, it.hd, it.hd, m4, m4, sl) : 0.0;
+    const double acc = group_sum<LPR, F>(part);
     if (ok && sl == 0) it.w[r] = acc;
 }
 
 // h = H w + h_update (HPSAlgorithm.hpp:1098-1117), compact H rows already in WESN order; the
 // compact H row p is contiguous: its first s entries multiply w on interface Ia, the rest Ib
-template <bool VEC, int LPR>
+template <bool VEC, int LPR, int F>
 __global__ void __launch_bounds__(kGemvThreads) k_gemv_h(const MergeItem* __restrict__ items, int s, long long nrows) {
     pdl_begin();
-    const int sl = threadIdx.x & (LPR - 1);
-    const long long g = group_row<LPR>();
+    const int sl = threadIdx.x & (F * LPR - 1);
+    const long long g = group_row<F * LPR>();
     const bool ok = g < nrows;
     const int m8 = 8 * s;
     const int item = ok ? int(g / m8) : 0, p = ok ? int(g - (long long)item * m8) : 0;
@@ -311,14 +307,14 @@ __global__ void __launch_bounds__(kGemvThreads) k_gemv_h(const MergeItem* __rest
     int c, q, Ia, Ib;
     ext_map(p, s, c, q);
     child_ifaces(c, Ia, Ib);
-    const double part = ok ? group_dot<VEC, LPR>(it.H + (long long)p * (2LL * s), it.w + Ia * s, it.w + Ib * s, s, 2 * s, sl) : 0.0;
-    const double acc = group_sum<LPR>(part);
+    const double part = ok ? group_dot<VEC, LPR, F>(it.H + (long long)p * (2LL * s), it.w + Ia * s, it.w + Ib * s, s, 2 * s, sl) : 0.0;
+    const double acc = group_sum<LPR, F>(part);
     if (ok && sl == 0) it.h[p] = acc + it.hc[c][q];
 }
 
 // u_Gamma = S g + w (HPSAlgorithm.hpp:1197-1204) scattered to the children's interface data; the
 // leading threads also copy the exterior data of the children (HPSAlgorithm.hpp:1214-1227)
-template <bool VEC, int LPR>
+template <bool VEC, int LPR, int F>
 __global__ void __launch_bounds__(kGemvThreads) k_gemv_down(const MergeItem* __restrict__ items, int s,
                                                             long long nrows, int nitems, int add_w) {
     pdl_begin();
@@ -331,13 +327,13 @@ __global__ void __launch_bounds__(kGemvThreads) k_gemv_down(const MergeItem* __r
         ext_map(p, s, c, q);
         it.gc[c][q] = it.gf[p];
     }
-    const int sl = threadIdx.x & (LPR - 1);
-    const long long g = group_row<LPR>();
+    const int sl = threadIdx.x & (F * LPR - 1);
+    const long long g = group_row<F * LPR>();
     const bool ok = g < nrows;
     const int item = ok ? int(g / m4) : 0, r = ok ? int(g - (long long)item * m4) : 0;
     const MergeItem& it = items[item];
-    const double part = ok ? group_dot<VEC, LPR>(it.RHS + (long long)r * (12LL * s), it.gf, it.gf, m8, m8, sl) : 0.0;
-    const double acc = group_sum<LPR>(part);
+    const double part = ok ? group_dot<VEC, LPR, F>(it.RHS + (long long)r * (12LL * s), it.gf, it.gf, m8, m8, sl) : 0.0;
+    const double acc = group_sum<LPR, F>(part);
     if (ok && sl == 0) {
         const double u = add_w ? acc + it.w[r] : acc;
         const int I = r / s, o = r - I * s;
@@ -346,22 +342,60 @@ __global__ void __launch_bounds__(kGemvThreads) k_gemv_down(const MergeItem* __r
     }
 }
 
-// lanes per row for a row of `len` doubles: eight loads per lane where the row allows
+// lanes per row for a row of `len` doubles: sixteen units per lane where the row allows
 inline int pick_lpr(int len, bool vec) {
     const int units = vec ? len / 2 : len;
-    if (units >= 256) return 32;
-    if (units >= 128) return 16;
-    if (units >= 64) return 8;
-    return 4;
+    if (units >= 512) return 32;
+    if (units >= 256) return 16;
+    if (units >= 128) return 8;
+    if (units >= 64) return 4;
+    return 2;
 }
 
-#define EF_LPR_DISPATCH(KERNEL, VEC, LPR, GRID, ...)                                       \
-    do {                                                                                    \
-        if (LPR == 32) launch_chained(Chain::few, KERNEL<VEC, 32>, dim3(GRID), kGemvThreads, 0, st, __VA_ARGS__);         \
-        else if (LPR == 16) launch_chained(Chain::few, KERNEL<VEC, 16>, dim3(GRID), kGemvThreads, 0, st, __VA_ARGS__);    \
-        else if (LPR == 8) launch_chained(Chain::few, KERNEL<VEC, 8>, dim3(GRID), kGemvThreads, 0, st, __VA_ARGS__);      \
-        else launch_chained(Chain::few, KERNEL<VEC, 4>, dim3(GRID), kGemvThreads, 0, st, __VA_ARGS__);                    \
+// Real lanes per lane of the sum: four while the level keeps within the blocks that are chained to the launch before
+// or, where one lane is too many for that, a quarter of the SMs' threads; two up to half of them.
+// Levels 3 to 6 with 16 x 16 leaves, us, against one line at the chained blocks alone: 55 / 98 / 196 / 457 and
+// 59 / 119 / 211 / 455.
+inline int pick_share(long long rows, int lpr, bool vec) {
+    if (!vec || lpr == 32) return 1;
+    const long long threads = rows * lpr, chained = kChainedBlocks * (long long)kGemvThreads;
+    const long long four = threads <= chained ? chained : 152 * 512;
+    return threads * 4 <= four && lpr <= 8 ? 4 : threads * 2 <= 152 * 1024 ? 2 : 1;
+}
+
+#define EF_GEMV(KERNEL, VEC, LPR, F, NTHREADS, ...) \
+    launch_chained(Chain::few, KERNEL<VEC, LPR, F>, dim3(gemv_blocks(NTHREADS)), kGemvThreads, 0, st, __VA_ARGS__)
+// ROWS groups of F LPR lanes, at least LEAST threads
+#define EF_GEMV_DISPATCH(KERNEL, VEC, LPR, F, ROWS, LEAST, ...)                                                 \
+    do {                                                                                                        \
+        const long long nt_ = std::max<long long>((ROWS) * (LPR) * (F), (LEAST));                               \
+        if (!(VEC)) {                                                                                           \
+            if (LPR == 32) EF_GEMV(KERNEL, false, 32, 1, nt_, __VA_ARGS__);                                     \
+            else if (LPR == 16) EF_GEMV(KERNEL, false, 16, 1, nt_, __VA_ARGS__);                                \
+            else if (LPR == 8) EF_GEMV(KERNEL, false, 8, 1, nt_, __VA_ARGS__);                                  \
+            else if (LPR == 4) EF_GEMV(KERNEL, false, 4, 1, nt_, __VA_ARGS__);                                  \
+            else EF_GEMV(KERNEL, false, 2, 1, nt_, __VA_ARGS__);                                                \
+        } else if (F == 1) {                                                                                    \
+            if (LPR == 32) EF_GEMV(KERNEL, true, 32, 1, nt_, __VA_ARGS__);                                      \
+            else if (LPR == 16) EF_GEMV(KERNEL, true, 16, 1, nt_, __VA_ARGS__);                                 \
+            else if (LPR == 8) EF_GEMV(KERNEL, true, 8, 1, nt_, __VA_ARGS__);                                   \
+            else if (LPR == 4) EF_GEMV(KERNEL, true, 4, 1, nt_, __VA_ARGS__);                                   \
+            else EF_GEMV(KERNEL, true, 2, 1, nt_, __VA_ARGS__);                                                 \
+        } else if (F == 2) {                                                                                    \
+            if (LPR == 16) EF_GEMV(KERNEL, true, 16, 2, nt_, __VA_ARGS__);                                      \
+            else if (LPR == 8) EF_GEMV(KERNEL, true, 8, 2, nt_, __VA_ARGS__);                                   \
+            else if (LPR == 4) EF_GEMV(KERNEL, true, 4, 2, nt_, __VA_ARGS__);                                   \
+            else EF_GEMV(KERNEL, true, 2, 2, nt_, __VA_ARGS__);                                                 \
+        } else {                                                                                                \
+            if (LPR == 8) EF_GEMV(KERNEL, true, 8, 4, nt_, __VA_ARGS__);                                   \
+            else if (LPR == 4) EF_GEMV(KERNEL, true, 4, 4, nt_, __VA_ARGS__);                                   \
+            else EF_GEMV(KERNEL, true, 2, 4, nt_, __VA_ARGS__);                                                 \
+        }                                                                                                       \
     } while (0)
+
+inline unsigned gemv_blocks(long long threads) {
+    return unsigned(std::max(1LL, (threads + kGemvThreads - 1) / kGemvThreads));
+}
 
 __global__ void k_root_diag(int m, const double* a, const double* b, const double* r,
                             const double* h, double* g) {
@@ -398,9 +432,9 @@ __global__ void __launch_bounds__(256) k_root_gemv(int m, const double* __restri
                                                    double* out) {
     const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (r >= m) return;  // whole warp
-    double acc = (m & 1) == 0 ? group_dot<true, 32>(M + (long long)r * m, x, x, m, m, lane)
-                              : group_dot<false, 32>(M + (long long)r * m, x, x, m, m, lane);
-    acc = group_sum<32>(acc);
+    double acc = (m & 1) == 0 ? group_dot<true, 32, 1>(M + (long long)r * m, x, x, m, m, lane)
+                              : group_dot<false, 32, 1>(M + (long long)r * m, x, x, m, m, lane);
+    acc = group_sum<32, 1>(acc);
     if (lane == 0) out[r] = rhs ? rhs[r] - fma(b[r], acc, a[r] * x[r]) : add ? out[r] + acc : acc;
 }
 
@@ -419,8 +453,8 @@ __global__ void __launch_bounds__(256) k_root_check(int m, const double* __restr
         acc += p;
         mag += fabs(p);
     }
-    acc = group_sum<32>(acc);
-    mag = group_sum<32>(mag);
+    acc = group_sum<32, 1>(acc);
+    mag = group_sum<32, 1>(mag);
     if (lane == 0) {
         const double ay = a[r] * y[r], res = root_check_entry(r) - fma(b[r], acc, ay);
         if (!(fabs(res) <= 1e-12 * (1.0 + fabs(ay) + fabs(b[r]) * mag))) *info = 1;
@@ -565,25 +599,19 @@ void upward_hdiff(cudaStream_t st, const MergeItem* items, int nitems, int s) {
     ++g_kernel_launches;
 }
 
-inline unsigned gemv_blocks(long long threads) {
-    return unsigned(std::max(1LL, (threads + kGemvThreads - 1) / kGemvThreads));
-}
-
 void upward_w(cudaStream_t st, const MergeItem* items, int nitems, int s) {
     const long long rows = (long long)nitems * 4 * s;
     const bool vec = (s % 2 == 0);
-    const int lpr = pick_lpr(4 * s, vec);
-    if (vec) EF_LPR_DISPATCH(k_gemv_w, true, lpr, gemv_blocks(rows * lpr), items, s, rows);
-    else EF_LPR_DISPATCH(k_gemv_w, false, lpr, gemv_blocks(rows * lpr), items, s, rows);
+    const int lpr = pick_lpr(4 * s, vec), f = pick_share(rows, lpr, vec);
+    EF_GEMV_DISPATCH(k_gemv_w, vec, lpr, f, rows, 0, items, s, rows);
     ++g_kernel_launches;
 }
 
 void upward_h(cudaStream_t st, const MergeItem* items, int nitems, int s) {
     const long long rows = (long long)nitems * 8 * s;
     const bool vec = (s % 2 == 0);
-    const int lpr = pick_lpr(2 * s, vec);
-    if (vec) EF_LPR_DISPATCH(k_gemv_h, true, lpr, gemv_blocks(rows * lpr), items, s, rows);
-    else EF_LPR_DISPATCH(k_gemv_h, false, lpr, gemv_blocks(rows * lpr), items, s, rows);
+    const int lpr = pick_lpr(2 * s, vec), f = pick_share(rows, lpr, vec);
+    EF_GEMV_DISPATCH(k_gemv_h, vec, lpr, f, rows, 0, items, s, rows);
     ++g_kernel_launches;
 }
 
@@ -591,10 +619,8 @@ void upward_h(cudaStream_t st, const MergeItem* items, int nitems, int s) {
 void downward(cudaStream_t st, const MergeItem* items, int nitems, int s, int add_w) {
     const long long rows = (long long)nitems * 4 * s;
     const bool vec = (s % 2 == 0);
-    const int lpr = pick_lpr(8 * s, vec);
-    const unsigned nb = gemv_blocks(std::max(rows * lpr, (long long)nitems * 8 * s));
-    if (vec) EF_LPR_DISPATCH(k_gemv_down, true, lpr, nb, items, s, rows, nitems, add_w);
-    else EF_LPR_DISPATCH(k_gemv_down, false, lpr, nb, items, s, rows, nitems, add_w);
+    const int lpr = pick_lpr(8 * s, vec), f = pick_share(rows, lpr, vec);
+    EF_GEMV_DISPATCH(k_gemv_down, vec, lpr, f, rows, (long long)nitems * 8 * s, items, s, rows, nitems, add_w);
     ++g_kernel_launches;
 }
 
