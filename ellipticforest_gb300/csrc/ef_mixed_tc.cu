@@ -362,8 +362,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         const unsigned long long pol = tmap ? l2_evict_normal() : l2_evict_first();
         int cur_tile = -1;
         long long cur_blk = 0;
-        auto copy = [&](int g) {
-            const int u = g / cpu, c = g - u * cpu, tl = tile_of(u), sl = g % NS;
+        auto copy = [&](int g, int sl) {  // chunk g into stage sl = g mod NS
+            const int u = g / cpu, c = g - u * cpu, tl = tile_of(u);
             if (tl != cur_tile) {
                 cur_tile = tl;
                 cur_blk = (long long)(tmap ? __ldg(tmap + tl) : tl) * nkc + cbase;
@@ -378,41 +378,49 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         };
         bool ok = true;
         int issued = 0;
-        for (; issued < NS && issued < total; ++issued) copy(issued);
+        for (; issued < NS && issued < total; ++issued) copy(issued, issued);
         if (g_mx_inject_timeout && nunits > 0) ok = __all_sync(0xffffffffu, tc_wait(never, 0u, abort_flag, 1000000LL));
         const uint64_t d0 = tc_desc(smem_u32(base));
-        for (int gch = 0; gch < total && ok; ++gch) {
-            const int c = gch % cpu, bf = gch % NP, st = gch % NS;
-            const unsigned ph = unsigned(gch / NS) & 1u;
-            // the chunk's accumulator set was drained NP chunks ago
-            if (gch >= NP) ok = tc_wait(&acc_empty[bf], unsigned(gch / NP - 1) & 1u, abort_flag);
-            if (ok) ok = tc_wait(&a_full[st], ph, abort_flag) && tc_wait(&x_full[st], ph, abort_flag);
-            if (!(ok = __all_sync(0xffffffffu, ok))) break;
-            tc_fence_after();
-            const uint64_t da = d0 + uint64_t(unsigned(st) * (unsigned(SB) >> 4));
-            const uint64_t dx = da + uint64_t(3 * kPlaneA >> 4);
-            const unsigned dhi = tmem + unsigned(bf * 3 * ncol), dlo = dhi + unsigned(ncol);
-            const int kleft = K - (cbase + c) * kTK;
-            const int nk = kleft >= kTK ? kTK / 16 : (kleft + 15) / 16;
-            if (elect_one()) {
+        // the stages are unrolled, so that an operand's descriptor is the shared base plus a constant: computed per
+        // stage, the descriptors alone took as long as the MMAs
+        int c = 0, bf = 0, bf_turn = 0;
+        for (int g0 = 0, turn = 0; g0 < total && ok; g0 += NS, ++turn) {
 #pragma unroll
-                for (int kk = 0; kk < kTK / 16; ++kk) {
-                    if (kk < nk) {
-                        const uint64_t ko = uint64_t(2 * kk), x123 = dx + ko;
-                        // the three X planes are consecutive rows of one K-major operand: [x1 | x2 | x3]
-                        tc_mma(dhi, da + ko, x123, idesc3, kk > 0 ? 1u : 0u);  // D_hi = a1 x1, D_lo_a = a1 x2, D_lo_b = a1 x3
-                        tc_mma(dlo, da + uint64_t(kPlaneA >> 4) + ko, x123, idesc2, 1u);      // D_lo_a += a2 x1, D_lo_b += a2 x2
-                        tc_mma(dlo, da + uint64_t(2 * kPlaneA >> 4) + ko, x123, idesc1, 1u);  // D_lo_a += a3 x1
+            for (int st = 0; st < NS; ++st) {
+                const int gch = g0 + st;
+                if (gch >= total || !ok) break;
+                // the chunk's accumulator set was drained NP chunks ago
+                if (bf_turn > 0) ok = tc_wait(&acc_empty[bf], unsigned(bf_turn - 1) & 1u, abort_flag);
+                if (ok) ok = tc_wait(&a_full[st], unsigned(turn) & 1u, abort_flag) && tc_wait(&x_full[st], unsigned(turn) & 1u, abort_flag);
+                if (!(ok = __all_sync(0xffffffffu, ok))) break;
+                tc_fence_after();
+                const uint64_t da = d0 + uint64_t(unsigned(st) * (unsigned(SB) >> 4));
+                const uint64_t dx = da + uint64_t(3 * kPlaneA >> 4);
+                const unsigned dhi = tmem + unsigned(bf * 3 * ncol), dlo = dhi + unsigned(ncol);
+                const int kleft = K - (cbase + c) * kTK;
+                const int nk = kleft >= kTK ? kTK / 16 : (kleft + 15) / 16;
+                if (elect_one()) {
+#pragma unroll
+                    for (int kk = 0; kk < kTK / 16; ++kk) {
+                        if (kk < nk) {
+                            const uint64_t ko = uint64_t(2 * kk), x123 = dx + ko;
+                            // the three X planes are consecutive rows of one K-major operand: [x1 | x2 | x3]
+                            tc_mma(dhi, da + ko, x123, idesc3, kk > 0 ? 1u : 0u);  // D_hi = a1 x1, D_lo_a = a1 x2, D_lo_b = a1 x3
+                            tc_mma(dlo, da + uint64_t(kPlaneA >> 4) + ko, x123, idesc2, 1u);      // D_lo_a += a2 x1, D_lo_b += a2 x2
+                            tc_mma(dlo, da + uint64_t(2 * kPlaneA >> 4) + ko, x123, idesc1, 1u);  // D_lo_a += a3 x1
+                        }
                     }
+                    tc_commit(&empty[st]);
+                    tc_commit(&acc_full[bf]);
                 }
-                tc_commit(&empty[st]);
-                tc_commit(&acc_full[bf]);
-            }
-            __syncwarp();
-            // refill the stage of the chunk before, whose MMAs complete while this chunk's run
-            if (gch > 0 && issued < total) {
-                ok = __all_sync(0xffffffffu, tc_wait(&empty[(gch - 1) % NS], unsigned((gch - 1) / NS) & 1u, abort_flag));
-                if (ok) copy(issued++);
+                __syncwarp();
+                if (++c == cpu) c = 0;
+                if (++bf == NP) { bf = 0; ++bf_turn; }
+                // refill the stage of the chunk before, whose MMAs complete while this chunk's run
+                if (gch > 0 && issued < total) {
+                    ok = __all_sync(0xffffffffu, tc_wait(&empty[(st + NS - 1) % NS], unsigned(st > 0 ? turn : turn - 1) & 1u, abort_flag));
+                    if (ok) copy(issued++, (st + NS - 1) % NS);
+                }
             }
         }
         if (!ok) {
