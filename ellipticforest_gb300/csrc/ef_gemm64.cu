@@ -35,15 +35,17 @@ constexpr int kDigits = 8;
 constexpr int kMT = 128, kNT = 32, kKB = 64;             // tile rows, tile columns, k per block
 constexpr int kPlane = kMT * kKB * 2;                    // one digit of an A block: 16 KB
 constexpr int kBBlock = kDigits * kNT * kKB * 2;         // all digits of a B block: 32 KB
-constexpr int kASlots = 6, kBSlots = 2, kSets = 2;       // rings: A digits, B blocks, accumulator sets
+constexpr int kASlots = kDigits, kBSlots = 2, kSets = 2; // rings: A digits, B blocks, accumulator sets
 constexpr int kFlush = 2;                                // k blocks per accumulator set (128 values of k)
 constexpr int kNotFinite = 1 << 20;                      // exponent of a row that holds an infinity or NaN
 constexpr int kCollect = 256, kGemmThreads = kCollect + 64;  // collecting threads, then the copy and MMA warps
 constexpr int kHalf = kNT / 2;                           // columns per collecting thread
 constexpr int kMaxOps = 8, kMaxGemms = 4;
 enum Add : int { ADD_NONE = 0, ADD_D = 1, ADD_IDENTITY = 2 };
-constexpr int kSums = kMT * kNT * 16;                    // a tile's integer sums on their way to rows of C
+constexpr int kPass = kHalf / 2;                         // of them, columns per pass of the write-out
+constexpr int kSums = kCollect * kPass * 16;             // a pass's integer sums on their way to rows of C
 constexpr size_t kSmem = 1024 + size_t(kASlots) * kPlane + size_t(kBSlots) * kBBlock + kSums + 512;
+static_assert(kBSlots == 2 && kFlush == 2, "a digit's slot is full in even blocks with parity 0, in odd ones with 1");
 static_assert(kSmem <= 227 * 1024, "shared memory of one CTA");
 static_assert(2 * kSmem > 228 * 1024, "one CTA per SM: each takes all of TMEM");
 
@@ -273,7 +275,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm64(const __grid_constan
     unsigned char* base = g_smem + ((1024u - (smem_u32(g_smem) & 1023u)) & 1023u);
     unsigned char* bbase = base + size_t(kASlots) * kPlane;
     int4* sums = reinterpret_cast<int4*>(bbase + size_t(kBSlots) * kBBlock);
-    unsigned long long* bars = reinterpret_cast<unsigned long long*>(sums + kMT * kNT);
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(sums + kCollect * kPass);
     unsigned long long *a_full = bars, *a_empty = a_full + kASlots, *b_full = a_empty + kASlots,
                        *b_empty = b_full + kBSlots, *acc_full = b_empty + kBSlots, *acc_empty = acc_full + kSets,
                        *drain = acc_empty + kSets;
@@ -347,40 +349,50 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm64(const __grid_constan
             atomicExch(err, 1);
         }
     } else if (warp == 9) {
-        unsigned sa = 0, sb = 0, pa = 0, pb = 0, ns = 0;
+        unsigned ns = 0;
         bool ok = true;
-        // operand descriptors differ in their address field only
+        // Operand descriptors differ in their address field only, by constants: a digit's slot is its number, and
+        // the loop over the k blocks is unrolled over the B slots (an FP64 build of a 7-level tree of 16 x 16
+        // leaves: 28.6 ms with slots taken round robin, 27.5 now; an MMA took 96 clocks on average against 72 of
+        // the tensor cores).
         const uint64_t da0 = tc_desc(smem_u32(base)), db0 = tc_desc(smem_u32(bbase));
-        for (int t = blockIdx.x; t < L.tiles && ok; t += gridDim.x) {
-            const int nkb = (L.op[tile_at(L, t).o].K + kKB - 1) / kKB;
-            for (int kb = 0; kb < nkb && ok; ++kb) {
+        int t = blockIdx.x, kb = 0, nkb = t < L.tiles ? (L.op[tile_at(L, t).o].K + kKB - 1) / kKB : 0;
+        for (unsigned turn = 0; t < L.tiles && ok; ++turn) {
+#pragma unroll
+            for (int sb = 0; sb < kBSlots; ++sb) {
+                if (t >= L.tiles || !ok) break;
                 const unsigned set = ns % kSets;
-                if (kb % kFlush == 0 && ns >= kSets) ok = tc_wait(acc_empty + set, (ns / kSets - 1) & 1u, abort_flag);
-                if (ok) ok = tc_wait(b_full + sb, pb, abort_flag);
+                const bool fresh = kb % kFlush == 0, last = kb == nkb - 1;
+                if (fresh && ns >= kSets) ok = tc_wait(acc_empty + set, (ns / kSets - 1) & 1u, abort_flag);
+                if (ok) ok = tc_wait(b_full + sb, turn & 1u, abort_flag);
                 const uint64_t db = db0 + uint64_t(sb * (kBBlock >> 4));
                 const unsigned d = tmem + set * 256u;
 #pragma unroll
                 for (int i = 0; i < kDigits; ++i) {
-                    if (ok) ok = tc_wait(a_full + sa, pa, abort_flag);
+                    if (ok) ok = tc_wait(a_full + i, unsigned(sb & 1), abort_flag);
                     if (!(ok = __all_sync(0xffffffffu, ok))) break;
                     tc_fence_after();
-                    const uint64_t da = da0 + uint64_t(sa * (kPlane >> 4));
+                    const uint64_t da = da0 + uint64_t(i * (kPlane >> 4));
                     if (elect_one()) {
 #pragma unroll
                         for (int kk = 0; kk < kKB / 16; ++kk)
                             tc_mma(d + unsigned(i * kNT), da + uint64_t(2 * kk), db + uint64_t(2 * kk),
-                                   tc_idesc(kMT, kNT * (kDigits - i)), kb % kFlush == 0 && i == 0 && kk == 0 ? 0u : 1u);
-                        tc_commit(a_empty + sa);
+                                   tc_idesc(kMT, kNT * (kDigits - i)), i == 0 && kk == 0 ? (fresh ? 0u : 1u) : 1u);
+                        tc_commit(a_empty + i);
                         if (i == kDigits - 1) {
                             tc_commit(b_empty + sb);
-                            if (kb % kFlush == kFlush - 1 || kb == nkb - 1) tc_commit(acc_full + set);
+                            if (!fresh || last) tc_commit(acc_full + set);
                         }
                     }
                     __syncwarp();
-                    if (++sa == kASlots) { sa = 0; pa ^= 1u; }
                 }
-                if (++sb == kBSlots) { sb = 0; pb ^= 1u; }
-                if (kb % kFlush == kFlush - 1 || kb == nkb - 1) ++ns;
+                if (!fresh || last) ++ns;
+                ++kb;
+                if (last) {
+                    t += gridDim.x;
+                    kb = 0;
+                    if (t < L.tiles) nkb = (L.op[tile_at(L, t).o].K + kKB - 1) / kKB;
+                }
             }
         }
         // every MMA issued has completed before TMEM is freed
@@ -393,7 +405,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm64(const __grid_constan
         // warps w and w + 4 hold the same 32 rows (TMEM lanes 32 (w mod 4) ..), columns 0-15 and 16-31
         const int wr = warp & 3, c0 = warp < 4 ? 0 : kHalf;
         const unsigned acc0 = tmem + (unsigned(wr * 32) << 16) + unsigned(c0);
-        int4* own = sums + (warp * 32) * kHalf;
+        int4* own = sums + (warp * 32) * kPass;
         unsigned ns = 0;
         bool ok = true;
         for (int t = blockIdx.x; t < L.tiles && ok; t += gridDim.x) {
@@ -428,66 +440,71 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm64(const __grid_constan
                 mbar_arrive(acc_empty + set);
             }
             if (!ok) break;
-            // the sums change hands inside the warp, so that lanes take consecutive columns of two rows: this
-            // thread's row goes to shared memory with its 16-byte entries swizzled by the row
-#pragma unroll
-            for (int c = 0; c < kHalf; ++c) {
-                const long long h = hi[c] + (lo[c] >> 32);  // the carry of lo first
-                own[lane * kHalf + (c ^ (lane & 15))] = make_int4(int(h), int(h >> 32), int(lo[c]), 0);
-            }
-            __syncwarp();
-            const int row0 = at.m * kMT + 32 * wr, n = at.n * kNT + c0 + (lane & 15), odd_row = lane >> 4;
-            const bool col = n < g.N;
+            // the sums change hands inside the warp, eight columns at a time, so that lanes take consecutive columns
+            // of four rows: this thread's row goes to shared memory with its 16-byte entries swizzled by the row
+            const int row0 = at.m * kMT + 32 * wr, quad = lane >> 3;
             const int ea = g.ea[(long long)at.b * g.eastride + min(row0 + lane, g.M - 1)];
-            const int eb = g.eb[(long long)at.b * g.ebstride + min(n, g.N - 1)];
             const int add = g.add, crs = g.c.rs, drs = g.d.rs, rows = min(32, g.M - row0);
             const long long cld = g.c.ld, cdr = g.c.dr, dld = g.d.ld, ddr = g.d.dr;
             const unsigned flip = g.neg ? 0x80000000u : 0u;
-            double* C = table_ptr(g.c.base, at.b) + g.c.off + n + (n >= g.c.ks ? g.c.dk : 0);
-            double v[16], old[16];
-            if (add == ADD_D) {
-                const double* D = table_ptr(g.d.base, at.b) + g.d.off + n + (n >= g.d.ks ? g.d.dk : 0);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const int i = 2 * j + odd_row, r = row0 + i;
-                    old[j] = col && i < rows ? D[r * dld + (r >= drs ? ddr : 0)] : 0.0;
+            for (int ps = 0; ps < kHalf / kPass; ++ps) {
+#pragma unroll
+                for (int k = 0; k < kPass; ++k) {
+                    const int c = ps * kPass + k;
+                    const long long h = hi[c] + (lo[c] >> 32);  // the carry of lo first
+                    own[lane * kPass + (k ^ (lane & 7))] = make_int4(int(h), int(h >> 32), int(lo[c]), 0);
                 }
-            } else {
+                __syncwarp();
+                const int n = at.n * kNT + c0 + ps * kPass + (lane & 7);
+                const bool col = n < g.N;
+                const int eb = g.eb[(long long)at.b * g.ebstride + min(n, g.N - 1)];
+                double* C = table_ptr(g.c.base, at.b) + g.c.off + n + (n >= g.c.ks ? g.c.dk : 0);
+                double v[8], old[8];
+                if (add == ADD_D) {
+                    const double* D = table_ptr(g.d.base, at.b) + g.d.off + n + (n >= g.d.ks ? g.d.dk : 0);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) old[j] = n == row0 + 2 * j + odd_row ? 1.0 : 0.0;
-            }
-            // all sixteen conversions before any branch: a branch per entry would run them one after another
-            unsigned odd = 0;
+                    for (int j = 0; j < 8; ++j) {
+                        const int i = 4 * j + quad, r = row0 + i;
+                        old[j] = col && i < rows ? D[r * dld + (r >= drs ? ddr : 0)] : 0.0;
+                    }
+                } else {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const int i = 2 * j + odd_row;
-                const int4 q = own[i * kHalf + ((lane & 15) ^ (i & 15))];
-                const int e1 = __shfl_sync(0xffffffffu, ea, i);
-                bool o;
-                v[j] = fixed_to_double(join(q), unsigned(q.z), e1 + eb - 36, o);  // (h + f 2^-32) 2^(e1 + eb - 36)
-                odd |= o || e1 >= kNotFinite || eb >= kNotFinite ? 1u << j : 0u;
-            }
-            if (__any_sync(0xffffffffu, odd != 0)) {
+                    for (int j = 0; j < 8; ++j) old[j] = n == row0 + 4 * j + quad ? 1.0 : 0.0;
+                }
+                // all conversions before any branch: a branch per entry would run them one after another
+                unsigned odd = 0;
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const int i = 2 * j + odd_row;
-                    const int4 q = own[i * kHalf + ((lane & 15) ^ (i & 15))];
+                for (int j = 0; j < 8; ++j) {
+                    const int i = 4 * j + quad;
+                    const int4 q = own[i * kPass + ((lane & 7) ^ (i & 7))];
                     const int e1 = __shfl_sync(0xffffffffu, ea, i);
-                    if ((odd >> j) & 1u) v[j] = fixed_to_double_any(join(q), unsigned(q.z), e1, eb);
+                    bool o;
+                    v[j] = fixed_to_double(join(q), unsigned(q.z), e1 + eb - 36, o);  // (h + f 2^-32) 2^(e1 + eb - 36)
+                    odd |= o || e1 >= kNotFinite || eb >= kNotFinite ? 1u << j : 0u;
                 }
-            }
+                if (__any_sync(0xffffffffu, odd != 0)) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = __hiloint2double(int(unsigned(__double2hiint(v[j])) ^ flip), __double2loint(v[j]));
-            if (add) {
+                    for (int j = 0; j < 8; ++j) {
+                        const int i = 4 * j + quad;
+                        const int4 q = own[i * kPass + ((lane & 7) ^ (i & 7))];
+                        const int e1 = __shfl_sync(0xffffffffu, ea, i);
+                        if ((odd >> j) & 1u) v[j] = fixed_to_double_any(join(q), unsigned(q.z), e1, eb);
+                    }
+                }
 #pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] = old[j] + v[j];
-            }
+                for (int j = 0; j < 8; ++j) v[j] = __hiloint2double(int(unsigned(__double2hiint(v[j])) ^ flip), __double2loint(v[j]));
+                if (add) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const int i = 2 * j + odd_row, r = row0 + i;
-                if (col && i < rows) C[r * cld + (r >= crs ? cdr : 0)] = v[j];
+                    for (int j = 0; j < 8; ++j) v[j] = old[j] + v[j];
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int i = 4 * j + quad, r = row0 + i;
+                    if (col && i < rows) C[r * cld + (r >= crs ? cdr : 0)] = v[j];
+                }
+                __syncwarp();
             }
-            __syncwarp();
         }
         if (!ok) atomicExch(err, 1);
     }
