@@ -594,11 +594,24 @@ __global__ void __launch_bounds__(64) k_inv_small(const __grid_constant__ InvLis
     if (tid == 0 && bad) info[blockIdx.y] = 1;
 }
 
-// x 2^k for a finite x, by the exponent bits (zero where the result would be below the smallest normal number)
-__device__ __forceinline__ double shift_exponent(double x, int k) {
-    const int hi = __double2hiint(x), e = (hi >> 20) & 0x7ff;
-    if (e == 0 || e + k < 1) return 0.0;
-    return __hiloint2double(e + k > 2046 ? (hi & int(0x80000000u)) | 0x7fe00000 : hi + (k << 20), __double2loint(x));
+// x 2^-e rounded to nearest, for |x| < 2^e (zero where it would be subnormal; NaN where asked)
+__device__ __forceinline__ float scaled_float(double x, int e, bool nan) {
+    const int hi = __double2hiint(x);
+    const unsigned lo = unsigned(__double2loint(x));
+    const int top = (hi & 0x7fffffff) - ((e + 896) << 20);  // float exponent and leading 20 bits of the significand
+    const unsigned bits = ((unsigned(top) << 3) | (lo >> 29)) + ((lo >> 28) & 1u);
+    return __uint_as_float(nan ? 0x7fc00000u : (unsigned(hi) & 0x80000000u) | (top < (1 << 20) ? 0u : bits));
+}
+
+// x 2^-e (zero below the smallest normal number, the largest power of two above the range; PLAIN: |e| is at most
+// 800, so that neither happens to a normal x)
+template <bool PLAIN>
+__device__ __forceinline__ double scaled_double(float x, int e) {
+    const unsigned b = __float_as_uint(x), u = b & 0x7fffffffu;
+    const int ex = int(u >> 23) + 896 - e;
+    const bool zero = u < 0x00800000u || (!PLAIN && ex < 1), large = !PLAIN && ex > 2046;
+    const unsigned hi = zero ? 0u : large ? 0x7fe00000u : (u >> 3) + (unsigned(896 - e) << 20);
+    return __hiloint2double(int((b & 0x80000000u) | hi), zero || large ? 0 : int(u << 29));
 }
 
 constexpr int kStartLd = 132;
@@ -614,10 +627,11 @@ __device__ __forceinline__ void fma2(float& x, float& y, float a, float p, float
 
 // FP32 inverse of one matrix of at most 128 rows per block: the start of the iteration of `invert`.  Gauss-Jordan
 // in steps of 32 rows: one warp inverts the diagonal block in registers (a row per lane, pivots inside the
-// block, rows exchanged by shuffles), the block's row panel is multiplied by it, and all 256 threads update
-// their 8 x 8 entries with 32 columns at once.  Rows are brought to magnitudes below one by powers of two
-// first, so any scaling of the rows is harmless.  Column by column over the whole matrix (two block barriers
-// and ~1000 clocks per column) it took 76 us for 128 rows.
+// block, the pivot row through shared memory), the block's row panel is multiplied by it, and all 256 threads
+// update their 8 x 8 entries with 32 columns at once.  Rows are brought to magnitudes below one by powers of two
+// first, so any scaling of the rows is harmless.  One block, so it is a chain of latencies: of 97,000 clocks for
+// 128 rows (51 us; 61 us with a branch per converted entry), the diagonal blocks take 42,000 (320 per pivot, by
+// shuffles as much), the updates 23,000 (16,400 of FP32 multiply-adds), the rest is loads, panels and stores.
 __global__ void __launch_bounds__(256) k_inv_start(const __grid_constant__ InvList L, int n, int* __restrict__ info) {
     pdl_begin();
     constexpr int PB = 32, LD = kStartLd;  // panel width; row stride (16-byte rows, no bank conflicts)
@@ -631,26 +645,36 @@ __global__ void __launch_bounds__(256) k_inv_start(const __grid_constant__ InvLi
     float (*s_row)[LD] = reinterpret_cast<float (*)[LD]>(is_smem + 128 * LD);  // row panel, then times the inverse block
     float (*s_colT)[LD] = reinterpret_cast<float (*)[LD]>(is_smem + 160 * LD); // column panel, transposed
     __shared__ __align__(16) float s_inv[PB][PB + 4];
+    __shared__ __align__(16) float s_piv[2][PB + 4];
     __shared__ int s_e[128];
     // rows and columns of a thread: 4 t .. 4 t + 3 and 64 more, so that 16-byte reads of a row or column by the
     // 16 threads of a direction touch every bank once
     // (the loops over rows and steps stay rolled: the block runs each a few times at most, and fetching
     // straight-line code would take longer than running it)
-#pragma unroll 4
-    for (int r = warp; r < 128; r += 8) {
-        double x[4];
-        unsigned m = 0;
+    // (eight rows of a warp in flight; the conversions are integer steps without a branch: one per entry would
+    // run them one after another)
+#pragma unroll 1
+    for (int r0 = warp; r0 < 128; r0 += 64) {
+        double x[8][4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int c = lane + 32 * q;
-            x[q] = r < n && c < n ? A[(long long)r * V.ld + c] : (r == c ? 1.0 : 0.0);
-            m = max(m, unsigned(__double2hiint(x[q])) & 0x7fffffffu);
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int r = r0 + 8 * i, c = lane + 32 * q;
+                x[i][q] = r < n && c < n ? A[(long long)r * V.ld + c] : (r == c ? 1.0 : 0.0);
+            }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int r = r0 + 8 * i;
+            unsigned m = 0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) m = max(m, unsigned(__double2hiint(x[i][q])) & 0x7fffffffu);
+            m = __reduce_max_sync(0xffffffffu, m);
+            const int e = max(int(m >> 20), 1) - 1022;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) s_all[r][lane + 32 * q] = scaled_float(x[i][q], e, m >= 0x7ff00000u);
+            if (lane == 0) s_e[r] = e;
         }
-        m = __reduce_max_sync(0xffffffffu, m);
-        const int e = max(int(m >> 20), 1) - 1022;  // a row that is not finite keeps its infinities and NaNs
-#pragma unroll
-        for (int q = 0; q < 4; ++q) s_all[r][lane + 32 * q] = d2f_rn_bits(m < 0x7ff00000u ? shift_exponent(x[q], -e) : x[q]);
-        if (lane == 0) s_e[r] = e;
     }
     __syncthreads();
     float a[8][8];
@@ -667,15 +691,23 @@ __global__ void __launch_bounds__(256) k_inv_start(const __grid_constant__ InvLi
         // rows (columns) k0 .. k0 + 31 are entries 4 .. 7 or 0 .. 3 of the threads of eight rows (columns)
         const int t0 = (k0 & 63) >> 2, hi = k0 >= 64 ? 4 : 0;
         const bool mine_r = ty >= t0 && ty < t0 + 8, mine_c = tx >= t0 && tx < t0 + 8;
+        // published: the rows R with the identity for the block itself, the columns as -C with the identity in the
+        // block's rows (A <- A - C R then turns them into R), the block
         if (mine_r) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int r = 4 * (ty - t0) + i;
 #pragma unroll
-                for (int j = 0; j < 8; j += 4)
-                    *reinterpret_cast<float4*>(&s_row[r][4 * tx + 16 * j]) =
-                        hi ? make_float4(a[i + 4][j], a[i + 4][j + 1], a[i + 4][j + 2], a[i + 4][j + 3])
-                           : make_float4(a[i][j], a[i][j + 1], a[i][j + 2], a[i][j + 3]);
+                for (int j = 0; j < 8; j += 4) {
+                    float4 v = hi ? make_float4(a[i + 4][j], a[i + 4][j + 1], a[i + 4][j + 2], a[i + 4][j + 3])
+                                  : make_float4(a[i][j], a[i][j + 1], a[i][j + 2], a[i][j + 3]);
+                    if (mine_c && j == hi) {
+                        const int c = 4 * (tx - t0);
+                        *reinterpret_cast<float4*>(&s_inv[r][c]) = v;
+                        v = make_float4(r == c, r == c + 1, r == c + 2, r == c + 3);
+                    }
+                    *reinterpret_cast<float4*>(&s_row[r][4 * tx + 16 * j]) = v;
+                }
             }
         }
         if (mine_c) {
@@ -683,10 +715,15 @@ __global__ void __launch_bounds__(256) k_inv_start(const __grid_constant__ InvLi
             for (int j = 0; j < 4; ++j) {
                 const int c = 4 * (tx - t0) + j;
 #pragma unroll
-                for (int i = 0; i < 8; i += 4)
-                    *reinterpret_cast<float4*>(&s_colT[c][4 * ty + 16 * i]) =
-                        hi ? make_float4(a[i][j + 4], a[i + 1][j + 4], a[i + 2][j + 4], a[i + 3][j + 4])
-                           : make_float4(a[i][j], a[i + 1][j], a[i + 2][j], a[i + 3][j]);
+                for (int i = 0; i < 8; i += 4) {
+                    float4 v = hi ? make_float4(-a[i][j + 4], -a[i + 1][j + 4], -a[i + 2][j + 4], -a[i + 3][j + 4])
+                                  : make_float4(-a[i][j], -a[i + 1][j], -a[i + 2][j], -a[i + 3][j]);
+                    if (mine_r && i == hi) {
+                        const int r = 4 * (ty - t0);
+                        v = make_float4(r == c, r + 1 == c, r + 2 == c, r + 3 == c);
+                    }
+                    *reinterpret_cast<float4*>(&s_colT[c][4 * ty + 16 * i]) = v;
+                }
             }
         }
         __syncthreads();
@@ -695,27 +732,68 @@ __global__ void __launch_bounds__(256) k_inv_start(const __grid_constant__ InvLi
             // rows not used yet (leading 26 bits, then the row), row k of the result comes from that row
             float d[PB];
 #pragma unroll
-            for (int j = 0; j < PB; ++j) d[j] = s_row[lane][k0 + j];
+            for (int j = 0; j < PB; j += 4) {
+                const float4 t = *reinterpret_cast<const float4*>(&s_inv[lane][j]);
+                d[j] = t.x; d[j + 1] = t.y; d[j + 2] = t.z; d[j + 3] = t.w;
+            }
             bool used = false;
             int my_k = 0, my_p = 0;  // the step this row is the pivot of; the pivot row of step `lane`
+            unsigned best = 0;
+            float my_inv = 0.f;
+            auto candidate = [&](float v) {
+                const unsigned h = __float_as_uint(v) & 0x7fffffffu;
+                my_inv = __fdividef(1.f, v);
+                best = __reduce_max_sync(0xffffffffu, used ? 0u : ((h << 1) & ~63u) | unsigned(63 - lane));
+            };
+            candidate(d[0]);
+            // The pivot row goes round through shared memory, and a step leaves the columns where they are, two to
+            // an instruction; after two steps they move down two registers and the steps' own go to the end.
 #pragma unroll 1
-            for (int k = 0; k < PB; ++k) {
-                // column k is d[0]: every step moves the columns one register down and its own to the end
-                const unsigned h = __float_as_uint(d[0]) & 0x7fffffffu;
-                const unsigned best = __reduce_max_sync(0xffffffffu, used ? 0u : ((h << 1) & ~63u) | unsigned(63 - lane));
-                const int p = 63 - int(best & 63u);
-                const float piv = __shfl_sync(0xffffffffu, d[0], p);
-                if (!(fabsf(piv) > 0.f) || best >= 0xff000000u) bad = true;
-                const float inv = __fdividef(1.f, piv);
-                const bool pr = lane == p;
-                if (pr) { used = true; my_k = k; }
-                if (lane == k) my_p = p;
-                // every row loses c times the scaled pivot row; the pivot row keeps 1 / piv of itself with c = piv - 1;
-                // the entries of column k count as those of a unit vector
-                const float c = (pr ? piv - 1.f : d[0]) * inv;
+            for (int k = 0; k < PB; k += 2) {
 #pragma unroll
-                for (int j = 1; j < PB; ++j) d[j - 1] = fmaf(-c, __shfl_sync(0xffffffffu, d[j], p), d[j]);
-                d[PB - 1] = (pr ? 1.f : 0.f) - c;
+                for (int o = 0; o < 2; ++o) {
+                    const int p = 63 - int(best & 63u);
+                    const bool pr = lane == p;
+                    if (pr) {
+                        used = true;
+                        my_k = k + o;
+#pragma unroll
+                        for (int j = 0; j < PB; j += 4)
+                            *reinterpret_cast<float4*>(&s_piv[o][j]) = make_float4(d[j], d[j + 1], d[j + 2], d[j + 3]);
+                        s_piv[o][PB] = my_inv;
+                    }
+                    if (lane == k + o) my_p = p;
+                    __syncwarp();
+                    const float inv = s_piv[o][PB];
+                    float r[PB];
+#pragma unroll
+                    for (int j = 0; j < PB; j += 4) {
+                        const float4 t = *reinterpret_cast<const float4*>(&s_piv[o][j]);
+                        r[j] = t.x; r[j + 1] = t.y; r[j + 2] = t.z; r[j + 3] = t.w;
+                    }
+                    if (!(fabsf(r[o]) > 0.f) || best >= 0xff000000u) bad = true;
+                    // every row loses c times the scaled pivot row; the pivot row keeps 1 / piv of itself with
+                    // c = piv - 1; the entries of the step's column count as those of a unit vector
+                    const float c = (pr ? r[o] - 1.f : d[o]) * inv, own = (pr ? 1.f : 0.f) - c;
+                    // the next column first, and the search for its pivot between the others
+                    if (o == 0) {
+                        d[1] = fmaf(-c, r[1], d[1]);
+                        d[0] = own;
+                        candidate(d[1]);
+#pragma unroll
+                        for (int j = 2; j < PB; j += 2) fma2(d[j], d[j + 1], -c, r[j], r[j + 1]);
+                    } else {
+                        const float first = fmaf(-c, r[0], d[0]);
+                        fma2(d[2], d[3], -c, r[2], r[3]);
+                        candidate(d[2]);
+#pragma unroll
+                        for (int j = 4; j < PB; j += 2) fma2(d[j], d[j + 1], -c, r[j], r[j + 1]);
+#pragma unroll
+                        for (int j = 2; j < PB; ++j) d[j - 2] = d[j];
+                        d[PB - 2] = first;
+                        d[PB - 1] = own;
+                    }
+                }
             }
 #pragma unroll
             for (int j = 0; j < PB; ++j) {
@@ -724,21 +802,26 @@ __global__ void __launch_bounds__(256) k_inv_start(const __grid_constant__ InvLi
             }
         }
         __syncthreads();
-        // panel x inverse block (the block itself replaced by the identity): 32 x 128, 4 x 4 entries per thread
+        // panel x inverse block: 32 x 128, 4 x 4 entries per thread
         {
             const int r0 = 4 * (tid >> 5), c0 = 4 * lane;
             float s[4][4] = {};
-            const bool inside = c0 >= k0 && c0 < k0 + PB;
-#pragma unroll 8
-            for (int k = 0; k < PB; ++k) {
-                float4 p = *reinterpret_cast<const float4*>(&s_row[k][c0]);
-                if (inside)
-                    p = make_float4(c0 - k0 == k, c0 + 1 - k0 == k, c0 + 2 - k0 == k, c0 + 3 - k0 == k);
+#pragma unroll 2
+            for (int k4 = 0; k4 < PB; k4 += 4) {
+                float v[4][4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const float v = s_inv[r0 + i][k];
-                    fma2(s[i][0], s[i][1], v, p.x, p.y);
-                    fma2(s[i][2], s[i][3], v, p.z, p.w);
+                    const float4 t = *reinterpret_cast<const float4*>(&s_inv[r0 + i][k4]);
+                    v[i][0] = t.x; v[i][1] = t.y; v[i][2] = t.z; v[i][3] = t.w;
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const float4 p = *reinterpret_cast<const float4*>(&s_row[k4 + u][c0]);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        fma2(s[i][0], s[i][1], v[i][u], p.x, p.y);
+                        fma2(s[i][2], s[i][3], v[i][u], p.z, p.w);
+                    }
                 }
             }
             __syncthreads();
@@ -747,7 +830,7 @@ __global__ void __launch_bounds__(256) k_inv_start(const __grid_constant__ InvLi
                 *reinterpret_cast<float4*>(&s_row[r0 + i][c0]) = make_float4(s[i][0], s[i][1], s[i][2], s[i][3]);
         }
         __syncthreads();
-        // the block's columns start from zero, its rows become the panel: A <- A - C R with C = -I in those rows
+        // the block's columns and rows start from zero
         if (mine_c) {
 #pragma unroll
             for (int i = 0; i < 8; ++i)
@@ -774,20 +857,12 @@ __global__ void __launch_bounds__(256) k_inv_start(const __grid_constant__ InvLi
                 const float4 t = *reinterpret_cast<const float4*>(&s_row[k][4 * tx + 16 * j]);
                 rj[j] = t.x; rj[j + 1] = t.y; rj[j + 2] = t.z; rj[j + 3] = t.w;
                 const float4 u = *reinterpret_cast<const float4*>(&s_colT[k][4 * ty + 16 * j]);
-                ci[j] = -u.x; ci[j + 1] = -u.y; ci[j + 2] = -u.z; ci[j + 3] = -u.w;
-            }
-            if (mine_r) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float one = 4 * (ty - t0) + i == k ? 1.f : 0.f;
-                    if (hi) ci[i + 4] = one;
-                    else ci[i] = one;
-                }
+                ci[j] = u.x; ci[j + 1] = u.y; ci[j + 2] = u.z; ci[j + 3] = u.w;
             }
 #pragma unroll
             for (int i = 0; i < 8; ++i)
 #pragma unroll
-                for (int j = 0; j < 8; j += 2) fma2(a[i][j], a[i][j + 1], ci[i], rj[j], rj[j + 1]);
+                for (int j = 0; j < 8; ++j) a[i][j] = fmaf(ci[i], rj[j], a[i][j]);
         }
         __syncthreads();
     }
@@ -798,14 +873,28 @@ __global__ void __launch_bounds__(256) k_inv_start(const __grid_constant__ InvLi
             *reinterpret_cast<float4*>(&s_all[4 * ty + (i & 3) + 16 * (i & 4)][4 * tx + 16 * j]) =
                 make_float4(a[i][j], a[i][j + 1], a[i][j + 2], a[i][j + 3]);
     __syncthreads();
-#pragma unroll 4
-    for (int r = warp; r < n; r += 8)
+    int ec[4];  // a column of A^-1 takes the scale of that row of A
+    bool plain = true;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int c = lane + 32 * q;
-            // a column of A^-1 takes the scale of that row of A
-            if (c < n) out[(long long)r * O.ld + c] = shift_exponent(f2d_bits(s_all[r][c]), -s_e[c]);
-        }
+    for (int q = 0; q < 4; ++q) {
+        ec[q] = s_e[lane + 32 * q];
+        plain = plain && ec[q] >= -800 && ec[q] <= 800;
+    }
+    plain = __all_sync(0xffffffffu, plain);
+    double* o = out + (long long)warp * O.ld + lane;
+    if (plain) {
+#pragma unroll 2
+        for (int r = warp; r < n; r += 8, o += 8LL * O.ld)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (lane + 32 * q < n) o[32 * q] = scaled_double<true>(s_all[r][lane + 32 * q], ec[q]);
+    } else {
+#pragma unroll 1
+        for (int r = warp; r < n; r += 8, o += 8LL * O.ld)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (lane + 32 * q < n) o[32 * q] = scaled_double<false>(s_all[r][lane + 32 * q], ec[q]);
+    }
     if (tid < 32 && bad && lane == 0) info[blockIdx.y] = 1;
 }
 
