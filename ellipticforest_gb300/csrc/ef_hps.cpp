@@ -49,14 +49,14 @@ void leaf_tables(int n, double dx, double dy, double lambda, double* V, double* 
             const double c = (k == n - 1) ? std::sqrt(1.0 / n) : std::sqrt(2.0 / n);
             V[i * n + k] = c * std::sin(M_PI * (k + 1) * (i + 0.5) / n);
         }
+    double mux[64], muy[64];  // n <= 64
+    for (int k = 0; k < n; ++k) {
+        const double sn = std::sin(M_PI * (k + 1) / (2.0 * n));
+        mux[k] = -(4.0 / (dx * dx)) * sn * sn;
+        muy[k] = -(4.0 / (dy * dy)) * sn * sn;
+    }
     for (int k = 0; k < n; ++k)
-        for (int l = 0; l < n; ++l) {
-            const double sx = std::sin(M_PI * (k + 1) / (2.0 * n));
-            const double sy = std::sin(M_PI * (l + 1) / (2.0 * n));
-            const double mux = -(4.0 / (dx * dx)) * sx * sx;
-            const double muy = -(4.0 / (dy * dy)) * sy * sy;
-            Dinv[k * n + l] = 1.0 / (mux + muy + lambda);
-        }
+        for (int l = 0; l < n; ++l) Dinv[k * n + l] = 1.0 / (mux[k] + muy[l] + lambda);
 }
 
 void Hps::check(cudaError_t e, const char* what) {

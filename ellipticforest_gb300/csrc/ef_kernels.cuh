@@ -119,7 +119,12 @@ int leaf_dtn_lu(cudaStream_t st, int n, double lambda, const std::vector<double>
                 const std::vector<double*>& T);
 // rows 0..7 of the 16 x 16 sine basis into constant memory (ordered on st, synchronous); required
 // before leaf_eigen runs NEUMANN or SOLVE on 16 x 16 leaves
-void leaf_set_basis16(cudaStream_t st);
+// (wait: until it has arrived; the host values are staged on return either way)
+void leaf_set_basis16(cudaStream_t st, bool wait = true);
+
+// static device memory of kPatchBytes on the current device (a solve or a DtN application of one patch)
+constexpr size_t kPatchBytes = 144 * 1024;
+cudaError_t patch_memory(char** p);
 
 // Variable-coefficient leaf (FivePointStencil): coefficients sampled per cell, banded LU of the
 // 5-point operator (bandwidth n, no pivoting), triangular solves one warp per (leaf, RHS).

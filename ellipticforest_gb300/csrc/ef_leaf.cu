@@ -397,7 +397,7 @@ void launch_leaf(cudaStream_t st, const LeafType* types, const LeafItem* items, 
 
 }  // namespace
 
-void leaf_set_basis16(cudaStream_t st) {
+void leaf_set_basis16(cudaStream_t st, bool wait) {
     // uploaded by every tree set-up and single-patch call (1 KB): the values never change, and a
     // context reset by the caller cannot leave the table empty
     double V[8 * 16];
@@ -407,8 +407,15 @@ void leaf_set_basis16(cudaStream_t st) {
             V[i * 16 + k] = c * std::sin(M_PI * (k + 1) * (i + 0.5) / 16);
         }
     if (cudaMemcpyToSymbolAsync(c_V16d, V, sizeof(V), 0, cudaMemcpyHostToDevice, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
+        (wait && cudaStreamSynchronize(st) != cudaSuccess))
         throw std::runtime_error("leaf basis upload failed");
+}
+
+namespace {
+__device__ __align__(256) unsigned char g_patch_memory[kPatchBytes];
+}
+cudaError_t patch_memory(char** p) {
+    return cudaGetSymbolAddress(reinterpret_cast<void**>(p), g_patch_memory);
 }
 
 void leaf_eigen(cudaStream_t st, int mode, const LeafType* types, const LeafItem* items, int nitems,
