@@ -509,7 +509,7 @@ private:
         bool tc[3] = {false, false, false};  // per kind (W, H, DOWN)
         TcPlanes pl[3];
         int* rep[3] = {nullptr, nullptr, nullptr};  // device: source row tile of each stored tile
-        std::vector<int> tile[3], first[3];         // their tables
+        std::vector<int> tile[3], first[3], pair[3];  // their tables
     };
     struct MStep {
         int level = 0, nf = 0, count = 0;

@@ -270,12 +270,16 @@ struct TcPlanes {
     void* planes = nullptr;
     int* tile = nullptr;  // device: stored tile of each of the group's row tiles; null: all stored, in order
     int count = 0;        // stored tiles (with `tile`)
+    int* pair = nullptr;  // device: two row tiles (or one and -1) of one stored tile, npairs times; null: by tiles
+    int npairs = 0;
 };
 bool mx_tc_supported(int kind, int s);
 int mx_tc_max_split(int kind, int s);
 long long mx_tc_plane_elems(int ntiles, int K);
 // stored tile per row tile and the first row tile of each stored one, for nodes of operator classes cls
 void mx_tc_tiles(int kind, int s, const std::vector<int>& cls, std::vector<int>& tile, std::vector<int>& rep);
+// row tiles two by two where enough of them share a stored tile, else none
+std::vector<int> mx_tc_pairs(int kind, int s, const std::vector<int>& tile, int stored);
 // rep (device, with dst.tile): source row tile of each stored one
 void mx_tc_split(cudaStream_t st, int kind, const float* src, const TcPlanes& dst, const int* rep, long long rows, int K, int s);
 // failure-path test switch of both GEMM forms (process-wide): every CTA's first wait runs out

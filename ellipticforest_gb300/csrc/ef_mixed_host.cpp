@@ -194,6 +194,9 @@ MixedSolver::MixedSolver(Hps& hps, int bmax, const MixedSolver* share)
                 if (fewer) {
                     mg.pl[kind].tile = cv.get<int>(mg.tile[kind].size());
                     mg.rep[kind] = cv.get<int>(mg.first[kind].size());
+                    mg.pair[kind] = mx_tc_pairs(kind, g.s, mg.tile[kind], int(mg.first[kind].size()));
+                    mg.pl[kind].npairs = int(mg.pair[kind].size() / 2);
+                    mg.pl[kind].pair = mg.pair[kind].empty() ? nullptr : cv.get<int>(mg.pair[kind].size());
                 }
             }
             for (size_t i = 0; i < cnt; ++i) {
@@ -458,6 +461,8 @@ MixedSolver::MixedSolver(Hps& hps, int bmax, const MixedSolver* share)
             if (g.pl[kind].tile) {
                 ck(upload_sync(st, g.pl[kind].tile, g.tile[kind].data(), g.tile[kind].size() * sizeof(int)), "tiles");
                 ck(upload_sync(st, g.rep[kind], g.first[kind].data(), g.first[kind].size() * sizeof(int)), "tiles");
+                if (g.pl[kind].pair)
+                    ck(upload_sync(st, g.pl[kind].pair, g.pair[kind].data(), g.pair[kind].size() * sizeof(int)), "pairs");
             }
             mx_tc_split(st, kind, op[kind], g.pl[kind], g.rep[kind], rows[kind], Ks[kind], g.s);
         }

@@ -70,7 +70,7 @@ constexpr int kTK = 64;                   // K per stage: 64 bf16 = one 128-byte
 constexpr int kTB = 32;                   // requests per right-hand-side block (MMA N per block)
 constexpr int kPlaneA = kTM * kTK * 2;    // bytes of one A plane per stage (16 KB)
 constexpr int kPlaneX = kTB * kTK * 2;    // bytes of one X plane per block per stage (4 KB)
-constexpr int kTcThreads = 256;
+constexpr int kTcThreads = 288;
 constexpr int kStageThreads = 96;  // warps 4-6
 constexpr int kMaxSeg = 2;
 constexpr int kXRing = 3;  // FP32 request-block chunks in the staging ring
@@ -272,6 +272,25 @@ __device__ __forceinline__ void tc_store_row(const MixItem* __restrict__ items, 
     }
 }
 
+// K split: a thread's 32 partial sums in shared memory, four to a vector and vector i of all n threads together (with
+// a thread's own next to each other the 32 lanes of a warp met in one bank, 13 us of a launch), and the sum of
+// another rank's added to its own
+__device__ __forceinline__ void put_partial(unsigned char* red, const float (&v)[32], int t, int n) {
+    float4* r = reinterpret_cast<float4*>(red) + t;
+#pragma unroll
+    for (int q = 0; q < 32; q += 4) r[q / 4 * n] = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
+}
+__device__ __forceinline__ void add_partial(const unsigned char* red, float (&v)[32], int t, int n) {
+    const float4* r = reinterpret_cast<const float4*>(red) + t;
+    float4 x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = r[i * n];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        v[4 * i] += x[i].x; v[4 * i + 1] += x[i].y; v[4 * i + 2] += x[i].z; v[4 * i + 3] += x[i].w;
+    }
+}
+
 template <int KIND, int NSEG>
 __global__ void __launch_bounds__(kTcThreads, 1)
     k_mx_umma(const __nv_bfloat16* __restrict__ A3, const MixItem* __restrict__ items, int s, int B, int cnt,
@@ -354,31 +373,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     bool ep_ok = true;
 
     if (warp == 7) {
-        // ---- the warp stays converged and elects a lane for the bulk copies of the A planes and the MMAs: a
-        //      branch on the lane number has the compiler move every operand into uniform registers
-        //      through a loop over the active lanes (~100 clocks per MMA, 12 of them per chunk) ----
-        const long long pstride = (long long)nplanes * nkc * (kTM * kTK);  // elements per plane
-        // planes that several tiles read stay in L2; the others are read once per pass and go first
-        const unsigned long long pol = tmap ? l2_evict_normal() : l2_evict_first();
-        int cur_tile = -1;
-        long long cur_blk = 0;
-        auto copy = [&](int g, int sl) {  // chunk g into stage sl = g mod NS
-            const int u = g / cpu, c = g - u * cpu, tl = tile_of(u);
-            if (tl != cur_tile) {
-                cur_tile = tl;
-                cur_blk = (long long)(tmap ? __ldg(tmap + tl) : tl) * nkc + cbase;
-            }
-            const __nv_bfloat16* src = A3 + (cur_blk + c) * (kTM * kTK);
-            if (elect_one()) {
-                unsigned char* sa = base + size_t(sl) * SB;
-                mbar_expect_tx(&a_full[sl], 3u * kPlaneA);
-                for (int p = 0; p < 3; ++p) bulk_load(sa + p * kPlaneA, src + p * pstride, kPlaneA, &a_full[sl], pol);
-            }
-            __syncwarp();
-        };
+        // ---- the warp stays converged and elects a lane for the MMAs: a branch on the lane number has the compiler
+        //      move every operand into uniform registers through a loop over the active lanes (~100 clocks
+        //      per MMA, 12 of them per chunk).  The bulk copies of the A planes have a warp of their own ----
         bool ok = true;
-        int issued = 0;
-        for (; issued < NS && issued < total; ++issued) copy(issued, issued);
         if (g_mx_inject_timeout && nunits > 0) ok = __all_sync(0xffffffffu, tc_wait(never, 0u, abort_flag, 1000000LL));
         const uint64_t d0 = tc_desc(smem_u32(base));
         // the stages are unrolled, so that an operand's descriptor is the shared base plus a constant: computed per
@@ -416,25 +414,41 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 __syncwarp();
                 if (++c == cpu) c = 0;
                 if (++bf == NP) { bf = 0; ++bf_turn; }
-                // refill the stage of the chunk before, whose MMAs complete while this chunk's run
-                if (gch > 0 && issued < total) {
-                    ok = __all_sync(0xffffffffu, tc_wait(&empty[(st + NS - 1) % NS], unsigned(st > 0 ? turn : turn - 1) & 1u, abort_flag));
-                    if (ok) copy(issued++, (st + NS - 1) % NS);
-                }
             }
-        }
-        if (!ok) {
-            // let the loads still in flight land before the shared memory goes away
-            // (only the last NS loads can be pending: a stage is reloaded after its MMAs completed)
-            volatile int never_set = 0;
-            for (int q = issued > NS ? issued - NS : 0; q < issued; ++q)
-                (void)tc_wait(&a_full[q % NS], unsigned(q / NS) & 1u, &never_set);
         }
         // every MMA issued has completed before TMEM is freed
         if (elect_one()) tc_commit(drain);
         __syncwarp();
         volatile int never_set = 0;
         if (!tc_wait(drain, 0u, &never_set)) ok = false;
+        if (!ok && lane == 0) atomicExch(err, 1);
+    } else if (warp == 8) {
+        const long long pstride = (long long)nplanes * nkc * (kTM * kTK);  // elements per plane
+        // planes that several tiles read stay in L2; the others are read once per pass and go first
+        const unsigned long long pol = tmap ? l2_evict_normal() : l2_evict_first();
+        bool ok = true;
+        int issued = 0, sl = 0;
+        unsigned ph = 1;
+        for (int u = 0; u < nunits && ok; ++u) {
+            const int tl = tile_of(u);
+            const __nv_bfloat16* src = A3 + ((long long)(tmap ? __ldg(tmap + tl) : tl) * nkc + cbase) * (kTM * kTK);
+            for (int c = 0; c < cpu; ++c, src += kTM * kTK) {
+                if (issued >= NS) ok = tc_wait(&empty[sl], ph, abort_flag);
+                if (!(ok = __all_sync(0xffffffffu, ok))) break;
+                if (elect_one()) {
+                    unsigned char* sa = base + size_t(sl) * SB;
+                    mbar_expect_tx(&a_full[sl], 3u * kPlaneA);
+                    for (int p = 0; p < 3; ++p) bulk_load(sa + p * kPlaneA, src + p * pstride, kPlaneA, &a_full[sl], pol);
+                }
+                __syncwarp();
+                ++issued;
+                if (++sl == NS) { sl = 0; ph ^= 1u; }
+            }
+        }
+        // the loads still in flight land before the shared memory goes away
+        volatile int never_set = 0;
+        for (int q = issued > NS ? issued - NS : 0; q < issued; ++q)
+            if (!tc_wait(&a_full[q % NS], unsigned(q / NS) & 1u, &never_set)) ok = false;
         if (!ok && lane == 0) atomicExch(err, 1);
     } else if (warp >= 4) {
         // ---- warps 4-6: stage X.  FP32 request rows travel by cp.async into a ring of kXRing
@@ -568,10 +582,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             if (ksplit > 1) {
                 // partial tiles -> rank 0 of the cluster through distributed shared memory, in rank
                 // order (deterministic); the stage memory is free once every MMA has completed
-                float* red = reinterpret_cast<float*>(base);
-#pragma unroll
-                for (int q = 0; q < 32; q += 4)
-                    *reinterpret_cast<float4*>(red + t * 32 + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
+                put_partial(base, v, t, 128);
                 break;  // the cluster reduction and the epilogue follow below
             }
             const int grow = tile * kTM + t;
@@ -587,21 +598,14 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         cg::cluster_group cluster = cg::this_cluster();
         if (nunits == 0 && tid < 128) {
             // a rank without K chunks adds zeros
-            float* red = reinterpret_cast<float*>(base);
 #pragma unroll
-            for (int q = 0; q < 32; q += 4) *reinterpret_cast<float4*>(red + tid * 32 + q) = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int q = 0; q < 32; ++q) v[q] = 0.f;
+            put_partial(base, v, tid, 128);
         }
         cluster.sync();
         if (cluster.block_rank() == 0 && tid < 128 && nunits > 0 && !*abort_flag) {
             const int t = tid;
-            float* red = reinterpret_cast<float*>(base);
-#pragma unroll
-            for (int q = 0; q < 32; ++q) v[q] = red[t * 32 + q];
-            for (int rk = 1; rk < ksplit; ++rk) {
-                const float* rr = cluster.map_shared_rank(red, rk);
-#pragma unroll
-                for (int q = 0; q < 32; ++q) v[q] += rr[t * 32 + q];
-            }
+            for (int rk = 1; rk < ksplit; ++rk) add_partial(cluster.map_shared_rank(base, rk), v, t, 128);
             const int tile = first_tile;
             const int grow = tile * kTM + t;
             if (grow < R) tc_store_row<KIND>(items, s, B, b0, sh.rows_item, grow, v, pre, vec);
@@ -613,6 +617,316 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     __syncthreads();
     tc_fence_after();
     if (warp == 7) tmem_dealloc(tmem, unsigned(tcols));
+}
+
+// ---- two nodes with equal operators per tile --------------------------------------------------------------
+// The same sums as k_mx_umma (term for term: bit-identical results) for the two nodes of a pair of row tiles that
+// share a stored tile: an A chunk (48 KB) is loaded once for both, and one MMA takes the 64 requests of both.  The
+// bound is shared memory: 96 KB read by the MMAs of a chunk and 72 KB written for them, 1,340 clocks at 128 bytes
+// per clock, against 1,180 for one node in k_mx_umma (measured: about 1,800 and 1,950).  Per stage 48 KB of A
+// and 24 KB of X; the rows of X come straight into registers one chunk ahead (an FP32 copy in shared memory would
+// cost the third stage and its bandwidth).  All node GEMMs of a block of 32 requests on a 7-level tree with
+// 16 x 16 leaves, two passes: 1.65 ms by single tiles, 1.39 ms.
+// Roles: warps 0-7 collect and write (four per node), warps 8-15 stage X, warp 16 issues the MMAs, warp 17 copies A.
+constexpr int kPairThreads = 576, kPairStage = 256, kPairStages = 3, kPairSets = 2;
+constexpr int kPairCols = 2 * kTB;  // right-hand side columns per plane
+constexpr int kPairStageBytes = 3 * kPlaneA + 3 * 2 * kPlaneX;
+constexpr size_t kPairSmem = 1024 + size_t(kPairStages) * kPairStageBytes + 256;
+static_assert(kPairSmem <= 227 * 1024, "shared memory of one CTA");
+static_assert(2 * kPairSmem > 228 * 1024, "one CTA per SM: each takes all of TMEM");
+static_assert(kPairSets * 3 * kPairCols <= 512, "accumulator sets");
+
+// Rows of both nodes are whole tiles (128 rows or more per segment), K is a multiple of 64.
+bool pair_supported(int kind, int s) {
+    const TcShape sh = tc_shape(kind, s);
+    return sh.nseg == 1 && sh.K % kTK == 0;
+}
+
+// *p where `get`, else zero; a load in any case, never a branch
+__device__ __forceinline__ float load_if(const float* p, bool get) {
+    float x;
+    asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n mov.f32 %0, 0f00000000;\n @p ld.global.cg.f32 %0, [%1];\n}\n"
+                 : "=f"(x)
+                 : "l"(p), "r"(unsigned(get))
+                 : "memory");
+    return x;
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(kPairThreads, 1)
+    k_mx_umma_pair(const __nv_bfloat16* __restrict__ A3, const MixItem* __restrict__ items, int s, int B, int cnt,
+                   int ksplit, const int2* __restrict__ pairs, int npairs, const int* __restrict__ tmap, int nplanes,
+                   int* __restrict__ err) {
+    const TcShape sh = tc_shape(KIND, s);
+    const int K = sh.K, R = cnt * sh.rows_item, nkc = K / kTK;
+    constexpr int NS = kPairStages, SB = kPairStageBytes, NP = kPairSets, ncol = kPairCols;
+    constexpr unsigned idesc1 = tc_idesc(kTM, ncol), idesc2 = tc_idesc(kTM, 2 * ncol), idesc3 = tc_idesc(kTM, 3 * ncol);
+    extern __shared__ unsigned char tc_smem[];
+    unsigned char* base = tc_smem + ((1024u - (smem_u32(tc_smem) & 1023u)) & 1023u);
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(base + size_t(NS) * SB);
+    unsigned long long *a_full = bars, *x_full = a_full + NS, *empty = x_full + NS, *acc_full = empty + NS,
+                       *acc_empty = acc_full + NP, *drain = acc_empty + NP, *never = drain + 1;
+    unsigned* tmem_slot = reinterpret_cast<unsigned*>(never + 1);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    int first, step, nunits, cpu, cbase;
+    if (ksplit > 1) {
+        const int kp = blockIdx.x % ksplit, cpp = (nkc + ksplit - 1) / ksplit;
+        first = blockIdx.x / ksplit;
+        step = 0;
+        nunits = 1;
+        cbase = min(nkc, kp * cpp);
+        cpu = min(nkc, cbase + cpp) - cbase;
+    } else {
+        first = blockIdx.x;
+        step = gridDim.x;
+        nunits = first < npairs ? (npairs - 1 - first) / step + 1 : 0;
+        cbase = 0;
+        cpu = nkc;
+    }
+    if (cpu <= 0) nunits = 0;
+    const int total = nunits * cpu, b0 = blockIdx.y * kTB;
+    const bool vec = (B & 3) == 0;
+    if (tid == 0) {
+        for (int i = 0; i < NS; ++i) {
+            mbar_init(a_full + i, 1);
+            mbar_init(x_full + i, kPairStage);
+            mbar_init(empty + i, 1);
+        }
+        for (int i = 0; i < NP; ++i) {
+            mbar_init(acc_full + i, 1);
+            mbar_init(acc_empty + i, 256);
+        }
+        mbar_init(drain, 1);
+        mbar_init(never, 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    }
+    if (warp == 16) {
+        tmem_alloc(tmem_slot, 512u);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const unsigned tmem = *tmem_slot;
+
+    float v[32];  // collecting threads: the row's sums
+    bool ep_ok = true;
+    if (warp == 16) {
+        // converged, one elected lane issuing; stages and accumulator sets unrolled (constant descriptors).  The copies
+        // have a warp of their own: issuing them here took 400 of 2,200 clocks per chunk from the MMAs.
+        bool ok = true;
+        if (g_mx_inject_timeout && nunits > 0) ok = __all_sync(0xffffffffu, tc_wait(never, 0u, abort_flag, 1000000LL));
+        const uint64_t d0 = tc_desc(smem_u32(base));
+        constexpr int UN = 6;  // a multiple of NS and NP
+        static_assert(UN % NS == 0 && UN % NP == 0 && (UN / NS) % 2 == 0, "phases of the unrolled chunks");
+        for (int g0 = 0, turn = 0; g0 < total && ok; g0 += UN, ++turn) {
+#pragma unroll
+            for (int o = 0; o < UN; ++o) {
+                const int g = g0 + o;
+                if (g >= total || !ok) break;
+                constexpr int perset = UN / NP;  // uses of a set per turn
+                const int st = o % NS, bf = o % NP;
+                const unsigned ph = unsigned(o / NS) & 1u;
+                if (g >= NP) ok = tc_wait(acc_empty + bf, unsigned(turn * perset + o / NP + 1) & 1u, abort_flag);
+                if (ok) ok = tc_wait(a_full + st, ph, abort_flag) && tc_wait(x_full + st, ph, abort_flag);
+                if (!(ok = __all_sync(0xffffffffu, ok))) break;
+                tc_fence_after();
+                const uint64_t da = d0 + uint64_t(unsigned(st) * (unsigned(SB) >> 4)), dx = da + uint64_t(3 * kPlaneA >> 4);
+                const unsigned dhi = tmem + unsigned(bf * 3 * ncol), dlo = dhi + unsigned(ncol);
+                if (elect_one()) {
+#pragma unroll
+                    for (int kk = 0; kk < kTK / 16; ++kk) {
+                        const uint64_t ko = uint64_t(2 * kk), x123 = dx + ko;
+                        tc_mma(dhi, da + ko, x123, idesc3, kk > 0 ? 1u : 0u);
+                        tc_mma(dlo, da + uint64_t(kPlaneA >> 4) + ko, x123, idesc2, 1u);
+                        tc_mma(dlo, da + uint64_t(2 * kPlaneA >> 4) + ko, x123, idesc1, 1u);
+                    }
+                    tc_commit(empty + st);
+                    tc_commit(acc_full + bf);
+                }
+                __syncwarp();
+            }
+        }
+        volatile int never_set = 0;
+        if (elect_one()) tc_commit(drain);
+        __syncwarp();
+        if (!tc_wait(drain, 0u, &never_set)) ok = false;
+        if (!ok && lane == 0) atomicExch(err, 1);
+    } else if (warp == 17) {
+        const long long pstride = (long long)nplanes * nkc * (kTM * kTK);
+        const unsigned long long pol = l2_evict_normal();
+        bool ok = true;
+        int issued = 0, sl = 0;
+        unsigned ph = 1;
+        for (int u = 0; u < nunits && ok; ++u) {
+            const __nv_bfloat16* src = A3 + ((long long)__ldg(tmap + pairs[first + u * step].x) * nkc + cbase) * (kTM * kTK);
+            for (int c = 0; c < cpu; ++c, src += kTM * kTK) {
+                if (issued >= NS) ok = tc_wait(empty + sl, ph, abort_flag);
+                if (!(ok = __all_sync(0xffffffffu, ok))) break;
+                if (elect_one()) {
+                    unsigned char* sa = base + size_t(sl) * SB;
+                    mbar_expect_tx(a_full + sl, 3u * kPlaneA);
+                    for (int p = 0; p < 3; ++p) bulk_load(sa + p * kPlaneA, src + p * pstride, kPlaneA, a_full + sl, pol);
+                }
+                __syncwarp();
+                ++issued;
+                if (++sl == NS) { sl = 0; ph ^= 1u; }
+            }
+        }
+        // the loads still in flight land before the shared memory goes away
+        volatile int never_set = 0;
+        for (int q = issued > NS ? issued - NS : 0; q < issued; ++q)
+            if (!tc_wait(a_full + q % NS, unsigned(q / NS) & 1u, &never_set)) ok = false;
+        if (!ok && lane == 0) atomicExch(err, 1);
+    } else if (warp >= 8) {
+        // ---- X: thread = (8 consecutive k, request) of both nodes; the next chunk's rows are loaded before this
+        //      chunk's are split
+        const int t = tid - 256, n = t & 31, kg = t >> 5;
+        const bool in = b0 + n < B;
+        float xa[2][8], xb[2][8];
+        const float *p1[2], *p2[2];  // this thread's rows of the next chunk, for k < kb and from there on
+        bool have[2];
+        int kb = 0, lu = 0, lc = 0;  // the next chunk to load: lc of unit lu
+        const long long row = (long long)B;
+        auto load = [&](float (&x)[2][8]) {
+            if (lc == 0 && lu < nunits) {
+                const int2 pr = pairs[first + lu * step];
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const int tile = j ? pr.y : pr.x;
+                    have[j] = tile >= 0 && in;
+                    const TcSeg sg = tc_seg<KIND>(items, s, B, max(tile, 0) * kTM / sh.seg_rows);
+                    const long long off = (long long)(cbase * kTK + 8 * kg) * B + b0 + (in ? n : 0);
+                    p1[j] = sg.X1 + off;
+                    p2[j] = sg.X2 + off;
+                    kb = sg.kb;
+                }
+            }
+            const bool one = (cbase + lc) * kTK + 8 * kg < kb;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const float* p = one ? p1[j] : p2[j];
+                const bool get = have[j] && lu < nunits;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) x[j][i] = load_if(p + i * row, get);
+                p1[j] += kTK * row;
+                p2[j] += kTK * row;
+            }
+            if (++lc == cpu) { lc = 0; ++lu; }
+        };
+        bool ok = true;
+        int st = 0;
+        unsigned ph = 0;
+        auto stage = [&](int g, const float (&x)[2][8]) {
+            if (g >= NS && !tc_wait(empty + st, ph ^ 1u, abort_flag)) return false;
+            unsigned char* sx = base + size_t(st) * SB + 3 * kPlaneA;
+            constexpr unsigned xp = 2u * kPlaneX;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                uint4 c0, c1, c2;
+                split3x2(x[j][0], x[j][1], c0.x, c1.x, c2.x);
+                split3x2(x[j][2], x[j][3], c0.y, c1.y, c2.y);
+                split3x2(x[j][4], x[j][5], c0.z, c1.z, c2.z);
+                split3x2(x[j][6], x[j][7], c0.w, c1.w, c2.w);
+                const unsigned off = unsigned(j) * kPlaneX + unsigned(n) * 128u + ((unsigned(kg) ^ unsigned(n & 7)) << 4);
+                *reinterpret_cast<uint4*>(sx + off) = c0;
+                *reinterpret_cast<uint4*>(sx + xp + off) = c1;
+                *reinterpret_cast<uint4*>(sx + 2 * xp + off) = c2;
+            }
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            mbar_arrive(x_full + st);
+            if (++st == NS) { st = 0; ph ^= 1u; }
+            return true;
+        };
+        if (total > 0) load(xa);
+        for (int g = 0; g < total; g += 2) {
+            load(xb);  // (nothing past the last chunk)
+            if (!(ok = stage(g, xa)) || g + 1 >= total) break;
+            load(xa);
+            if (!(ok = stage(g + 1, xb))) break;
+        }
+        if (!ok) atomicExch(err, 1);
+    } else {
+        // ---- collect: warps 0-3 the first node's columns, 4-7 the second's; warp w holds rows 32 (w mod 4) ..
+        const int t = tid & 127, j = tid >> 7;
+        float rlo[32];
+#pragma unroll
+        for (int q = 0; q < 32; ++q) { v[q] = 0.f; rlo[q] = 0.f; }
+        const unsigned acc = tmem + (unsigned((warp & 3) * 32) << 16) + unsigned(j * kTB);
+        int c = 0, u = 0;
+        for (int g = 0; g < total; ++g) {
+            const int bf = g % NP;
+            if (!(ep_ok = tc_wait(acc_full + bf, unsigned(g / NP) & 1u, abort_flag))) break;
+            tc_fence_after();
+            const unsigned col = acc + unsigned(bf * 3 * ncol);
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+                float x[16];
+                tmem_ld16(col + unsigned(16 * hf), x);
+#pragma unroll
+                for (int q = 0; q < 16; ++q) v[16 * hf + q] += x[q];
+                tmem_ld16(col + unsigned(ncol + 16 * hf), x);
+#pragma unroll
+                for (int q = 0; q < 16; ++q) rlo[16 * hf + q] += x[q];
+                tmem_ld16(col + unsigned(2 * ncol + 16 * hf), x);
+#pragma unroll
+                for (int q = 0; q < 16; ++q) rlo[16 * hf + q] += x[q];
+            }
+            tc_fence_before();
+            mbar_arrive(acc_empty + bf);
+            if (++c < cpu) continue;
+            c = 0;
+#pragma unroll
+            for (int q = 0; q < 32; ++q) {
+                v[q] += rlo[q];
+                rlo[q] = 0.f;
+            }
+            if (ksplit > 1) break;  // the cluster's reduction and the epilogue follow below
+            const int2 pr = pairs[first + u * step];
+            const int tile = j ? pr.y : pr.x, grow = tile * kTM + t;
+            if (tile >= 0 && grow < R) {
+                float pre[32];
+                tc_prefetch_row<KIND>(items, s, B, b0, sh.rows_item, grow, pre, vec);
+                tc_store_row<KIND>(items, s, B, b0, sh.rows_item, grow, v, pre, vec);
+            }
+            ++u;
+#pragma unroll
+            for (int q = 0; q < 32; ++q) v[q] = 0.f;
+        }
+        if (!ep_ok) atomicExch(err, 1);
+    }
+
+    // ---- K split: rank 0 of the cluster adds the partial tiles in rank order and runs the epilogue ----
+    if (ksplit > 1) {
+        cg::cluster_group cluster = cg::this_cluster();
+        __syncthreads();  // every MMA has completed (drain): the stages are free
+        if (tid < 256) {
+            if (nunits == 0) {
+#pragma unroll
+                for (int q = 0; q < 32; ++q) v[q] = 0.f;
+            }
+            put_partial(base, v, tid, 256);
+        }
+        cluster.sync();
+        if (cluster.block_rank() == 0 && tid < 256 && nunits > 0 && !*abort_flag) {
+            for (int rk = 1; rk < ksplit; ++rk) add_partial(cluster.map_shared_rank(base, rk), v, tid, 256);
+            const int2 pr = pairs[first];
+            const int tile = tid >> 7 ? pr.y : pr.x, grow = tile * kTM + (tid & 127);
+            if (tile >= 0 && grow < R) {
+                float pre[32];
+                tc_prefetch_row<KIND>(items, s, B, b0, sh.rows_item, grow, pre, vec);
+                tc_store_row<KIND>(items, s, B, b0, sh.rows_item, grow, v, pre, vec);
+            }
+        }
+        cluster.sync();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 16) tmem_dealloc(tmem, 512u);
 }
 
 // A planes of one group: three bf16 planes with src[R][K] = plane 0 + plane 1 + plane 2, each stored
@@ -690,10 +1004,41 @@ void launch_umma_n(cudaStream_t st, const TcPlanes& A, const MixItem* items, int
 }
 
 template <int KIND>
+void launch_pair(cudaStream_t st, const TcPlanes& A, const MixItem* items, int cnt, int s, int B, int* err, int ksplit) {
+    const int chunks = (B + kTB - 1) / kTB;
+    cudaFuncSetAttribute(k_mx_umma_pair<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPairSmem));
+    int sms = 0, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(ksplit > 1 ? A.npairs * ksplit : std::max(1, std::min(A.npairs, std::max(1, sms / chunks)))),
+                       unsigned(chunks));
+    cfg.blockDim = dim3(kPairThreads);
+    cfg.dynamicSmemBytes = kPairSmem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = unsigned(ksplit);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = ksplit > 1 ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_mx_umma_pair<KIND>, reinterpret_cast<const __nv_bfloat16*>(A.planes), items, s,
+                                             B, cnt, ksplit, reinterpret_cast<const int2*>(A.pair), A.npairs, A.tile, A.count, err);
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        throw std::runtime_error(std::string("tensor-core node GEMM launch (pairs, K split ") + std::to_string(ksplit) +
+                                 "): " + cudaGetErrorString(e));
+    }
+    ++g_kernel_launches;
+}
+
+template <int KIND>
 void launch_umma(cudaStream_t st, const TcPlanes& A, const MixItem* items, int cnt, int s, int B, int* err,
                  int ksplit) {
     const int nseg = tc_shape(KIND, s).nseg;
-    if (nseg == 1) launch_umma_n<KIND, 1>(st, A, items, cnt, s, B, err, ksplit);
+    if (A.pair) launch_pair<KIND>(st, A, items, cnt, s, B, err, ksplit);
+    else if (nseg == 1) launch_umma_n<KIND, 1>(st, A, items, cnt, s, B, err, ksplit);
     else launch_umma_n<KIND, 2>(st, A, items, cnt, s, B, err, ksplit);
 }
 
@@ -735,6 +1080,21 @@ void mx_tc_tiles(int kind, int s, const std::vector<int>& cls, std::vector<int>&
         if (it.second) rep.push_back(t);
         tile.push_back(it.first->second);
     }
+}
+
+std::vector<int> mx_tc_pairs(int kind, int s, const std::vector<int>& tile, int stored) {
+    std::vector<int> pairs;
+    if (!pair_supported(kind, s)) return pairs;
+    std::vector<std::vector<int>> users(stored);
+    for (size_t t = 0; t < tile.size(); ++t) users[tile[t]].push_back(int(t));
+    for (const auto& u : users)
+        for (size_t i = 0; i < u.size(); i += 2) {
+            pairs.push_back(u[i]);
+            pairs.push_back(i + 1 < u.size() ? u[i + 1] : -1);
+        }
+    // a pair costs about what one tile does, a tile alone in its pair a little more
+    if (pairs.size() / 2 * 4 > tile.size() * 3) pairs.clear();
+    return pairs;
 }
 
 void mx_tc_split(cudaStream_t st, int kind, const float* src, const TcPlanes& dst, const int* rep, long long R, int K, int s) {
