@@ -155,118 +155,148 @@ __device__ __forceinline__ TcSeg tc_seg(const MixItem* __restrict__ items, int s
     return t;
 }
 
-// Prefetch of the operand a row's epilogue reads (issued when the row's tile starts, so that its
-// latency hides behind the K loop): w for DOWN, the child's particular flux hc for H.
+// ---- epilogue of 32 tile rows by one warp ----------------------------------------------------------
+// A lane holds a row's sums for the 32 requests of a block.  Rows are 128 bytes (B = 32) in memory, so with 16-byte
+// accesses by rows every instruction touched 32 of them.  With B a multiple of 4 the warp therefore exchanges
+// its 4-request pieces first: lane (piece c = lane / 4, a = lane mod 4) gets piece c of the rows 4 i + a, i = 0 .. 7, and
+// an instruction covers four whole rows (L7 block 4.00 -> 3.94 ms).  Otherwise the lane keeps its row, one request
+// at a time.
+
+// where a tile row reads and writes: its addresses, null for a row past the group's end
+struct TcRow {
+    const float* src;  // added to the sums: H the child's particular flux hc, DOWN w
+    float *d0, *d1;    // W: w; H: h; DOWN: both children's interface rows
+    double* state;     // DOWN: the FP64 interface state (null: one launch adds the whole pass's values at its end)
+};
 template <int KIND>
-__device__ __forceinline__ void tc_prefetch_row(const MixItem* __restrict__ items, int s, int B, int b0, int rows_item,
-                                                int grow, float (&pre)[32], bool vec) {
-    if (KIND == MX_W) return;
+__device__ __forceinline__ TcRow tc_row(const MixItem* __restrict__ items, int s, int B, int rows_item, int grow, bool in) {
+    TcRow t{nullptr, nullptr, nullptr, nullptr};
+    if (!in) return t;
     const int item = grow / rows_item, r = grow - item * rows_item;
     const MixItem& it = items[item];
-    const int nb = min(32, B - b0);
-    const float* src;
-    if (KIND == MX_H) {
+    if (KIND == MX_W) {
+        t.d0 = it.w + (long long)r * B;
+    } else if (KIND == MX_H) {
+        const int p = tc_h_unpermute(r, s);
         int c, q2;
-        mx_ext_map(tc_h_unpermute(r, s), s, c, q2);
-        src = it.hc[c] + (long long)q2 * B + b0;
+        mx_ext_map(p, s, c, q2);
+        t.src = it.hc[c] + (long long)q2 * B;
+        t.d0 = it.h + (long long)p * B;
     } else {
-        src = it.w + (long long)r * B + b0;
+        const int I = r / s, o = r - I * s;
+        t.src = it.w + (long long)r * B;
+        t.d0 = it.gc[mx_lower_child(I)] + (long long)mx_q_lower(I, o, s) * B;
+        t.d1 = it.gc[mx_upper_child(I)] + (long long)mx_q_upper(I, o, s) * B;
+        if (it.uG) t.state = it.uG + (long long)r * B;
+    }
+    return t;
+}
+template <class T>
+__device__ __forceinline__ T* row_of_lane(T* p, int lane) {
+    return reinterpret_cast<T*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(p), lane));
+}
+
+// the operand that the epilogue adds, in the layout of the accesses (issued early, so that its latency is hidden)
+template <int KIND>
+__device__ __forceinline__ void tc_prefetch(const TcRow& row, int B, int b0, float (&pre)[32], bool vec) {
+    if (KIND == MX_W) return;
+    const int lane = threadIdx.x & 31, nb = min(32, B - b0);
+    if (KIND == MX_DOWN && row.state) {  // its 256 bytes to L2: read once more per sweep only
+        asm volatile("prefetch.global.L2 [%0];\n" ::"l"(row.state + b0));
+        asm volatile("prefetch.global.L2 [%0];\n" ::"l"(row.state + b0 + nb - 1));
     }
     if (vec) {
+        const int c = lane >> 2, a = lane & 3;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            const float4 x = 4 * i < nb ? *reinterpret_cast<const float4*>(src + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float* p = row_of_lane(row.src, 4 * i + a);
+            const float4 x = p && 4 * c < nb ? *reinterpret_cast<const float4*>(p + b0 + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
             pre[4 * i] = x.x; pre[4 * i + 1] = x.y; pre[4 * i + 2] = x.z; pre[4 * i + 3] = x.w;
         }
     } else {
 #pragma unroll
-        for (int q = 0; q < 32; ++q) pre[q] = q < nb ? src[q] : 0.f;
+        for (int q = 0; q < 32; ++q) pre[q] = row.src && q < nb ? row.src[b0 + q] : 0.f;
     }
 }
 
-// Epilogue of one tile row: v[q] = (A X)[row][b0 + q] for the 32 requests of this request block,
-// pre[q] the prefetched operand (tc_prefetch_row).  The FP64 interface state of DOWN rows is read
-// and written in two halves of 16 requests, each with its loads ahead of its stores; 16-byte
-// accesses when B % 4 == 0.
+// v[q] = (A X)[row][b0 + q] of this lane's row (v is used up)
 template <int KIND>
-__device__ __forceinline__ void tc_store_row(const MixItem* __restrict__ items, int s, int B, int b0, int rows_item,
-                                             int grow, const float (&v)[32], const float (&pre)[32], bool vec) {
-    const int item = grow / rows_item, r = grow - item * rows_item;
-    const MixItem& it = items[item];
-    const int nb = min(32, B - b0);
-    const long long cb = (long long)b0;
-    if (KIND == MX_W) {
-        float* dst = it.w + (long long)r * B + cb;
-        if (vec) {
+__device__ __forceinline__ void tc_store(const TcRow& row, int B, int b0, float (&v)[32], const float (&pre)[32], bool vec) {
+    const int lane = threadIdx.x & 31, nb = min(32, B - b0);
+    if (vec) {
+        const int c = lane >> 2, a = lane & 3;
+        // piece bits and lane bits change places
 #pragma unroll
-            for (int q = 0; q < 32; q += 4)
-                if (q < nb) *reinterpret_cast<float4*>(dst + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
-        } else {
+        for (int k = 0; k < 3; ++k) {
+            const int bit = 1 << k;
+            const bool up = (lane >> 2) & bit;
 #pragma unroll
-            for (int q = 0; q < 32; ++q)
-                if (q < nb) dst[q] = v[q];
+            for (int i = 0; i < 8; ++i) {
+                if (i & bit) continue;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    float &x = v[4 * i + e], &y = v[4 * (i | bit) + e];
+                    const float got = __shfl_xor_sync(0xffffffffu, up ? x : y, 4 * bit);
+                    if (up) x = got;
+                    else y = got;
+                }
+            }
         }
-    } else if (KIND == MX_H) {
-        float* dst = it.h + (long long)tc_h_unpermute(r, s) * B + cb;
-        if (vec) {
+        if (KIND != MX_W) {
 #pragma unroll
-            for (int q = 0; q < 32; q += 4)
-                if (q < nb)
-                    *reinterpret_cast<float4*>(dst + q) =
-                        make_float4(v[q] + pre[q], v[q + 1] + pre[q + 1], v[q + 2] + pre[q + 2], v[q + 3] + pre[q + 3]);
-        } else {
-#pragma unroll
-            for (int q = 0; q < 32; ++q)
-                if (q < nb) dst[q] = v[q] + pre[q];
+            for (int q = 0; q < 32; ++q) v[q] += pre[q];
         }
-    } else {
-        const int I = r / s, o = r - (r / s) * s;
-        float* d0 = it.gc[mx_lower_child(I)] + (long long)mx_q_lower(I, o, s) * B + cb;
-        float* d1 = it.gc[mx_upper_child(I)] + (long long)mx_q_upper(I, o, s) * B + cb;
-        // the FP64 state (none: one launch adds the whole pass's values at its end)
-        double* ug = it.uG ? it.uG + (long long)r * B + cb : nullptr;
+        const bool in = 4 * c < nb;
+        const int at = b0 + 4 * c;
 #pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-            const int q0 = 16 * hf;
-            float uu[16];
+        for (int i = 0; i < 8; ++i) {
+            float* d0 = row_of_lane(row.d0, 4 * i + a);
+            float* d1 = KIND == MX_DOWN ? row_of_lane(row.d1, 4 * i + a) : nullptr;
+            if (d0 && in) {
+                const float4 o = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                *reinterpret_cast<float4*>(d0 + at) = o;
+                if (KIND == MX_DOWN) *reinterpret_cast<float4*>(d1 + at) = o;
+            }
+        }
+        if (KIND == MX_DOWN && __any_sync(0xffffffffu, row.state != nullptr)) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) uu[i] = v[q0 + i] + pre[q0 + i];
-            if (vec && !ug) {
+            for (int i = 0; i < 8; i += 2) {
+                double* st[2];
+                double2 u[2][2];
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (q0 + 4 * i < nb) {
-                        const float4 o4 = make_float4(uu[4 * i], uu[4 * i + 1], uu[4 * i + 2], uu[4 * i + 3]);
-                        *reinterpret_cast<float4*>(d0 + q0 + 4 * i) = o4;
-                        *reinterpret_cast<float4*>(d1 + q0 + 4 * i) = o4;
+                for (int k = 0; k < 2; ++k) {
+                    st[k] = row_of_lane(row.state, 4 * (i + k) + a);
+                    st[k] = st[k] && in ? st[k] + at : nullptr;
+                    if (st[k]) {
+                        u[k][0] = *reinterpret_cast<const double2*>(st[k]);
+                        u[k][1] = *reinterpret_cast<const double2*>(st[k] + 2);
                     }
-            } else if (vec) {
-                double2 u2[8];
+                }
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    u2[i] = q0 + 2 * i < nb ? *reinterpret_cast<const double2*>(ug + q0 + 2 * i) : make_double2(0.0, 0.0);
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (q0 + 4 * i < nb) {
-                        const float4 o4 = make_float4(uu[4 * i], uu[4 * i + 1], uu[4 * i + 2], uu[4 * i + 3]);
-                        *reinterpret_cast<float4*>(d0 + q0 + 4 * i) = o4;
-                        *reinterpret_cast<float4*>(d1 + q0 + 4 * i) = o4;
+                for (int k = 0; k < 2; ++k)
+                    if (st[k]) {
+                        const float* w = v + 4 * (i + k);
+                        *reinterpret_cast<double2*>(st[k]) = make_double2(u[k][0].x + f2d_bits(w[0]), u[k][0].y + f2d_bits(w[1]));
+                        *reinterpret_cast<double2*>(st[k] + 2) = make_double2(u[k][1].x + f2d_bits(w[2]), u[k][1].y + f2d_bits(w[3]));
                     }
+            }
+        }
+    } else if (row.d0) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    if (q0 + 2 * i < nb)
-                        *reinterpret_cast<double2*>(ug + q0 + 2 * i) =
-                            make_double2(u2[i].x + f2d_bits(uu[2 * i]), u2[i].y + f2d_bits(uu[2 * i + 1]));
-            } else {
-                double uv[16];
+        for (int h = 0; h < 32; h += 4) {
+            double u[4];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) uv[i] = (ug && q0 + i < nb) ? ug[q0 + i] : 0.0;
+            for (int i = 0; i < 4; ++i) u[i] = KIND == MX_DOWN && row.state && h + i < nb ? row.state[b0 + h + i] : 0.0;
 #pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    if (q0 + i < nb) {
-                        d0[q0 + i] = uu[i];
-                        d1[q0 + i] = uu[i];
-                        if (ug) ug[q0 + i] = uv[i] + f2d_bits(uu[i]);
-                    }
+            for (int i = 0; i < 4; ++i) {
+                const int q = h + i;
+                if (q >= nb) continue;
+                const float x = KIND == MX_W ? v[q] : v[q] + pre[q];
+                row.d0[b0 + q] = x;
+                if (KIND == MX_DOWN) {
+                    row.d1[b0 + q] = x;
+                    if (row.state) row.state[b0 + q] = u[i] + f2d_bits(x);
+                }
             }
         }
     }
@@ -370,6 +400,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     // the row's result at a unit's end) and its prefetched epilogue operand (w for DOWN, hc for H)
     float v[32];
     float pre[32];
+    TcRow row{};
     bool ep_ok = true;
 
     if (warp == 7) {
@@ -550,7 +581,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             const int u = gch / cpu;
             if (gch - u * cpu == 0) {
                 const int grow = tile_of(u) * kTM + t;
-                if (grow < R) tc_prefetch_row<KIND>(items, s, B, b0, sh.rows_item, grow, pre, vec);
+                row = tc_row<KIND>(items, s, B, sh.rows_item, grow, grow < R);
+                tc_prefetch<KIND>(row, B, b0, pre, vec);
             }
             const int bf = gch % NP;
             if (!(ep_ok = tc_wait(&acc_full[bf], unsigned(gch / NP) & 1u, abort_flag))) break;
@@ -573,7 +605,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             mbar_arrive(&acc_empty[bf]);
             if ((gch + 1) % cpu != 0) continue;
             // ---- epilogue of the unit ----
-            const int tile = tile_of(u);
 #pragma unroll
             for (int q = 0; q < 32; ++q) {
                 v[q] += rlo[q];
@@ -585,8 +616,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 put_partial(base, v, t, 128);
                 break;  // the cluster reduction and the epilogue follow below
             }
-            const int grow = tile * kTM + t;
-            if (grow < R) tc_store_row<KIND>(items, s, B, b0, sh.rows_item, grow, v, pre, vec);
+            tc_store<KIND>(row, B, b0, v, pre, vec);
 #pragma unroll
             for (int q = 0; q < 32; ++q) v[q] = 0.f;
         }
@@ -603,12 +633,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             put_partial(base, v, tid, 128);
         }
         cluster.sync();
-        if (cluster.block_rank() == 0 && tid < 128 && nunits > 0 && !*abort_flag) {
+        if (cluster.block_rank() == 0 && tid < 128 && nunits > 0 && __all_sync(0xffffffffu, !*abort_flag)) {
             const int t = tid;
             for (int rk = 1; rk < ksplit; ++rk) add_partial(cluster.map_shared_rank(base, rk), v, t, 128);
-            const int tile = first_tile;
-            const int grow = tile * kTM + t;
-            if (grow < R) tc_store_row<KIND>(items, s, B, b0, sh.rows_item, grow, v, pre, vec);
+            tc_store<KIND>(row, B, b0, v, pre, vec);
         }
         cluster.sync();
     }
@@ -887,10 +915,11 @@ __global__ void __launch_bounds__(kPairThreads, 1)
             if (ksplit > 1) break;  // the cluster's reduction and the epilogue follow below
             const int2 pr = pairs[first + u * step];
             const int tile = j ? pr.y : pr.x, grow = tile * kTM + t;
-            if (tile >= 0 && grow < R) {
+            {
                 float pre[32];
-                tc_prefetch_row<KIND>(items, s, B, b0, sh.rows_item, grow, pre, vec);
-                tc_store_row<KIND>(items, s, B, b0, sh.rows_item, grow, v, pre, vec);
+                const TcRow row = tc_row<KIND>(items, s, B, sh.rows_item, grow, tile >= 0 && grow < R);
+                tc_prefetch<KIND>(row, B, b0, pre, vec);
+                tc_store<KIND>(row, B, b0, v, pre, vec);
             }
             ++u;
 #pragma unroll
@@ -911,14 +940,15 @@ __global__ void __launch_bounds__(kPairThreads, 1)
             put_partial(base, v, tid, 256);
         }
         cluster.sync();
-        if (cluster.block_rank() == 0 && tid < 256 && nunits > 0 && !*abort_flag) {
+        if (cluster.block_rank() == 0 && tid < 256 && nunits > 0 && __all_sync(0xffffffffu, !*abort_flag)) {
             for (int rk = 1; rk < ksplit; ++rk) add_partial(cluster.map_shared_rank(base, rk), v, tid, 256);
             const int2 pr = pairs[first];
             const int tile = tid >> 7 ? pr.y : pr.x, grow = tile * kTM + (tid & 127);
-            if (tile >= 0 && grow < R) {
+            {
                 float pre[32];
-                tc_prefetch_row<KIND>(items, s, B, b0, sh.rows_item, grow, pre, vec);
-                tc_store_row<KIND>(items, s, B, b0, sh.rows_item, grow, v, pre, vec);
+                const TcRow row = tc_row<KIND>(items, s, B, sh.rows_item, grow, tile >= 0 && grow < R);
+                tc_prefetch<KIND>(row, B, b0, pre, vec);
+                tc_store<KIND>(row, B, b0, v, pre, vec);
             }
         }
         cluster.sync();
