@@ -422,8 +422,9 @@ void leaf_eigen(cudaStream_t st, int mode, const LeafType* types, const LeafItem
                 int nmax) {
     if (nitems <= 0) return;
     if (nmax == 16 && (mode == LEAF_NEUMANN || mode == LEAF_SOLVE)) {
-        // up to about seven leaves per SM a block per leaf is faster (64 leaves 37 -> 9 us, 1024 leaves 40 -> 34 us)
-        if (nitems <= 1024) {
+        // up to six leaves per SM a block per leaf is faster (Neumann and solve steps: 64 leaves 12 and 12 us against 39
+        // and 48, 256 leaves 17 and 18 against 39 and 49; 1024 leaves 41 and 51 against 39 and 49)
+        if (nitems <= 6 * 152) {
             if (mode == LEAF_NEUMANN) launch_chained(Chain::few, k_leaf16d_wide<LEAF_NEUMANN>, dim3(unsigned(nitems)), 256, 0, st, types, items);
             else launch_chained(Chain::few, k_leaf16d_wide<LEAF_SOLVE>, dim3(unsigned(nitems)), 256, 0, st, types, items);
             ++g_kernel_launches;

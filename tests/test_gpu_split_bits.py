@@ -1,6 +1,6 @@
 """A right-hand side on a whole tree against the same tree as a top part and subtrees, bit for bit: the long levels of
 the whole tree and the short ones of a subtree share out their dot products in different ways (and 16 x 16 leaves are
-solved by another kernel up to 1024 of them), but add in one order."""
+solved by another kernel up to some hundreds of them), but add in one order."""
 import numpy as np
 import pytest
 
