@@ -846,7 +846,7 @@ void Hps::root_from_bc() {
     if (!same) {
         // A^-1 by the merges' block elimination where its residual is that of a pivoted LU, else the LU: the
         // factors' 2 x 4M steps of a solve are a chain, a product with A^-1 is not (1280 x 1280: 18 ms for LU and
-        // one solve, 3.8 ms for the inverse, its check and a solve)
+        // one solve, 2.8 ms for the inverse, its check and a solve)
         root_assemble(st_, m, d_bca_, d_bcb_, nodes_[0].T, d_rootA_);
         check(cudaMemsetAsync(d_rootinfo_, 0, sizeof(int), st_), "memset root info");
         root_inverse_ = false;

@@ -149,7 +149,8 @@ __device__ __forceinline__ void copy8_async(double* dst, const double* src) {
 // with y_{I-1} and y_I in registers (the loops are unrolled to NP >= n rows), every band entry read once per
 // warp as a broadcast; the backward substitution the same with U_II, U_{I,I+1}.  y goes through `scratch` (4n
 // consecutive values per row, one n^2 x 4n slot per block) between the two.  FP64 pipe bound: 2 n^3 multiply-adds
-// per column, two per clock and SM.  Warps whose columns start in a later block (data on E) skip the blocks before it.
+// per column, two per clock and SM (1024 leaves of 32 x 32 cells: 174 ms with a column per warp, 15.9 ms).  Warps whose
+// columns start in a later block (data on E) skip the blocks before it.
 // The staged rows are spread to NP (zeros where a block row has no entry), so the loops need no bounds.
 template <int NP>
 __global__ void __launch_bounds__(128) k_fp_columns(const FpLeaf* __restrict__ leaves, const LeafItem* __restrict__ items,
@@ -373,7 +374,8 @@ __device__ __forceinline__ double rows_sum(int n, F&& coef, const double* x) {
 // In a block the n products with the previous block's values run in all lanes at once; the triangle then takes
 // one shuffle and one multiply-add per row (and the quotient by U's diagonal on the way back, from reciprocals
 // taken for the block together).  Latency bound: 2 n^2 steps of ~100 to 300 clocks, several leaves per SM, where
-// a row at a time took two reductions over the warp from global memory per row.
+// a row at a time took two reductions over the warp from global memory per row.  Solve and Neumann step of 1024 leaves
+// of 32 x 32 cells: 0.8 ms each.
 template <int MODE>
 __global__ void __launch_bounds__(32) k_fp_solve_blocks(const FpLeaf* __restrict__ leaves,
                                                         const LeafItem* __restrict__ items) {

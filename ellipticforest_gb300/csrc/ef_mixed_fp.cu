@@ -84,7 +84,9 @@ constexpr int kFpStages = 3;  // block rows in flight
 // read.  Per k a lane reads its two matrix entries and, as broadcasts, the eight right-hand sides and the
 // eight previous values of row k: six shared-memory wavefronts for 512 multiply-adds, which bounds the kernel
 // (the matrices' 512 MB of a 1024-leaf, 32 x 32 tree would take 75 us).  A warp exchanges rows inside itself, so
-// the only block barrier of a step is the ring's.  y goes through `scratch` between the sweeps.
+// the only block barrier of a step is the ring's.  y goes through `scratch` between the sweeps.  A block of 16
+// requests on that tree, four leaf solves and the rest: 5.4 ms with a group's vectors in shared memory and 2n dependent
+// products, 1.7 ms.
 // NEUMANN: g = 0, load q, write h32 = DtN(0, q).  SOLVE: load q + boundary terms of g32, add (or store,
 // accumulate == 0) the solution to u64.
 template <int MODE>
