@@ -10,6 +10,8 @@
 //     U = V [ (V^T F V) ./ (mu_x[k] + mu_y[l] + lambda) ] V^T.
 // The Neumann data follow FiniteVolumeSolver.cpp:296-353: h_W = (2/dx)(u_W - g_W),
 // h_E = -(2/dx)(u_E - g_E), h_S = (2/dy)(u_S - g_S), h_N = -(2/dy)(u_N - g_N).
+#include <cooperative_groups.h>
+
 #include <cmath>
 #include <stdexcept>
 
@@ -20,10 +22,15 @@ namespace efgb {
 
 namespace {
 
+// One leaf per cluster of `parts` blocks: a block takes a range of the rows k of V^T F and (V^T F) V, fetches the others'
+// rows of the result through distributed shared memory, and takes the same range of the rows i of U.  Every entry is
+// the same sum whatever `parts` is.  FP64 pipe bound, two multiply-adds per clock and SM (4 n^3 of them), so few
+// leaves are spread over the SMs.  A block per leaf and several, us: a right-hand side of 4 leaves of 32 x 32 cells
+// 96 / 47, of 64 of them 137 / 107; solve and DtN application of one 64 x 64 patch from host arrays 728 / 267.
 template <int MODE>
 __global__ void __launch_bounds__(256) k_leaf_eigen(const LeafType* __restrict__ types,
-                                                    const LeafItem* __restrict__ items) {
-    const LeafItem it = items[blockIdx.x];
+                                                    const LeafItem* __restrict__ items, int parts) {
+    const LeafItem it = items[blockIdx.x / parts];
     const LeafType ty = types[it.type];
     const int n = ty.n, nn = n * n;
     extern __shared__ double sm[];
@@ -31,6 +38,8 @@ __global__ void __launch_bounds__(256) k_leaf_eigen(const LeafType* __restrict__
     double* F = sm + nn;
     double* W = sm + 2 * nn;
     const int tid = threadIdx.x, nt = blockDim.x;
+    const int part = blockIdx.x % parts, per = (n + parts - 1) / parts;
+    const int r0 = min(n, part * per), r1 = min(n, r0 + per);  // this block's rows
     const double cx = 1.0 / (ty.dx * ty.dx), cy = 1.0 / (ty.dy * ty.dy);
 
     // boundary value of side `side` at position `pos` (WESN)
@@ -58,7 +67,7 @@ __global__ void __launch_bounds__(256) k_leaf_eigen(const LeafType* __restrict__
     }
     __syncthreads();
     // W = V^T F
-    for (int e = tid; e < nn; e += nt) {
+    for (int e = r0 * n + tid; e < r1 * n; e += nt) {
         const int k = e / n, j = e - (e / n) * n;
         double acc = 0.0;
         for (int i = 0; i < n; ++i) acc = fma(V[i * n + k], F[i * n + j], acc);
@@ -66,15 +75,25 @@ __global__ void __launch_bounds__(256) k_leaf_eigen(const LeafType* __restrict__
     }
     __syncthreads();
     // F = (W V) ./ D
-    for (int e = tid; e < nn; e += nt) {
+    for (int e = r0 * n + tid; e < r1 * n; e += nt) {
         const int k = e / n, l = e - (e / n) * n;
         double acc = 0.0;
         for (int j = 0; j < n; ++j) acc = fma(W[k * n + j], V[j * n + l], acc);
         F[e] = acc * ty.Dinv[e];
     }
-    __syncthreads();
+    if (parts > 1) {
+        auto cluster = cooperative_groups::this_cluster();
+        cluster.sync();
+        for (int e = tid; e < nn; e += nt) {
+            const int owner = e / n / per;
+            if (owner != part) F[e] = cluster.map_shared_rank(F, owner)[e];
+        }
+        cluster.sync();  // the others have read this block's rows (and all threads have written theirs)
+    } else {
+        __syncthreads();
+    }
     // W = V F
-    for (int e = tid; e < nn; e += nt) {
+    for (int e = r0 * n + tid; e < r1 * n; e += nt) {
         const int i = e / n, l = e - (e / n) * n;
         double acc = 0.0;
         for (int k = 0; k < n; ++k) acc = fma(V[i * n + k], F[k * n + l], acc);
@@ -83,7 +102,7 @@ __global__ void __launch_bounds__(256) k_leaf_eigen(const LeafType* __restrict__
     __syncthreads();
     if (MODE == LEAF_SOLVE) {
         // U = W V^T
-        for (int e = tid; e < nn; e += nt) {
+        for (int e = r0 * n + tid; e < r1 * n; e += nt) {
             const int i = e / n, j = e - (e / n) * n;
             double acc = 0.0;
             for (int l = 0; l < n; ++l) acc = fma(W[i * n + l], V[j * n + l], acc);
@@ -100,6 +119,7 @@ __global__ void __launch_bounds__(256) k_leaf_eigen(const LeafType* __restrict__
             else if (side == 1) { i = n - 1; j = pos; }
             else if (side == 2) { i = pos; j = 0; }
             else { i = pos; j = n - 1; }
+            if (i < r0 || i >= r1) continue;
             double u = 0.0;
             for (int l = 0; l < n; ++l) u = fma(W[i * n + l], V[j * n + l], u);
             const double gv = gval(side, pos);
@@ -391,7 +411,23 @@ void launch_leaf(cudaStream_t st, const LeafType* types, const LeafItem* items, 
     // set on every call (cheap, and the current device may change between calls); a once-only flag
     // would be shared unsynchronised by host threads
     cudaFuncSetAttribute(k_leaf_eigen<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    k_leaf_eigen<MODE><<<nitems, 256, smem, st>>>(types, items);
+    // parts of a leaf: blocks for the SMs, eight rows or more each
+    int parts = 1;
+    while (parts < 8 && 2LL * parts * nitems <= 152 && nmax / (2 * parts) >= 8) parts *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(nitems) * parts);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = unsigned(parts);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = parts > 1 ? 1 : 0;
+    // (a launch that fails is found by the caller's cudaGetLastError)
+    cudaLaunchKernelEx(&cfg, k_leaf_eigen<MODE>, types, items, parts);
     ++g_kernel_launches;
 }
 

@@ -1,6 +1,6 @@
 """A right-hand side on a whole tree against the same tree as a top part and subtrees, bit for bit: the long levels of
-the whole tree and the short ones of a subtree share out their dot products in different ways (and 16 x 16 leaves are
-solved by another kernel up to some hundreds of them), but add in one order."""
+the whole tree and the short ones of a subtree share out their dot products in different ways, and few leaves are spread
+over more blocks (16 x 16 ones by a kernel of their own), but every sum is added in one order."""
 import numpy as np
 import pytest
 
@@ -10,7 +10,7 @@ from ellipticforest_gb300 import _lib
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("L, n, cut", [(6, 16, 2), (6, 10, 3), (5, 13, 2), (5, 32, 2), (5, 7, 1)])
+@pytest.mark.parametrize("L, n, cut", [(6, 16, 2), (6, 10, 3), (5, 13, 2), (5, 32, 2), (5, 7, 1), (4, 33, 2), (3, 64, 2)])
 def test_subtrees_equal_the_whole_tree(L, n, cut):
     solver = ef.FiniteVolumeSolver(solver_type=ef.FISHPACK90)
     mesh = ef.Mesh().uniform(L, ef.FiniteVolumePatch(ef.FiniteVolumeGrid(n, -1.0, 1.0, n, -1.0, 1.0)))
