@@ -654,7 +654,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 // per clock, against 1,180 for one node in k_mx_umma (measured: about 1,800 and 1,950).  Per stage 48 KB of A
 // and 24 KB of X; the rows of X come straight into registers one chunk ahead (an FP32 copy in shared memory would
 // cost the third stage and its bandwidth).  All node GEMMs of a block of 32 requests on a 7-level tree with
-// 16 x 16 leaves, two passes: 1.65 ms by single tiles, 1.39 ms.
+// 16 x 16 leaves, two passes: 1.65 ms by single tiles, 1.39 ms (1.32 since the epilogue exchanges pieces).
 // Roles: warps 0-7 collect and write (four per node), warps 8-15 stage X, warp 16 issues the MMAs, warp 17 copies A.
 constexpr int kPairThreads = 576, kPairStage = 256, kPairStages = 3, kPairSets = 2;
 constexpr int kPairCols = 2 * kTB;  // right-hand side columns per plane
