@@ -271,7 +271,9 @@ void Hps::allocate() {
 
     const bool fp = solver_type_ == SOLVER_FIVE_POINT;
     auto layout = [&](Carver& cv) {
-        for (auto& ty : types_) ty.T = cv.get<double>(size_t(16) * nn);
+        // (without gaps: one launch writes the maps of many types)
+        double* T = cv.get<double>(types_.size() * 16 * nn);
+        for (size_t t = 0; t < types_.size(); ++t) types_[t].T = T ? T + t * 16 * nn : nullptr;
         if (fp) {
             // per leaf: coefficients [alpha | beta W,E,S,N | lambda], band LU, boundary coefficients
             d_coef_ = cv.get<double>(size_t(L) * 6 * nn);
@@ -579,21 +581,26 @@ void Hps::build_leaf_types() {
         pe(double(types_.size()) * 16 * n * n * 8, double(nitems_dtn_) * (6 * n * n * n + 8 * n * n));
         return;
     }
-    // one DtN per distinct leaf geometry (the types' T lie one after another)
-    std::vector<double> dx, dy;
+    // One DtN per distinct leaf geometry.  Which form a type takes depends on the type alone, never on the others of the
+    // tree: an incremental build and a subtree take over maps of trees with other leaves.
+    std::vector<double> dx, dy;  // of the types whose maps come from an LU
     std::vector<double*> T;
-    for (const auto& ty : types_) {
-        dx.push_back(ty.dx);
-        dy.push_back(ty.dy);
-        T.push_back(ty.T);
-    }
     const double nn = n * n, nt = double(types_.size());
-    bool modes = true;
-    for (size_t t = 0; t < types_.size(); ++t)
-        modes = modes && leaf_dtn_definite(n_, lambda_, dx[t], dy[t]) && T[t] == T[0] + t * 16 * size_t(n_) * n_;
     pb("leaf_dtn");
-    if (modes) leaf_dtn_modes(st_, n_, lambda_, d_types_, int(types_.size()), T[0]);
-    else leaf_singular_ = leaf_dtn_lu(st_, n_, lambda_, dx, dy, T);
+    for (size_t t = 0; t < types_.size();) {
+        if (!leaf_dtn_definite(n_, lambda_, types_[t].dx, types_[t].dy)) {
+            dx.push_back(types_[t].dx);
+            dy.push_back(types_[t].dy);
+            T.push_back(types_[t].T);
+            ++t;
+            continue;
+        }
+        size_t end = t + 1;
+        while (end < types_.size() && leaf_dtn_definite(n_, lambda_, types_[end].dx, types_[end].dy)) ++end;
+        leaf_dtn_modes(st_, n_, lambda_, d_types_ + t, int(end - t), types_[t].T);
+        t = end;
+    }
+    if (!T.empty()) leaf_singular_ = leaf_dtn_lu(st_, n_, lambda_, dx, dy, T);
     pe(nt * 8 * (2 * nn * nn + 2 * nn * 4 * n + 16 * n * n),
        nt * (2.0 / 3.0 * nn * nn * nn + 2.0 * nn * nn * 4 * n));
 }
