@@ -607,6 +607,7 @@ void Hps::build_leaf_types() {
 
 void Hps::build() {
     root_lu_valid_ = false;
+    built_ = false;  // until it succeeds
     top_level_ = -1;
     for (const auto& g : groups_) merge_workspace(g.distinct, g.s);
     build_leaf_types();
@@ -620,6 +621,7 @@ void Hps::build() {
     if (merges_rejected(mesh_.max_level)) {
         merge_levels(mesh_.max_level - 1, true, true);
         check(cudaStreamSynchronize(st_), "build sync");
+        check_merge_waits();
     }
     singular_ = count_singular(mesh_.max_level, true) + leaf_singular_;
     if (solver_type_ == SOLVER_FIVE_POINT) {
@@ -668,14 +670,18 @@ bool Hps::merge_workspace(int cnt, int s) {
     return !merge64_supported(s) || reserve(merge64_workspace(cnt, s));
 }
 
-bool Hps::merges_rejected(int below) {
-    if (!d_ws_) return false;
+void Hps::check_merge_waits() {
+    if (!d_ws_) return;
     int err = 0;
     check(cudaMemcpy(&err, d_wserr_, sizeof(int), cudaMemcpyDeviceToHost), "merge error");
-    if (err) {
-        check(cudaMemset(d_wserr_, 0, sizeof(int)), "merge error");
-        throw std::runtime_error("CUDA error in build: an operand copy of a merge did not complete");
-    }
+    if (!err) return;
+    check(cudaMemset(d_wserr_, 0, sizeof(int)), "merge error");
+    throw std::runtime_error("CUDA error in build: an operand copy of a merge did not complete");
+}
+
+bool Hps::merges_rejected(int below) {
+    check_merge_waits();
+    if (!d_ws_) return false;
     for (auto& g : groups_) {
         if (g.level >= below || !merge64_supported(g.s)) continue;
         std::vector<int> info(g.nodes.size());
@@ -721,6 +727,7 @@ void Hps::merge_nodes(const MergeTables& t, int cnt, int s, bool careful) {
     merge64(st_, t.items, cnt, s, t.info, d_ws_, d_wserr_);
     pe(c * 8 * 12 * dm * dm, c * 8.0 * dm * dm * dm);
     if (!careful) return;
+    if (inject_merge_error_) check(cudaMemsetAsync(d_wserr_, 1, sizeof(int), st_), "merge error test");
     std::vector<int> info(cnt);
     check(cudaMemcpyAsync(info.data(), t.info, cnt * sizeof(int), cudaMemcpyDeviceToHost, st_), "merge info");
     check(cudaStreamSynchronize(st_), "merge info");

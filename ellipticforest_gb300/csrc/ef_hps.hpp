@@ -234,6 +234,7 @@ public:
     int solver_type() const { return solver_type_; }
     cudaStream_t stream() const { return st_; }
     void set_homogeneous_rhs(bool v) { homogeneous_ = v; }
+    void set_inject_merge_error(bool v) { inject_merge_error_ = v; }
     // true when the boundary coefficient b of a*u + b*du/dn = r is not identically zero
     void set_bc_general(bool v) { bc_general_ = v; }
     bool homogeneous_rhs() const { return homogeneous_; }
@@ -323,6 +324,7 @@ private:
     bool merge_workspace(int cnt, int s);  // room for merge64; false: not available, merge by LU
     bool reserve(size_t bytes);            // d_ws_ of at least that many bytes
     bool merges_rejected(int below);       // block elimination set info in some merge of levels < below
+    void check_merge_waits();              // throws where a wait of the merges' kernels gave up (after a sync)
     void upward_levels(int top);      // upward pass of levels top .. 0
     void downward_levels(int bottom, bool uncoarsen_bottom);  // split from the root to level `bottom`
     int count_singular(int below, bool distinct);  // zero pivots among the merges of levels < below
@@ -364,6 +366,7 @@ private:
     size_t ws_bytes_ = 0;
     int* d_wserr_ = nullptr;
     bool ws_refused_ = false;
+    bool inject_merge_error_ = false;  // failure-path test: careful merges set the error word
     bool equal_operators_ = false;  // nodes of equal subtrees have equal operators
 
     double *d_f_ = nullptr, *d_u_ = nullptr;

@@ -52,6 +52,7 @@ void Hps::build_from(const Hps& old) {
         old.mesh_.yl != mesh_.yl || old.mesh_.yu != mesh_.yu)
         throw std::invalid_argument("incremental build: domain, patch size or lambda differ");
     root_lu_valid_ = false;
+    built_ = false;  // until it succeeds
     top_level_ = -1;
     const std::vector<uint64_t> sn = signatures(mesh_), so = signatures(old.mesh_);
     std::map<std::tuple<int, int64_t, int64_t>, int> old_id;
@@ -119,8 +120,12 @@ void Hps::build_from(const Hps& old) {
     const size_t ncopy = cdst.size();
     const size_t c_src = reserve(ncopy * sizeof(void*)), c_dst = reserve(ncopy * sizeof(void*)),
                  c_len = reserve(ncopy * sizeof(long long));
-    unsigned char* dev = nullptr;
-    cki(cudaMalloc(&dev, host.size() + 256), "cudaMalloc(incremental tables)");
+    struct Tables {
+        unsigned char* p = nullptr;
+        ~Tables() { cudaFree(p); }
+    } tables;
+    cki(cudaMalloc(&tables.p, host.size() + 256), "cudaMalloc(incremental tables)");
+    unsigned char* const dev = tables.p;
     static const int cb[8] = {0, 2, 1, 3, 0, 1, 2, 3};
     static const int ia[4] = {0, 1, 0, 1}, ib[4] = {2, 2, 3, 3};
     std::vector<MergeItem> all_items;
@@ -202,15 +207,15 @@ void Hps::build_from(const Hps& old) {
         }
         return n;
     };
-    merges_rejected(0);  // a wait that gave up
+    check_merge_waits();
     int bad = marked();
     if (bad > 0) {
         merge_dirty(true);
         cki(cudaStreamSynchronize(st_), "incremental build sync");
+        check_merge_waits();
         bad = marked();
     }
     singular_ = leaf_singular_ + bad;
-    cudaFree(dev);
     equal_operators_ = false;  // the reused operators come from another tree
     built_ = true;
 }

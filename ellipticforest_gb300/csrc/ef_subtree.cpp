@@ -84,6 +84,7 @@ void Hps::build_top(int level, const double* const* T_host) {
     if (merges_rejected(level)) {
         merge_levels(level - 1, false, true);
         check(cudaStreamSynchronize(st_), "top build sync");
+        check_merge_waits();
     }
     singular_ = count_singular(level, false);
     top_level_ = level;
