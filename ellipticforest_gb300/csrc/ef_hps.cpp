@@ -825,7 +825,7 @@ void Hps::root_from_bc() {
     pb("root_general");
     if (!d_rootA_) {
         const size_t bytes = align_up(size_t(m) * m * 8) + 4 * align_up(size_t(m) * 8) +
-                             2 * align_up(size_t(m) * 4) + 2 * align_up(sizeof(int)) + 4 * align_up(sizeof(void*));
+                             2 * align_up(size_t(m) * 4) + 2 * align_up(sizeof(int)) + 5 * align_up(sizeof(void*));
         check(cudaMalloc(&d_rootA_, bytes), "cudaMalloc(root)");
         Carver cv;
         cv.base = reinterpret_cast<char*>(d_rootA_);
@@ -840,6 +840,7 @@ void Hps::root_from_bc() {
         d_rootb_ = cv.get<double>(m);
         d_rootA_arr_ = cv.get<double*>(1);
         d_rootrhs_arr_ = cv.get<double*>(1);
+        d_roottmp_arr_ = cv.get<double*>(1);
         d_rootpiv_arr_ = cv.get<int*>(1);
         d_rootperm_arr_ = cv.get<int*>(1);
         check(upload_sync(st_, d_rootA_arr_, &d_rootA_, sizeof(void*)), "root arr");
@@ -861,19 +862,21 @@ void Hps::root_from_bc() {
         // A^-1 by the merges' block elimination where its residual is that of a pivoted LU, else the LU: the
         // factors' 2 x 4M steps of a solve are a chain, a product with A^-1 is not (1280 x 1280: 18 ms for LU and
         // one solve, 2.8 ms for the inverse, its check and a solve)
+        root_lu_valid_ = false;  // what was kept is overwritten from here on
         root_assemble(st_, m, d_bca_, d_bcb_, nodes_[0].T, d_rootA_);
         check(cudaMemsetAsync(d_rootinfo_, 0, sizeof(int), st_), "memset root info");
         root_inverse_ = false;
         const size_t digits = (invert64_workspace(m) + 1023) / 1024 * 1024, tmp = invert64_tmp(m) * sizeof(double);
         if (m <= 32768 && reserve(digits + tmp)) {
             double* t = reinterpret_cast<double*>(d_ws_ + digits);
-            check(upload_sync(st_, d_rootrhs_arr_, &t, sizeof(void*)), "root tmp");
-            invert64(st_, d_rootA_arr_, d_rootrhs_arr_, m, d_rootinfo_, d_ws_, d_wserr_);
+            check(upload_sync(st_, d_roottmp_arr_, &t, sizeof(void*)), "root tmp");
+            invert64(st_, d_rootA_arr_, d_roottmp_arr_, m, d_rootinfo_, d_ws_, d_wserr_);
+            if (inject_merge_error_) check(cudaMemsetAsync(d_wserr_, 1, sizeof(int), st_), "root error test");
             root_check(st_, m, nodes_[0].T, d_bca_, d_bcb_, d_rootA_, d_rootrhs_, nodes_[0].g, d_rootinfo_);
             int info = 0, err = 0;
             check(cudaMemcpyAsync(&info, d_rootinfo_, sizeof(int), cudaMemcpyDeviceToHost, st_), "root info");
             check(cudaMemcpyAsync(&err, d_wserr_, sizeof(int), cudaMemcpyDeviceToHost, st_), "root error");
-            check(upload_sync(st_, d_rootrhs_arr_, &d_rootrhs_, sizeof(void*)), "root arr");
+            check(cudaStreamSynchronize(st_), "root info");
             if (err) {
                 check(cudaMemsetAsync(d_wserr_, 0, sizeof(int), st_), "root error");
                 throw std::runtime_error("CUDA error in the root solve: an operand copy did not complete");

@@ -366,7 +366,7 @@ private:
     size_t ws_bytes_ = 0;
     int* d_wserr_ = nullptr;
     bool ws_refused_ = false;
-    bool inject_merge_error_ = false;  // failure-path test: careful merges set the error word
+    bool inject_merge_error_ = false;  // failure-path test: careful merges and the root's inverse set the error word
     bool equal_operators_ = false;  // nodes of equal subtrees have equal operators
 
     double *d_f_ = nullptr, *d_u_ = nullptr;
@@ -381,6 +381,7 @@ private:
     long long root_factorizations_ = 0;
     double** d_rootA_arr_ = nullptr;
     double** d_rootrhs_arr_ = nullptr;
+    double** d_roottmp_arr_ = nullptr;
     int** d_rootpiv_arr_ = nullptr;
     int** d_rootperm_arr_ = nullptr;
 

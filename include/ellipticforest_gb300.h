@@ -87,7 +87,8 @@ int ef_hps_set_coefficients(ef_hps* hps, const double* alpha, const double* beta
  * without coarsening steps (which otherwise read and difference them in place).  Both give the same
  * results bit for bit; "inject-wait-timeout" 1 makes the tensor-core GEMMs' first wait run out
  * (failure-path test: the solve returns EF_ERR_CUDA).  "inject-merge-error" 1 (this handle) sets the
- * merges' error word while a build redoes rejected merges (the build then returns EF_ERR_CUDA). */
+ * merges' error word while a build redoes rejected merges or a solve inverts a general root operator
+ * (the call then returns EF_ERR_CUDA). */
 int ef_hps_set_option(ef_hps* hps, const char* key, int value);
 /* Use an external CUDA stream (cudaStream_t) for all work of this handle; NULL = default stream. */
 int ef_hps_set_stream(ef_hps* hps, void* cuda_stream);
