@@ -85,7 +85,7 @@ void Hps::allocate32() {
     Carver32 dry;
     layout(dry);
     arena32_bytes_ = dry.off;
-    ck32(cudaMalloc(&arena32_, arena32_bytes_), "cudaMalloc(FP32 operators)");
+    ck32(device_alloc(reinterpret_cast<void**>(&arena32_), arena32_bytes_), "cudaMalloc(FP32 operators)");
     Carver32 real;
     real.base = arena32_;
     layout(real);

@@ -376,6 +376,12 @@ int ef_hps_set_option(ef_hps* h, const char* key, int value) {
         });
     } else if (k == "inject-merge-error") {
         h->hps->set_inject_merge_error(value != 0);  // failure-path test of the build's second pass
+    } else if (k == "workspace-limit-mb") {
+        if (value < 0) return fail(EF_ERR_INVALID, "workspace-limit-mb: 0 none, else at least 1");
+        return guarded([&] {
+            h->hps->set_workspace_limit(value == 0 ? ~size_t(0) : size_t(value) << 20);
+            return EF_OK;
+        });
     } else if (k == "tensor-cores") {
         if (value < 0 || value > 2) return fail(EF_ERR_INVALID, "tensor-cores: 0 off, 1 tuned, 2 forced");
         h->hps->set_tensor_cores(value);  // block solvers created from now on

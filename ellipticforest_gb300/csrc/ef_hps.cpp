@@ -12,6 +12,7 @@
 #include <cmath>
 #include <cstring>
 #include <map>
+#include <new>
 #include <stdexcept>
 #include <string>
 
@@ -600,7 +601,14 @@ void Hps::build_leaf_types() {
         leaf_dtn_modes(st_, n_, lambda_, d_types_ + t, int(end - t), types_[t].T);
         t = end;
     }
-    if (!T.empty()) leaf_singular_ = leaf_dtn_lu(st_, n_, lambda_, dx, dy, T);
+    if (!T.empty()) {
+        try {
+            leaf_singular_ = leaf_dtn_lu(st_, n_, lambda_, dx, dy, T);
+        } catch (const std::bad_alloc&) {
+            if (!release_workspace()) throw;
+            leaf_singular_ = leaf_dtn_lu(st_, n_, lambda_, dx, dy, T);
+        }
+    }
     pe(nt * 8 * (2 * nn * nn + 2 * nn * 4 * n + 16 * n * n),
        nt * (2.0 / 3.0 * nn * nn * nn + 2.0 * nn * nn * 4 * n));
 }
@@ -609,8 +617,10 @@ void Hps::build() {
     root_lu_valid_ = false;
     built_ = false;  // until it succeeds
     top_level_ = -1;
-    for (const auto& g : groups_) merge_workspace(g.distinct, g.s);
     build_leaf_types();
+    std::vector<int> counts;
+    for (const auto& g : groups_) counts.push_back(g.distinct);
+    reserve_merges(counts);
     // the merges of every level (a fixed launch sequence for this tree) replay as a CUDA graph from
     // the third build on (first eager, second captured); the leaf DtN maps above stay eager
     const long long l0 = g_kernel_launches.load();
@@ -648,26 +658,67 @@ std::vector<int> Hps::operator_classes(size_t group) const {
 bool Hps::reserve(size_t need) {
     need = (need + 1023) / 1024 * 1024 + 1024;  // and the error word
     if (need <= ws_bytes_) return true;
-    if (ws_refused_) return false;
+    if (need > ws_limit_) return false;
     check(cudaStreamSynchronize(st_), "workspace sync");
-    graph_build_.clear();  // the captured merges point into the old workspace
-    if (d_ws_) cudaFree(d_ws_);
+    auto take = [&](size_t bytes) {
+        char* p = nullptr;
+        if (cudaMalloc(&p, bytes) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        release_workspace();
+        graph_build_.clear();  // merges captured without a workspace
+        d_ws_ = p;
+        ws_bytes_ = bytes;
+        d_wserr_ = reinterpret_cast<int*>(d_ws_ + bytes - 1024);
+        check(cudaMemsetAsync(d_wserr_, 0, sizeof(int), st_), "memset workspace error");
+        return true;
+    };
+    // beside the one there is, which stays where the larger one is refused
+    if (take(need)) return true;
+    size_t free = 0, total = 0;
+    if (!d_ws_ || cudaMemGetInfo(&free, &total) != cudaSuccess || free + ws_bytes_ < need) return false;
+    const size_t had = ws_bytes_;
+    release_workspace();
+    if (take(need)) return true;
+    (void)take(had);
+    return false;
+}
+
+bool Hps::release_workspace() {
+    if (!d_ws_) return false;
+    check(cudaStreamSynchronize(st_), "workspace sync");
+    graph_build_.clear();  // the captured merges point into it
+    cudaFree(d_ws_);
     d_ws_ = nullptr;
+    d_wserr_ = nullptr;
     ws_bytes_ = 0;
-    if (cudaMalloc(&d_ws_, need) != cudaSuccess) {
-        (void)cudaGetLastError();
-        d_ws_ = nullptr;
-        ws_refused_ = true;
-        return false;
-    }
-    ws_bytes_ = need;
-    d_wserr_ = reinterpret_cast<int*>(d_ws_ + need - 1024);
-    check(cudaMemsetAsync(d_wserr_, 0, sizeof(int), st_), "memset workspace error");
     return true;
 }
 
-bool Hps::merge_workspace(int cnt, int s) {
-    return !merge64_supported(s) || reserve(merge64_workspace(cnt, s));
+void Hps::set_workspace_limit(size_t bytes) {
+    ws_limit_ = bytes;
+    if (ws_bytes_ > bytes) release_workspace();
+}
+
+cudaError_t Hps::device_alloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && d_ws_) {
+        (void)cudaGetLastError();
+        release_workspace();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
+void Hps::reserve_merges(const std::vector<int>& counts) {
+    size_t most = 0;
+    for (size_t g = 0; g < groups_.size(); ++g)
+        if (counts[g] > 0 && merge64_supported(groups_[g].s)) most = std::max(most, merge64_workspace(counts[g], groups_[g].s));
+    if (!most || reserve(most)) return;
+    // what the smaller groups need, where the largest gets no room
+    for (size_t g = 0; g < groups_.size(); ++g)
+        if (counts[g] > 0 && merge64_supported(groups_[g].s)) (void)reserve(merge64_workspace(counts[g], groups_[g].s));
 }
 
 void Hps::check_merge_waits() {
@@ -826,7 +877,7 @@ void Hps::root_from_bc() {
     if (!d_rootA_) {
         const size_t bytes = align_up(size_t(m) * m * 8) + 4 * align_up(size_t(m) * 8) +
                              2 * align_up(size_t(m) * 4) + 2 * align_up(sizeof(int)) + 5 * align_up(sizeof(void*));
-        check(cudaMalloc(&d_rootA_, bytes), "cudaMalloc(root)");
+        check(device_alloc(reinterpret_cast<void**>(&d_rootA_), bytes), "cudaMalloc(root)");
         Carver cv;
         cv.base = reinterpret_cast<char*>(d_rootA_);
         cv.get<double>(size_t(m) * m);

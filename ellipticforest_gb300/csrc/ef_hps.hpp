@@ -296,7 +296,12 @@ public:
     int indefinite_count() const { return indefinite_; }
     // LU factorisations of the general root matrix diag(a) + diag(b) T so far (cached across solves)
     long long root_factorizations() const { return root_factorizations_; }
-    size_t device_bytes() const { return arena_bytes_; }
+    size_t device_bytes() const { return arena_bytes_ + ws_bytes_; }
+    // The workspace of builds and general root solves is grown to what they need and kept: up to 0.5 GB for merges,
+    // 1.6 GB for a root operator of 8192 rows.  Where there is no room for it, merges and root operators are
+    // factored by the pivoted LU.
+    void set_workspace_limit(size_t bytes);
+    bool release_workspace();  // true: there was one
 
     // Counters for the roofline: flops of the build by kernel family (FP64).
     double build_flops() const;
@@ -321,9 +326,12 @@ private:
     void merge_levels(int top, bool distinct, bool careful);
     void merge_nodes(const MergeTables& t, int cnt, int s, bool careful);
     void merge_lu(const MergeTables& t, int cnt, int s);  // from the gathered X, H and T_LHS on
-    bool merge_workspace(int cnt, int s);  // room for merge64; false: not available, merge by LU
-    bool reserve(size_t bytes);            // d_ws_ of at least that many bytes
+    // room for merge64 of counts[g] nodes of each group g, as far as it can be had (without it a group merges by LU)
+    void reserve_merges(const std::vector<int>& counts);
+    bool reserve(size_t bytes);            // d_ws_ of at least that many bytes; false: refused, what there was stays
     bool merges_rejected(int below);       // block elimination set info in some merge of levels < below
+    // device memory, giving back the workspace where there is none left
+    cudaError_t device_alloc(void** p, size_t bytes);
     void check_merge_waits();              // throws where a wait of the merges' kernels gave up (after a sync)
     void upward_levels(int top);      // upward pass of levels top .. 0
     void downward_levels(int bottom, bool uncoarsen_bottom);  // split from the root to level `bottom`
@@ -361,11 +369,11 @@ private:
     LeafItem *d_items_dtn_ = nullptr, *d_items_neu_ = nullptr, *d_items_solve_ = nullptr;
     int nitems_dtn_ = 0;
 
-    // digits of the merges' products, grown to what a build needs, and the error word of their waits
+    // digits of the merges' products, grown to what a build needs, and the error word of their waits (at its end)
     char* d_ws_ = nullptr;
     size_t ws_bytes_ = 0;
     int* d_wserr_ = nullptr;
-    bool ws_refused_ = false;
+    size_t ws_limit_ = ~size_t(0);
     bool inject_merge_error_ = false;  // failure-path test: careful merges and the root's inverse set the error word
     bool equal_operators_ = false;  // nodes of equal subtrees have equal operators
 

@@ -124,7 +124,7 @@ void Hps::build_from(const Hps& old) {
         unsigned char* p = nullptr;
         ~Tables() { cudaFree(p); }
     } tables;
-    cki(cudaMalloc(&tables.p, host.size() + 256), "cudaMalloc(incremental tables)");
+    cki(device_alloc(reinterpret_cast<void**>(&tables.p), host.size() + 256), "cudaMalloc(incremental tables)");
     unsigned char* const dev = tables.p;
     static const int cb[8] = {0, 2, 1, 3, 0, 1, 2, 3};
     static const int ia[4] = {0, 1, 0, 1}, ib[4] = {2, 2, 3, 3};
@@ -173,8 +173,9 @@ void Hps::build_from(const Hps& old) {
     copy_batched(st_, reinterpret_cast<const double* const*>(at(c_src)), reinterpret_cast<double* const*>(at(c_dst)),
                  reinterpret_cast<const long long*>(at(c_len)), int(ncopy), std::accumulate(clen.begin(), clen.end(), 0LL));
     const int maxL = mesh_.max_level;
-    for (size_t gi = 0; gi < groups_.size(); ++gi)
-        if (sub[gi].cnt) merge_workspace(sub[gi].cnt, groups_[gi].s);
+    std::vector<int> counts;
+    for (const auto& sb : sub) counts.push_back(sb.cnt);
+    reserve_merges(counts);
     auto merge_dirty = [&](bool careful) {
         for (int lvl = maxL - 1; lvl >= 0; --lvl) {
             for (size_t k = 0; k < tsteps_.size(); ++k)

@@ -21,6 +21,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <new>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -263,7 +264,12 @@ int leaf_dtn_lu(cudaStream_t st, int n, double lambda, const std::vector<double>
                  oQ = oP + up(nt * nn * 4), oI = oQ + up(nt * nn * 4), oDx = oI + up(nt * 4),
                  oDy = oDx + up(nt * 8), oArr = oDy + up(nt * 8), total = oArr + up(6 * nt * sizeof(void*));
     char* buf = nullptr;
-    ck(cudaMalloc(&buf, total), "cudaMalloc(leaf DtN LU)");
+    const cudaError_t got = cudaMalloc(&buf, total);
+    if (got == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        throw std::bad_alloc();
+    }
+    ck(got, "cudaMalloc(leaf DtN LU)");
     std::vector<void*> arr(6 * nt);
     for (int t = 0; t < nt; ++t) {
         arr[0 * nt + t] = buf + oA + t * nn * nn * 8;  // A (LU in place)

@@ -232,7 +232,7 @@ MixedSolver::MixedSolver(Hps& hps, int bmax, const MixedSolver* share)
     MxCarver dry;
     layout(dry);
     bytes_ = dry.off;
-    ck(cudaMalloc(&arena_, bytes_), "cudaMalloc(mixed arena)");
+    ck(hps.device_alloc(reinterpret_cast<void**>(&arena_), bytes_), "cudaMalloc(mixed arena)");
     MxCarver real;
     real.base = arena_;
     layout(real);
@@ -253,7 +253,7 @@ MixedSolver::MixedSolver(Hps& hps, int bmax, const MixedSolver* share)
         std::vector<double> V(nn), D(nn);
         std::vector<float> Vf(nn), Df(nn);
         float* tab = nullptr;
-        ck(cudaMalloc(&tab, 2 * nn * t32.size() * sizeof(float)), "cudaMalloc(fp32 tables)");
+        ck(hps.device_alloc(reinterpret_cast<void**>(&tab), 2 * nn * t32.size() * sizeof(float)), "cudaMalloc(fp32 tables)");
         tables_ = tab;
         for (size_t t = 0; t < t32.size(); ++t) {
             leaf_tables(n, hps.types_[t].dx, hps.types_[t].dy, hps.lambda_, V.data(), D.data());
@@ -609,7 +609,7 @@ void MixedSolver::set_root_operator(const double* a, const double* b) {
     auto up = [](size_t x) { return (x + 255) / 256 * 256; };
     if (!robin_mem_) {
         const size_t bytes = up(2 * m * 8) + up(m * 4) + up(mm * 4) + 2 * up(size_t(m) * cap_ * 4) + up(3 * sizeof(void*));
-        ck(cudaMalloc(&robin_mem_, bytes), "cudaMalloc(mixed Robin root)");
+        ck(h.device_alloc(reinterpret_cast<void**>(&robin_mem_), bytes), "cudaMalloc(mixed Robin root)");
         char* p = robin_mem_;
         ra64_ = reinterpret_cast<double*>(p); rb64_ = ra64_ + m; p += up(2 * m * 8);
         rb32_ = reinterpret_cast<float*>(p); p += up(m * 4);
@@ -630,7 +630,7 @@ void MixedSolver::set_root_operator(const double* a, const double* b) {
     // Z = (diag a + diag b T)^{-1} in FP64 (LU with partial pivoting, then the solve of P I), kept in FP32
     char* tmp = nullptr;
     const size_t tbytes = 2 * up(mm * 8) + 2 * up(size_t(m) * 4) + up(4) + up(4 * sizeof(void*));
-    ck(cudaMalloc(&tmp, tbytes), "cudaMalloc(Robin factor)");
+    ck(h.device_alloc(reinterpret_cast<void**>(&tmp), tbytes), "cudaMalloc(Robin factor)");
     double* A = reinterpret_cast<double*>(tmp);
     double* Z = reinterpret_cast<double*>(tmp + up(mm * 8));
     int* piv = reinterpret_cast<int*>(tmp + 2 * up(mm * 8));

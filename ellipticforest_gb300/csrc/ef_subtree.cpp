@@ -76,8 +76,9 @@ void Hps::build_top(int level, const double* const* T_host) {
         check(cudaMemcpyAsync(nd.T, T_host[k], m * m * sizeof(double), cudaMemcpyHostToDevice, st_), "copy T block");
     }
     // the T blocks come from outside: no two are known to be equal
-    for (const auto& g : groups_)
-        if (g.level < level) merge_workspace(int(g.nodes.size()), g.s);
+    std::vector<int> counts;
+    for (const auto& g : groups_) counts.push_back(g.level < level ? int(g.nodes.size()) : 0);
+    reserve_merges(counts);
     merge_levels(level - 1, false, false);
     check(cudaGetLastError(), "top build launch");
     check(cudaStreamSynchronize(st_), "top build sync");

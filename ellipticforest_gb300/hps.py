@@ -392,12 +392,19 @@ class HPSAlgorithm:
         check(lib.ef_hps_create(mesh.handle, _solver_code(patch_solver.solver_type),
                                 float(patch_solver.lambda_function(0, 0)), C.byref(h)))
         self._h = h
-        nl, n, M, nb = C.c_int(), C.c_int(), C.c_int(), C.c_longlong()
-        check(lib.ef_hps_info(h, C.byref(nl), C.byref(n), C.byref(M), C.byref(nb)))
-        self.num_leaves, self.n, self.M, self.device_bytes = nl.value, n.value, M.value, nb.value
+        nl, n, M = C.c_int(), C.c_int(), C.c_int()
+        check(lib.ef_hps_info(h, C.byref(nl), C.byref(n), C.byref(M), None))
+        self.num_leaves, self.n, self.M = nl.value, n.value, M.value
         self._apply_options()
         if patch_solver.solver_type == FivePointStencil:
             self._set_coefficients()
+
+    @property
+    def device_bytes(self) -> int:
+        """Device memory of the tree's arrays and of the scratch that builds and general root solves have kept so far."""
+        nb = C.c_longlong()
+        check(_lib.load().ef_hps_info(self._h, None, None, None, C.byref(nb)))
+        return nb.value
 
     def save(self, path: str):
         """Solve-time operators of the built tree and its mesh to `path` (no reference counterpart)."""
@@ -411,9 +418,9 @@ class HPSAlgorithm:
         check(lib.ef_hps_load(str(path).encode(), C.byref(mh), C.byref(hh)))
         self = cls.__new__(cls)
         self._h = hh
-        nl, n, M, nb = C.c_int(), C.c_int(), C.c_int(), C.c_longlong()
-        check(lib.ef_hps_info(hh, C.byref(nl), C.byref(n), C.byref(M), C.byref(nb)))
-        self.num_leaves, self.n, self.M, self.device_bytes = nl.value, n.value, M.value, nb.value
+        nl, n, M = C.c_int(), C.c_int(), C.c_int()
+        check(lib.ef_hps_info(hh, C.byref(nl), C.byref(n), C.byref(M), None))
+        self.num_leaves, self.n, self.M = nl.value, n.value, M.value
         mesh = Mesh()
         mesh._h = mh
         boxes = []

@@ -81,6 +81,8 @@ int ef_hps_set_coefficients(ef_hps* hps, const double* alpha, const double* beta
  * Added key "tensor-cores" (default 1) for the mixed block solvers created afterwards: 0 CUDA-core
  * node GEMMs only, 1 the faster of the CUDA-core and tcgen05 GEMM per node group (timed), 2 the
  * tcgen05 GEMM wherever it supports the shape.
+ * Added key "workspace-limit-mb" (default 0, none): device memory that builds and general root solves may
+ * keep for their scratch; what finds no room in it is factored by a pivoted LU, which takes longer.
  * Verification keys (process-wide, default 0): "general-leaf-residual" 1 runs the exact residual of
  * 16 x 16 leaves through the general leaf-size kernel; "per-level-interface" 1 makes mixed block
  * solvers created afterwards move the residual's interface rows level by level even on trees
@@ -92,6 +94,7 @@ int ef_hps_set_coefficients(ef_hps* hps, const double* alpha, const double* beta
 int ef_hps_set_option(ef_hps* hps, const char* key, int value);
 /* Use an external CUDA stream (cudaStream_t) for all work of this handle; NULL = default stream. */
 int ef_hps_set_stream(ef_hps* hps, void* cuda_stream);
+/* device_bytes: the tree's arrays and the scratch that builds and general root solves have kept so far. */
 int ef_hps_info(const ef_hps* hps, int* num_leaves, int* leaf_n, int* root_M, long long* device_bytes);
 /* Number of LU factorisations of the general root matrix diag(a) + diag(b) T_root made so far.  The
  * reference factors it on every solve with b != 0 (HPSAlgorithm.hpp:402-420); here the factors are
