@@ -209,27 +209,28 @@ __device__ __forceinline__ double group_sum(double v) {
     return v;
 }
 
-// One turn of group_dot: eight units from unit `at` on, in U = double2 or double; those from n on count nothing
-// (FULL: there are none).
-template <bool FULL, int LPR, int F, class U>
-__device__ __forceinline__ void group_turn(const U* __restrict__ row, const U* __restrict__ xa, const U* __restrict__ xb,
-                                           int split, int n, int at, int lane, double* a) {
+// T half turns of group_dot from unit `at` on, in U = double2 or double, every load before the first product; units
+// from n on count nothing (FULL: there are none).
+template <bool FULL, int T, int LPR, int F, class U>
+__device__ __forceinline__ void group_batch(const U* __restrict__ row, const U* __restrict__ xa, const U* __restrict__ xb,
+                                            int split, int n, int at, int lane, double* a) {
     constexpr int NA = 4 / F;
     const int first = at + lane / LPR * NA * LPR, base = first + (lane & (LPR - 1));
-    U m[2 * NA], v[2 * NA];
+    U m[T * NA], v[T * NA];
 #pragma unroll
-    for (int u = 0; u < 2 * NA; ++u) {
+    for (int u = 0; u < T * NA; ++u) {
         const int i = base + (u % NA + 4 * (u / NA)) * LPR;
-        m[u] = FULL || i < n ? __ldcs(row + i) : U{};
+        if (FULL || i < n) m[u] = __ldcs(row + i);
     }
 #pragma unroll
-    for (int u = 0; u < 2 * NA; ++u) {
+    for (int u = 0; u < T * NA; ++u) {
         const int i = base + (u % NA + 4 * (u / NA)) * LPR;
-        v[u] = FULL || i < n ? __ldg((i < split ? xa : xb) + i) : U{};
+        if (FULL || i < n) v[u] = __ldg((i < split ? xa : xb) + i);
     }
 #pragma unroll
-    for (int u = 0; u < 2 * NA; ++u) {
-        if (!FULL && first + (u % NA + 4 * (u / NA)) * LPR >= n) continue;
+    for (int u = 0; u < T * NA; ++u) {
+        const int i = base + (u % NA + 4 * (u / NA)) * LPR;
+        if (!FULL && i >= n) continue;
         if constexpr (sizeof(U) == 16) {
             a[u % NA] = fma(m[u].x, v[u].x, a[u % NA]);
             a[u % NA] = fma(m[u].y, v[u].y, a[u % NA]);
@@ -254,9 +255,17 @@ __device__ __forceinline__ double group_dot(const double* __restrict__ row, cons
 #pragma unroll
     for (int k = 0; k < NA; ++k) a[k] = 0.0;
     int at = 0;
-#pragma unroll F
-    for (; at + 8 * LPR <= n; at += 8 * LPR) group_turn<true, LPR, F>(r, ua, ub, split / W, n, at, lane, a);
-    if (at < n) group_turn<false, LPR, F>(r, ua, ub, split / W, n, at, lane, a);
+    // whole turns by F, so that a lane has eight loads in flight, then the row's end: half as many where they are there,
+    // and the rest unit by unit.  Rows that end inside a turn (leaves of 9, 10, 17, 18 .. cells a side, on every level)
+    // took a whole guarded turn for their end before, one turn of a lane at a time, and odd sides no shared lanes:
+    // trees of 15 x 15 leaves 4 levels deep 115 -> 93 us, 17 x 17 113 -> 100, 18 x 18 5 levels deep 261 -> 248, 6 levels
+    // 801 -> 757; 16 x 16, 4 levels, 95 -> 82, 7 levels the same.
+    for (; at + 8 * F * LPR <= n; at += 8 * F * LPR) group_batch<true, 2 * F, LPR, F>(r, ua, ub, split / W, n, at, lane, a);
+    if (at + 4 * F * LPR <= n) {
+        group_batch<true, F, LPR, F>(r, ua, ub, split / W, n, at, lane, a);
+        at += 4 * F * LPR;
+    }
+    if (at < n) group_batch<false, F, LPR, F>(r, ua, ub, split / W, n, at, lane, a);
     return NA == 4 ? (a[0] + a[1]) + (a[NA - 2] + a[NA - 1]) : NA == 2 ? a[0] + a[NA - 1] : a[0];
 }
 
@@ -355,9 +364,9 @@ inline int pick_lpr(int len, bool vec) {
 // Real lanes per lane of the sum: four while the level keeps within the blocks that are chained to the launch before
 // or, where one lane is too many for that, a quarter of the SMs' threads; two up to half of them.
 // Levels 3 to 6 with 16 x 16 leaves, us, against one line at the chained blocks alone: 55 / 98 / 196 / 457 and
-// 59 / 119 / 211 / 455.
-inline int pick_share(long long rows, int lpr, bool vec) {
-    if (!vec || lpr == 32) return 1;
+// 59 / 119 / 211 / 455.  (Leaves of 4 to 32 cells a side and trees of 1 to 6 levels: none slower than with one lane.)
+inline int pick_share(long long rows, int lpr) {
+    if (lpr == 32) return 1;
     const long long threads = rows * lpr, chained = kChainedBlocks * (long long)kGemvThreads;
     const long long four = threads <= chained ? chained : 152 * 512;
     return threads * 4 <= four && lpr <= 8 ? 4 : threads * 2 <= 152 * 1024 ? 2 : 1;
@@ -366,31 +375,26 @@ inline int pick_share(long long rows, int lpr, bool vec) {
 #define EF_GEMV(KERNEL, VEC, LPR, F, NTHREADS, ...) \
     launch_chained(Chain::few, KERNEL<VEC, LPR, F>, dim3(gemv_blocks(NTHREADS)), kGemvThreads, 0, st, __VA_ARGS__)
 // ROWS groups of F LPR lanes, at least LEAST threads
-#define EF_GEMV_DISPATCH(KERNEL, VEC, LPR, F, ROWS, LEAST, ...)                                                 \
-    do {                                                                                                        \
-        const long long nt_ = std::max<long long>((ROWS) * (LPR) * (F), (LEAST));                               \
-        if (!(VEC)) {                                                                                           \
-            if (LPR == 32) EF_GEMV(KERNEL, false, 32, 1, nt_, __VA_ARGS__);                                     \
-            else if (LPR == 16) EF_GEMV(KERNEL, false, 16, 1, nt_, __VA_ARGS__);                                \
-            else if (LPR == 8) EF_GEMV(KERNEL, false, 8, 1, nt_, __VA_ARGS__);                                  \
-            else if (LPR == 4) EF_GEMV(KERNEL, false, 4, 1, nt_, __VA_ARGS__);                                  \
-            else EF_GEMV(KERNEL, false, 2, 1, nt_, __VA_ARGS__);                                                \
-        } else if (F == 1) {                                                                                    \
-            if (LPR == 32) EF_GEMV(KERNEL, true, 32, 1, nt_, __VA_ARGS__);                                      \
-            else if (LPR == 16) EF_GEMV(KERNEL, true, 16, 1, nt_, __VA_ARGS__);                                 \
-            else if (LPR == 8) EF_GEMV(KERNEL, true, 8, 1, nt_, __VA_ARGS__);                                   \
-            else if (LPR == 4) EF_GEMV(KERNEL, true, 4, 1, nt_, __VA_ARGS__);                                   \
-            else EF_GEMV(KERNEL, true, 2, 1, nt_, __VA_ARGS__);                                                 \
-        } else if (F == 2) {                                                                                    \
-            if (LPR == 16) EF_GEMV(KERNEL, true, 16, 2, nt_, __VA_ARGS__);                                      \
-            else if (LPR == 8) EF_GEMV(KERNEL, true, 8, 2, nt_, __VA_ARGS__);                                   \
-            else if (LPR == 4) EF_GEMV(KERNEL, true, 4, 2, nt_, __VA_ARGS__);                                   \
-            else EF_GEMV(KERNEL, true, 2, 2, nt_, __VA_ARGS__);                                                 \
-        } else {                                                                                                \
-            if (LPR == 8) EF_GEMV(KERNEL, true, 8, 4, nt_, __VA_ARGS__);                                   \
-            else if (LPR == 4) EF_GEMV(KERNEL, true, 4, 4, nt_, __VA_ARGS__);                                   \
-            else EF_GEMV(KERNEL, true, 2, 4, nt_, __VA_ARGS__);                                                 \
-        }                                                                                                       \
+#define EF_GEMV_SHARED(KERNEL, VEC, LPR, F, NT, ...)                       \
+    do {                                                                   \
+        if (F == 1) EF_GEMV(KERNEL, VEC, LPR, 1, NT, __VA_ARGS__);         \
+        else if (F == 2) EF_GEMV(KERNEL, VEC, LPR, 2, NT, __VA_ARGS__);    \
+        else if constexpr (LPR <= 8) EF_GEMV(KERNEL, VEC, LPR, 4, NT, __VA_ARGS__); \
+    } while (0)
+#define EF_GEMV_LANES(KERNEL, VEC, LPR, F, NT, ...)                        \
+    do {                                                                   \
+        if (LPR == 32) EF_GEMV(KERNEL, VEC, 32, 1, NT, __VA_ARGS__);       \
+        else if (LPR == 16) EF_GEMV_SHARED(KERNEL, VEC, 16, F, NT, __VA_ARGS__); \
+        else if (LPR == 8) EF_GEMV_SHARED(KERNEL, VEC, 8, F, NT, __VA_ARGS__);   \
+        else if (LPR == 4) EF_GEMV_SHARED(KERNEL, VEC, 4, F, NT, __VA_ARGS__);   \
+        else EF_GEMV_SHARED(KERNEL, VEC, 2, F, NT, __VA_ARGS__);           \
+    } while (0)
+// ROWS groups of F LPR lanes, at least LEAST threads
+#define EF_GEMV_DISPATCH(KERNEL, VEC, LPR, F, ROWS, LEAST, ...)                                 \
+    do {                                                                                        \
+        const long long nt_ = std::max<long long>((ROWS) * (LPR) * (F), (LEAST));               \
+        if (VEC) EF_GEMV_LANES(KERNEL, true, LPR, F, nt_, __VA_ARGS__);                         \
+        else EF_GEMV_LANES(KERNEL, false, LPR, F, nt_, __VA_ARGS__);                            \
     } while (0)
 
 inline unsigned gemv_blocks(long long threads) {
@@ -602,7 +606,7 @@ void upward_hdiff(cudaStream_t st, const MergeItem* items, int nitems, int s) {
 void upward_w(cudaStream_t st, const MergeItem* items, int nitems, int s) {
     const long long rows = (long long)nitems * 4 * s;
     const bool vec = (s % 2 == 0);
-    const int lpr = pick_lpr(4 * s, vec), f = pick_share(rows, lpr, vec);
+    const int lpr = pick_lpr(4 * s, vec), f = pick_share(rows, lpr);
     EF_GEMV_DISPATCH(k_gemv_w, vec, lpr, f, rows, 0, items, s, rows);
     ++g_kernel_launches;
 }
@@ -610,7 +614,7 @@ void upward_w(cudaStream_t st, const MergeItem* items, int nitems, int s) {
 void upward_h(cudaStream_t st, const MergeItem* items, int nitems, int s) {
     const long long rows = (long long)nitems * 8 * s;
     const bool vec = (s % 2 == 0);
-    const int lpr = pick_lpr(2 * s, vec), f = pick_share(rows, lpr, vec);
+    const int lpr = pick_lpr(2 * s, vec), f = pick_share(rows, lpr);
     EF_GEMV_DISPATCH(k_gemv_h, vec, lpr, f, rows, 0, items, s, rows);
     ++g_kernel_launches;
 }
@@ -619,7 +623,7 @@ void upward_h(cudaStream_t st, const MergeItem* items, int nitems, int s) {
 void downward(cudaStream_t st, const MergeItem* items, int nitems, int s, int add_w) {
     const long long rows = (long long)nitems * 4 * s;
     const bool vec = (s % 2 == 0);
-    const int lpr = pick_lpr(8 * s, vec), f = pick_share(rows, lpr, vec);
+    const int lpr = pick_lpr(8 * s, vec), f = pick_share(rows, lpr);
     EF_GEMV_DISPATCH(k_gemv_down, vec, lpr, f, rows, (long long)nitems * 8 * s, items, s, rows, nitems, add_w);
     ++g_kernel_launches;
 }
