@@ -95,8 +95,6 @@ void Hps::allocate32() {
     for (size_t t = 0; t < types_.size(); ++t) t64[t] = types_[t].T;
     upload(st_, d_tT64_, t64, "type T64");
     upload(st_, d_tT32_, typeT, "type T32");
-    static const int cb[8] = {0, 2, 1, 3, 0, 1, 2, 3};
-    static const int ia[4] = {0, 1, 0, 1}, ib[4] = {2, 2, 3, 3};
     for (size_t gi = 0; gi < groups_.size(); ++gi) {
         const Group& g = groups_[gi];
         const int cnt = int(g.nodes.size());
@@ -121,10 +119,10 @@ void Hps::allocate32() {
             X[i] = m.X;
             R[i] = m.RHS;
             for (int b = 0; b < 8; ++b) {
-                const int c = cb[b];
+                const int c = kRunChild[b];
                 gA[8 * i + b] = m.H + size_t(b) * sz * 2 * sz;
-                gB[8 * i + b] = m.RHS + size_t(ia[c]) * sz * 12 * sz;
-                gB2[8 * i + b] = m.RHS + size_t(ib[c]) * sz * 12 * sz;
+                gB[8 * i + b] = m.RHS + size_t(kRunIa[c]) * sz * 12 * sz;
+                gB2[8 * i + b] = m.RHS + size_t(kRunIb[c]) * sz * 12 * sz;
                 gC[8 * i + b] = m.T + size_t(b) * sz * 8 * sz;
             }
         }

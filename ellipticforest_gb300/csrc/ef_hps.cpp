@@ -475,18 +475,16 @@ void Hps::upload_tables() {
         // (W: alpha, gamma; E: beta, omega; S: alpha, beta; N: gamma, omega), whose interfaces are
         // alpha: I0, I2; beta: I1, I2; gamma: I0, I3; omega: I1, I3.
         {
-            static const int cb[8] = {0, 2, 1, 3, 0, 1, 2, 3};
-            static const int ia[4] = {0, 1, 0, 1}, ib[4] = {2, 2, 3, 3};
             const size_t sz = size_t(g.s);
             std::vector<const double*> gA(8 * cnt), gB(8 * cnt), gB2(8 * cnt);
             std::vector<double*> gC(8 * cnt);
             for (int i = 0; i < cnt; ++i) {
                 const NodeDev& nd = nodes_[g.nodes[i]];
                 for (int b = 0; b < 8; ++b) {
-                    const int c = cb[b];
+                    const int c = kRunChild[b];
                     gA[8 * i + b] = nd.H + size_t(b) * sz * 2 * sz;
-                    gB[8 * i + b] = nd.RHS + size_t(ia[c]) * sz * 12 * sz;
-                    gB2[8 * i + b] = nd.RHS + size_t(ib[c]) * sz * 12 * sz;
+                    gB[8 * i + b] = nd.RHS + size_t(kRunIa[c]) * sz * 12 * sz;
+                    gB2[8 * i + b] = nd.RHS + size_t(kRunIb[c]) * sz * 12 * sz;
                     gC[8 * i + b] = nd.T + size_t(b) * sz * 8 * sz;
                 }
             }
@@ -624,15 +622,12 @@ void Hps::build() {
     // the merges of every level (a fixed launch sequence for this tree) replay as a CUDA graph from
     // the third build on (first eager, second captured); the leaf DtN maps above stay eager
     const long long l0 = g_kernel_launches.load();
-    graph_build_.run(st_, 1, graphs_ && !prof_, [&] { merge_levels(mesh_.max_level - 1, true, false); });
+    const std::vector<MergePart> parts = group_parts(mesh_.max_level, true);
+    graph_build_.run(st_, 1, graphs_ && !prof_, [&] { merge_pass(parts, mesh_.max_level - 1, false); });
     build_launches_ = g_kernel_launches.load() - l0;
     check(cudaGetLastError(), "build launch");
     check(cudaStreamSynchronize(st_), "build sync");
-    if (merges_rejected(mesh_.max_level)) {
-        merge_levels(mesh_.max_level - 1, true, true);
-        check(cudaStreamSynchronize(st_), "build sync");
-        check_merge_waits();
-    }
+    redo_rejected(parts);
     singular_ = count_singular(mesh_.max_level, true) + leaf_singular_;
     if (solver_type_ == SOLVER_FIVE_POINT) {
         std::vector<int> info(num_leaves());
@@ -730,17 +725,17 @@ void Hps::check_merge_waits() {
     throw std::runtime_error("CUDA error in build: an operand copy of a merge did not complete");
 }
 
-bool Hps::merges_rejected(int below) {
+int Hps::rejected_level(const std::vector<MergePart>& parts) {
     check_merge_waits();
-    if (!d_ws_) return false;
-    for (auto& g : groups_) {
-        if (g.level >= below || !merge64_supported(g.s)) continue;
-        std::vector<int> info(g.nodes.size());
-        check(cudaMemcpy(info.data(), g.d_info, info.size() * sizeof(int), cudaMemcpyDeviceToHost), "info");
+    int deepest = -1;
+    for (const auto& p : parts) {
+        if (groups_[p.group].level <= deepest || !by_products(p)) continue;
+        std::vector<int> info(p.cnt);
+        check(cudaMemcpy(info.data(), p.t.info, info.size() * sizeof(int), cudaMemcpyDeviceToHost), "info");
         for (int v : info)
-            if (v) return true;
+            if (v) deepest = groups_[p.group].level;
     }
-    return false;
+    return deepest;
 }
 
 void Hps::merge_lu(const MergeTables& t, int cnt, int s) {
@@ -764,57 +759,149 @@ void Hps::merge_lu(const MergeTables& t, int cnt, int s) {
     pe(c * 8 * (dm * dm / 2 + dm * 2 * dm + 2 * 4 * dm * dm), c * 2.0 * (2 * dm) * (2 * dm) * (dm / 2));
 }
 
-void Hps::merge_nodes(const MergeTables& t, int cnt, int s, bool careful) {
+bool Hps::by_products(const MergePart& p) const {
+    const int s = groups_[p.group].s;
+    return merge64_supported(s) && ws_bytes_ >= merge64_workspace(p.cnt, s) + 1024;
+}
+
+void Hps::merge_part(const MergePart& p) {
+    const int cnt = p.cnt, s = groups_[p.group].s;
     const double c = cnt, dm = 4.0 * s;
     pb("gather_xht");
-    merge_gather_xht(st_, t.items, cnt, s);
+    merge_gather_xht(st_, p.t.items, cnt, s);
     pe(c * 8 * (dm * dm + 2 * dm * dm + 4 * dm * dm) * 1.5, 0);
-    check(cudaMemsetAsync(t.info, 0, cnt * sizeof(int), st_), "memset info");
-    if (!merge64_supported(s) || ws_bytes_ < merge64_workspace(cnt, s) + 1024) {
-        merge_lu(t, cnt, s);
+    check(cudaMemsetAsync(p.t.info, 0, cnt * sizeof(int), st_), "memset info");
+    if (!by_products(p)) {
+        merge_lu(p.t, cnt, s);
         return;
     }
     pb("merge64");
-    merge64(st_, t.items, cnt, s, t.info, d_ws_, d_wserr_);
+    merge64(st_, p.t.items, cnt, s, p.t.info, d_ws_, d_wserr_);
     pe(c * 8 * 12 * dm * dm, c * 8.0 * dm * dm * dm);
-    if (!careful) return;
-    if (inject_merge_error_) check(cudaMemsetAsync(d_wserr_, 1, sizeof(int), st_), "merge error test");
-    std::vector<int> info(cnt);
-    check(cudaMemcpyAsync(info.data(), t.info, cnt * sizeof(int), cudaMemcpyDeviceToHost, st_), "merge info");
-    check(cudaStreamSynchronize(st_), "merge info");
-    for (int i = 0; i < cnt; ++i) {
-        if (!info[i]) continue;
-        const MergeTables one = t.from(i);
-        merge_gather_xht(st_, one.items, 1, s);
-        check(cudaMemsetAsync(one.info, 0, sizeof(int), st_), "memset info");
-        merge_lu(one, 1, s);
-    }
 }
 
-// every merge of the tree levels top .. 0, deepest first (HPSAlgorithm.hpp:497-518 per node): the
-// children's T of level top + 1 must be in place
-void Hps::merge_levels(int top, bool distinct, bool careful) {
+namespace {
+
+// Tables of the k merges idx of t, made from their items.
+struct PickedMerges {
+    char* p = nullptr;
+    MergeTables t{};
+    ~PickedMerges() { cudaFree(p); }
+    static size_t bytes(size_t k) { return align_up(k * sizeof(MergeItem)) + align_up(36 * k * sizeof(void*)) + k * sizeof(int); }
+    void fill(cudaStream_t st, const std::vector<MergeItem>& items, int s) {
+        const size_t k = items.size(), s2 = size_t(s) * s;
+        std::vector<const void*> ptr(36 * k);  // X, RHS, piv, perm, then eight each of gA, gB, gB2, gC
+        for (size_t j = 0; j < k; ++j) {
+            const MergeItem& it = items[j];
+            ptr[j] = it.X;
+            ptr[k + j] = it.RHS;
+            ptr[2 * k + j] = it.piv;
+            ptr[3 * k + j] = it.perm;
+            for (int b = 0; b < 8; ++b) {
+                const int c = kRunChild[b];
+                const void** q = ptr.data() + 4 * k + 8 * j + b;
+                q[0] = it.H + size_t(b) * 2 * s2;
+                q[8 * k] = it.RHS + size_t(kRunIa[c]) * 12 * s2;
+                q[16 * k] = it.RHS + size_t(kRunIb[c]) * 12 * s2;
+                q[24 * k] = it.T + size_t(b) * 8 * s2;
+            }
+        }
+        void** q = reinterpret_cast<void**>(p + align_up(k * sizeof(MergeItem)));
+        int* info = reinterpret_cast<int*>(reinterpret_cast<char*>(q) + align_up(ptr.size() * sizeof(void*)));
+        if (upload_sync(st, p, items.data(), k * sizeof(MergeItem)) != cudaSuccess ||
+            upload_sync(st, q, ptr.data(), ptr.size() * sizeof(void*)) != cudaSuccess)
+            throw std::runtime_error("CUDA error in build: tables of rejected merges");
+        auto dd = [&](size_t at) { return reinterpret_cast<double* const*>(q + at * k); };
+        auto cd = [&](size_t at) { return reinterpret_cast<const double* const*>(q + at * k); };
+        auto ii = [&](size_t at) { return reinterpret_cast<int* const*>(q + at * k); };
+        t = {reinterpret_cast<const MergeItem*>(p), dd(0), dd(1), ii(2), ii(3), info, cd(4), cd(12), cd(20), dd(28)};
+    }
+};
+
+}  // namespace
+
+// The merges of p that block elimination gave up, all at once (one at a time the pivoted LU is a chain of small
+// launches per merge: a build of 1024 leaves of 16 x 16 cells with random coefficients over eight decades 183 ms, now 53).
+bool Hps::merge_rejected(const MergePart& p) {
+    const int s = groups_[p.group].s, cnt = p.cnt;
+    std::vector<int> info(cnt), idx;
+    check(cudaMemcpyAsync(info.data(), p.t.info, cnt * sizeof(int), cudaMemcpyDeviceToHost, st_), "merge info");
+    check(cudaStreamSynchronize(st_), "merge info");
+    for (int i = 0; i < cnt; ++i)
+        if (info[i]) idx.push_back(i);
+    if (idx.empty()) return false;
+    const int k = int(idx.size());
+    PickedMerges picked;
+    const bool run = idx.back() - idx.front() + 1 == k;  // their tables are part of p's
+    if (!run) {
+        std::vector<MergeItem> all(cnt), items;
+        check(cudaMemcpy(all.data(), p.t.items, cnt * sizeof(MergeItem), cudaMemcpyDeviceToHost), "merge items");
+        for (int i : idx) items.push_back(all[i]);
+        check(device_alloc(reinterpret_cast<void**>(&picked.p), PickedMerges::bytes(k)), "cudaMalloc(rejected merges)");
+        picked.fill(st_, items, s);
+    }
+    const MergeTables t = run ? p.t.from(idx.front()) : picked.t;
+    merge_gather_xht(st_, t.items, k, s);
+    check(cudaMemsetAsync(t.info, 0, k * sizeof(int), st_), "memset info");
+    merge_lu(t, k, s);
+    if (run) return true;
+    std::vector<int> lu(k);
+    check(cudaMemcpyAsync(lu.data(), t.info, k * sizeof(int), cudaMemcpyDeviceToHost, st_), "merge info");
+    check(cudaStreamSynchronize(st_), "merge info");
+    for (int j = 0; j < k; ++j) info[idx[j]] = lu[j];
+    check(upload_sync(st_, p.t.info, info.data(), cnt * sizeof(int)), "merge info");
+    return true;
+}
+
+std::vector<Hps::MergePart> Hps::group_parts(int below, bool distinct) const {
+    std::vector<MergePart> parts;
+    for (size_t gi = 0; gi < groups_.size(); ++gi) {
+        const Group& g = groups_[gi];
+        if (g.level >= below) continue;
+        parts.push_back({gi, {g.d_items, g.d_X, g.d_RHS, g.d_piv, g.d_perm, g.d_info, g.d_gA, g.d_gB, g.d_gB2, g.d_gC},
+                         distinct ? g.distinct : int(g.nodes.size()), distinct});
+    }
+    return parts;
+}
+
+// Merges of `parts`, deepest level first (HPSAlgorithm.hpp:497-518 per node), from level `top` on: the children's T of
+// level top + 1 must be in place.  redo: the pass before gave up merges of level `top` and none below it; those go
+// through the pivoted LU, the levels above start again, and what is given up there follows.
+void Hps::merge_pass(const std::vector<MergePart>& parts, int top, bool redo) {
+    if (redo && inject_merge_error_ && d_ws_) check(cudaMemsetAsync(d_wserr_, 1, sizeof(int), st_), "merge error test");
     for (int lvl = top; lvl >= 0; --lvl) {
-        for (size_t k = 0; k < tsteps_.size(); ++k)
+        const bool done = redo && lvl == top;
+        for (size_t k = 0; k < tsteps_.size() && !done; ++k)
             if (tsteps_[k].level == lvl + 1) {
                 const double nf = tsteps_[k].nf, cnt = tsteps_[k].count;
                 pb("coarsen_T");
                 coarsen_T(st_, tsteps_[k].d_in, tsteps_[k].d_out, tsteps_[k].count, tsteps_[k].nf);
                 pe(cnt * 8 * (16 * nf * nf + 4 * nf * nf), cnt * 4 * nf * nf * 10);
             }
-        for (auto& g : groups_) {
+        for (const auto& p : parts) {
+            const Group& g = groups_[p.group];
             if (g.level != lvl) continue;
-            const int all = int(g.nodes.size()), cnt = distinct ? g.distinct : all, s = g.s;
-            if (cnt < all) check(cudaMemsetAsync(g.d_info + cnt, 0, (all - cnt) * sizeof(int), st_), "memset info");
-            merge_nodes({g.d_items, g.d_X, g.d_RHS, g.d_piv, g.d_perm, g.d_info, g.d_gA, g.d_gB, g.d_gB2, g.d_gC}, cnt, s,
-                        careful);
-            if (distinct && g.ncopy > 0) {
+            const int all = int(g.nodes.size());
+            if (!done) {
+                if (p.copies && p.cnt < all) check(cudaMemsetAsync(g.d_info + p.cnt, 0, (all - p.cnt) * sizeof(int), st_), "memset info");
+                merge_part(p);
+            }
+            const bool again = redo && by_products(p) && merge_rejected(p);
+            if (p.copies && g.ncopy > 0 && (!done || again)) {
                 pb("copy_equal");
-                copy_batched(st_, g.d_csrc, g.d_cdst, g.d_clen, g.ncopy, 128LL * s * s * (all - cnt));
-                pe(double(all - cnt) * 2 * 8 * 128 * s * s, 0);
+                copy_batched(st_, g.d_csrc, g.d_cdst, g.d_clen, g.ncopy, 128LL * g.s * g.s * (all - p.cnt));
+                pe(double(all - p.cnt) * 2 * 8 * 128 * g.s * g.s, 0);
             }
         }
     }
+}
+
+void Hps::redo_rejected(const std::vector<MergePart>& parts) {
+    const int level = rejected_level(parts);
+    if (level < 0) return;
+    merge_pass(parts, level, true);
+    check(cudaStreamSynchronize(st_), "build sync");
+    check_merge_waits();
 }
 
 // interface LUs with a zero pivot among the merges of the levels below `below` (synchronous)

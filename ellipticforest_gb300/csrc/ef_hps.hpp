@@ -48,6 +48,10 @@ struct NodeDev {
     std::vector<double*> Tsteps, hsteps, gsteps;  // intermediate (un)coarsening buffers
 };
 
+// T += H S by rows: the child of each run of s rows of the parent's WESN order, and the interfaces of each child
+constexpr int kRunChild[8] = {0, 2, 1, 3, 0, 1, 2, 3};
+constexpr int kRunIa[4] = {0, 1, 0, 1}, kRunIb[4] = {2, 2, 3, 3};
+
 struct Group {
     int level = 0, s = 0;
     std::vector<int> nodes;
@@ -321,15 +325,24 @@ public:
     void profile_reset();
 
 private:
-    // merges of levels top .. 0; `distinct`: one merge per distinct operator, copied to its equals;
-    // `careful`: after every group, the merges that block elimination gave up go through the pivoted LU
-    void merge_levels(int top, bool distinct, bool careful);
-    void merge_nodes(const MergeTables& t, int cnt, int s, bool careful);
+    // merges of one group: all its nodes or some; copies: of a whole group's distinct nodes, copied to their equals
+    struct MergePart {
+        size_t group;
+        MergeTables t;
+        int cnt;
+        bool copies;
+    };
+    std::vector<MergePart> group_parts(int below, bool distinct) const;  // of the levels < below
+    void merge_pass(const std::vector<MergePart>& parts, int top, bool redo);
+    void redo_rejected(const std::vector<MergePart>& parts);  // after a pass and a sync: what block elimination gave up, by LU
+    int rejected_level(const std::vector<MergePart>& parts);  // the deepest level with such a merge, -1: none
+    bool by_products(const MergePart& p) const;               // merged by digit products, else by the pivoted LU
+    void merge_part(const MergePart& p);
+    bool merge_rejected(const MergePart& p);                  // false: there were none
     void merge_lu(const MergeTables& t, int cnt, int s);  // from the gathered X, H and T_LHS on
     // room for merge64 of counts[g] nodes of each group g, as far as it can be had (without it a group merges by LU)
     void reserve_merges(const std::vector<int>& counts);
     bool reserve(size_t bytes);            // d_ws_ of at least that many bytes; false: refused, what there was stays
-    bool merges_rejected(int below);       // block elimination set info in some merge of levels < below
     // device memory, giving back the workspace where there is none left
     cudaError_t device_alloc(void** p, size_t bytes);
     void check_merge_waits();              // throws where a wait of the merges' kernels gave up (after a sync)

@@ -126,8 +126,6 @@ void Hps::build_from(const Hps& old) {
     } tables;
     cki(device_alloc(reinterpret_cast<void**>(&tables.p), host.size() + 256), "cudaMalloc(incremental tables)");
     unsigned char* const dev = tables.p;
-    static const int cb[8] = {0, 2, 1, 3, 0, 1, 2, 3};
-    static const int ia[4] = {0, 1, 0, 1}, ib[4] = {2, 2, 3, 3};
     std::vector<MergeItem> all_items;
     for (size_t gi = 0; gi < groups_.size(); ++gi) {
         const Sub& s = sub[gi];
@@ -148,10 +146,10 @@ void Hps::build_from(const Hps& old) {
             std::memcpy(&host[s.piv + k * sizeof(void*)], &nd.piv, sizeof(void*));
             std::memcpy(&host[s.perm + k * sizeof(void*)], &nd.perm, sizeof(void*));
             for (int b = 0; b < 8; ++b) {
-                const int c = cb[b];
+                const int c = kRunChild[b];
                 const double* A = nd.H + size_t(b) * sz * 2 * sz;
-                const double* Bp = nd.RHS + size_t(ia[c]) * sz * 12 * sz;
-                const double* B2 = nd.RHS + size_t(ib[c]) * sz * 12 * sz;
+                const double* Bp = nd.RHS + size_t(kRunIa[c]) * sz * 12 * sz;
+                const double* B2 = nd.RHS + size_t(kRunIb[c]) * sz * 12 * sz;
                 double* Cp = nd.T + size_t(b) * sz * 8 * sz;
                 std::memcpy(&host[s.gA + (8 * k + b) * sizeof(void*)], &A, sizeof(void*));
                 std::memcpy(&host[s.gB + (8 * k + b) * sizeof(void*)], &Bp, sizeof(void*));
@@ -172,51 +170,32 @@ void Hps::build_from(const Hps& old) {
     // the reused operators first: parents read their children's T when they merge
     copy_batched(st_, reinterpret_cast<const double* const*>(at(c_src)), reinterpret_cast<double* const*>(at(c_dst)),
                  reinterpret_cast<const long long*>(at(c_len)), int(ncopy), std::accumulate(clen.begin(), clen.end(), 0LL));
-    const int maxL = mesh_.max_level;
     std::vector<int> counts;
     for (const auto& sb : sub) counts.push_back(sb.cnt);
     reserve_merges(counts);
-    auto merge_dirty = [&](bool careful) {
-        for (int lvl = maxL - 1; lvl >= 0; --lvl) {
-            for (size_t k = 0; k < tsteps_.size(); ++k)
-                if (tsteps_[k].level == lvl + 1) coarsen_T(st_, tsteps_[k].d_in, tsteps_[k].d_out, tsteps_[k].count, tsteps_[k].nf);
-            for (size_t gi = 0; gi < groups_.size(); ++gi) {
-                const Sub& sb = sub[gi];
-                if (groups_[gi].level != lvl || !sb.cnt) continue;
-                const MergeTables t{reinterpret_cast<const MergeItem*>(at(sb.items)), reinterpret_cast<double* const*>(at(sb.X)),
-                                    reinterpret_cast<double* const*>(at(sb.RHS)), reinterpret_cast<int* const*>(at(sb.piv)),
-                                    reinterpret_cast<int* const*>(at(sb.perm)), reinterpret_cast<int*>(at(sb.info)),
-                                    reinterpret_cast<const double* const*>(at(sb.gA)),
-                                    reinterpret_cast<const double* const*>(at(sb.gB)),
-                                    reinterpret_cast<const double* const*>(at(sb.gB2)),
-                                    reinterpret_cast<double* const*>(at(sb.gC))};
-                merge_nodes(t, sb.cnt, groups_[gi].s, careful);
-            }
-        }
-    };
-    merge_dirty(false);
+    std::vector<MergePart> parts;
+    for (size_t gi = 0; gi < groups_.size(); ++gi) {
+        const Sub& sb = sub[gi];
+        if (!sb.cnt) continue;
+        parts.push_back({gi,
+                         {reinterpret_cast<const MergeItem*>(at(sb.items)), reinterpret_cast<double* const*>(at(sb.X)),
+                          reinterpret_cast<double* const*>(at(sb.RHS)), reinterpret_cast<int* const*>(at(sb.piv)),
+                          reinterpret_cast<int* const*>(at(sb.perm)), reinterpret_cast<int*>(at(sb.info)),
+                          reinterpret_cast<const double* const*>(at(sb.gA)), reinterpret_cast<const double* const*>(at(sb.gB)),
+                          reinterpret_cast<const double* const*>(at(sb.gB2)), reinterpret_cast<double* const*>(at(sb.gC))},
+                         sb.cnt,
+                         false});
+    }
+    merge_pass(parts, mesh_.max_level - 1, false);
     cki(cudaGetLastError(), "incremental build launch");
     cki(cudaStreamSynchronize(st_), "incremental build sync");
-    auto marked = [&] {
-        int n = 0;
-        for (size_t gi = 0; gi < groups_.size(); ++gi) {
-            const Sub& sb = sub[gi];
-            if (!sb.cnt) continue;
-            std::vector<int> info(sb.cnt);
-            cki(cudaMemcpy(info.data(), at(sb.info), sb.cnt * sizeof(int), cudaMemcpyDeviceToHost), "info");
-            for (int v : info) n += (v != 0);
-        }
-        return n;
-    };
-    check_merge_waits();
-    int bad = marked();
-    if (bad > 0) {
-        merge_dirty(true);
-        cki(cudaStreamSynchronize(st_), "incremental build sync");
-        check_merge_waits();
-        bad = marked();
+    redo_rejected(parts);
+    singular_ = leaf_singular_;
+    for (const auto& p : parts) {
+        std::vector<int> info(p.cnt);
+        cki(cudaMemcpy(info.data(), p.t.info, p.cnt * sizeof(int), cudaMemcpyDeviceToHost), "info");
+        for (int v : info) singular_ += (v != 0);
     }
-    singular_ = leaf_singular_ + bad;
     equal_operators_ = false;  // the reused operators come from another tree
     built_ = true;
 }

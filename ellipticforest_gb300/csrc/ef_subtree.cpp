@@ -79,14 +79,11 @@ void Hps::build_top(int level, const double* const* T_host) {
     std::vector<int> counts;
     for (const auto& g : groups_) counts.push_back(g.level < level ? int(g.nodes.size()) : 0);
     reserve_merges(counts);
-    merge_levels(level - 1, false, false);
+    const std::vector<MergePart> parts = group_parts(level, false);
+    merge_pass(parts, level - 1, false);
     check(cudaGetLastError(), "top build launch");
     check(cudaStreamSynchronize(st_), "top build sync");
-    if (merges_rejected(level)) {
-        merge_levels(level - 1, false, true);
-        check(cudaStreamSynchronize(st_), "top build sync");
-        check_merge_waits();
-    }
+    redo_rejected(parts);
     singular_ = count_singular(level, false);
     top_level_ = level;
     equal_operators_ = false;  // the T blocks come from outside
