@@ -115,24 +115,47 @@ __global__ void k_dtn_extract(int n, const double* __restrict__ dxs, const doubl
 struct dd {
     double h, l;
 };
+// A compiler may fuse a product with a sum that it feeds, which these steps cannot stand: on the device they are
+// written with the operations that are never fused, on the host the products are fused multiply-adds already.
+__host__ __device__ inline double add_rn(double a, double b) {
+#ifdef __CUDA_ARCH__
+    return __dadd_rn(a, b);
+#else
+    return a + b;
+#endif
+}
+__host__ __device__ inline double fma_rn(double a, double b, double c) {
+#ifdef __CUDA_ARCH__
+    return __fma_rn(a, b, c);
+#else
+    return std::fma(a, b, c);
+#endif
+}
+__host__ __device__ inline double mul_rn(double a, double b) {
+#ifdef __CUDA_ARCH__
+    return __dmul_rn(a, b);
+#else
+    return std::fma(a, b, 0.0);
+#endif
+}
 __host__ __device__ inline dd quick_sum(double a, double b) {  // |a| >= |b|
-    const double s = a + b;
-    return {s, b - (s - a)};
+    const double s = add_rn(a, b);
+    return {s, add_rn(b, -add_rn(s, -a))};
 }
 __host__ __device__ inline dd two_sum(double a, double b) {
-    const double s = a + b, t = s - a;
-    return {s, (a - (s - t)) + (b - t)};
+    const double s = add_rn(a, b), t = add_rn(s, -a);
+    return {s, add_rn(add_rn(a, -add_rn(s, -t)), add_rn(b, -t))};
 }
 __host__ __device__ inline dd operator+(dd a, dd b) {
     const dd s = two_sum(a.h, b.h), t = two_sum(a.l, b.l);
-    const dd u = quick_sum(s.h, s.l + t.h);
-    return quick_sum(u.h, u.l + t.l);
+    const dd u = quick_sum(s.h, add_rn(s.l, t.h));
+    return quick_sum(u.h, add_rn(u.l, t.l));
 }
 __host__ __device__ inline dd operator-(dd a) { return {-a.h, -a.l}; }
 __host__ __device__ inline dd operator-(dd a, dd b) { return a + (-b); }
 __host__ __device__ inline dd operator*(dd a, dd b) {
-    const double p = a.h * b.h;
-    return quick_sum(p, fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h));
+    const double p = mul_rn(a.h, b.h);
+    return quick_sum(p, add_rn(fma_rn(a.h, b.h, -p), fma_rn(a.h, b.l, mul_rn(a.l, b.h))));
 }
 __host__ __device__ inline dd operator/(dd a, dd b) {
     const double q1 = a.h / b.h;
