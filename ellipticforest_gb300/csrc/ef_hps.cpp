@@ -709,11 +709,11 @@ cudaError_t Hps::device_alloc(void** p, size_t bytes) {
 void Hps::reserve_merges(const std::vector<int>& counts) {
     size_t most = 0;
     for (size_t g = 0; g < groups_.size(); ++g)
-        if (counts[g] > 0 && merge64_supported(groups_[g].s)) most = std::max(most, merge64_workspace(counts[g], groups_[g].s));
+        if (counts[g] > 0) most = std::max(most, products_need(counts[g], groups_[g].s));
     if (!most || reserve(most)) return;
     // what the smaller groups need, where the largest gets no room
     for (size_t g = 0; g < groups_.size(); ++g)
-        if (counts[g] > 0 && merge64_supported(groups_[g].s)) (void)reserve(merge64_workspace(counts[g], groups_[g].s));
+        if (counts[g] > 0) (void)reserve(products_need(counts[g], groups_[g].s));
 }
 
 void Hps::check_merge_waits() {
@@ -759,9 +759,17 @@ void Hps::merge_lu(const MergeTables& t, int cnt, int s) {
     pe(c * 8 * (dm * dm / 2 + dm * 2 * dm + 2 * 4 * dm * dm), c * 2.0 * (2 * dm) * (2 * dm) * (dm / 2));
 }
 
-bool Hps::by_products(const MergePart& p) const {
-    const int s = groups_[p.group].s;
-    return merge64_supported(s) && ws_bytes_ >= merge64_workspace(p.cnt, s) + 1024;
+// workspace of cnt merges by digit products, 0: they are not for this size.  Kept (it is a dry run of the whole merge, some
+// 2 us, asked for several times per group and build).
+size_t Hps::products_need(int cnt, int s) {
+    const auto it = products_need_.emplace(std::make_pair(cnt, s), 0);
+    if (it.second && merge64_supported(s)) it.first->second = merge64_workspace(cnt, s);
+    return it.first->second;
+}
+
+bool Hps::by_products(const MergePart& p) {
+    const size_t need = products_need(p.cnt, groups_[p.group].s);
+    return need > 0 && ws_bytes_ >= need + 1024;
 }
 
 void Hps::merge_part(const MergePart& p) {

@@ -10,8 +10,10 @@
 
 #include <array>
 #include <cstdint>
+#include <map>
 #include <memory>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "ef_kernels.cuh"
@@ -336,7 +338,9 @@ private:
     void merge_pass(const std::vector<MergePart>& parts, int top, bool redo);
     void redo_rejected(const std::vector<MergePart>& parts);  // after a pass and a sync: what block elimination gave up, by LU
     int rejected_level(const std::vector<MergePart>& parts);  // the deepest level with such a merge, -1: none
-    bool by_products(const MergePart& p) const;               // merged by digit products, else by the pivoted LU
+    bool by_products(const MergePart& p);                     // merged by digit products, else by the pivoted LU
+    size_t products_need(int cnt, int s);
+    std::map<std::pair<int, int>, size_t> products_need_;
     void merge_part(const MergePart& p);
     bool merge_rejected(const MergePart& p);                  // false: there were none
     void merge_lu(const MergeTables& t, int cnt, int s);  // from the gathered X, H and T_LHS on
