@@ -65,6 +65,9 @@ CUtensorMap make_map(float* base, long long rows, int cols, int box_rows) {
     return tm;
 }
 
+// a block of B requests is run with up to a sixth more to make a multiple of four of it
+bool worth_filling(int B) { return B >= 5 && 6 * ((B + 3) / 4 * 4 - B) <= B; }
+
 }  // namespace
 
 MixedSolver::MixedSolver(Hps& hps, int bmax, const MixedSolver* share)
@@ -80,10 +83,11 @@ MixedSolver::MixedSolver(Hps& hps, int bmax, const MixedSolver* share)
         throw std::invalid_argument("mixed solver: FivePointStencil leaves of at most 32 x 32 cells");
     if (n % 4 != 0 || n > 64)
         throw std::invalid_argument("mixed solver: the leaf size must be a multiple of 4 and at most 64");
-    // room for the requests that fill a block up to a multiple of four (see filled), where the limits allow it
+    // room for the requests that fill a block up to a multiple of four, where it is (see filled) and the limits allow it
     const int up4 = (bmax + 3) / 4 * 4;
-    if (bmax >= 5 && (long long)L * up4 < (1LL << 31) && 12LL * hps.node(0).nx * up4 < (1LL << 31)) cap_ = up4;
-    const size_t nn = size_t(n) * n, B = size_t(cap_);
+    if (worth_filling(bmax) && (long long)L * up4 < (1LL << 31) && 12LL * hps.node(0).nx * up4 < (1LL << 31)) cap_ = up4;
+    const size_t nn = size_t(n) * n;
+    size_t B = size_t(cap_);
     const int M = hps.root_M();
     const Mesh& mesh = hps.mesh();
     mn_.assign(N, MNode());
@@ -229,10 +233,20 @@ MixedSolver::MixedSolver(Hps& hps, int bmax, const MixedSolver* share)
             st.out64 = cv.get<void*>(st.count);
         }
     };
-    MxCarver dry;
-    layout(dry);
-    bytes_ = dry.off;
-    ck(hps.device_alloc(reinterpret_cast<void**>(&arena_), bytes_), "cudaMalloc(mixed arena)");
+    auto allocate = [&] {
+        MxCarver dry;
+        layout(dry);
+        bytes_ = dry.off;
+        return hps.device_alloc(reinterpret_cast<void**>(&arena_), bytes_);
+    };
+    cudaError_t got = allocate();
+    if (got == cudaErrorMemoryAllocation && cap_ > bmax) {  // without the room to fill up
+        (void)cudaGetLastError();
+        cap_ = bmax;
+        B = size_t(bmax);
+        got = allocate();
+    }
+    ck(got, "cudaMalloc(mixed arena)");
     MxCarver real;
     real.base = arena_;
     layout(real);
@@ -805,10 +819,7 @@ void MixedSolver::pass(int B, bool first, bool neumann_done, bool last) {
     h.pe(items * (nn * (first ? 12.0 : 20.0) + 4.0 * n * 4), items * 2.0 * 4 * nn * n, st);
 }
 
-int MixedSolver::filled(int B) const {
-    const int up4 = (B + 3) / 4 * 4;
-    return B == bmax_ && B >= 5 && 6 * (up4 - B) <= B && up4 <= cap_ ? up4 : B;
-}
+int MixedSolver::filled(int B) const { return B == bmax_ ? cap_ : B; }
 
 void MixedSolver::solve(int batch, int sweeps) {
     if (batch < 1 || batch > bmax_) throw std::invalid_argument("mixed solver: batch size out of range");
