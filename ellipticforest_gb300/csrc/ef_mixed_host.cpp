@@ -252,6 +252,11 @@ MixedSolver::MixedSolver(Hps& hps, int bmax, const MixedSolver* share)
     layout(real);
     cudaStream_t st = st_;
     ck(cudaMemsetAsync(arena_, 0, bytes_, st), "memset(mixed arena)");
+    if (cap_ > bmax) {
+        // the requests that fill a block up are solved too: no load, root data 1 u = 0
+        const std::vector<double> one(size_t(cap_ - bmax) * 4 * M, 1.0);
+        ck(upload_sync(st, a_ + size_t(bmax) * 4 * M, one.data(), one.size() * sizeof(double)), "root data of the filling requests");
+    }
 
     if (fp) {
         std::vector<MixFp> fl(L);
@@ -825,7 +830,7 @@ void MixedSolver::solve(int batch, int sweeps) {
     if (batch < 1 || batch > bmax_) throw std::invalid_argument("mixed solver: batch size out of range");
     // The interface rows of a block are accessed in 16-byte pieces, and the tensor-core GEMMs' right-hand sides
     // copied in them, when the request count is a multiple of four: a full block that is nearly one takes the
-    // places behind the caller's along (requests do not mix, and nobody reads those).  Adaptive tree, 23
+    // zero requests behind the caller's along (requests do not mix, and nobody reads those).  Adaptive tree, 23
     // requests: 3.95 -> 3.34 ms; beyond a sixth more requests the leaf passes would cost more than the rows save.
     const int B = filled(batch);
     if (sweeps < 0 || sweeps + 1 > kMaxPasses) throw std::invalid_argument("mixed solver: too many sweeps");
