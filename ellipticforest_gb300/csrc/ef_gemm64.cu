@@ -9,11 +9,15 @@
 //   * the products of digit i of A and digit j of B carry the weight 256^-(i+j).  All pairs of one weight
 //     w = i + j add up in one FP32 accumulator: at most 8 pairs x 128 values of k x 2^14 = 2^24, so every
 //     partial sum is an integer that FP32 holds exactly, whatever the order;
-//   * pairs with w > 7 are left out: they are below 2^-62 of (row maximum) x (column maximum);
+//   * pairs with w > 7 are left out;
 //   * after every 128 values of k the eight sums per entry go to two 64-bit integers (exact), and the entry
 //     is rounded to a double once, at the end.
-// An entry's error is K 2^-62 of its row maximum times its column maximum plus one rounding; a chain of
-// FP64 FMAs errs by up to K 2^-53 of the sum of its |products|.
+// With the row's largest entry in [2^61, 2^62) of its scale, the seven pairs of weight 8 come to 7 x 2^-62 of the two
+// scales' product per k, rounding both operands to 2^-63 to one more, and a scale is up to twice the largest entry: an
+// entry's error is at most 33 K 2^-62 (K 2^-57) of its row maximum times its column maximum, plus one rounding; for
+// digits without a pattern it is some sqrt(K) 2^-60.  This is a bound by norms: a chain of FP64 FMAs errs by up to K 2^-53
+// of the sum of its |products|, which is less where every product is far below the two maxima (entries of graded rows and
+// columns).  The merges check the inverses they form with these products by their residuals, S and T follow from them.
 #include <cuda_bf16.h>
 
 #include <algorithm>
