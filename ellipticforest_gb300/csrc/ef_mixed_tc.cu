@@ -35,12 +35,12 @@
 // four children) puts the blocks side by side in N (32 requests each) and keeps each row's own
 // block in the epilogue.
 //
-// Roles (256 threads, eight warps: two per SM sub-partition, so up to 255 registers a thread):
+// Roles (288 threads, nine warps, so up to 224 registers a thread):
 // warps 0-3 add each chunk's accumulators to registers and run the epilogue (warp w reads TMEM lanes
 // 32w..32w+31; the operands a row's epilogue reads are prefetched when its tile starts; the
 // exterior rows of DOWN's children are copied by their own launch, k_mx_ext32), warps 4-6
 // stage X (the next chunk's loads in flight while the current one is split and written), warp 7
-// allocates TMEM and issues the bulk copies and the MMAs.  Stages
+// allocates TMEM and issues the MMAs, warp 8 the bulk copies of the A planes.  Stages
 // are handed over through mbarriers; the MMA issuer frees a stage with tcgen05.commit.  Every wait
 // gives up after about one second: the kernel then sets the error word, lets its copies and MMAs in
 // flight finish (bounded waits), frees its TMEM and returns.
@@ -94,7 +94,6 @@ __host__ __device__ constexpr int tc_stage_bytes(int nseg) { return 3 * kPlaneA 
 __host__ __device__ constexpr size_t tc_smem_bytes(int nseg) {
     return 1024 + size_t(tc_stages(nseg)) * tc_stage_bytes(nseg) + 256 + size_t(kXRing) * nseg * kTK * kTB * 4;
 }
-// two chunk buffers x (D_hi, D_lo) x 32 nseg columns
 // accumulator sets of a chunk: D_hi, D_lo_a, D_lo_b of 32 nseg columns each, as many as fit in 512
 __host__ __device__ constexpr int tc_acc_sets(int nseg) { return 512 / (3 * kTB * nseg); }
 __host__ __device__ constexpr int tc_tmem_cols(int) { return 512; }
@@ -159,8 +158,8 @@ __device__ __forceinline__ TcSeg tc_seg(const MixItem* __restrict__ items, int s
 // A lane holds a row's sums for the 32 requests of a block.  Rows are 128 bytes (B = 32) in memory, so with 16-byte
 // accesses by rows every instruction touched 32 of them.  With B a multiple of 4 the warp therefore exchanges
 // its 4-request pieces first: lane (piece c = lane / 4, a = lane mod 4) gets piece c of the rows 4 i + a, i = 0 .. 7, and
-// an instruction covers four whole rows (L7 block 4.00 -> 3.94 ms).  Otherwise the lane keeps its row, one request
-// at a time.
+// an instruction covers four whole rows (L7 block 4.00 -> 3.94 ms).  Blocks of single units keep their rows (see
+// tc_access), and where B is no multiple of 4 the lane takes its row one request at a time.
 
 // where a tile row reads and writes: its addresses, null for a row past the group's end
 struct TcRow {
@@ -196,16 +195,31 @@ __device__ __forceinline__ T* row_of_lane(T* p, int lane) {
     return reinterpret_cast<T*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(p), lane));
 }
 
+// How the epilogue accesses memory: one request at a time, in 16-byte pieces of a lane's own row, or in pieces exchanged
+// first.  The exchange and its addresses are some 110 shuffles, which a block with one unit has nothing to hide behind:
+// blocks of 12 requests on trees of 16 x 16 leaves, 1 / 2 / 3 / 5 levels, us: 82 / 121 / 168 / 375 with the exchange
+// throughout, 76 / 117 / 162 / 366 without it for single units; 7 levels, 32 requests: 3928 and 3932 (3960 without it).
+enum TcAccess : int { TC_SINGLE = 0, TC_ROWS = 1, TC_EXCHANGED = 2 };
+__device__ __forceinline__ TcAccess tc_access(int B, int nunits) {
+    return (B & 3) != 0 ? TC_SINGLE : nunits <= 1 ? TC_ROWS : TC_EXCHANGED;
+}
+
 // the operand that the epilogue adds, in the layout of the accesses (issued early, so that its latency is hidden)
 template <int KIND>
-__device__ __forceinline__ void tc_prefetch(const TcRow& row, int B, int b0, float (&pre)[32], bool vec) {
+__device__ __forceinline__ void tc_prefetch(const TcRow& row, int B, int b0, float (&pre)[32], TcAccess acc) {
     if (KIND == MX_W) return;
     const int lane = threadIdx.x & 31, nb = min(32, B - b0);
     if (KIND == MX_DOWN && row.state) {  // its 256 bytes to L2: read once more per sweep only
         asm volatile("prefetch.global.L2 [%0];\n" ::"l"(row.state + b0));
         asm volatile("prefetch.global.L2 [%0];\n" ::"l"(row.state + b0 + nb - 1));
     }
-    if (vec) {
+    if (acc == TC_ROWS) {
+#pragma unroll
+        for (int q = 0; q < 32; q += 4) {
+            const float4 x = row.src && q < nb ? *reinterpret_cast<const float4*>(row.src + b0 + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+            pre[q] = x.x; pre[q + 1] = x.y; pre[q + 2] = x.z; pre[q + 3] = x.w;
+        }
+    } else if (acc == TC_EXCHANGED) {
         const int c = lane >> 2, a = lane & 3;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -221,9 +235,38 @@ __device__ __forceinline__ void tc_prefetch(const TcRow& row, int B, int b0, flo
 
 // v[q] = (A X)[row][b0 + q] of this lane's row (v is used up)
 template <int KIND>
-__device__ __forceinline__ void tc_store(const TcRow& row, int B, int b0, float (&v)[32], const float (&pre)[32], bool vec) {
+__device__ __forceinline__ void tc_store(const TcRow& row, int B, int b0, float (&v)[32], const float (&pre)[32], TcAccess acc) {
     const int lane = threadIdx.x & 31, nb = min(32, B - b0);
-    if (vec) {
+    if (acc == TC_ROWS) {
+        if (!row.d0) return;
+        if (KIND != MX_W) {
+#pragma unroll
+            for (int q = 0; q < 32; ++q) v[q] += pre[q];
+        }
+#pragma unroll
+        for (int q = 0; q < 32; q += 4) {
+            if (q >= nb) continue;
+            const float4 o = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
+            *reinterpret_cast<float4*>(row.d0 + b0 + q) = o;
+            if (KIND == MX_DOWN) *reinterpret_cast<float4*>(row.d1 + b0 + q) = o;
+        }
+        if (KIND == MX_DOWN && row.state) {
+#pragma unroll
+            for (int h = 0; h < 32; h += 8) {
+                double2 u[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    u[i] = h + 2 * i < nb ? *reinterpret_cast<const double2*>(row.state + b0 + h + 2 * i) : make_double2(0.0, 0.0);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (h + 2 * i < nb)
+                        *reinterpret_cast<double2*>(row.state + b0 + h + 2 * i) =
+                            make_double2(u[i].x + f2d_bits(v[h + 2 * i]), u[i].y + f2d_bits(v[h + 2 * i + 1]));
+            }
+        }
+        return;
+    }
+    if (acc == TC_EXCHANGED) {
         const int c = lane >> 2, a = lane & 3;
         // piece bits and lane bits change places
 #pragma unroll
@@ -336,7 +379,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     unsigned char* base = tc_smem + ((1024u - (smem_u32(tc_smem) & 1023u)) & 1023u);
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(base + size_t(NS) * SB);
     unsigned long long* a_full = bars;             // [NS] bulk-copy transaction barriers
-    unsigned long long* x_full = bars + NS;        // [NS] 128 staging arrivals
+    unsigned long long* x_full = bars + NS;        // [NS] kStageThreads staging arrivals
     unsigned long long* empty = bars + 2 * NS;     // [NS] MMA commit
     unsigned long long* acc_full = bars + 3 * NS;   // [NP] MMA commit at the end of a chunk
     unsigned long long* acc_empty = acc_full + NP;  // [NP] 128 epilogue arrivals
@@ -366,6 +409,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const int total = nunits * cpu;
     const int b0 = blockIdx.y * kTB;
     const bool vec = (B & 3) == 0;
+    const TcAccess access = tc_access(B, nunits);
 
     if (tid == 0) {
         for (int i = 0; i < NS; ++i) {
@@ -582,7 +626,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             if (gch - u * cpu == 0) {
                 const int grow = tile_of(u) * kTM + t;
                 row = tc_row<KIND>(items, s, B, sh.rows_item, grow, grow < R);
-                tc_prefetch<KIND>(row, B, b0, pre, vec);
+                tc_prefetch<KIND>(row, B, b0, pre, access);
             }
             const int bf = gch % NP;
             if (!(ep_ok = tc_wait(&acc_full[bf], unsigned(gch / NP) & 1u, abort_flag))) break;
@@ -616,7 +660,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 put_partial(base, v, t, 128);
                 break;  // the cluster reduction and the epilogue follow below
             }
-            tc_store<KIND>(row, B, b0, v, pre, vec);
+            tc_store<KIND>(row, B, b0, v, pre, access);
 #pragma unroll
             for (int q = 0; q < 32; ++q) v[q] = 0.f;
         }
@@ -636,7 +680,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         if (cluster.block_rank() == 0 && tid < 128 && nunits > 0 && __all_sync(0xffffffffu, !*abort_flag)) {
             const int t = tid;
             for (int rk = 1; rk < ksplit; ++rk) add_partial(cluster.map_shared_rank(base, rk), v, t, 128);
-            tc_store<KIND>(row, B, b0, v, pre, vec);
+            tc_store<KIND>(row, B, b0, v, pre, access);
         }
         cluster.sync();
     }
@@ -715,6 +759,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     if (cpu <= 0) nunits = 0;
     const int total = nunits * cpu, b0 = blockIdx.y * kTB;
     const bool vec = (B & 3) == 0;
+    const TcAccess access = vec ? TC_EXCHANGED : TC_SINGLE;
     if (tid == 0) {
         for (int i = 0; i < NS; ++i) {
             mbar_init(a_full + i, 1);
@@ -918,8 +963,8 @@ __global__ void __launch_bounds__(kPairThreads, 1)
             {
                 float pre[32];
                 const TcRow row = tc_row<KIND>(items, s, B, sh.rows_item, grow, tile >= 0 && grow < R);
-                tc_prefetch<KIND>(row, B, b0, pre, vec);
-                tc_store<KIND>(row, B, b0, v, pre, vec);
+                tc_prefetch<KIND>(row, B, b0, pre, access);
+                tc_store<KIND>(row, B, b0, v, pre, access);
             }
             ++u;
 #pragma unroll
@@ -947,8 +992,8 @@ __global__ void __launch_bounds__(kPairThreads, 1)
             {
                 float pre[32];
                 const TcRow row = tc_row<KIND>(items, s, B, sh.rows_item, grow, tile >= 0 && grow < R);
-                tc_prefetch<KIND>(row, B, b0, pre, vec);
-                tc_store<KIND>(row, B, b0, v, pre, vec);
+                tc_prefetch<KIND>(row, B, b0, pre, access);
+                tc_store<KIND>(row, B, b0, v, pre, access);
             }
         }
         cluster.sync();
