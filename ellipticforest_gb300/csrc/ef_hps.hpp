@@ -557,7 +557,7 @@ private:
     void node_gemm(cudaStream_t st, const MGroup& g, int kind, int B, int code);
     int filled(int B) const;  // requests a block of B is run with
     double gemm_bytes(const MGroup& g, int kind, int B, int code) const;
-    // times the K-split candidates of every node GEMM (CUDA events, block of min(bmax, 32)) and keeps
+    // times the K-split candidates of every node GEMM (CUDA events, block of min(bmax, 64)) and keeps
     // the fastest per group and kind in the tree
     void tune();
 

@@ -511,9 +511,11 @@ void Hps::set_mx_plan(const std::vector<std::array<int, 3>>& codes) {
 
 void MixedSolver::tune() {
     // per group and kind, the fastest of the CUDA-core GEMM (K split 1, 2, 4, ...: code > 0) and the
-    // tensor-core GEMM (code < 0: split -code), timed with CUDA events on a block of min(bmax, 32)
+    // tensor-core GEMM (code < 0: split -code), timed with CUDA events on a block of min(bmax, 64)
     Hps& h = H_;
-    const int B = std::min(filled(bmax_), 32);
+    // (64: two columns of tiles.  Timed with one, a K split that fills the SMs by itself wins there and loses with two:
+    // 64 requests, 16 x 16 leaves, 5 levels 794 us with the plan of 32, 734 with its own)
+    const int B = std::min(filled(bmax_), 64);
     std::vector<std::array<int, 3>> best(groups_.size(), std::array<int, 3>{1, 1, 1});
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     ck(cudaEventCreate(&e0), "tune event");
