@@ -493,19 +493,23 @@ void Hps::upload_tables() {
             check(upload_sync(st_, g.d_gB2, gB2.data(), gB2.size() * sizeof(void*)), "gB2");
             check(upload_sync(st_, g.d_gC, gC.data(), gC.size() * sizeof(void*)), "gC");
         }
-        std::vector<const double*> csrc;
-        std::vector<double*> cdst;
-        std::vector<long long> clen;
+        // sources, targets and lengths lie one after another: one copy
         const long long s2 = (long long)g.s * g.s;
+        char* const first = reinterpret_cast<char*>(g.d_csrc);
+        std::vector<char> jobs(reinterpret_cast<char*>(g.d_clen + g.ncopy) - first);
+        auto put = [&](void* table, size_t i, const void* v) { std::memcpy(jobs.data() + (static_cast<char*>(table) - first) + 8 * i, v, 8); };
         for (size_t k = 0; k < g.same.size(); ++k) {
             const NodeDev &a = nodes_[g.nodes[g.same[k]]], &b = nodes_[g.nodes[g.distinct + k]];
-            csrc.push_back(a.T); cdst.push_back(b.T); clen.push_back(64 * s2);
-            csrc.push_back(a.RHS); cdst.push_back(b.RHS); clen.push_back(48 * s2);
-            csrc.push_back(a.H); cdst.push_back(b.H); clen.push_back(16 * s2);
+            const double* src[3] = {a.T, a.RHS, a.H};
+            double* dst[3] = {b.T, b.RHS, b.H};
+            const long long len[3] = {64 * s2, 48 * s2, 16 * s2};
+            for (int q = 0; q < 3; ++q) {
+                put(g.d_csrc, 3 * k + q, &src[q]);
+                put(g.d_cdst, 3 * k + q, &dst[q]);
+                put(g.d_clen, 3 * k + q, &len[q]);
+            }
         }
-        check(upload_sync(st_, g.d_csrc, csrc.data(), csrc.size() * sizeof(void*)), "copy src");
-        check(upload_sync(st_, g.d_cdst, cdst.data(), cdst.size() * sizeof(void*)), "copy dst");
-        check(upload_sync(st_, g.d_clen, clen.data(), clen.size() * sizeof(long long)), "copy len");
+        if (g.ncopy) check(upload_sync(st_, first, jobs.data(), jobs.size()), "copies of equal operators");
     }
     for (size_t k = 0; k < tsteps_.size(); ++k) {
         const int t = step_index_t_[k];

@@ -478,10 +478,13 @@ MixedSolver::MixedSolver(Hps& hps, int bmax, const MixedSolver* share)
         for (int kind = 0; kind < 3; ++kind) {
             if (!g.tc[kind]) continue;
             if (g.pl[kind].tile) {
-                ck(upload_sync(st, g.pl[kind].tile, g.tile[kind].data(), g.tile[kind].size() * sizeof(int)), "tiles");
-                ck(upload_sync(st, g.rep[kind], g.first[kind].data(), g.first[kind].size() * sizeof(int)), "tiles");
-                if (g.pl[kind].pair)
-                    ck(upload_sync(st, g.pl[kind].pair, g.pair[kind].data(), g.pair[kind].size() * sizeof(int)), "pairs");
+                // (the tables are members: no need to wait for each copy)
+                auto up = [&](int* dst, const std::vector<int>& v) {
+                    ck(cudaMemcpyAsync(dst, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice, st), "tiles");
+                };
+                up(g.pl[kind].tile, g.tile[kind]);
+                up(g.rep[kind], g.first[kind]);
+                if (g.pl[kind].pair) up(g.pl[kind].pair, g.pair[kind]);
             }
             mx_tc_split(st, kind, op[kind], g.pl[kind], g.rep[kind], rows[kind], Ks[kind], g.s);
         }
