@@ -151,7 +151,7 @@ __device__ __forceinline__ void copy8_async(double* dst, const double* src) {
 // consecutive values per row, one n^2 x 4n slot per block) between the two.  Sums run from the far, small factors to the
 // near, large ones and add y last (from the near ones on, with y first, the solutions of trees of 20 x 20 to 32 x 32
 // leaves erred 2 to 5% more; now 0 to 2% less than with a column per warp).  FP64 pipe bound: 2 n^3 multiply-adds
-// per column, two per clock and SM (1024 leaves of 32 x 32 cells: 174 ms with a column per warp, 15.9 ms).  Warps whose
+// per column, two per clock and SM (1024 leaves of 32 x 32 cells: 174 ms with a column per warp, 16.1 ms).  Warps whose
 // columns start in a later block (data on E) skip the blocks before it.
 // The staged rows are spread to NP (zeros where a block row has no entry), so the loops need no bounds.
 template <int NP>
