@@ -89,7 +89,8 @@ constexpr int kFpStages = 3;  // block rows in flight
 // products, 1.7 ms.
 // NEUMANN: g = 0, load q, write h32 = DtN(0, q).  SOLVE: load q + boundary terms of g32, add (or store,
 // accumulate == 0) the solution to u64.
-template <int MODE>
+// FEW: the loop over k unrolled by eight, both products side by side; else by four, one after the other (the same sums).
+template <int MODE, bool FEW>
 __global__ void __launch_bounds__(32 * kFpWarps) k_mx_fp_leaf32(const MixFp* __restrict__ fps, const MixLeaf* __restrict__ leaves,
                                                               int L, int B, int n, const float* __restrict__ q,
                                                               double* __restrict__ u64, float* __restrict__ scratch,
@@ -141,15 +142,26 @@ __global__ void __launch_bounds__(32 * kFpWarps) k_mx_fp_leaf32(const MixFp* __r
         float sub[kFpReq];
 #pragma unroll
         for (int r = 0; r < kFpReq; ++r) acc[r] = sub[r] = 0.f;
-        auto add = [](float (&c)[kFpReq], float x, const float* p) {
-            const float4 p0 = *reinterpret_cast<const float4*>(p), p1 = *reinterpret_cast<const float4*>(p + 4);
+        auto add = [](float (&c)[kFpReq], float x, const float4& p0, const float4& p1) {
             c[0] = fmaf(x, p0.x, c[0]); c[1] = fmaf(x, p0.y, c[1]); c[2] = fmaf(x, p0.z, c[2]); c[3] = fmaf(x, p0.w, c[3]);
             c[4] = fmaf(x, p1.x, c[4]); c[5] = fmaf(x, p1.y, c[5]); c[6] = fmaf(x, p1.z, c[6]); c[7] = fmaf(x, p1.w, c[7]);
         };
-#pragma unroll 4
-        for (int k = 0; k < n; ++k) {
-            add(acc, m1[k * n], sq + k * kFpReq);
-            add(sub, m2[k * n], sy + k * kFpReq);
+        auto row4 = [](const float* p, int k, int h) { return *reinterpret_cast<const float4*>(p + k * kFpReq + 4 * h); };
+        if (FEW) {
+#pragma unroll 8
+            for (int k = 0; k < n; ++k) {
+                const float x = m1[k * n], y = m2[k * n];
+                const float4 p0 = row4(sq, k, 0), p1 = row4(sq, k, 1), t0 = row4(sy, k, 0), t1 = row4(sy, k, 1);
+                add(acc, x, p0, p1);
+                add(sub, y, t0, t1);
+            }
+        } else {
+            for (int k = 0; k < n; k += 4) {  // n is a multiple of four
+#pragma unroll
+                for (int o = 0; o < 4; ++o) add(acc, m1[(k + o) * n], row4(sq, k + o, 0), row4(sq, k + o, 1));
+#pragma unroll
+                for (int o = 0; o < 4; ++o) add(sub, m2[(k + o) * n], row4(sy, k + o, 0), row4(sy, k + o, 1));
+            }
         }
 #pragma unroll
         for (int r = 0; r < kFpReq; ++r) acc[r] -= sub[r];
@@ -368,10 +380,12 @@ void mx_fp_leaf32(cudaStream_t st, int mode, const MixFp* fps, const MixLeaf* le
                   const float* q, double* u64, float* scratch, int accumulate) {
     const size_t smem = (size_t(kFpStages) * 2 * n * n + size_t(kFpWarps) * 2 * 32 * kFpReq) * sizeof(float);
     dim3 grid(unsigned(L), unsigned((B + kFpGroup - 1) / kFpGroup));
-    if (mode == LEAF_NEUMANN)
-        k_mx_fp_leaf32<LEAF_NEUMANN><<<grid, 32 * kFpWarps, smem, st>>>(fps, leaves, L, B, n, q, u64, scratch, 0);
-    else
-        k_mx_fp_leaf32<LEAF_SOLVE><<<grid, 32 * kFpWarps, smem, st>>>(fps, leaves, L, B, n, q, u64, scratch, accumulate);
+    // up to five blocks per SM, all at once at the unrolled form's registers, a step's latency counts (64 leaves of 32 x 32
+    // cells, 23 requests: 638 us by fours, 597 unrolled); beyond, the blocks per SM (1024 leaves, 16 requests: 1712 and 1935)
+    const bool few = (long long)grid.x * grid.y <= 5 * 152;
+    auto kernel = mode == LEAF_NEUMANN ? (few ? k_mx_fp_leaf32<LEAF_NEUMANN, true> : k_mx_fp_leaf32<LEAF_NEUMANN, false>)
+                                       : (few ? k_mx_fp_leaf32<LEAF_SOLVE, true> : k_mx_fp_leaf32<LEAF_SOLVE, false>);
+    kernel<<<grid, 32 * kFpWarps, smem, st>>>(fps, leaves, L, B, n, q, u64, scratch, mode == LEAF_NEUMANN ? 0 : accumulate);
     ++g_kernel_launches;
 }
 
