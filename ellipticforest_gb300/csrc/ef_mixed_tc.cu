@@ -158,8 +158,8 @@ __device__ __forceinline__ TcSeg tc_seg(const MixItem* __restrict__ items, int s
 // A lane holds a row's sums for the 32 requests of a block.  Rows are 128 bytes (B = 32) in memory, so with 16-byte
 // accesses by rows every instruction touched 32 of them.  With B a multiple of 4 the warp therefore exchanges
 // its 4-request pieces first: lane (piece c = lane / 4, a = lane mod 4) gets piece c of the rows 4 i + a, i = 0 .. 7, and
-// an instruction covers four whole rows (L7 block 4.00 -> 3.94 ms).  Blocks of single units keep their rows (see
-// tc_access), and where B is no multiple of 4 the lane takes its row one request at a time.
+// an instruction covers four whole rows (L7 block 4.00 -> 3.94 ms).  Launches with single units per block keep their
+// rows (see tc_access), and where B is no multiple of 4 the lane takes its row one request at a time.
 
 // where a tile row reads and writes: its addresses, null for a row past the group's end
 struct TcRow {
@@ -200,26 +200,23 @@ __device__ __forceinline__ T* row_of_lane(T* p, int lane) {
 // blocks of 12 requests on trees of 16 x 16 leaves, 1 / 2 / 3 / 5 levels, us: 82 / 121 / 168 / 375 with the exchange
 // throughout, 76 / 117 / 162 / 366 without it for single units; 7 levels, 32 requests: 3928 and 3932 (3960 without it).
 enum TcAccess : int { TC_SINGLE = 0, TC_ROWS = 1, TC_EXCHANGED = 2 };
-__device__ __forceinline__ TcAccess tc_access(int B, int nunits) {
-    return (B & 3) != 0 ? TC_SINGLE : nunits <= 1 ? TC_ROWS : TC_EXCHANGED;
-}
 
 // the operand that the epilogue adds, in the layout of the accesses (issued early, so that its latency is hidden)
-template <int KIND>
-__device__ __forceinline__ void tc_prefetch(const TcRow& row, int B, int b0, float (&pre)[32], TcAccess acc) {
+template <int KIND, TcAccess ACC>
+__device__ __forceinline__ void tc_prefetch(const TcRow& row, int B, int b0, float (&pre)[32]) {
     if (KIND == MX_W) return;
     const int lane = threadIdx.x & 31, nb = min(32, B - b0);
     if (KIND == MX_DOWN && row.state) {  // its 256 bytes to L2: read once more per sweep only
         asm volatile("prefetch.global.L2 [%0];\n" ::"l"(row.state + b0));
         asm volatile("prefetch.global.L2 [%0];\n" ::"l"(row.state + b0 + nb - 1));
     }
-    if (acc == TC_ROWS) {
+    if constexpr (ACC == TC_ROWS) {
 #pragma unroll
         for (int q = 0; q < 32; q += 4) {
             const float4 x = row.src && q < nb ? *reinterpret_cast<const float4*>(row.src + b0 + q) : make_float4(0.f, 0.f, 0.f, 0.f);
             pre[q] = x.x; pre[q + 1] = x.y; pre[q + 2] = x.z; pre[q + 3] = x.w;
         }
-    } else if (acc == TC_EXCHANGED) {
+    } else if constexpr (ACC == TC_EXCHANGED) {
         const int c = lane >> 2, a = lane & 3;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -234,10 +231,10 @@ __device__ __forceinline__ void tc_prefetch(const TcRow& row, int B, int b0, flo
 }
 
 // v[q] = (A X)[row][b0 + q] of this lane's row (v is used up)
-template <int KIND>
-__device__ __forceinline__ void tc_store(const TcRow& row, int B, int b0, float (&v)[32], const float (&pre)[32], TcAccess acc) {
+template <int KIND, TcAccess ACC>
+__device__ __forceinline__ void tc_store(const TcRow& row, int B, int b0, float (&v)[32], const float (&pre)[32]) {
     const int lane = threadIdx.x & 31, nb = min(32, B - b0);
-    if (acc == TC_ROWS) {
+    if constexpr (ACC == TC_ROWS) {
         if (!row.d0) return;
         if (KIND != MX_W) {
 #pragma unroll
@@ -266,7 +263,7 @@ __device__ __forceinline__ void tc_store(const TcRow& row, int B, int b0, float 
         }
         return;
     }
-    if (acc == TC_EXCHANGED) {
+    if constexpr (ACC == TC_EXCHANGED) {
         const int c = lane >> 2, a = lane & 3;
         // piece bits and lane bits change places
 #pragma unroll
@@ -364,7 +361,7 @@ __device__ __forceinline__ void add_partial(const unsigned char* red, float (&v)
     }
 }
 
-template <int KIND, int NSEG>
+template <int KIND, int NSEG, TcAccess ACC>
 __global__ void __launch_bounds__(kTcThreads, 1)
     k_mx_umma(const __nv_bfloat16* __restrict__ A3, const MixItem* __restrict__ items, int s, int B, int cnt,
               int ksplit, int ntiles, const int* __restrict__ tmap, int nplanes, int* __restrict__ err) {
@@ -408,8 +405,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     if (cpu <= 0) nunits = 0;
     const int total = nunits * cpu;
     const int b0 = blockIdx.y * kTB;
-    const bool vec = (B & 3) == 0;
-    const TcAccess access = tc_access(B, nunits);
 
     if (tid == 0) {
         for (int i = 0; i < NS; ++i) {
@@ -553,7 +548,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 }
                 const int k0 = (cbase + c) * kTK;
                 float* dst = ring + (g % kXRing) * RC;
-                if (vec) {
+                if constexpr (ACC != TC_SINGLE) {
                     // 16-byte pieces: 8 per row of 32 requests (B % 4 == 0: a piece is all in or all out)
 #pragma unroll
                     for (int j = 0; j < NSEG; ++j)
@@ -626,7 +621,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             if (gch - u * cpu == 0) {
                 const int grow = tile_of(u) * kTM + t;
                 row = tc_row<KIND>(items, s, B, sh.rows_item, grow, grow < R);
-                tc_prefetch<KIND>(row, B, b0, pre, access);
+                tc_prefetch<KIND, ACC>(row, B, b0, pre);
             }
             const int bf = gch % NP;
             if (!(ep_ok = tc_wait(&acc_full[bf], unsigned(gch / NP) & 1u, abort_flag))) break;
@@ -660,7 +655,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 put_partial(base, v, t, 128);
                 break;  // the cluster reduction and the epilogue follow below
             }
-            tc_store<KIND>(row, B, b0, v, pre, access);
+            tc_store<KIND, ACC>(row, B, b0, v, pre);
 #pragma unroll
             for (int q = 0; q < 32; ++q) v[q] = 0.f;
         }
@@ -680,7 +675,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         if (cluster.block_rank() == 0 && tid < 128 && nunits > 0 && __all_sync(0xffffffffu, !*abort_flag)) {
             const int t = tid;
             for (int rk = 1; rk < ksplit; ++rk) add_partial(cluster.map_shared_rank(base, rk), v, t, 128);
-            tc_store<KIND>(row, B, b0, v, pre, access);
+            tc_store<KIND, ACC>(row, B, b0, v, pre);
         }
         cluster.sync();
     }
@@ -724,7 +719,7 @@ __device__ __forceinline__ float load_if(const float* p, bool get) {
     return x;
 }
 
-template <int KIND>
+template <int KIND, TcAccess ACC>
 __global__ void __launch_bounds__(kPairThreads, 1)
     k_mx_umma_pair(const __nv_bfloat16* __restrict__ A3, const MixItem* __restrict__ items, int s, int B, int cnt,
                    int ksplit, const int2* __restrict__ pairs, int npairs, const int* __restrict__ tmap, int nplanes,
@@ -758,8 +753,6 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     }
     if (cpu <= 0) nunits = 0;
     const int total = nunits * cpu, b0 = blockIdx.y * kTB;
-    const bool vec = (B & 3) == 0;
-    const TcAccess access = vec ? TC_EXCHANGED : TC_SINGLE;
     if (tid == 0) {
         for (int i = 0; i < NS; ++i) {
             mbar_init(a_full + i, 1);
@@ -963,8 +956,8 @@ __global__ void __launch_bounds__(kPairThreads, 1)
             {
                 float pre[32];
                 const TcRow row = tc_row<KIND>(items, s, B, sh.rows_item, grow, tile >= 0 && grow < R);
-                tc_prefetch<KIND>(row, B, b0, pre, access);
-                tc_store<KIND>(row, B, b0, v, pre, access);
+                tc_prefetch<KIND, ACC>(row, B, b0, pre);
+                tc_store<KIND, ACC>(row, B, b0, v, pre);
             }
             ++u;
 #pragma unroll
@@ -992,8 +985,8 @@ __global__ void __launch_bounds__(kPairThreads, 1)
             {
                 float pre[32];
                 const TcRow row = tc_row<KIND>(items, s, B, sh.rows_item, grow, tile >= 0 && grow < R);
-                tc_prefetch<KIND>(row, B, b0, pre, access);
-                tc_store<KIND>(row, B, b0, v, pre, access);
+                tc_prefetch<KIND, ACC>(row, B, b0, pre);
+                tc_store<KIND, ACC>(row, B, b0, v, pre);
             }
         }
         cluster.sync();
@@ -1041,6 +1034,16 @@ __global__ void k_tc_split(const float* __restrict__ src, __nv_bfloat16* __restr
     }
 }
 
+// The form of the epilogue's accesses.  The exchange and its addresses are some 110 shuffles, which a launch without a
+// second unit per block has nothing to hide behind; and a kernel for each form fetches less code (and spills less) than one
+// with all three.  Blocks of 12 requests on trees of 16 x 16 leaves, 1 / 3 / 5 levels, us: 80 / 168 / 371 with the exchange
+// throughout, 80 / 164 / 364 with rows for single units in the same kernel, 74 / 158 / 359 now; of 5 requests on 7 levels
+// 1616 and 1555, of 32 3932 and 3917 (3960 without the exchange).  Pairs of nodes exchange always: without it for single
+// units blocks of 64 requests on 5 levels take 736 us against 721.
+TcAccess tc_access(int B, int ksplit, long long units, long long blocks) {
+    return (B & 3) != 0 ? TC_SINGLE : ksplit > 1 || units <= blocks ? TC_ROWS : TC_EXCHANGED;
+}
+
 template <int KIND, int NSEG>
 void launch_umma_n(cudaStream_t st, const TcPlanes& A, const MixItem* items, int cnt, int s, int B, int* err,
                    int ksplit) {
@@ -1049,13 +1052,16 @@ void launch_umma_n(cudaStream_t st, const TcPlanes& A, const MixItem* items, int
     const int ntiles = int((R + kTM - 1) / kTM);
     const int chunks = (B + kTB - 1) / kTB;
     const size_t smem = tc_smem_bytes(NSEG);
-    cudaFuncSetAttribute(k_mx_umma<KIND, NSEG>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     int sms = 0, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     unsigned gx;
     if (ksplit > 1) gx = unsigned(ntiles * ksplit);
     else gx = unsigned(std::max(1, std::min(ntiles, std::max(1, sms / chunks))));
+    const TcAccess access = tc_access(B, ksplit, ntiles, gx);
+    const auto kernel = access == TC_SINGLE ? k_mx_umma<KIND, NSEG, TC_SINGLE>
+                        : access == TC_ROWS ? k_mx_umma<KIND, NSEG, TC_ROWS> : k_mx_umma<KIND, NSEG, TC_EXCHANGED>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(gx, unsigned(chunks));
     cfg.blockDim = dim3(kTcThreads);
@@ -1068,7 +1074,7 @@ void launch_umma_n(cudaStream_t st, const TcPlanes& A, const MixItem* items, int
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = ksplit > 1 ? 1 : 0;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_mx_umma<KIND, NSEG>, reinterpret_cast<const __nv_bfloat16*>(A.planes),
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, reinterpret_cast<const __nv_bfloat16*>(A.planes),
                                              items, s, B, cnt, ksplit, ntiles, A.tile, A.tile ? A.count : ntiles, err);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
@@ -1081,7 +1087,8 @@ void launch_umma_n(cudaStream_t st, const TcPlanes& A, const MixItem* items, int
 template <int KIND>
 void launch_pair(cudaStream_t st, const TcPlanes& A, const MixItem* items, int cnt, int s, int B, int* err, int ksplit) {
     const int chunks = (B + kTB - 1) / kTB;
-    cudaFuncSetAttribute(k_mx_umma_pair<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPairSmem));
+    const auto kernel = (B & 3) != 0 ? k_mx_umma_pair<KIND, TC_SINGLE> : k_mx_umma_pair<KIND, TC_EXCHANGED>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPairSmem));
     int sms = 0, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1098,7 +1105,7 @@ void launch_pair(cudaStream_t st, const TcPlanes& A, const MixItem* items, int c
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = ksplit > 1 ? 1 : 0;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_mx_umma_pair<KIND>, reinterpret_cast<const __nv_bfloat16*>(A.planes), items, s,
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, reinterpret_cast<const __nv_bfloat16*>(A.planes), items, s,
                                              B, cnt, ksplit, reinterpret_cast<const int2*>(A.pair), A.npairs, A.tile, A.count, err);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
